@@ -9,10 +9,14 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "capi/capi_common.hpp"
 #include "core/log.hpp"
 #include "gpu/cuda_driver.hpp"
+#include "gpu/pdl.cuh"
+
+using namespace cclx;
 
 namespace {
 
@@ -23,73 +27,140 @@ __device__ __forceinline__ float warp_sum_f(float v) {
     return v;
 }
 
-// One warp per row, V 16-byte packs per lane (row length D = 256 * V).  Lane l holds packs l, l+32, ...
-template <int V>
-__device__ __forceinline__ void load_row(const __nv_bfloat16* row, int lane, float (&x)[V * 8]) {
-    const uint4* p = reinterpret_cast<const uint4*>(row);
+__device__ __forceinline__ void unpack8(const uint4& u, float (&x)[8]) {
+    const uint32_t w[4] = { u.x, u.y, u.z, u.w };
 #pragma unroll
-    for (int v = 0; v < V; v++) {
-        const uint4 u = p[lane + v * 32];
-        const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&u);
-#pragma unroll
-        for (int e = 0; e < 8; e++)
-            x[v * 8 + e] = __bfloat162float(h[e]);
+    for (int i = 0; i < 4; i++) { // bf16 is the upper half of an fp32 word
+        x[2 * i] = __uint_as_float(w[i] << 16);
+        x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
     }
 }
 
-template <int V>
-__device__ __forceinline__ void store_row(__nv_bfloat16* row, int lane, const float (&x)[V * 8]) {
-    uint4* p = reinterpret_cast<uint4*>(row);
+// pairs of fp32 values: one instruction adds or multiplies both (fma.rn.f32x2 and relatives)
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpair(f32x2 v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack4x2(const uint4& u, f32x2 (&x)[4]) {
+    const uint32_t w[4] = { u.x, u.y, u.z, u.w };
 #pragma unroll
-    for (int v = 0; v < V; v++) {
-        uint4 u;
-        __nv_bfloat16* h = reinterpret_cast<__nv_bfloat16*>(&u);
+    for (int i = 0; i < 4; i++) // bf16 is the upper half of an fp32 word
+        x[i] = pair(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
+}
+__device__ __forceinline__ uint4 pack4x2(const f32x2 (&x)[4]) {
+    uint32_t w[4];
 #pragma unroll
-        for (int e = 0; e < 8; e++)
-            h[e] = __float2bfloat16_rn(x[v * 8 + e]);
-        p[lane + v * 32] = u;
+    for (int i = 0; i < 4; i++) {
+        float lo, hi;
+        unpair(x[i], lo, hi);
+        const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+        w[i] = *reinterpret_cast<const uint32_t*>(&h);
     }
+    return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// y = (x - mean) * rstd * w + b ; optionally x = x + residual first (the sum is written to `sum_out`)
+__device__ __forceinline__ uint4 pack8(const float (&x)[8]) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
+        w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// y = (x - mean) * rstd * w + b ; optionally x = x + residual first (the sum is written to `sum_out`).
+//
+// Bound by memory: x (and the residual) in, y (and the sum) out.  One warp owns a row, lane l holds the 16-byte packs
+// l, l + 32, ... of it (V = packs per lane, the last one partial when the width is no multiple of 256), so the two
+// reductions are shuffles and nothing synchronises.  The row stays packed while it waits and gamma / beta are
+// re-read from L1 for every row, which leaves enough warps per SM to keep the loads of some 20 rows in flight.
 template <int V>
-__global__ void __launch_bounds__(256) ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
-                                                     const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
-                                                     __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ sum_out,
+__global__ void __launch_bounds__(128) ln_fwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res,
+                                                     const uint4* __restrict__ w, const uint4* __restrict__ b,
+                                                     uint4* __restrict__ y, uint4* __restrict__ sum_out,
                                                      float* __restrict__ mean, float* __restrict__ rstd, size_t rows,
-                                                     float eps) {
-    constexpr int D = V * 256;
+                                                     int packs, float inv_d, float eps) {
     const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    float wv[V * 8], bv[V * 8];
-    load_row<V>(w, lane, wv);
-    load_row<V>(b, lane, bv);
+    const bool last_on = lane + (V - 1) * 32 < packs;
     for (size_t r = (size_t)blockIdx.x * wpb + (threadIdx.x >> 5); r < rows; r += (size_t)gridDim.x * wpb) {
-        float xv[V * 8];
-        load_row<V>(x + r * D, lane, xv);
-        if (res) {
-            float rv[V * 8];
-            load_row<V>(res + r * D, lane, rv);
+        const size_t base = r * packs + lane;
+        uint4 u[V], q[V];
 #pragma unroll
-            for (int i = 0; i < V * 8; i++)
-                xv[i] = __bfloat162float(__float2bfloat16_rn(xv[i] + rv[i])); // the sum lives in bf16
-            store_row<V>(sum_out + r * D, lane, xv);
-        }
+        for (int v = 0; v < V; v++)
+            u[v] = v < V - 1 || last_on ? x[base + v * 32] : make_uint4(0, 0, 0, 0);
         float s = 0.f;
+        if (res) {
 #pragma unroll
-        for (int i = 0; i < V * 8; i++)
-            s += xv[i];
-        const float m = warp_sum_f(s) * (1.0f / D);
-        float q = 0.f;
+            for (int v = 0; v < V; v++)
+                q[v] = v < V - 1 || last_on ? res[base + v * 32] : make_uint4(0, 0, 0, 0);
 #pragma unroll
-        for (int i = 0; i < V * 8; i++) {
-            const float d = xv[i] - m;
-            q += d * d;
+            for (int v = 0; v < V; v++) {
+                float a[8], c[8];
+                unpack8(u[v], a);
+                unpack8(q[v], c);
+#pragma unroll
+                for (int e = 0; e < 8; e++)
+                    a[e] += c[e];
+                u[v] = pack8(a); // the sum lives in bf16
+                if (v < V - 1 || last_on)
+                    sum_out[base + v * 32] = u[v];
+            }
         }
-        const float rs = rsqrtf(warp_sum_f(q) * (1.0f / D) + eps);
 #pragma unroll
-        for (int i = 0; i < V * 8; i++)
-            xv[i] = (xv[i] - m) * rs * wv[i] + bv[i];
-        store_row<V>(y + r * D, lane, xv);
+        for (int v = 0; v < V; v++) {
+            float a[8];
+            unpack8(u[v], a);
+#pragma unroll
+            for (int e = 0; e < 8; e++)
+                s += a[e];
+        }
+        const float m = warp_sum_f(s) * inv_d;
+        float var = 0.f;
+#pragma unroll
+        for (int v = 0; v < V; v++) {
+            float a[8];
+            unpack8(u[v], a);
+            if (v < V - 1 || last_on) {
+#pragma unroll
+                for (int e = 0; e < 8; e++)
+                    var = fmaf(a[e] - m, a[e] - m, var);
+            }
+        }
+        const float rs = rsqrtf(warp_sum_f(var) * inv_d + eps);
+#pragma unroll
+        for (int v = 0; v < V; v++) {
+            if (v < V - 1 || last_on) {
+                float a[8], wv[8], bv[8];
+                unpack8(u[v], a);
+                unpack8(__ldg(w + lane + v * 32), wv);
+                unpack8(__ldg(b + lane + v * 32), bv);
+#pragma unroll
+                for (int e = 0; e < 8; e++)
+                    a[e] = fmaf((a[e] - m) * rs, wv[e], bv[e]);
+                y[base + v * 32] = pack8(a);
+            }
+        }
         if (lane == 0) {
             mean[r] = m;
             rstd[r] = rs;
@@ -97,91 +168,246 @@ __global__ void __launch_bounds__(256) ln_fwd_kernel(const __nv_bfloat16* __rest
     }
 }
 
-// dx = rstd * (g - mean(g) - xhat * mean(g * xhat)), g = dy * w;  partial dgamma / dbeta per block.
-// `dres` (optional) is added to dx: the gradient that reached the residual branch.
-template <int V>
-__global__ void __launch_bounds__(256) ln_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                                                     const __nv_bfloat16* __restrict__ w, const float* __restrict__ mean,
-                                                     const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ dres,
-                                                     __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, size_t rows) {
-    constexpr int D = V * 256;
-    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5, warp = threadIdx.x >> 5;
-    float wv[V * 8], dg[V * 8], db[V * 8];
-    load_row<V>(w, lane, wv);
+// Sums NV values over the warp at once: each exchange halves the number of values a lane still carries, so 8 values
+// take 9 shuffles instead of 40.  Lane l ends with the total of value (l * NV / 32).
+template <int NV>
+__device__ __forceinline__ float warp_sum_many(float (&v)[NV], int lane) {
 #pragma unroll
-    for (int i = 0; i < V * 8; i++)
-        dg[i] = db[i] = 0.f;
-    for (size_t r = (size_t)blockIdx.x * wpb + warp; r < rows; r += (size_t)gridDim.x * wpb) {
-        float xv[V * 8], gv[V * 8];
-        load_row<V>(x + r * D, lane, xv);
-        load_row<V>(dy + r * D, lane, gv);
-        const float m = mean[r], rs = rstd[r];
-        float s1 = 0.f, s2 = 0.f;
+    for (int n = NV / 2, o = 16; n > 0; n >>= 1, o >>= 1) {
+        const bool up = lane & o;
 #pragma unroll
-        for (int i = 0; i < V * 8; i++) {
-            const float xh = (xv[i] - m) * rs;
-            db[i] += gv[i];
-            dg[i] += gv[i] * xh;
-            const float g = gv[i] * wv[i];
-            s1 += g;
-            s2 += g * xh;
-            xv[i] = xh;
-            gv[i] = g;
+        for (int i = 0; i < n; i++) {
+            const float send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
         }
-        s1 = warp_sum_f(s1) * (1.0f / D);
-        s2 = warp_sum_f(s2) * (1.0f / D);
-#pragma unroll
-        for (int i = 0; i < V * 8; i++)
-            gv[i] = rs * (gv[i] - s1 - xv[i] * s2);
-        if (dres) {
-            load_row<V>(dres + r * D, lane, xv);
-#pragma unroll
-            for (int i = 0; i < V * 8; i++)
-                gv[i] += xv[i];
-        }
-        store_row<V>(dx + r * D, lane, gv);
     }
-    // block partials: warps add into shared memory one after the other (fixed order), then one row out
-    __shared__ float sh[2][D];
-    for (int k = 0; k < wpb; k++) {
-        if (warp == k) {
 #pragma unroll
-            for (int v = 0; v < V; v++)
+    for (int o = 16 / NV; o > 0; o >>= 1)
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+
+__device__ __forceinline__ void copy16_async(void* smem, const void* gmem, bool on) {
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(gmem), "r"(on ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_commit() {
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void copy_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+constexpr int LN_BWD_ROWS = 2; // rows per step of a group
+constexpr int LN_BWD_STAGES = 4; // steps in flight or in use
+constexpr int LN_BWD_BLOCKS = 2; // resident blocks per SM
+
+// dx = rstd * (g - mean(g) - xhat * mean(g * xhat)), g = dy * w;  partial dgamma / dbeta (and column sums of dx) per
+// block.  `dres` (optional) is added to dx: the gradient that reached the residual branch.
+//
+// Bound by memory: dy, x, dres in, dx out.  A thread owns 8 columns (one 16-byte pack) of every row its group of `tpr`
+// threads works on, so the column sums cost 8 registers each, and a group takes R rows per step: one block barrier
+// per R rows (the row sums cross the warps of a group through shared memory, double-buffered).  Every thread
+// copies its own packs of the next three steps into shared memory with cp.async and reads back only those, so no
+// barrier guards the ring and 147 KB per SM are in flight whatever the registers hold.  The instruction rate is the next limit (0.74 issued per
+// scheduler and cycle with scalar arithmetic), hence the packed pairs.  A warp per row with the whole
+// row and its column sums in registers needed 191 of them, had 8 warps per SM and ran at half the copy rate.
+template <int R, bool COLSUM>
+__global__ void __launch_bounds__(256, LN_BWD_BLOCKS)
+    ln_bwd_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ x, const uint4* __restrict__ w,
+                  const float* __restrict__ mean, const float* __restrict__ rstd, const uint4* __restrict__ dres,
+                  uint4* __restrict__ dx, float* __restrict__ partial, size_t rows, int packs, int tpr, float inv_d) {
+    constexpr int NS = COLSUM ? 3 : 2;
+    extern __shared__ __align__(16) float sh[]; // ring, then the row sums; the block's column sums at the end
+    const int groups = blockDim.x / tpr;
+    const int grp = threadIdx.x / tpr, c = threadIdx.x - grp * tpr;
+    const int lane = threadIdx.x & 31, gw = c >> 5;
+    const bool on = c < packs;
+    uint4* ring = reinterpret_cast<uint4*>(sh); // [stage][tensor][row][thread]
+    float* sums = sh + (size_t)LN_BWD_STAGES * 3 * R * blockDim.x * 4; // [2][group][2 R][8]: up to 8 warps' shares, zeros behind
+    for (int i = threadIdx.x; i < 2 * groups * 2 * R * 8; i += blockDim.x)
+        sums[i] = 0.f;
+    __syncthreads();
+    gpu::pdl_trigger(); // the final sum may be scheduled as soon as SMs fall idle; it waits for this grid's end
+    f32x2 wv[4], acc2[NS][4];
+    unpack4x2(on ? w[c] : make_uint4(0, 0, 0, 0), wv);
 #pragma unroll
-                for (int e = 0; e < 8; e++) {
-                    const int col = (lane + v * 32) * 8 + e;
-                    sh[0][col] = (k == 0 ? 0.f : sh[0][col]) + dg[v * 8 + e];
-                    sh[1][col] = (k == 0 ? 0.f : sh[1][col]) + db[v * 8 + e];
-                }
+    for (int i = 0; i < NS; i++)
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            acc2[i][e] = 0;
+    const size_t step = (size_t)gridDim.x * groups * R;
+    const size_t first = ((size_t)blockIdx.x * groups + grp) * R;
+    auto at = [&](int stage, int tensor, int k) { return ring + ((size_t)(stage * 3 + tensor) * R + k) * blockDim.x + threadIdx.x; };
+    auto fetch = [&](size_t r0, int stage) { // rows behind the end arrive as zeros
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+            const bool ok = on && r0 + k < rows;
+            const size_t i = ok ? (r0 + k) * packs + c : 0;
+            copy16_async(at(stage, 0, k), x + i, ok);
+            copy16_async(at(stage, 1, k), dy + i, ok);
+            if (dres)
+                copy16_async(at(stage, 2, k), dres + i, ok);
         }
+        copy_commit();
+    };
+    float m[R], rs[R];
+    auto fetch_stats = [&](size_t r0) {
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+            m[k] = r0 + k < rows ? mean[r0 + k] : 0.f;
+            rs[k] = r0 + k < rows ? rstd[r0 + k] : 0.f;
+        }
+    };
+#pragma unroll
+    for (int s = 0; s < LN_BWD_STAGES - 1; s++)
+        fetch(first + s * step, s);
+    fetch_stats(first);
+    int stage = 0, buf = 0;
+    size_t r0 = first;
+    for (size_t base = (size_t)blockIdx.x * groups * R; base < rows; base += step, r0 += step, buf ^= 1) {
+        fetch(r0 + (LN_BWD_STAGES - 1) * step, (stage + LN_BWD_STAGES - 1) % LN_BWD_STAGES);
+        copy_wait<LN_BWD_STAGES - 1>();
+        float s[2 * R];
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+            f32x2 a[4], g[4], s1 = 0, s2 = 0;
+            unpack4x2(*at(stage, 0, k), a);
+            unpack4x2(*at(stage, 1, k), g);
+            const f32x2 nm = pair(-m[k], -m[k]);
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const f32x2 t = mul2(g[e], wv[e]);
+                s1 = add2(s1, t);
+                s2 = fma2(t, add2(a[e], nm), s2);
+            }
+            float p, q;
+            unpair(s1, p, q);
+            s[2 * k] = on ? p + q : 0.f;
+            unpair(s2, p, q);
+            s[2 * k + 1] = on ? (p + q) * rs[k] : 0.f;
+        }
+        const float tot = warp_sum_many<2 * R>(s, lane);
+        float* slot = sums + ((size_t)buf * groups + grp) * 2 * R * 8;
+        if ((lane & (16 / R - 1)) == 0)
+            slot[lane * (2 * R) / 32 * 8 + gw] = tot;
         __syncthreads();
+        float c1[R], c2[R], cm[R], cr[R];
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+            const float4* t = reinterpret_cast<const float4*>(slot + 2 * k * 8);
+            c1[k] = (((t[0].x + t[0].y) + (t[0].z + t[0].w)) + ((t[1].x + t[1].y) + (t[1].z + t[1].w))) * inv_d;
+            c2[k] = (((t[2].x + t[2].y) + (t[2].z + t[2].w)) + ((t[3].x + t[3].y) + (t[3].z + t[3].w))) * inv_d;
+            cm[k] = m[k];
+            cr[k] = rs[k];
+        }
+        fetch_stats(r0 + step); // of the next step: used after the next wait
+#pragma unroll
+        for (int k = 0; k < R; k++) {
+            // with x' = x - mean and the row's constants: dx = dres + rstd g - rstd c1 - (rstd^2 c2) x'
+            f32x2 a[4], g[4], d[4];
+            unpack4x2(*at(stage, 0, k), a);
+            unpack4x2(*at(stage, 1, k), g);
+            unpack4x2(dres ? *at(stage, 2, k) : make_uint4(0, 0, 0, 0), d);
+            const float h0 = -cr[k] * c1[k], h1 = -cr[k] * cr[k] * c2[k];
+            const f32x2 nm = pair(-cm[k], -cm[k]), r2 = pair(cr[k], cr[k]), k0 = pair(h0, h0), k1 = pair(h1, h1);
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const f32x2 xc = add2(a[e], nm), gr = mul2(g[e], r2);
+                acc2[0][e] = fma2(gr, xc, acc2[0][e]);
+                acc2[1][e] = add2(acc2[1][e], g[e]);
+                d[e] = fma2(gr, wv[e], add2(d[e], fma2(xc, k1, k0)));
+            }
+            if (on && r0 + k < rows) {
+                const uint4 o = pack4x2(d);
+                dx[(r0 + k) * packs + c] = o;
+                if (COLSUM) {
+                    unpack4x2(o, d); // the sums are those of the bf16 values that dx holds
+#pragma unroll
+                    for (int e = 0; e < 4; e++)
+                        acc2[NS - 1][e] = add2(acc2[NS - 1][e], d[e]);
+                }
+            }
+        }
+        stage = (stage + 1) % LN_BWD_STAGES;
     }
-    for (int c = threadIdx.x; c < D; c += blockDim.x) {
-        partial[((size_t)blockIdx.x * 2 + 0) * D + c] = sh[0][c];
-        partial[((size_t)blockIdx.x * 2 + 1) * D + c] = sh[1][c];
+    copy_wait<0>();
+    float acc[NS][8];
+#pragma unroll
+    for (int i = 0; i < NS; i++)
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            unpair(acc2[i][e], acc[i][2 * e], acc[i][2 * e + 1]);
+    // block partials: the groups' sums meet in shared memory in a fixed order
+    const int cols = packs * 8;
+    float* out = partial + (size_t)blockIdx.x * NS * cols;
+    if (groups == 1) {
+        if (on)
+#pragma unroll
+            for (int i = 0; i < NS; i++)
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                    *reinterpret_cast<float4*>(out + (size_t)i * cols + c * 8 + h * 4) =
+                        make_float4(acc[i][4 * h], acc[i][4 * h + 1], acc[i][4 * h + 2], acc[i][4 * h + 3]);
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < NS; i++) {
+        __syncthreads();
+        if (on)
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                *reinterpret_cast<float4*>(sh + (size_t)grp * cols + c * 8 + h * 4) =
+                    make_float4(acc[i][4 * h], acc[i][4 * h + 1], acc[i][4 * h + 2], acc[i][4 * h + 3]);
+        __syncthreads();
+        for (int col = threadIdx.x; col < cols; col += blockDim.x) {
+            float t = 0.f;
+            for (int q = 0; q < groups; q++)
+                t += sh[(size_t)q * cols + col];
+            out[(size_t)i * cols + col] = t;
+        }
     }
 }
 
-// out[c] = sum over `n` partial rows (fixed order per column); two outputs interleaved as in ln_bwd_kernel.
-// A block owns 32 columns of one output: 8 row groups add their share of the partial rows, a fixed tree
-// in shared memory joins them.  grid = (D / 32, 2).
-__global__ void __launch_bounds__(256) ln_bwd_final_kernel(const float* __restrict__ partial, int n, int D,
-                                                           __nv_bfloat16* __restrict__ dgamma, __nv_bfloat16* __restrict__ dbeta) {
+// out[which][col] (+)= sum over `n` partial rows in a fixed order.  A block owns 32 columns of one output: 8 row groups
+// add their share of the partial rows (8 loads in flight each), shared memory joins them.  grid = (cols / 32, outputs).
+struct partial_outs {
+    __nv_bfloat16* out[3];
+    int add; // 1: add to what the outputs hold
+};
+
+__global__ void __launch_bounds__(256) partial_rows_sum_kernel(const float* __restrict__ partial, int n, int cols, partial_outs o) {
     const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
     const int c = blockIdx.x * 32 + lane, which = blockIdx.y;
+    gpu::pdl_wait();
     float a = 0.f;
-    if (c < D)
-        for (int k = grp; k < n; k += 8)
-            a += partial[((size_t)k * 2 + which) * D + c];
+    if (c < cols) {
+        const float* p = partial + (size_t)which * cols + c;
+        const size_t pitch = (size_t)gridDim.y * cols;
+        int k = grp;
+        for (; k + 56 < n; k += 64) {
+            float t[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                t[i] = __ldcg(p + (size_t)(k + 8 * i) * pitch);
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                a += t[i];
+        }
+        for (; k < n; k += 8)
+            a += __ldcg(p + (size_t)k * pitch);
+    }
     __shared__ float sh[8][32];
     sh[grp][lane] = a;
     __syncthreads();
-    if (grp == 0 && c < D) {
+    if (grp == 0 && c < cols) {
         float s = 0.f;
 #pragma unroll
         for (int g = 0; g < 8; g++)
             s += sh[g][lane];
-        (which == 0 ? dgamma : dbeta)[c] = __float2bfloat16_rn(s);
+        __nv_bfloat16* out = (which == 0 ? o.out[0] : which == 1 ? o.out[1] : o.out[2]) + c;
+        *out = __float2bfloat16_rn(o.add ? __bfloat162float(*out) + s : s);
     }
 }
 
@@ -289,63 +515,108 @@ int sm_count_now() {
     return sms;
 }
 
+// dynamic shared memory above the default 48 KB, granted to the kernel once per device
+template <auto KERNEL>
+void allow_smem(size_t bytes) {
+    static std::atomic<bool> done[64];
+    int dev = 0;
+    CUDA_CHECK(cudaGetDevice(&dev));
+    if (dev < 64 && done[dev].load(std::memory_order_acquire))
+        return;
+    CUDA_CHECK(cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    if (dev < 64)
+        done[dev].store(true, std::memory_order_release);
+}
+
 } // namespace
 
 // ---- C entry points -----------------------------------------------------------------------------
-// D must be 256, 512, 768 or 1024.  mean / rstd: fp32 [rows].  res / sum_out may be null (no residual).
+// D: a multiple of 8 up to 2048; 16-byte aligned rows.  mean / rstd: fp32 [rows].  res / sum_out may be null (no residual).
 CCLX_API int cclx_layer_norm_fwd(const void* x, const void* res, const void* w, const void* b, void* y, void* sum_out,
                                  float* mean, float* rstd, size_t rows, int D, float eps, void* stream) {
     return cclx::capi::guard([&] {
-        CCL_THROW_IF_NOT(D % 256 == 0 && D >= 256 && D <= 1024, "fused LayerNorm supports 256, 512, 768 and 1024 columns");
+        CCL_THROW_IF_NOT(D % 8 == 0 && D >= 8 && D <= 2048, "fused LayerNorm supports multiples of 8 up to 2048 columns");
         CCL_THROW_IF_NOT((res == nullptr) == (sum_out == nullptr), "residual input and sum output go together");
         if (rows == 0)
             return;
-        const int blocks = (int)std::min<size_t>((rows + 7) / 8, (size_t)sm_count_now() * 4);
+        // four warps per block; up to 24 warps per SM, after which warps take several rows
+        const int blocks = (int)std::min<size_t>((rows + 3) / 4, (size_t)sm_count_now() * 6);
         cudaStream_t st = (cudaStream_t)stream;
-#define LN_FWD(V)                                                                                                          \
-    ln_fwd_kernel<V><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (const __nv_bfloat16*)w, \
-                                             (const __nv_bfloat16*)b, (__nv_bfloat16*)y, (__nv_bfloat16*)sum_out, mean,   \
-                                             rstd, rows, eps)
-        switch (D / 256) {
-            case 1: LN_FWD(1); break;
-            case 2: LN_FWD(2); break;
-            case 3: LN_FWD(3); break;
-            default: LN_FWD(4); break;
+#define LN_FWD(V)                                                                                                     \
+    case V:                                                                                                           \
+        ln_fwd_kernel<V><<<blocks, 128, 0, st>>>((const uint4*)x, (const uint4*)res, (const uint4*)w, (const uint4*)b, \
+                                                 (uint4*)y, (uint4*)sum_out, mean, rstd, rows, D / 8, 1.0f / D, eps); \
+        break
+        switch ((D + 255) / 256) {
+            LN_FWD(1);
+            LN_FWD(2);
+            LN_FWD(3);
+            LN_FWD(4);
+            LN_FWD(5);
+            LN_FWD(6);
+            LN_FWD(7);
+            LN_FWD(8);
         }
 #undef LN_FWD
         CUDA_CHECK(cudaGetLastError());
     });
 }
 
-// workspace: fp32 [cclx_layer_norm_bwd_blocks(rows) * 2 * D].  dres may be null.
+// rows of the backward workspace: an upper bound of the blocks that any width launches
 CCLX_API int cclx_layer_norm_bwd_blocks(size_t rows) {
-    return (int)std::min<size_t>((rows + 7) / 8, (size_t)sm_count_now());
+    return (int)std::min<size_t>(rows, (size_t)sm_count_now() * LN_BWD_BLOCKS);
+}
+
+namespace {
+template <int R, bool COLSUM>
+int launch_ln_bwd(const void* dy, const void* x, const void* w, const float* mean, const float* rstd, const void* dres,
+                  void* dx, float* workspace, size_t rows, int D, cudaStream_t st) {
+    const int packs = D / 8, tpr = (packs + 31) / 32 * 32;
+    const int groups = std::max(1, 256 / tpr), threads = groups * tpr;
+    const size_t ring = (size_t)LN_BWD_STAGES * 3 * R * threads * 16;
+    const size_t smem = std::max(ring + (size_t)2 * groups * 2 * R * 8 * 4, groups > 1 ? (size_t)groups * D * 4 : 0);
+    const size_t want = (rows + (size_t)groups * R - 1) / ((size_t)groups * R);
+    const int blocks = (int)std::min<size_t>(want, (size_t)sm_count_now() * LN_BWD_BLOCKS);
+    allow_smem<ln_bwd_kernel<R, COLSUM>>((size_t)LN_BWD_STAGES * 3 * R * 256 * 16 + 2048);
+    ln_bwd_kernel<R, COLSUM><<<blocks, threads, smem, st>>>((const uint4*)dy, (const uint4*)x, (const uint4*)w, mean, rstd,
+                                                            (const uint4*)dres, (uint4*)dx, workspace, rows, packs, tpr,
+                                                            1.0f / D);
+    CUDA_CHECK(cudaGetLastError());
+    return blocks;
+}
+} // namespace
+
+// workspace: fp32 [cclx_layer_norm_bwd_blocks(rows) * (dxsum ? 3 : 2) * D].  dres may be null.  dxsum (optional): column
+// sums of dx, the bias gradient of the linear layer whose output the residual addition took.  `add`: the three column
+// results are added to what dgamma / dbeta / dxsum hold.
+CCLX_API int cclx_layer_norm_bwd_sums(const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
+                                      const void* dres, void* dx, void* dgamma, void* dbeta, void* dxsum, int add,
+                                      float* workspace, size_t rows, int D, void* stream) {
+    return cclx::capi::guard([&] {
+        CCL_THROW_IF_NOT(D % 8 == 0 && D >= 8 && D <= 2048, "fused LayerNorm supports multiples of 8 up to 2048 columns");
+        if (rows == 0)
+            return;
+        cudaStream_t st = (cudaStream_t)stream;
+        // Two rows per step halve the barriers; with too few rows to give every SM several steps, one row at a time
+        // spreads them over the chip instead (64 rows of 1024: 32 blocks, not 16).
+        const bool wide = rows >= (size_t)sm_count_now() * 16;
+        int n;
+        if (dxsum)
+            n = wide ? launch_ln_bwd<LN_BWD_ROWS, true>(dy, x, w, mean, rstd, dres, dx, workspace, rows, D, st)
+                     : launch_ln_bwd<1, true>(dy, x, w, mean, rstd, dres, dx, workspace, rows, D, st);
+        else
+            n = wide ? launch_ln_bwd<LN_BWD_ROWS, false>(dy, x, w, mean, rstd, dres, dx, workspace, rows, D, st)
+                     : launch_ln_bwd<1, false>(dy, x, w, mean, rstd, dres, dx, workspace, rows, D, st);
+        partial_outs o{ { (__nv_bfloat16*)dgamma, (__nv_bfloat16*)dbeta, (__nv_bfloat16*)dxsum }, add };
+        gpu::launch_dependent(partial_rows_sum_kernel, dim3((D + 31) / 32, dxsum ? 3 : 2), dim3(256), 0, st,
+                              (const float*)workspace, n, D, o);
+    });
 }
 
 CCLX_API int cclx_layer_norm_bwd(const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
                                  const void* dres, void* dx, void* dgamma, void* dbeta, float* workspace, size_t rows, int D,
                                  void* stream) {
-    return cclx::capi::guard([&] {
-        CCL_THROW_IF_NOT(D % 256 == 0 && D >= 256 && D <= 1024, "fused LayerNorm supports 256, 512, 768 and 1024 columns");
-        if (rows == 0)
-            return;
-        const int blocks = cclx_layer_norm_bwd_blocks(rows);
-        cudaStream_t st = (cudaStream_t)stream;
-#define LN_BWD(V)                                                                                                      \
-    ln_bwd_kernel<V><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, \
-                                             mean, rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, workspace, rows)
-        switch (D / 256) {
-            case 1: LN_BWD(1); break;
-            case 2: LN_BWD(2); break;
-            case 3: LN_BWD(3); break;
-            default: LN_BWD(4); break;
-        }
-#undef LN_BWD
-        CUDA_CHECK(cudaGetLastError());
-        ln_bwd_final_kernel<<<dim3((D + 31) / 32, 2), 256, 0, st>>>(workspace, blocks, D, (__nv_bfloat16*)dgamma,
-                                                                   (__nv_bfloat16*)dbeta);
-        CUDA_CHECK(cudaGetLastError());
-    });
+    return cclx_layer_norm_bwd_sums(dy, x, w, mean, rstd, dres, dx, dgamma, dbeta, nullptr, 0, workspace, rows, D, stream);
 }
 
 // workspace: fp32 [64 * N]; counters: (N + 255) / 256 zero-initialised words that the kernel leaves zero

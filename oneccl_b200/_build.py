@@ -1,6 +1,6 @@
 """In-tree build of the native libraries.
 
-Two artefacts, both placed in ``oneccl_b200/lib`` so that they travel with the
+Three artefacts, all placed in ``oneccl_b200/lib`` so that they travel with the
 source tree:
 
 * ``libccl_b200.so``   - the collective library itself (C++17 host runtime and
@@ -9,6 +9,8 @@ source tree:
   the Python bindings.
 * ``_ccl_torch.so``    - the torch.distributed backend ("ccl" ProcessGroup),
   built against the installed torch headers.
+* ``_ccl_ops.so``      - the host code of ``oneccl_b200.ops`` (autograd functions and
+  their calls into the library), built the same way.
 
 The build is driven by a generated ninja file: one object per source, rebuilt
 only when the source or a header changes.  ``python -m oneccl_b200._build``
@@ -115,25 +117,34 @@ rule link
 
 def build_torch_backend(verbose: bool = False) -> Path:
     """Compile the c10d backend against the installed torch and link it to libccl_b200.so."""
+    return _build_torch_extension("_ccl_torch", ROOT / "oneccl_b200" / "torch_backend", verbose)
+
+
+def build_torch_ops(verbose: bool = False) -> Path:
+    """Compile the operators' host code against the installed torch and link it to libccl_b200.so."""
+    return _build_torch_extension("_ccl_ops", ROOT / "oneccl_b200" / "torch_ops", verbose)
+
+
+def _build_torch_extension(name: str, src_dir: Path, verbose: bool) -> Path:
     import torch
     from torch.utils import cpp_extension as ce
 
     build_native(verbose)
-    bdir = BUILD / "torch"
+    bdir = BUILD / ("torch" if name == "_ccl_torch" else name)
     bdir.mkdir(parents=True, exist_ok=True)
-    srcs = sorted((ROOT / "oneccl_b200" / "torch_backend").glob("*.cpp"))
+    srcs = sorted(src_dir.glob("*.cpp"))
     if not srcs:
-        raise RuntimeError("no torch backend sources")
+        raise RuntimeError(f"no sources of {name}")
     incs = ce.include_paths() + [str(CSRC), str(CSRC / "include"), "/usr/local/cuda/include",
                                  sysconfig.get_paths()["include"]]
     inc = " ".join(f"-I{p}" for p in incs)
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
     cxxflags = (
         f"-std=c++17 -O2 -fPIC -Wall -Wno-unused-function -Wno-sign-compare -pthread {inc} "
-        f"-D_GLIBCXX_USE_CXX11_ABI={abi} -DTORCH_EXTENSION_NAME=_ccl_torch -DTORCH_API_INCLUDE_EXTENSION_H -DUSE_C10D_NCCL=0"
+        f"-D_GLIBCXX_USE_CXX11_ABI={abi} -DTORCH_EXTENSION_NAME={name} -DTORCH_API_INCLUDE_EXTENSION_H -DUSE_C10D_NCCL=0"
     )
     tlib = Path(torch.__file__).parent / "lib"
-    ext = LIBDIR / "_ccl_torch.so"
+    ext = LIBDIR / f"{name}.so"
     ldflags = (
         f"-shared -L{tlib} -L{LIBDIR} -Wl,-rpath,{tlib} '-Wl,-rpath,$$ORIGIN' "
         f"-lc10 -lc10_cuda -ltorch_cpu -ltorch_cuda -ltorch -ltorch_python -lccl_b200"
@@ -187,6 +198,7 @@ def build_all(verbose: bool = False):
     build_native(verbose)
     if (ROOT / "oneccl_b200" / "torch_backend").exists():
         build_torch_backend(verbose)
+        build_torch_ops(verbose)
 
 
 if __name__ == "__main__":

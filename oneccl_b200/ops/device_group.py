@@ -14,27 +14,22 @@ flavours that share every kernel:
 from __future__ import annotations
 
 import ctypes as C
-import threading
 from typing import Optional, Sequence
 
 import torch
 
 from .. import _lib
 from ..dtypes import GPU_ALGO, COLL, reduce_op_code, torch_to_ccl
+from ..torch_ops import native
 
 
 def _stream_ptr(stream=None) -> int:
     """Raw handle of the launch stream; also points the library's own CUDA runtime
     (per-thread current device) at the caller's device."""
-    s = stream if stream is not None else torch.cuda.current_stream()
-    idx = s.device.index if s.device.index is not None else torch.cuda.current_device()
-    if getattr(_tls, "device", None) != idx:  # the library's runtime keeps the device per thread too
-        _lib.load().cclx_set_device(idx)
-        _tls.device = idx
-    return s.cuda_stream
-
-
-_tls = threading.local()
+    if stream is None:
+        return native().stream_ptr()
+    native().set_device(stream.device_index)
+    return stream.cuda_stream
 
 
 class _SymmStorage:

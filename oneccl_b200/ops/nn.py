@@ -8,7 +8,7 @@
 * ``split_qkv``: views of a packed QKV projection for the attention call, whose backward assembles the
   packed gradient with one strided copy kernel instead of a concatenation.
 
-Shapes the kernels do not cover (LayerNorm width not a multiple of 256 or above 1024, non-bf16, CPU)
+Shapes the kernels do not cover (LayerNorm width not a multiple of 8, below 256 or above 2048, non-bf16, CPU)
 fall back to the equivalent PyTorch ops."""
 from __future__ import annotations
 
@@ -18,84 +18,25 @@ import torch
 import torch.nn.functional as F
 
 from .. import _lib
+from ..torch_ops import native
 from .device_group import _stream_ptr
 from . import train as _train
 
 
-def _ln_ok(x: torch.Tensor, D: int) -> bool:
-    return x.is_cuda and x.dtype == torch.bfloat16 and D % 256 == 0 and 256 <= D <= 1024
-
-
-class _AddLayerNorm(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, res, weight, bias, eps):
-        D = x.shape[-1]
-        x2 = x.reshape(-1, D)
-        x2 = x2 if x2.is_contiguous() else x2.contiguous()
-        rows = x2.shape[0]
-        y = torch.empty_like(x2)
-        mean = torch.empty(rows, dtype=torch.float32, device=x.device)
-        rstd = torch.empty_like(mean)
-        lib = _lib.load()
-        if res is not None:
-            r2 = res.reshape(-1, D)
-            r2 = r2 if r2.is_contiguous() else r2.contiguous()
-            total = torch.empty_like(x2)
-            _lib.check(lib.cclx_layer_norm_fwd(x2.data_ptr(), r2.data_ptr(), weight.data_ptr(), bias.data_ptr(),
-                                               y.data_ptr(), total.data_ptr(), mean.data_ptr(), rstd.data_ptr(), rows, D,
-                                               eps, _stream_ptr()))
-        else:
-            total = x2
-            _lib.check(lib.cclx_layer_norm_fwd(x2.data_ptr(), 0, weight.data_ptr(), bias.data_ptr(), y.data_ptr(), 0,
-                                               mean.data_ptr(), rstd.data_ptr(), rows, D, eps, _stream_ptr()))
-        _train._bump()
-        ctx.save_for_backward(total, weight, mean, rstd)
-        ctx.has_res = res is not None
-        ctx.shape = x.shape
-        if res is not None:
-            return y.view(x.shape), total.view(x.shape)
-        return y.view(x.shape)
-
-    @staticmethod
-    def backward(ctx, dy, dsum=None):
-        total, weight, mean, rstd = ctx.saved_tensors
-        rows, D = total.shape
-        lib = _lib.load()
-        dy2 = dy.reshape(rows, D)
-        dy2 = dy2 if dy2.is_contiguous() else dy2.contiguous()
-        dres = None
-        if ctx.has_res and dsum is not None:
-            dres = dsum.reshape(rows, D)
-            dres = dres if dres.is_contiguous() else dres.contiguous()
-        dx = torch.empty_like(total)
-        dgamma = torch.empty_like(weight)
-        dbeta = torch.empty_like(weight)
-        blocks = lib.cclx_layer_norm_bwd_blocks(rows)
-        ws = torch.empty(blocks * 2 * D, dtype=torch.float32, device=total.device)
-        _lib.check(lib.cclx_layer_norm_bwd(dy2.data_ptr(), total.data_ptr(), weight.data_ptr(), mean.data_ptr(),
-                                           rstd.data_ptr(), 0 if dres is None else dres.data_ptr(), dx.data_ptr(),
-                                           dgamma.data_ptr(), dbeta.data_ptr(), ws.data_ptr(), rows, D, _stream_ptr()))
-        _train._bump(2)
-        dx = dx.view(ctx.shape)
-        if ctx.has_res:
-            return dx, dx, dgamma, dbeta, None
-        return dx, None, dgamma, dbeta, None
-
-
 def layer_norm(x, weight, bias, eps: float = 1e-5):
-    if not _ln_ok(x, x.shape[-1]):
-        return F.layer_norm(x, (x.shape[-1],), weight, bias, eps)
-    return _AddLayerNorm.apply(x, None, weight, bias, eps)
+    y = native().add_layer_norm(x, None, weight, bias, eps)
+    return F.layer_norm(x, (x.shape[-1],), weight, bias, eps) if y is None else y
 
 
 def add_layer_norm(x, res, weight, bias, eps: float = 1e-5):
     """Returns (LayerNorm(x + res), x + res)."""
     if res is None:
         return layer_norm(x, weight, bias, eps), x
-    if not _ln_ok(x, x.shape[-1]):
+    out = native().add_layer_norm(x, res, weight, bias, eps)
+    if out is None:
         s = x + res
         return F.layer_norm(s, (s.shape[-1],), weight, bias, eps), s
-    return _AddLayerNorm.apply(x, res, weight, bias, eps)
+    return out
 
 
 def colsum(dy2: torch.Tensor) -> torch.Tensor:

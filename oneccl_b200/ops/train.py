@@ -1,22 +1,29 @@
 """Training-step kernels next to the gradient collective: fused softmax
 cross-entropy (logits become their own gradient in place), squared gradient
 norm and flat fused AdamW with fp32 master weights.  All three are native
-kernels from ``csrc/gpu/train_kernels.cu``; ``launch_count`` lets callers
-report how many of them ran."""
+kernels from ``csrc/gpu/train_kernels.cu``; ``launch_count`` (kernels launched by this
+package's training and layer operators so far) lets callers report how many of them ran."""
 from __future__ import annotations
 
 import torch
 
 from .. import _lib
 from ..dtypes import torch_to_ccl
+from ..torch_ops import native
 from .device_group import _stream_ptr
 
-launch_count = 0
+_py_launches = 0
 
 
 def _bump(n=1):
-    global launch_count
-    launch_count += n
+    global _py_launches
+    _py_launches += n
+
+
+def __getattr__(name):
+    if name == "launch_count":
+        return _py_launches + native().launch_count()
+    raise AttributeError(name)
 
 
 class _SoftmaxXent(torch.autograd.Function):

@@ -1,0 +1,71 @@
+// Shared pieces of the torch-side operators (host code of oneccl_b200.ops in C++): stream and device of a call, error
+// translation, the launch counter, prototypes of the kernel entry points in libccl_b200.so.
+//
+// Why C++: an operator of a small tensor costs more host time than GPU time.  Written as Python autograd functions over
+// ctypes, LayerNorm forward + backward took 125 to 190 us of host time around 42 us of kernels.
+#pragma once
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/extension.h>
+
+#include <atomic>
+#include <optional>
+#include <stdexcept>
+#include <string>
+
+extern "C" {
+const char* cclx_last_error();
+int cclx_set_device(int dev);
+int cclx_layer_norm_fwd(const void* x, const void* res, const void* w, const void* b, void* y, void* sum_out, float* mean,
+                        float* rstd, size_t rows, int D, float eps, void* stream);
+int cclx_layer_norm_bwd_blocks(size_t rows);
+int cclx_layer_norm_bwd_sums(const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
+                             const void* dres, void* dx, void* dgamma, void* dbeta, void* dxsum, int add,
+                             float* workspace, size_t rows, int D, void* stream);
+}
+
+namespace cclx_ops {
+
+using at::Tensor;
+
+// becomes oneccl_b200.CclError in Python
+struct ccl_error : std::runtime_error {
+    using std::runtime_error::runtime_error;
+};
+
+inline void check(int rc) {
+    if (rc != 0)
+        throw ccl_error(cclx_last_error());
+}
+
+// The library has its own CUDA runtime, whose current device is per thread as well: it follows the device of the call
+// (autograd runs backward on threads of its own).
+inline void set_device(int dev) {
+    thread_local int current = -1;
+    if (current != dev) {
+        check(cclx_set_device(dev));
+        current = dev;
+    }
+}
+
+inline void* stream_of(const Tensor& t) {
+    const int dev = t.get_device();
+    set_device(dev);
+    return at::cuda::getCurrentCUDAStream(dev).stream();
+}
+
+extern std::atomic<long long> launches; // kernels of the library launched through this module
+
+inline bool aligned16(const Tensor& t) {
+    return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+}
+
+// an uninitialised contiguous tensor on the device of `like`, without the dispatcher's round trip
+inline Tensor empty_on(const Tensor& like, at::IntArrayRef sizes, at::ScalarType dtype) {
+    return at::detail::empty_cuda(sizes, dtype, like.device(), std::nullopt);
+}
+
+void bind_nn(pybind11::module_& m);
+
+} // namespace cclx_ops

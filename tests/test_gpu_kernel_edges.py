@@ -1,0 +1,45 @@
+"""The kernels at the sizes where their tiling can go wrong: edges, remainders, smallest and largest of a range."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _bf16(g, *shape, scale=1.0):
+    return (torch.randn(*shape, generator=g, device="cuda") * scale).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("D", [256, 264, 512, 1032, 1280, 1600, 2048])
+@pytest.mark.parametrize("rows", [1, 3, 149, 2369, 4801])  # below / above the two-rows-per-step switch, odd remainders
+def test_layer_norm_widths(rows, D):
+    from oneccl_b200.ops.nn import add_layer_norm
+
+    g = torch.Generator(device="cuda").manual_seed(rows * D)
+    x, r, dy, ds = (_bf16(g, rows, D) for _ in range(4))
+    w, b = 1 + _bf16(g, D, scale=0.1), _bf16(g, D, scale=0.1)
+    ins = [t.requires_grad_(True) for t in (x, r, w, b)]
+    y, s = add_layer_norm(*ins)
+    got = torch.autograd.grad([y, s], ins, [dy, ds])
+    tot = (x + r).detach()
+    ref = [t.detach().float().requires_grad_(True) for t in (tot, w, b)]
+    yr = torch.nn.functional.layer_norm(ref[0], (D,), ref[1], ref[2])
+    want = torch.autograd.grad([yr, ref[0] * 1.0], ref, [dy.float(), ds.float()])
+    assert torch.equal(s, tot) and torch.equal(got[0], got[1])
+    torch.testing.assert_close(y.float(), yr, rtol=2e-2, atol=2e-2)
+    torch.testing.assert_close(got[0].float(), want[0], rtol=2e-2, atol=3e-2)
+    for a, c in zip(got[2:], want[1:]):
+        torch.testing.assert_close(a.float(), c, rtol=1e-2, atol=1e-2 * max(1.0, rows ** 0.5))
+
+
+def test_layer_norm_unused_outputs():
+    from oneccl_b200.ops.nn import add_layer_norm
+
+    g = torch.Generator(device="cuda").manual_seed(0)
+    ins = [t.requires_grad_(True) for t in (_bf16(g, 2, 5, 512), _bf16(g, 2, 5, 512), _bf16(g, 512), _bf16(g, 512))]
+    d = _bf16(g, 2, 5, 512)
+    _, s = add_layer_norm(*ins)  # only the sum is used: its gradient passes through
+    assert torch.equal(torch.autograd.grad(s, ins[0], d)[0], d)
+    y, _ = add_layer_norm(*ins)
+    y2 = torch.nn.functional.layer_norm((ins[0] + ins[1]), (512,), ins[2], ins[3])
+    for a, c in zip(torch.autograd.grad(y, ins, d), torch.autograd.grad(y2, ins, d)):
+        torch.testing.assert_close(a.float(), c.float(), rtol=3e-2, atol=3e-2)
