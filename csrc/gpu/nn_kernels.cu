@@ -9,14 +9,16 @@
 #include <stdint.h>
 
 #include <algorithm>
-#include <atomic>
 
 #include "capi/capi_common.hpp"
 #include "core/log.hpp"
+#include "gpu/async_copy.cuh"
 #include "gpu/cuda_driver.hpp"
-#include "gpu/pdl.cuh"
+#include "gpu/f32x2.cuh"
+#include "gpu/launch_util.cuh"
 
 using namespace cclx;
+using namespace cclx::gpu;
 
 namespace {
 
@@ -34,49 +36,6 @@ __device__ __forceinline__ void unpack8(const uint4& u, float (&x)[8]) {
         x[2 * i] = __uint_as_float(w[i] << 16);
         x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
     }
-}
-
-// pairs of fp32 values: one instruction adds or multiplies both (fma.rn.f32x2 and relatives)
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pair(float lo, float hi) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpair(f32x2 v, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ void unpack4x2(const uint4& u, f32x2 (&x)[4]) {
-    const uint32_t w[4] = { u.x, u.y, u.z, u.w };
-#pragma unroll
-    for (int i = 0; i < 4; i++) // bf16 is the upper half of an fp32 word
-        x[i] = pair(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
-}
-__device__ __forceinline__ uint4 pack4x2(const f32x2 (&x)[4]) {
-    uint32_t w[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        float lo, hi;
-        unpair(x[i], lo, hi);
-        const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-        w[i] = *reinterpret_cast<const uint32_t*>(&h);
-    }
-    return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
 __device__ __forceinline__ uint4 pack8(const float (&x)[8]) {
@@ -187,18 +146,6 @@ __device__ __forceinline__ float warp_sum_many(float (&v)[NV], int lane) {
     return v[0];
 }
 
-__device__ __forceinline__ void copy16_async(void* smem, const void* gmem, bool on) {
-    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(gmem), "r"(on ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void copy_commit() {
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
-template <int N>
-__device__ __forceinline__ void copy_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
 constexpr int LN_BWD_ROWS = 2; // rows per step of a group
 constexpr int LN_BWD_STAGES = 4; // steps in flight or in use
 constexpr int LN_BWD_BLOCKS = 2; // resident blocks per SM
@@ -229,7 +176,7 @@ __global__ void __launch_bounds__(256, LN_BWD_BLOCKS)
     for (int i = threadIdx.x; i < 2 * groups * 2 * R * 8; i += blockDim.x)
         sums[i] = 0.f;
     __syncthreads();
-    gpu::pdl_trigger(); // the final sum may be scheduled as soon as SMs fall idle; it waits for this grid's end
+    pdl_trigger(); // the final sum may be scheduled as soon as SMs fall idle; it waits for this grid's end
     f32x2 wv[4], acc2[NS][4];
     unpack4x2(on ? w[c] : make_uint4(0, 0, 0, 0), wv);
 #pragma unroll
@@ -380,7 +327,7 @@ struct partial_outs {
 __global__ void __launch_bounds__(256) partial_rows_sum_kernel(const float* __restrict__ partial, int n, int cols, partial_outs o) {
     const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
     const int c = blockIdx.x * 32 + lane, which = blockIdx.y;
-    gpu::pdl_wait();
+    pdl_wait();
     float a = 0.f;
     if (c < cols) {
         const float* p = partial + (size_t)which * cols + c;
@@ -515,19 +462,6 @@ int sm_count_now() {
     return sms;
 }
 
-// dynamic shared memory above the default 48 KB, granted to the kernel once per device
-template <auto KERNEL>
-void allow_smem(size_t bytes) {
-    static std::atomic<bool> done[64];
-    int dev = 0;
-    CUDA_CHECK(cudaGetDevice(&dev));
-    if (dev < 64 && done[dev].load(std::memory_order_acquire))
-        return;
-    CUDA_CHECK(cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    if (dev < 64)
-        done[dev].store(true, std::memory_order_release);
-}
-
 } // namespace
 
 // ---- C entry points -----------------------------------------------------------------------------
@@ -608,7 +542,7 @@ CCLX_API int cclx_layer_norm_bwd_sums(const void* dy, const void* x, const void*
             n = wide ? launch_ln_bwd<LN_BWD_ROWS, false>(dy, x, w, mean, rstd, dres, dx, workspace, rows, D, st)
                      : launch_ln_bwd<1, false>(dy, x, w, mean, rstd, dres, dx, workspace, rows, D, st);
         partial_outs o{ { (__nv_bfloat16*)dgamma, (__nv_bfloat16*)dbeta, (__nv_bfloat16*)dxsum }, add };
-        gpu::launch_dependent(partial_rows_sum_kernel, dim3((D + 31) / 32, dxsum ? 3 : 2), dim3(256), 0, st,
+        launch_dependent(partial_rows_sum_kernel, dim3((D + 31) / 32, dxsum ? 3 : 2), dim3(256), 0, st,
                               (const float*)workspace, n, D, o);
     });
 }

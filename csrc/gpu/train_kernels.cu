@@ -12,9 +12,17 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "capi/capi_common.hpp"
 #include "core/log.hpp"
+#include "gpu/async_copy.cuh"
 #include "gpu/cuda_driver.hpp"
+#include "gpu/f32x2.cuh"
+#include "gpu/launch_util.cuh"
+
+using namespace cclx;
+using namespace cclx::gpu;
 
 namespace {
 
@@ -267,130 +275,292 @@ __global__ void __launch_bounds__(1024)
     }
 }
 
-// Same contract as softmax_xent_kernel for rows that fit the register file: every thread keeps up
-// to PPT 16-byte packs of the row in registers, so the row is read from memory once.  The exponentials
-// are computed once (fp32, summed in fp32) and parked in the same registers as bf16 until the
-// normaliser is known; the gradient is bf16 anyway, the second rounding costs at most one more ulp.
-// Needs vocab % 8 == 0 columns handled as packs plus a scalar tail, ld % 8 == 0 and a 16-byte aligned base.
-template <int PPT>
-__global__ void __launch_bounds__(1024)
-    softmax_xent_regs_kernel(__nv_bfloat16* logits, const long long* targets, float* loss_rows, int vocab, size_t ld,
-                             float grad_scale, int pad_cols) {
-    constexpr float LOG2E = 1.4426950408889634f;
-    const size_t row = blockIdx.x;
-    __nv_bfloat16* x = logits + row * ld;
-    const long long tgt = targets[row];
-    __shared__ float red[32];
-    __shared__ float s_max, s_sum, s_tgt;
-    const int nv = vocab / 8;
-    uint4* xv = reinterpret_cast<uint4*>(x);
-    const int tail = nv * 8 + (int)threadIdx.x; // at most 7 leftover columns, one per thread
-    const bool has_tail = tail < vocab;
+// Softmax cross-entropy kernels.  A row of logits [rows, vocab] (bf16, row pitch ld) becomes its own gradient:
+// loss_row = logsumexp - logit[target], row <- (softmax - onehot) * grad_scale, all math in fp32.  Rows whose target is
+// outside [0, vocab) (ignored) have zero loss and zero gradient.  Columns [vocab, vocab + pad_cols) are alignment
+// padding and receive zeros.
+constexpr float LOG2E = 1.4426950408889634f;
 
-    uint4 u[PPT];
-#pragma unroll
-    for (int j = 0; j < PPT; j++) {
-        const int i = (int)threadIdx.x + j * 1024;
-        u[j] = i < nv ? xv[i] : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u); // -inf pairs
-    }
-    float xt = has_tail ? __bfloat162float(x[tail]) : -INFINITY;
-    if (threadIdx.x == 0)
-        s_tgt = (tgt >= 0 && tgt < vocab) ? __bfloat162float(x[tgt]) : 0.f;
+__device__ __forceinline__ float ex2(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 
-    float mx = xt;
-#pragma unroll
-    for (int j = 0; j < PPT; j++) {
-        const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&u[j]);
-#pragma unroll
-        for (int k = 0; k < 8; k++)
-            mx = fmaxf(mx, __bfloat162float(h[k]));
-    }
-    mx = warp_max(mx);
-    if ((threadIdx.x & 31) == 0)
-        red[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        float v = warp_max(red[threadIdx.x]);
-        if (threadIdx.x == 0)
-            s_max = v;
-    }
-    __syncthreads();
-    mx = s_max;
-    const float ms = mx * LOG2E;
+// largest of eight bf16 values
+__device__ __forceinline__ float max8(const uint4& u) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+    const __nv_bfloat162 m = __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3]));
+    return fmaxf(__low2float(m), __high2float(m));
+}
 
-    float sum = 0.f;
+// sum of 2^(x * log2(e) + shift) over eight bf16 values
+__device__ __forceinline__ float exp_sum8(const uint4& u, float shift) {
+    f32x2 x[4];
+    unpack4x2(u, x);
+    const f32x2 l2 = pair(LOG2E, LOG2E), sh = pair(shift, shift);
+    float a = 0.f;
 #pragma unroll
-    for (int j = 0; j < PPT; j++) {
-        __nv_bfloat16* h = reinterpret_cast<__nv_bfloat16*>(&u[j]);
+    for (int i = 0; i < 4; i++) {
+        float lo, hi;
+        unpair(fma2(x[i], l2, sh), lo, hi);
+        a += ex2(lo) + ex2(hi);
+    }
+    return a;
+}
+
+// 2^(x * log2(e) + shift) * inv, minus `hit` at element `at` (0 to 7, else nowhere)
+__device__ __forceinline__ uint4 grad8(const uint4& u, float shift, float inv, long long at, float hit) {
+    f32x2 x[4];
+    unpack4x2(u, x);
+    const f32x2 l2 = pair(LOG2E, LOG2E), sh = pair(shift, shift), k = pair(inv, inv);
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const float e = exp2f(fmaf(__bfloat162float(h[k]), LOG2E, -ms)); // exp2(-inf) = 0 for the filler
-            sum += e;
-            h[k] = __float2bfloat16_rn(e);
+    for (int i = 0; i < 4; i++) {
+        float lo, hi;
+        unpair(fma2(x[i], l2, sh), lo, hi);
+        x[i] = mul2(pair(ex2(lo), ex2(hi)), k);
+    }
+    if (at >= 0 && at < 8) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            float lo, hi;
+            unpair(x[i], lo, hi);
+            x[i] = pair(at == 2 * i ? lo - hit : lo, at == 2 * i + 1 ? hi - hit : hi);
         }
     }
-    const float et = has_tail ? exp2f(fmaf(xt, LOG2E, -ms)) : 0.f;
-    sum += et;
-    sum = warp_sum(sum);
-    if ((threadIdx.x & 31) == 0)
-        red[threadIdx.x >> 5] = sum;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        float v = warp_sum(red[threadIdx.x]);
-        if (threadIdx.x == 0)
-            s_sum = v;
+    return pack4x2(x);
+}
+
+// logit `at` (0 to 7) of a pack
+__device__ __forceinline__ float pick8(const uint4& u, int at) {
+    const uint32_t w = at < 2 ? u.x : at < 4 ? u.y : at < 6 ? u.z : u.w;
+    return __uint_as_float(at & 1 ? w & 0xffff0000u : w << 16);
+}
+
+// Running maximum and sum of exponentials below it: one more pack.  The maximum rarely moves after the first packs.
+__device__ __forceinline__ void online8(const uint4& u, float& m, float& shift, float& s) {
+    const float pm = max8(u);
+    if (pm > m) {
+        s = m == -INFINITY ? 0.f : s * ex2((m - pm) * LOG2E);
+        m = pm;
+        shift = -m * LOG2E;
     }
-    __syncthreads();
-    sum = s_sum;
-    const bool ignore = tgt < 0 || tgt >= vocab;
-    if (threadIdx.x == 0)
-        loss_rows[row] = ignore ? 0.f : (logf(sum) + mx - s_tgt);
-    const float inv = ignore ? 0.f : grad_scale / sum;
-    for (int i = vocab + threadIdx.x; i < vocab + pad_cols; i += blockDim.x)
-        x[i] = __float2bfloat16_rn(0.f);
-#pragma unroll
-    for (int j = 0; j < PPT; j++) {
-        const int i = (int)threadIdx.x + j * 1024;
-        if (i < nv) {
-            __nv_bfloat16* h = reinterpret_cast<__nv_bfloat16*>(&u[j]);
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                float p = __bfloat162float(h[k]) * inv;
-                if (!ignore && (long long)i * 8 + k == tgt)
-                    p -= grad_scale;
-                h[k] = __float2bfloat16_rn(p);
+    s += exp_sum8(u, shift);
+}
+__device__ __forceinline__ void online1(float x, float& m, float& shift, float& s) {
+    if (x > m) {
+        s = m == -INFINITY ? 0.f : s * ex2((m - x) * LOG2E);
+        m = x;
+        shift = -m * LOG2E;
+    }
+    s += ex2(fmaf(x, LOG2E, shift));
+}
+
+// Long rows.  Bound by memory (every logit read and written once) with the exponential unit close behind: two
+// exponentials per logit cost 187 of the 252 us that 8192 x 50304 logits need at the copy rate.  A block keeps one
+// row in shared memory.  Thread t owns packs t, t + T, ...; it copies them in with cp.async and is the only one to read
+// them, so the only block-wide step per row is the exchange of (maximum, sum) pairs.  While the gradient of a row goes
+// out, every pack read back is replaced at once by the same pack of the block's next row, so loads are in flight
+// during stores, and the packs of a row are consumed in four groups as they arrive.  Two blocks per SM (rows up to
+// 53 K logits) fill each other's gaps.  One block per row with the row in registers, which this replaces, left the
+// memory idle in all phases but one: 552 us for 8192 x 50257, now 300.
+template <int T>
+__global__ void __launch_bounds__(T, T == 1024 ? 1 : 1024 / T)
+    xent_stream_kernel(__nv_bfloat16* logits, const long long* __restrict__ targets, float* __restrict__ loss_rows, size_t rows,
+                       int vocab, size_t ld, float grad_scale, int pad_cols, int ppt) {
+    extern __shared__ uint4 ring[]; // [ppt][T]
+    __shared__ float2 part[2][32];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int nv = vocab / 8, per = (ppt + 3) / 4;
+    const int tail = nv * 8 + t; // at most 7 columns behind the packs, one per thread
+    pdl_trigger();
+    auto fetch = [&](size_t row, int j) {
+        const int i = t + j * T;
+        const bool ok = row < rows && i < nv;
+        copy16_async(ring + j * T + t, ok ? logits + row * ld + (size_t)i * 8 : logits, ok);
+    };
+    size_t row = blockIdx.x;
+    for (int g = 0; g < 4; g++) {
+        for (int j = g * per; j < min((g + 1) * per, ppt); j++)
+            fetch(row, j);
+        copy_commit();
+    }
+    int buf = 0;
+    for (; row < rows; row += gridDim.x, buf ^= 1) {
+        __nv_bfloat16* x = logits + row * ld;
+        const long long tgt = targets[row];
+        const float xt = tail < vocab ? __bfloat162float(x[tail]) : 0.f;
+        float m = -INFINITY, shift = 0.f, s = 0.f;
+        auto eat = [&](int g) {
+            for (int j = g * per; j < min((g + 1) * per, ppt); j++)
+                if (t + j * T < nv)
+                    online8(ring[j * T + t], m, shift, s);
+        };
+        copy_wait<3>();
+        eat(0);
+        copy_wait<2>();
+        eat(1);
+        copy_wait<1>();
+        eat(2);
+        copy_wait<0>();
+        eat(3);
+        if (tail < vocab)
+            online1(xt, m, shift, s);
+        const float wm = warp_max(m);
+        const float ws = warp_sum(m == -INFINITY ? 0.f : s * ex2((m - wm) * LOG2E));
+        if (lane == 0)
+            part[buf][warp] = make_float2(wm, ws);
+        __syncthreads();
+        const float2 p = lane < T / 32 ? part[buf][lane] : make_float2(-INFINITY, 0.f);
+        const float mx = warp_max(p.x);
+        const float sum = warp_sum(p.x == -INFINITY ? 0.f : p.y * ex2((p.x - mx) * LOG2E));
+        const bool ignore = tgt < 0 || tgt >= vocab;
+        const float inv = ignore ? 0.f : grad_scale / sum, hit = ignore ? 0.f : grad_scale;
+        shift = -mx * LOG2E;
+        if (ignore && t == 0)
+            loss_rows[row] = 0.f;
+        const long long at0 = ignore ? -1 : tgt;
+        for (int g = 0; g < 4; g++) {
+            for (int j = g * per; j < min((g + 1) * per, ppt); j++) {
+                const int i = t + j * T;
+                if (i < nv) {
+                    const uint4 u = ring[j * T + t];
+                    const long long at = at0 - (long long)i * 8;
+                    if (at >= 0 && at < 8)
+                        loss_rows[row] = logf(sum) + mx - pick8(u, (int)at);
+                    reinterpret_cast<uint4*>(x)[i] = grad8(u, shift, inv, at, hit);
+                }
+                fetch(row + gridDim.x, j);
             }
-            xv[i] = u[j];
+            copy_commit();
+        }
+        if (tail < vocab) {
+            float q = ex2(fmaf(xt, LOG2E, shift)) * inv;
+            if (tail == at0) {
+                loss_rows[row] = logf(sum) + mx - xt;
+                q -= hit;
+            }
+            x[tail] = __float2bfloat16_rn(q);
+        }
+        for (int i = vocab + t; i < vocab + pad_cols; i += T)
+            x[i] = __float2bfloat16_rn(0.f);
+    }
+    copy_wait<0>();
+}
+
+// Short rows (up to 256 * V logits): one warp per row, the row in registers, one exponential per logit, no barrier.
+// A block of 1024 threads per row spent most of its time waiting for itself: 317 x 1000 took 13 us, now 3.
+template <int V>
+__global__ void __launch_bounds__(128)
+    xent_warp_kernel(__nv_bfloat16* logits, const long long* __restrict__ targets, float* __restrict__ loss_rows, size_t rows,
+                     int vocab, size_t ld, float grad_scale, int pad_cols) {
+    const int lane = threadIdx.x & 31, nv = vocab / 8, tail = nv * 8 + lane;
+    pdl_trigger();
+    const size_t row = (size_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (row >= rows)
+        return;
+    __nv_bfloat16* x = logits + row * ld;
+    uint4* xv = reinterpret_cast<uint4*>(x);
+    const uint32_t ninf = 0xff80ff80u;
+    uint4 u[V];
+#pragma unroll
+    for (int v = 0; v < V; v++)
+        u[v] = lane + v * 32 < nv ? xv[lane + v * 32] : make_uint4(ninf, ninf, ninf, ninf);
+    const long long tgt = targets[row];
+    const float xt = tail < vocab ? __bfloat162float(x[tail]) : -INFINITY;
+    const bool ignore = tgt < 0 || tgt >= vocab;
+    float m = xt;
+#pragma unroll
+    for (int v = 0; v < V; v++)
+        m = fmaxf(m, max8(u[v]));
+    m = warp_max(m);
+    const float shift = -m * LOG2E;
+    float s = ex2(fmaf(xt, LOG2E, shift));
+#pragma unroll
+    for (int v = 0; v < V; v++)
+        s += exp_sum8(u[v], shift);
+    s = warp_sum(s);
+    const float inv = ignore ? 0.f : grad_scale / s, hit = ignore ? 0.f : grad_scale;
+    const long long at0 = ignore ? -1 : tgt;
+    if (ignore && lane == 0)
+        loss_rows[row] = 0.f;
+#pragma unroll
+    for (int v = 0; v < V; v++) {
+        const int i = lane + v * 32;
+        if (i < nv) {
+            const long long at = at0 - (long long)i * 8;
+            if (at >= 0 && at < 8)
+                loss_rows[row] = logf(s) + m - pick8(u[v], (int)at);
+            xv[i] = grad8(u[v], shift, inv, at, hit);
         }
     }
-    if (has_tail) {
-        float p = et * inv;
-        if (!ignore && tail == tgt)
-            p -= grad_scale;
-        x[tail] = __float2bfloat16_rn(p);
+    if (tail < vocab) {
+        float q = ex2(fmaf(xt, LOG2E, shift)) * inv;
+        if (tail == at0) {
+            loss_rows[row] = logf(s) + m - xt;
+            q -= hit;
+        }
+        x[tail] = __float2bfloat16_rn(q);
     }
+    for (int i = vocab + lane; i < vocab + pad_cols; i += 32)
+        x[i] = __float2bfloat16_rn(0.f);
+}
+
+int sm_count_now() {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+constexpr size_t XENT_SMEM = 226 * 1024; // shared memory of an SM that blocks can have, reserved parts aside
+
+template <int T>
+void launch_xent_stream(__nv_bfloat16* logits, const long long* targets, float* loss_rows, size_t rows, int vocab, size_t ld,
+                        float grad_scale, int pad_cols, cudaStream_t st) {
+    const int ppt = (vocab / 8 + T - 1) / T;
+    const size_t smem = (size_t)ppt * T * 16;
+    allow_smem<xent_stream_kernel<T>>(XENT_SMEM);
+    const int per_sm = std::max(1, std::min((int)(XENT_SMEM / (smem + 1536)), T == 1024 ? 1 : 1024 / T));
+    const int blocks = (int)std::min<size_t>(rows, (size_t)sm_count_now() * per_sm);
+    xent_stream_kernel<T><<<blocks, T, smem, st>>>(logits, targets, loss_rows, rows, vocab, ld, grad_scale, pad_cols, ppt);
 }
 
 void launch_softmax_xent(__nv_bfloat16* logits, const long long* targets, float* loss_rows, size_t rows, int vocab,
                          size_t ld, float grad_scale, int pad_cols, cudaStream_t st) {
     const bool vec = (ld % 8 == 0) && ((((uintptr_t)logits) & 15) == 0);
     const int nv = vocab / 8;
-    if (vec && nv <= 4 * 1024)
-        softmax_xent_regs_kernel<4><<<(unsigned)rows, 1024, 0, st>>>(logits, targets, loss_rows, vocab, ld, grad_scale,
-                                                                    pad_cols);
-    else if (vec && nv <= 7 * 1024)
-        softmax_xent_regs_kernel<7><<<(unsigned)rows, 1024, 0, st>>>(logits, targets, loss_rows, vocab, ld, grad_scale,
-                                                                    pad_cols);
+    const unsigned warp_blocks = (unsigned)((rows + 3) / 4);
+#define XENT_WARP(V) \
+    xent_warp_kernel<V><<<warp_blocks, 128, 0, st>>>(logits, targets, loss_rows, rows, vocab, ld, grad_scale, pad_cols)
+    // a warp's registers hold 2048 logits; longer rows stream through shared memory by a block whose threads own
+    // about four to thirteen packs each, up to what the shared memory of an SM takes (106 K logits); rows that are
+    // longer still or not 16-byte aligned are read three times
+    if (vec && nv <= 32)
+        XENT_WARP(1);
+    else if (vec && nv <= 64)
+        XENT_WARP(2);
+    else if (vec && nv <= 128)
+        XENT_WARP(4);
+    else if (vec && nv <= 256)
+        XENT_WARP(8);
+    else if (vec && nv <= 8 * 128)
+        launch_xent_stream<128>(logits, targets, loss_rows, rows, vocab, ld, grad_scale, pad_cols, st);
+    else if (vec && nv <= 8 * 256)
+        launch_xent_stream<256>(logits, targets, loss_rows, rows, vocab, ld, grad_scale, pad_cols, st);
+    else if (vec && nv <= 13 * 512)
+        launch_xent_stream<512>(logits, targets, loss_rows, rows, vocab, ld, grad_scale, pad_cols, st);
+    else if (vec && nv <= 13 * 1024)
+        launch_xent_stream<1024>(logits, targets, loss_rows, rows, vocab, ld, grad_scale, pad_cols, st);
     else
         softmax_xent_kernel<<<(unsigned)rows, 1024, 0, st>>>(logits, targets, loss_rows, vocab, ld, grad_scale,
                                                             pad_cols);
+#undef XENT_WARP
     CUDA_CHECK(cudaGetLastError());
 }
 
 int grid_for(size_t n, int threads) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count_now();
     size_t want = (n + threads - 1) / threads;
     size_t cap = (size_t)sms * 4;
     return (int)(want < cap ? (want ? want : 1) : cap);
@@ -459,6 +629,26 @@ CCLX_API int cclx_adamw_flat(float* master, const void* grad, int grad_dt, float
     });
 }
 
+namespace {
+// out[0] = sum(rows[0..n)) / n, fixed summation order (one block: strided partials, warps, then the first warp)
+__global__ void __launch_bounds__(1024) mean_rows_kernel(const float* rows, size_t n, float* out) {
+    __shared__ float part[32];
+    pdl_wait(); // launched while the kernel that fills `rows` still runs
+    float acc = 0.f;
+    for (size_t i = threadIdx.x; i < n; i += blockDim.x)
+        acc += __ldcg(rows + i);
+    acc = warp_sum(acc);
+    if ((threadIdx.x & 31) == 0)
+        part[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        acc = warp_sum(part[threadIdx.x]);
+        if (threadIdx.x == 0)
+            out[0] = acc / (float)n;
+    }
+}
+} // namespace
+
 CCLX_API int cclx_softmax_xent(void* logits_bf16, const long long* targets, float* loss_rows, size_t rows, int vocab,
                                size_t ld, float grad_scale, int pad_cols, void* stream) {
     return cclx::capi::guard([&] {
@@ -466,6 +656,17 @@ CCLX_API int cclx_softmax_xent(void* logits_bf16, const long long* targets, floa
             return;
         launch_softmax_xent((__nv_bfloat16*)logits_bf16, targets, loss_rows, rows, vocab, ld, grad_scale, pad_cols,
                             (cudaStream_t)stream);
+    });
+}
+
+// the same with the mean of the row losses in mean_loss[0] (loss_rows: fp32 scratch [rows])
+CCLX_API int cclx_softmax_xent_mean(void* logits_bf16, const long long* targets, float* loss_rows, float* mean_loss, size_t rows,
+                                    int vocab, size_t ld, float grad_scale, int pad_cols, void* stream) {
+    return cclx::capi::guard([&] {
+        CCL_THROW_IF_NOT(rows > 0, "the mean of no rows");
+        launch_softmax_xent((__nv_bfloat16*)logits_bf16, targets, loss_rows, rows, vocab, ld, grad_scale, pad_cols,
+                            (cudaStream_t)stream);
+        launch_dependent(mean_rows_kernel, dim3(1), dim3(1024), 0, (cudaStream_t)stream, (const float*)loss_rows, rows, mean_loss);
     });
 }
 
@@ -482,23 +683,6 @@ namespace {
 
 // scratch: one loss per row.  Lives in every device's copy of this module until the process ends.
 static __device__ __align__(256) float xent_row_scratch[CCLX_XENT_NOALLOC_MAX_ROWS];
-
-// out[0] = sum(rows[0..n)) / n, fixed summation order (one block, strided partials, tree in shared memory)
-__global__ void __launch_bounds__(1024) mean_rows_kernel(const float* rows, size_t n, float* out) {
-    __shared__ float part[1024];
-    float acc = 0.f;
-    for (size_t i = threadIdx.x; i < n; i += blockDim.x)
-        acc += rows[i];
-    part[threadIdx.x] = acc;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s)
-            part[threadIdx.x] += part[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        out[0] = part[0] / (float)n;
-}
 
 constexpr int XENT_MAX_DEVICES = 64;
 std::mutex xent_setup_mu;
@@ -537,7 +721,6 @@ CCLX_API int cclx_softmax_xent_mean_noalloc(void* logits_bf16, const long long* 
         float* scratch = xent_scratch_for_current_device();
         cudaStream_t st = (cudaStream_t)stream;
         launch_softmax_xent((__nv_bfloat16*)logits_bf16, targets, scratch, rows, vocab, ld, grad_scale, pad_cols, st);
-        mean_rows_kernel<<<1, 1024, 0, st>>>(scratch, rows, mean_loss);
-        CUDA_CHECK(cudaGetLastError());
+        launch_dependent(mean_rows_kernel, dim3(1), dim3(1024), 0, st, (const float*)scratch, rows, mean_loss);
     });
 }

@@ -12,6 +12,9 @@ from ..dtypes import torch_to_ccl
 from ..torch_ops import native
 from .device_group import _stream_ptr
 
+# the stored logit gradient assumes d(loss) = 1; True multiplies it by the upstream gradient
+scale_by_upstream = False
+
 _py_launches = 0
 
 
@@ -26,40 +29,12 @@ def __getattr__(name):
     raise AttributeError(name)
 
 
-class _SoftmaxXent(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, logits, targets, vocab):
-        assert logits.dtype == torch.bfloat16 and logits.dim() == 2 and logits.stride(1) == 1
-        rows, cols = logits.shape
-        ld = logits.stride(0)
-        loss_rows = torch.empty(rows, dtype=torch.float32, device=logits.device)
-        lib = _lib.load()
-        # the kernel overwrites `logits` with d(mean loss)/d(logits)
-        _lib.check(lib.cclx_softmax_xent(logits.data_ptr(), targets.data_ptr(), loss_rows.data_ptr(), rows, vocab, ld,
-                                         1.0 / rows, cols - vocab, _stream_ptr()))
-        _bump()
-        # autograd is not told about the in-place write: the producer of `logits` (a matmul)
-        # does not need its output for its own backward
-        ctx.save_for_backward(logits)
-        return loss_rows.mean()
-
-    @staticmethod
-    def backward(ctx, grad_out):
-        (grad_logits,) = ctx.saved_tensors
-        # the stored gradient assumes d(loss) = 1; scale only when the caller scaled the loss
-        if ctx.needs_input_grad[0] and grad_out is not None and _SoftmaxXent.scale_by_upstream:
-            grad_logits = grad_logits * grad_out.to(grad_logits.dtype)
-        return grad_logits, None, None
-
-    scale_by_upstream = False
-
-
 def softmax_cross_entropy(logits: torch.Tensor, targets: torch.Tensor, vocab: int | None = None) -> torch.Tensor:
     """Mean cross-entropy over the rows of ``logits`` ([rows, cols] bf16; only the
     first ``vocab`` columns are classes, the rest is alignment padding).  ``logits``
     is consumed: it holds the gradient afterwards.  ``targets`` int64."""
-    vocab = logits.shape[1] if vocab is None else vocab
-    return _SoftmaxXent.apply(logits, targets.contiguous(), vocab)
+    assert logits.dtype == torch.bfloat16 and logits.dim() == 2 and logits.stride(1) == 1
+    return native().softmax_xent(logits, targets, logits.shape[1] if vocab is None else vocab, scale_by_upstream)
 
 
 _partials = {}

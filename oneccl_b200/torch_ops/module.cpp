@@ -26,4 +26,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     }, "handle of the current stream; the library's runtime follows its device");
     m.def("set_device", [](int dev) { set_device(dev); });
     bind_nn(m);
+    bind_train(m);
 }

@@ -23,6 +23,8 @@ int cclx_layer_norm_bwd_blocks(size_t rows);
 int cclx_layer_norm_bwd_sums(const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
                              const void* dres, void* dx, void* dgamma, void* dbeta, void* dxsum, int add,
                              float* workspace, size_t rows, int D, void* stream);
+int cclx_softmax_xent_mean(void* logits_bf16, const long long* targets, float* loss_rows, float* mean_loss, size_t rows,
+                           int vocab, size_t ld, float grad_scale, int pad_cols, void* stream);
 }
 
 namespace cclx_ops {
@@ -67,5 +69,6 @@ inline Tensor empty_on(const Tensor& like, at::IntArrayRef sizes, at::ScalarType
 }
 
 void bind_nn(pybind11::module_& m);
+void bind_train(pybind11::module_& m);
 
 } // namespace cclx_ops

@@ -43,3 +43,27 @@ def test_layer_norm_unused_outputs():
     y2 = torch.nn.functional.layer_norm((ins[0] + ins[1]), (512,), ins[2], ins[3])
     for a, c in zip(torch.autograd.grad(y, ins, d), torch.autograd.grad(y2, ins, d)):
         torch.testing.assert_close(a.float(), c.float(), rtol=3e-2, atol=3e-2)
+
+
+@pytest.mark.parametrize("vocab,pad", [(1, 7), (7, 1), (9, 0), (256, 0), (263, 1), (513, 7), (1031, 1), (2049, 0), (2056, 64),
+                                       (8199, 1), (8200, 0), (16385, 7), (53255, 1), (53256, 0), (106503, 1), (106504, 0)])
+@pytest.mark.parametrize("rows", [1, 5, 301])  # 301: blocks that take a second row
+def test_softmax_xent_row_lengths(rows, vocab, pad):
+    """Around every limit of the dispatch (one warp per row up to 2048 logits, blocks of 128 to 1024 threads, the
+    three-pass kernel), with ignored rows, masked (-inf) logits and alignment padding."""
+    from oneccl_b200.ops.train import softmax_cross_entropy
+
+    g = torch.Generator(device="cuda").manual_seed(vocab + rows)
+    logits = _bf16(g, rows, vocab + pad, scale=3)
+    logits[:, : min(vocab - 1, 40)][:, ::3] = float("-inf")
+    tgt = torch.randint(max(0, vocab - 2), vocab, (rows,), generator=g, device="cuda")
+    tgt[rows // 2] = -100 if rows > 1 else tgt[0]
+    ref = logits[:, :vocab].float().requires_grad_(True)
+    loss_ref = torch.nn.functional.cross_entropy(ref, tgt, ignore_index=-100, reduction="sum") / rows
+    (want,) = torch.autograd.grad(loss_ref, ref)
+    x = logits.clone().requires_grad_(True)
+    loss = softmax_cross_entropy(x, tgt, vocab)
+    (got,) = torch.autograd.grad(loss, x)
+    torch.testing.assert_close(loss, loss_ref, rtol=1e-4, atol=1e-4)
+    torch.testing.assert_close(got[:, :vocab].float(), want, rtol=1e-2, atol=1e-6)
+    assert not pad or torch.count_nonzero(got[:, vocab:]) == 0
