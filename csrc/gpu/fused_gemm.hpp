@@ -19,6 +19,11 @@ void gemm_bf16_plain(const void* A, const void* B, void* C, int M, int N, int K,
 void gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int clusters,
                    uint32_t* err, cudaStream_t st, const int* rows_dev = nullptr);
 
+// the same product cut along K over clusters of CTAs, for few rows or a small C; and whether it is the faster choice
+void gemm_bf16_small(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, uint32_t* err, cudaStream_t st,
+                     const int* rows_dev = nullptr);
+bool gemm_small_preferred(int M, int N, int K, int sms);
+
 struct fused_plan; // opaque
 
 // mode 1: all-gather(X rows) -> GEMM.  M = total rows (world * rows per rank).

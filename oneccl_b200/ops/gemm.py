@@ -17,14 +17,16 @@ import ctypes as C
 import torch
 
 from .. import _lib
+from ..torch_ops import native
 from .device_group import DeviceGroup, _stream_ptr
 
 EPILOGUE = {None: 0, "none": 0, "silu": 1}
+_KERNEL = {"1sm": 1, "2sm": 2}
 _err_words = {}
 
 
 def _err_buffer(device) -> torch.Tensor:
-    key = torch.device(device).index or 0
+    key = device.index or 0
     if key not in _err_words:
         _err_words[key] = torch.zeros(4, dtype=torch.int32, device=device)
     return _err_words[key]
@@ -38,24 +40,9 @@ def gemm_bf16(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None,
     host never learns it; the other rows of ``out`` stay as they are)."""
     assert a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and a.is_cuda and w.is_cuda
     assert a.dim() == 2 and w.dim() == 2 and a.shape[1] == w.shape[1]
-    a = a.contiguous()
-    w = w.contiguous()
-    M, K = a.shape
-    N = w.shape[0]
-    if out is None:
-        out = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
+    assert rows is None or (rows.dtype == torch.int32 and rows.is_cuda)
     err = _err_buffer(a.device)
-    lib = _lib.load()
-    if rows is not None:
-        assert rows.dtype == torch.int32 and rows.is_cuda
-        _lib.check(lib.cclx_gemm_bf16_rows(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, EPILOGUE[epilogue],
-                                           rows.data_ptr(), err.data_ptr(), _stream_ptr()))
-    elif kernel == "2sm":
-        _lib.check(lib.cclx_gemm_bf16_2sm(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, EPILOGUE[epilogue],
-                                          ctas // 2, err.data_ptr(), _stream_ptr()))
-    else:
-        _lib.check(lib.cclx_gemm_bf16(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, EPILOGUE[epilogue],
-                                      -(ctas + 1) if kernel == "1sm" else ctas, err.data_ptr(), _stream_ptr()))
+    out = native().gemm_bf16(a, w, out, EPILOGUE[epilogue], ctas, _KERNEL.get(kernel, 0), rows, err)
     if check:
         code = int(err[0].item())
         if code != 0:

@@ -27,4 +27,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("set_device", [](int dev) { set_device(dev); });
     bind_nn(m);
     bind_train(m);
+    bind_gemm(m);
 }

@@ -23,6 +23,12 @@ int cclx_layer_norm_bwd_blocks(size_t rows);
 int cclx_layer_norm_bwd_sums(const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
                              const void* dres, void* dx, void* dgamma, void* dbeta, void* dxsum, int add,
                              float* workspace, size_t rows, int D, void* stream);
+int cclx_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int ctas, void* err_words,
+                   void* stream);
+int cclx_gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int clusters,
+                       void* err_words, void* stream);
+int cclx_gemm_bf16_rows(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, const void* rows_dev,
+                        void* err_words, void* stream);
 int cclx_softmax_xent_mean(void* logits_bf16, const long long* targets, float* loss_rows, float* mean_loss, size_t rows,
                            int vocab, size_t ld, float grad_scale, int pad_cols, void* stream);
 }
@@ -70,5 +76,6 @@ inline Tensor empty_on(const Tensor& like, at::IntArrayRef sizes, at::ScalarType
 
 void bind_nn(pybind11::module_& m);
 void bind_train(pybind11::module_& m);
+void bind_gemm(pybind11::module_& m);
 
 } // namespace cclx_ops

@@ -67,3 +67,20 @@ def test_softmax_xent_row_lengths(rows, vocab, pad):
     torch.testing.assert_close(loss, loss_ref, rtol=1e-4, atol=1e-4)
     torch.testing.assert_close(got[:, :vocab].float(), want, rtol=1e-2, atol=1e-6)
     assert not pad or torch.count_nonzero(got[:, vocab:]) == 0
+
+
+@pytest.mark.parametrize("M", [1, 15, 16, 17, 32, 33, 64, 65, 128, 129, 257, 700])  # tile widths 16 ... 256, one or more tiles
+@pytest.mark.parametrize("N,K", [(8, 8), (128, 64), (136, 264), (1024, 512), (1000, 2056), (4096, 1024)])  # 1 to 8 parts of K
+@pytest.mark.parametrize("rows", [None, 0.4])
+def test_gemm_few_rows(M, N, K, rows):
+    from oneccl_b200.ops.gemm import gemm_bf16
+
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a, w = _bf16(g, M, K), _bf16(g, N, K, scale=0.1)
+    out = torch.full((M, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    n = M if rows is None else int(M * rows)
+    dev = None if rows is None else torch.tensor([n], dtype=torch.int32, device="cuda")
+    gemm_bf16(a, w, out=out, epilogue="silu", rows=dev, check=True)
+    ref = torch.nn.functional.silu(a[:n].float() @ w.float().t())
+    torch.testing.assert_close(out[:n].float(), ref, rtol=1e-2, atol=2e-3 * K ** 0.5)
+    assert bool((out[n:] == 7.0).all())
