@@ -77,23 +77,13 @@ class FlatAdamW:
         self.lr, self.betas, self.eps, self.weight_decay, self.max_norm = lr, betas, eps, weight_decay, max_norm
         self.step_count = 0
         self._norm = torch.zeros(1, dtype=torch.float32, device=model_flat.device)
+        self._counter = torch.zeros(1, dtype=torch.int32, device=model_flat.device)  # arrivals of the norm's blocks
         self._step_dev = torch.zeros(1, dtype=torch.int32, device=model_flat.device) if device_step else None
 
     def step(self, flat_grad: torch.Tensor, grad_scale: float = 1.0):
         self.step_count += 1
-        lib = _lib.load()
-        norm_ptr = 0
-        if self.max_norm > 0:
-            self._norm.zero_()
-            sq_norm(flat_grad, self._norm)
-            norm_ptr = self._norm.data_ptr()
-        _lib.check(lib.cclx_adamw_flat(
-            self.master.data_ptr(), flat_grad.data_ptr(), torch_to_ccl(flat_grad.dtype), self.m.data_ptr(),
-            self.v.data_ptr(), 0 if self.model_flat is None else self.model_flat.data_ptr(), self.master.numel(),
-            self.n_decay, self.lr, self.betas[0], self.betas[1], self.eps, self.weight_decay, self.step_count,
-            grad_scale, self.max_norm, norm_ptr, 0 if self._step_dev is None else self._step_dev.data_ptr(),
-            _stream_ptr()))
-        _bump(1 if self._step_dev is None else 2)
+        native().adamw_step(self.master, flat_grad, self.m, self.v, self.model_flat, self.n_decay, self.lr, *self.betas, self.eps,
+                            self.weight_decay, self.step_count, grad_scale, self.max_norm, self._norm, self._counter, self._step_dev)
         if self._fp32_model is not None:
             self._fp32_model.copy_(self.master)
 

@@ -29,6 +29,11 @@ int cclx_gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int 
                        void* err_words, void* stream);
 int cclx_gemm_bf16_rows(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, const void* rows_dev,
                         void* err_words, void* stream);
+int cclx_adamw_step(float* master, const void* grad, int grad_dt, float* m, float* v, void* model_bf16, size_t n,
+                    size_t n_decay, float lr, float beta1, float beta2, float eps, float weight_decay, int step,
+                    float grad_scale, float max_norm, float* sq_norm, float* scratch, unsigned* counter,
+                    int* step_dev, void* stream);
+size_t cclx_adamw_step_scratch(size_t n, int grad_dt);
 int cclx_softmax_xent_mean(void* logits_bf16, const long long* targets, float* loss_rows, float* mean_loss, size_t rows,
                            int vocab, size_t ld, float grad_scale, int pad_cols, void* stream);
 }

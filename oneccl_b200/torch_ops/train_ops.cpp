@@ -41,9 +41,27 @@ Tensor softmax_xent(const Tensor& logits, const Tensor& targets, int64_t vocab, 
     return SoftmaxXent::apply(logits, t, vocab, scale)[0];
 }
 
+// one step of the flat AdamW: clipping norm (max_norm > 0) and update
+void adamw_step(const Tensor& master, const Tensor& grad, const Tensor& m, const Tensor& v, const std::optional<Tensor>& model,
+                int64_t n_decay, double lr, double beta1, double beta2, double eps, double weight_decay, int64_t step,
+                double grad_scale, double max_norm, const Tensor& norm, const Tensor& counter, const std::optional<Tensor>& step_dev) {
+    const int dt = grad.scalar_type() == at::kBFloat16 ? 11 : grad.scalar_type() == at::kFloat ? 9 : -1;
+    void* st = stream_of(master);
+    const bool clip = max_norm > 0;
+    const Tensor scratch =
+        clip ? empty_on(master, { (int64_t)cclx_adamw_step_scratch(master.numel(), dt) }, at::kFloat) : Tensor();
+    check(cclx_adamw_step(master.data_ptr<float>(), grad.data_ptr(), dt, m.data_ptr<float>(), v.data_ptr<float>(),
+                          model ? model->data_ptr() : nullptr, master.numel(), n_decay, (float)lr, (float)beta1, (float)beta2,
+                          (float)eps, (float)weight_decay, (int)step, (float)grad_scale, (float)max_norm, norm.data_ptr<float>(),
+                          clip ? scratch.data_ptr<float>() : nullptr, reinterpret_cast<unsigned*>(counter.data_ptr<int>()),
+                          step_dev ? step_dev->data_ptr<int>() : nullptr, st));
+    launches += clip || step_dev ? 2 : 1;
+}
+
 } // namespace
 
 void bind_train(pybind11::module_& m) {
+    m.def("adamw_step", &adamw_step);
     m.def("softmax_xent", &softmax_xent);
 }
 

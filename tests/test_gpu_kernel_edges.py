@@ -84,3 +84,33 @@ def test_gemm_few_rows(M, N, K, rows):
     ref = torch.nn.functional.silu(a[:n].float() @ w.float().t())
     torch.testing.assert_close(out[:n].float(), ref, rtol=1e-2, atol=2e-3 * K ** 0.5)
     assert bool((out[n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 2049, 1_000_003])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("aligned", [True, False])
+@pytest.mark.parametrize("max_norm", [0.5, 0.0])
+def test_flat_adamw_sizes(n, dtype, aligned, max_norm):
+    """Whole packs, remainders and unaligned gradients; the decay boundary inside a pack; the step number on the device."""
+    from oneccl_b200.ops.train import FlatAdamW
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    model = _bf16(g, n)
+    opt = FlatAdamW(model, n // 2, lr=1e-2, weight_decay=0.1, max_norm=max_norm, device_step=True)
+    p, m, v = model.double(), torch.zeros(n, device="cuda").double(), torch.zeros(n, device="cuda").double()
+    wd = torch.where(torch.arange(n, device="cuda") < n // 2, 0.1, 0.0)
+    for t in (1, 2):
+        store = torch.randn(n + 1, generator=g, device="cuda").to(dtype)
+        grad = store[:n] if aligned else store[1:]
+        opt.step(grad, grad_scale=0.5)
+        gd = grad.double() * 0.5
+        norm = gd.norm()
+        if max_norm:
+            torch.testing.assert_close(opt.grad_norm()[0].double() * 0.5, norm, rtol=1e-5, atol=1e-6)
+            gd = gd * min(1.0, max_norm / (norm.item() + 1e-6))
+        m, v = 0.9 * m + 0.1 * gd, 0.95 * v + 0.05 * gd * gd
+        p = p - 1e-2 * (wd * p + (m / (1 - 0.9**t)) / ((v / (1 - 0.95**t)).sqrt() + 1e-8))
+    assert int(opt._step_dev) == 2
+    torch.testing.assert_close(opt.master.double(), p, rtol=1e-5, atol=1e-5)
+    torch.testing.assert_close(opt.v.double(), v, rtol=1e-5, atol=1e-9)
+    assert torch.equal(model, opt.master.to(torch.bfloat16))
