@@ -269,8 +269,7 @@ __global__ void __launch_bounds__(256, LN_BWD_BLOCKS)
             if (on && r0 + k < rows) {
                 const uint4 o = pack4x2(d);
                 dx[(r0 + k) * packs + c] = o;
-                if (COLSUM) {
-                    unpack4x2(o, d); // the sums are those of the bf16 values that dx holds
+                if (COLSUM) { // of the fp32 values, before dx rounds them
 #pragma unroll
                     for (int e = 0; e < 4; e++)
                         acc2[NS - 1][e] = add2(acc2[NS - 1][e], d[e]);
@@ -321,7 +320,7 @@ __global__ void __launch_bounds__(256, LN_BWD_BLOCKS)
 // add their share of the partial rows (8 loads in flight each), shared memory joins them.  grid = (cols / 32, outputs).
 struct partial_outs {
     __nv_bfloat16* out[3];
-    int add; // 1: add to what the outputs hold
+    int add; // bit i: add to what output i holds
 };
 
 __global__ void __launch_bounds__(256) partial_rows_sum_kernel(const float* __restrict__ partial, int n, int cols, partial_outs o) {
@@ -354,7 +353,7 @@ __global__ void __launch_bounds__(256) partial_rows_sum_kernel(const float* __re
         for (int g = 0; g < 8; g++)
             s += sh[g][lane];
         __nv_bfloat16* out = (which == 0 ? o.out[0] : which == 1 ? o.out[1] : o.out[2]) + c;
-        *out = __float2bfloat16_rn(o.add ? __bfloat162float(*out) + s : s);
+        *out = __float2bfloat16_rn(o.add >> which & 1 ? __bfloat162float(*out) + s : s);
     }
 }
 
@@ -362,98 +361,144 @@ __global__ void __launch_bounds__(256) partial_rows_sum_kernel(const float* __re
 
 namespace {
 
-// column sums of a [rows, N] bf16 matrix (bias gradient): partial[chunk][N], then a fixed-order sum by the last block.
-// One warp covers 256 columns (a 16-byte pack per lane); grid = (N / 256, chunks).
-__global__ void __launch_bounds__(256) colsum_kernel(const __nv_bfloat16* __restrict__ dy, size_t rows, int N,
-                                                     float* __restrict__ partial, unsigned* __restrict__ counters,
-                                                     __nv_bfloat16* __restrict__ out) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-    const int col = (blockIdx.x * 32 + lane) * 8;
-    float acc[8] = { 0, 0, 0, 0, 0, 0, 0, 0 };
-    if (col < N) {
-        const size_t per = (rows + gridDim.y - 1) / gridDim.y;
-        const size_t r0 = (size_t)blockIdx.y * per, r1 = min(rows, r0 + per);
-        size_t r = r0 + warp;
-        for (; r + 3 * wpb < r1; r += 4 * wpb) { // four rows in flight per lane
-            uint4 u[4];
+// ---- elementwise passes over [rows, 8 * packs] that also sum their result over the rows (bias gradients) -------------
+//
+// Bound by memory.  A thread owns one 16-byte pack of columns and takes the rows of its block four at a time; blocks
+// are short (rows_per_block) and many, in launch order, and leave one row of partial sums each, which
+// partial_rows_sum_kernel adds in a fixed order.  The sum costs no pass of its own: reading the result again for it
+// took 13 us per 8192 rows of 1024 to 4096 columns.
+template <class F>
+__global__ void __launch_bounds__(128) map_colsum_kernel(F f, size_t rows, int packs, int rows_per_block, float* __restrict__ partial) {
+    const int pack = blockIdx.x * 128 + threadIdx.x;
+    pdl_trigger();
+    if (pack >= packs)
+        return;
+    const size_t r0 = (size_t)blockIdx.y * rows_per_block, r1 = min(rows, r0 + rows_per_block);
+    f32x2 acc[4] = { 0, 0, 0, 0 };
+    for (size_t r = r0; r < r1; r += 4) {
+        typename F::input in[4];
 #pragma unroll
-            for (int k = 0; k < 4; k++)
-                u[k] = *reinterpret_cast<const uint4*>(dy + (r + (size_t)k * wpb) * N + col);
+        for (int k = 0; k < 4; k++)
+            if (r + k < r1)
+                in[k] = f.load(r + k, pack);
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&u[k]);
+        for (int k = 0; k < 4; k++)
+            if (r + k < r1) {
+                f32x2 v[4];
+                f.apply(in[k], v);
+                f.store(r + k, pack, pack4x2(v));
 #pragma unroll
-                for (int e = 0; e < 8; e++)
-                    acc[e] += __bfloat162float(h[e]);
+                for (int e = 0; e < 4; e++)
+                    acc[e] = add2(acc[e], v[e]);
             }
-        }
-        for (; r < r1; r += wpb) {
-            const uint4 u = *reinterpret_cast<const uint4*>(dy + r * N + col);
-            const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&u);
+    }
+    float s[8];
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+        unpair(acc[e], s[2 * e], s[2 * e + 1]);
+    float4* out = reinterpret_cast<float4*>(partial + ((size_t)blockIdx.y * packs + pack) * 8);
+    out[0] = make_float4(s[0], s[1], s[2], s[3]);
+    out[1] = make_float4(s[4], s[5], s[6], s[7]);
+}
+
+// Gaussian error linear unit, tanh form: x * s with s = 1 / (1 + exp(-2 u)), u = sqrt(2 / pi) (x + 0.044715 x^3), which
+// is 0.5 x (1 + tanh(u)).
+__device__ __forceinline__ float gelu_gate(float x) {
+    constexpr float C = -2.f * 0.7978845608028654f * 1.4426950408889634f; // -2 sqrt(2 / pi) log2(e)
+    float e;
+    const float t = C * x * fmaf(0.044715f * x, x, 1.f);
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t));
+    return __fdividef(1.f, 1.f + fminf(e, 1e37f)); // within __fdividef's range
+}
+__device__ __forceinline__ float gelu_slope(float x) {
+    const float s = gelu_gate(x), x2 = x * x;
+    return fmaf(x * s * (1.f - s), 1.5957691216057308f * fmaf(0.134145f, x2, 1.f), s); // 2 sqrt(2 / pi) (1 + 3 * 0.044715 x^2)
+}
+
+__global__ void __launch_bounds__(256) gelu_fwd_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, size_t packs) {
+    const size_t i0 = (size_t)blockIdx.x * 512 + threadIdx.x;
+    uint4 u[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+        if (i0 + k * 256 < packs)
+            u[k] = x[i0 + k * 256];
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+        if (i0 + k * 256 < packs) {
+            float v[8];
+            unpack8(u[k], v);
 #pragma unroll
             for (int e = 0; e < 8; e++)
-                acc[e] += __bfloat162float(h[e]);
+                v[e] *= gelu_gate(v[e]);
+            y[i0 + k * 256] = pack8(v);
         }
-    }
-    __shared__ float sh[8][256];
-    __shared__ int last;
-#pragma unroll
-    for (int e = 0; e < 8; e++)
-        sh[warp][lane * 8 + e] = acc[e];
-    __syncthreads();
-    const int c = blockIdx.x * 256 + threadIdx.x;
-    if (c < N) {
-        float s = 0.f;
-        for (int k = 0; k < wpb; k++)
-            s += sh[k][threadIdx.x];
-        partial[(size_t)blockIdx.y * N + c] = s;
-    }
-    // the block that finishes last for this column tile adds the chunks in index order (the result does
-    // not depend on which block that is) and re-arms the counter for the next call
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0)
-        last = atomicAdd(counters + blockIdx.x, 1u) == gridDim.y - 1 ? 1 : 0;
-    __syncthreads();
-    if (last) {
-        __threadfence();
-        if (c < N) {
-            float s = 0.f;
-            for (unsigned k = 0; k < gridDim.y; k++)
-                s += __ldcg(partial + (size_t)k * N + c);
-            out[c] = __float2bfloat16_rn(s);
-        }
-        if (threadIdx.x == 0)
-            counters[blockIdx.x] = 0;
-    }
 }
 
-// dst[b, s, h, :] = src[b, s, h, :] for head rows of `dh` elements (dh % 8 == 0) with arbitrary element
-// strides of the three outer dimensions on both sides: assembles a packed QKV gradient from the three
-// attention gradients without a concatenation pass per tensor.
-struct head_copy_args {
-    const __nv_bfloat16* src[3];
-    long long sb[3], ss[3], sh[3]; // source strides of (batch, sequence, head)
-    __nv_bfloat16* dst[3];
-    long long db, ds, dh_stride; // destination strides (the same for the three parts)
-    int B, S, H, dh;
+// the matrix as it is: column sums alone
+struct sum_map {
+    const uint4* src;
+    int packs;
+    struct input {
+        uint4 u;
+    };
+    __device__ __forceinline__ input load(size_t r, int p) const {
+        return { src[r * packs + p] };
+    }
+    __device__ __forceinline__ void apply(const input& in, f32x2 (&v)[4]) const {
+        unpack4x2(in.u, v);
+    }
+    __device__ __forceinline__ void store(size_t, int, const uint4&) const {}
 };
 
-__global__ void __launch_bounds__(256) head_copy_kernel(head_copy_args a) {
-    const int ppr = a.dh / 8; // packs per head row
-    const size_t total = (size_t)a.B * a.S * a.H * ppr;
-    const int part = blockIdx.y;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int p = (int)(i % ppr);
-        size_t t = i / ppr;
-        const int h = (int)(t % a.H);
-        t /= a.H;
-        const int s = (int)(t % a.S);
-        const int b = (int)(t / a.S);
-        const uint4 v = *reinterpret_cast<const uint4*>(a.src[part] + b * a.sb[part] + s * a.ss[part] + h * a.sh[part] + p * 8);
-        *reinterpret_cast<uint4*>(a.dst[part] + b * a.db + s * a.ds + h * a.dh_stride + p * 8) = v;
+struct gelu_bwd_map {
+    const uint4 *dy, *x;
+    uint4* dx;
+    int packs;
+    struct input {
+        uint4 dy, x;
+    };
+    __device__ __forceinline__ input load(size_t r, int p) const {
+        return { dy[r * packs + p], x[r * packs + p] };
     }
-}
+    __device__ __forceinline__ void apply(const input& in, f32x2 (&v)[4]) const {
+        float a[8];
+        f32x2 g[4];
+        unpack8(in.x, a);
+        unpack4x2(in.dy, g);
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            v[e] = mul2(g[e], pair(gelu_slope(a[2 * e]), gelu_slope(a[2 * e + 1])));
+    }
+    __device__ __forceinline__ void store(size_t r, int p, const uint4& u) const {
+        dx[r * packs + p] = u;
+    }
+};
+
+// row (b, s) of a packed QKV gradient [B, S, 3, H, dh] from three gradients with element strides of their own
+struct qkv_map {
+    const __nv_bfloat16* src[3];
+    long long sb[3], ss[3], sh[3]; // source strides of (batch, sequence, head)
+    uint4* dst;
+    int S, H, ppr; // ppr: packs per head row
+    struct input {
+        uint4 u;
+    };
+    __device__ __forceinline__ input load(size_t r, int p) const {
+        const int head = p / ppr, part = head / H, h = head - part * H;
+        const size_t b = r / S, s = r - b * S;
+        const __nv_bfloat16* q = part == 0 ? src[0] : part == 1 ? src[1] : src[2];
+        const long long o = part == 0 ? b * sb[0] + s * ss[0] + h * sh[0]
+                            : part == 1 ? b * sb[1] + s * ss[1] + h * sh[1]
+                                        : b * sb[2] + s * ss[2] + h * sh[2];
+        return { *reinterpret_cast<const uint4*>(q + o + (p - head * ppr) * 8) };
+    }
+    __device__ __forceinline__ void apply(const input& in, f32x2 (&v)[4]) const {
+        unpack4x2(in.u, v);
+    }
+    __device__ __forceinline__ void store(size_t r, int p, const uint4& u) const {
+        dst[r * (size_t)(3 * H * ppr) + p] = u;
+    }
+};
 
 int sm_count_now() {
     int dev = 0, sms = 148;
@@ -521,8 +566,8 @@ int launch_ln_bwd(const void* dy, const void* x, const void* w, const float* mea
 } // namespace
 
 // workspace: fp32 [cclx_layer_norm_bwd_blocks(rows) * (dxsum ? 3 : 2) * D].  dres may be null.  dxsum (optional): column
-// sums of dx, the bias gradient of the linear layer whose output the residual addition took.  `add`: the three column
-// results are added to what dgamma / dbeta / dxsum hold.
+// sums of dx, the bias gradient of the linear layer whose output the residual addition took.  `add`: bits 0 to 2
+// say which of dgamma, dbeta and dxsum are added to what the outputs hold.
 CCLX_API int cclx_layer_norm_bwd_sums(const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
                                       const void* dres, void* dx, void* dgamma, void* dbeta, void* dxsum, int add,
                                       float* workspace, size_t rows, int D, void* stream) {
@@ -553,48 +598,85 @@ CCLX_API int cclx_layer_norm_bwd(const void* dy, const void* x, const void* w, c
     return cclx_layer_norm_bwd_sums(dy, x, w, mean, rstd, dres, dx, dgamma, dbeta, nullptr, 0, workspace, rows, D, stream);
 }
 
-// workspace: fp32 [64 * N]; counters: (N + 255) / 256 zero-initialised words that the kernel leaves zero
-CCLX_API int cclx_colsum_bf16(const void* dy, size_t rows, int N, void* out, float* workspace, unsigned* counters,
-                              void* stream) {
+namespace {
+int map_rows_per_block(size_t rows, int packs) {
+    // about six blocks of 128 threads per SM, between 8 and 64 rows each: fewer rows would spend more on partial sums
+    const size_t cols = (packs + 127) / 128;
+    const size_t per = rows * cols / ((size_t)sm_count_now() * 6);
+    return (int)std::min<size_t>(64, std::max<size_t>(8, (per + 3) / 4 * 4));
+}
+
+template <class F>
+void launch_map_colsum(const F& f, size_t rows, int packs, void* colsum, int add, float* workspace, cudaStream_t st) {
+    const int rpb = map_rows_per_block(rows, packs);
+    const int n = (int)((rows + rpb - 1) / rpb);
+    map_colsum_kernel<F><<<dim3((packs + 127) / 128, n), 128, 0, st>>>(f, rows, packs, rpb, workspace);
+    CUDA_CHECK(cudaGetLastError());
+    partial_outs o{ { (__nv_bfloat16*)colsum, nullptr, nullptr }, add };
+    launch_dependent(partial_rows_sum_kernel, dim3((packs * 8 + 31) / 32, 1), dim3(256), 0, st, (const float*)workspace, n,
+                     packs * 8, o);
+}
+} // namespace
+
+// floats of workspace that the entry points below need for a result of [rows, N]
+CCLX_API size_t cclx_map_colsum_workspace(size_t rows, int N) {
+    const int rpb = map_rows_per_block(rows, N / 8);
+    return (rows + rpb - 1) / rpb * (size_t)N;
+}
+
+// column sums of a [rows, N] bf16 matrix, added to what `out` holds if `add`
+CCLX_API int cclx_colsum(const void* x, void* out, int add, float* workspace, size_t rows, int N, void* stream) {
     return cclx::capi::guard([&] {
         CCL_THROW_IF_NOT(N % 8 == 0, "column count must be a multiple of 8");
         if (rows == 0 || N == 0)
             return;
-        const int chunks = (int)std::min<size_t>(64, (rows + 31) / 32);
-        colsum_kernel<<<dim3((N + 255) / 256, chunks), 256, 0, (cudaStream_t)stream>>>(
-            (const __nv_bfloat16*)dy, rows, N, workspace, counters, (__nv_bfloat16*)out);
+        launch_map_colsum(sum_map{ (const uint4*)x, N / 8 }, rows, N / 8, out, add, workspace, (cudaStream_t)stream);
+    });
+}
+
+CCLX_API int cclx_gelu_fwd(const void* x, void* y, size_t n, void* stream) {
+    return cclx::capi::guard([&] {
+        CCL_THROW_IF_NOT(n % 8 == 0, "the fused GELU takes whole 16-byte packs");
+        if (n == 0)
+            return;
+        gelu_fwd_kernel<<<(unsigned)((n / 8 + 511) / 512), 256, 0, (cudaStream_t)stream>>>((const uint4*)x, (uint4*)y, n / 8);
         CUDA_CHECK(cudaGetLastError());
     });
 }
 
-// three [B, H, S, dh]-indexed sources with element strides (sb, ss, sh) each -> three destinations sharing one
-// set of strides; strides: 9 source values (b, s, h per part) then 3 destination values.
-CCLX_API int cclx_head_copy3(const void* const* src, void* const* dst, const long long* strides, int B, int S, int H, int dh,
-                             void* stream) {
+// dx = dy * gelu'(x) over [rows, N], and its column sums (added to what `colsum` holds if `add`)
+CCLX_API int cclx_gelu_bwd_colsum(const void* dy, const void* x, void* dx, void* colsum, int add, float* workspace, size_t rows,
+                                  int N, void* stream) {
+    return cclx::capi::guard([&] {
+        CCL_THROW_IF_NOT(N % 8 == 0, "the fused GELU takes whole 16-byte packs");
+        if (rows == 0)
+            return;
+        gelu_bwd_map f{ (const uint4*)dy, (const uint4*)x, (uint4*)dx, N / 8 };
+        launch_map_colsum(f, rows, N / 8, colsum, add, workspace, (cudaStream_t)stream);
+    });
+}
+
+// packed QKV gradient out [B, S, 3, H, dh] from three [B, H, S, dh]-indexed gradients with 9 element strides (b, s, h per
+// part), and its column sums
+CCLX_API int cclx_qkv_grad_colsum(const void* const* src, const long long* strides, void* out, void* colsum, int add,
+                                  float* workspace, int B, int S, int H, int dh, void* stream) {
     return cclx::capi::guard([&] {
         CCL_THROW_IF_NOT(dh % 8 == 0, "head size must be a multiple of 8");
-        head_copy_args a;
+        if (B == 0 || S == 0)
+            return;
+        qkv_map f;
         for (int p = 0; p < 3; p++) {
-            a.src[p] = (const __nv_bfloat16*)src[p];
-            a.dst[p] = (__nv_bfloat16*)dst[p];
-            a.sb[p] = strides[p * 3 + 0];
-            a.ss[p] = strides[p * 3 + 1];
-            a.sh[p] = strides[p * 3 + 2];
-            CCL_THROW_IF_NOT(((uintptr_t)src[p] & 15) == 0 && ((uintptr_t)dst[p] & 15) == 0 && a.sb[p] % 8 == 0 &&
-                                 a.ss[p] % 8 == 0 && a.sh[p] % 8 == 0,
-                             "head copy needs 16-byte aligned rows");
+            f.src[p] = (const __nv_bfloat16*)src[p];
+            f.sb[p] = strides[p * 3 + 0];
+            f.ss[p] = strides[p * 3 + 1];
+            f.sh[p] = strides[p * 3 + 2];
+            CCL_THROW_IF_NOT(((uintptr_t)src[p] & 15) == 0 && f.sb[p] % 8 == 0 && f.ss[p] % 8 == 0 && f.sh[p] % 8 == 0,
+                             "the QKV gradient needs 16-byte aligned rows");
         }
-        a.db = strides[9];
-        a.ds = strides[10];
-        a.dh_stride = strides[11];
-        CCL_THROW_IF_NOT(a.db % 8 == 0 && a.ds % 8 == 0 && a.dh_stride % 8 == 0, "head copy needs 16-byte aligned rows");
-        a.B = B;
-        a.S = S;
-        a.H = H;
-        a.dh = dh;
-        const size_t total = (size_t)B * S * H * (dh / 8);
-        const int blocks = (int)std::min<size_t>((total + 255) / 256, (size_t)sm_count_now() * 8);
-        head_copy_kernel<<<dim3(blocks, 3), 256, 0, (cudaStream_t)stream>>>(a);
-        CUDA_CHECK(cudaGetLastError());
+        f.dst = (uint4*)out;
+        f.S = S;
+        f.H = H;
+        f.ppr = dh / 8;
+        launch_map_colsum(f, (size_t)B * S, 3 * H * dh / 8, colsum, add, workspace, (cudaStream_t)stream);
     });
 }

@@ -63,20 +63,29 @@ class Block(nn.Module):
         x = x + self.fc2(F.gelu(self.fc(h), approximate="tanh"))
         return x
 
-    def forward_fused(self, x, delta):
+    def forward_fused(self, x, delta, delta_bias):
         """``x`` is the residual stream without the previous block's MLP output ``delta`` (None for
-        the first block): the addition happens inside the LayerNorm kernel.  Returns (x, delta)."""
+        the first block): the addition happens inside the LayerNorm kernel, whose backward also sums the
+        gradient of ``delta``'s bias.  Returns (x, delta, its bias)."""
         from ..ops import nn as K
 
         B, S, D = x.shape
-        h, x = K.add_layer_norm(x, delta, self.ln1.weight, self.ln1.bias, self.ln1.eps)
-        q, k, v = K.split_qkv(K.linear(h, self.qkv.weight, self.qkv.bias), self.n_head)
+        h, x = K.add_layer_norm(x, delta, self.ln1.weight, self.ln1.bias, self.ln1.eps, delta_bias)
+        qkv = K.linear(h, self.qkv.weight, self.qkv.bias, defer_bias=True)
+        q, k, v = K.split_qkv(qkv, self.n_head, self.qkv.bias)
         a = F.scaled_dot_product_attention(q, k, v, is_causal=True)
-        attn = K.linear(a.transpose(1, 2).reshape(B, S, D), self.proj.weight, self.proj.bias)
-        h, x = K.add_layer_norm(x, attn, self.ln2.weight, self.ln2.bias, self.ln2.eps)
-        delta = K.linear(F.gelu(K.linear(h, self.fc.weight, self.fc.bias), approximate="tanh"), self.fc2.weight,
-                         self.fc2.bias)
-        return x, delta
+        attn = K.linear(a.transpose(1, 2).reshape(B, S, D), self.proj.weight, self.proj.bias, defer_bias=True)
+        h, x = K.add_layer_norm(x, attn, self.ln2.weight, self.ln2.bias, self.ln2.eps, self.proj.bias)
+        u = K.linear(h, self.fc.weight, self.fc.bias, defer_bias=True)
+        delta = K.linear(K.gelu(u, self.fc.bias), self.fc2.weight, self.fc2.bias, defer_bias=True)
+        return x, delta, self.fc2.bias
+
+    def fused_ok(self, x) -> bool:
+        """Whether ``forward_fused`` takes activations like ``x``."""
+        from ..ops import nn as K
+
+        dh = x.shape[-1] // self.n_head
+        return K.fused_width(x, self.ln1) and dh % 8 == 0 and self.fc.weight.dtype == torch.bfloat16
 
 
 class GPT2(nn.Module):
@@ -103,16 +112,19 @@ class GPT2(nn.Module):
             nn.init.normal_(m.weight, mean=0.0, std=0.02)
 
     def hidden(self, idx):
-        B, S = idx.shape
-        pos = torch.arange(S, device=idx.device)
-        x = self.wte(idx) + self.wpe(pos)
-        if self.fused_ops and x.is_cuda and x.dtype == torch.bfloat16:
-            from ..ops import nn as K
+        from ..ops import nn as K
 
-            delta = None
+        B, S = idx.shape
+        on_gpu = self.fused_ops and self.wte.weight.is_cuda and self.wte.weight.dtype == torch.bfloat16
+        if on_gpu:
+            x = K.embed(idx, self.wte.weight, self.wpe.weight)
+        else:
+            x = self.wte(idx) + self.wpe(torch.arange(S, device=idx.device))
+        if on_gpu and self.blocks and self.blocks[0].fused_ok(x):
+            delta = delta_bias = None
             for b in self.blocks:
-                x, delta = b.forward_fused(x, delta)
-            h, _ = K.add_layer_norm(x, delta, self.ln_f.weight, self.ln_f.bias, self.ln_f.eps)
+                x, delta, delta_bias = b.forward_fused(x, delta, delta_bias)
+            h, _ = K.add_layer_norm(x, delta, self.ln_f.weight, self.ln_f.bias, self.ln_f.eps, delta_bias)
             return h
         for b in self.blocks:
             x = b(x)
@@ -120,7 +132,12 @@ class GPT2(nn.Module):
 
     def logits(self, idx):
         x = self.hidden(idx)
-        return F.linear(x.view(-1, x.shape[-1]), self.wte.weight)  # [B*S, vocab_padded]
+        x = x.view(-1, x.shape[-1])
+        if self.fused_ops and x.is_cuda:  # [B*S, vocab_padded]; the embedding adds its part of the gradient later
+            from ..ops import nn as K
+
+            return K.linear(x, self.wte.weight, None, last_use=False)
+        return F.linear(x, self.wte.weight)
 
     def forward(self, idx, targets=None, fused_loss: bool = True):
         lg = self.logits(idx)

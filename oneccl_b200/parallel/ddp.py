@@ -28,6 +28,7 @@ memory, which is what makes the replay valid.
 """
 from __future__ import annotations
 
+import weakref
 from typing import List, Optional
 
 import torch
@@ -35,6 +36,7 @@ import torch.nn as nn
 
 from ..ops.device_group import DeviceGroup
 from ..ops.train import FlatAdamW
+from ..torch_ops import native
 
 # Thread blocks of a bucket allreduce.  Measured with oneccl_b200.benchmarks.ddp_overlap_bench on B200s:
 # the in-switch (NVLS) reduction of a 25 MB bucket among 8 GPUs is as fast from 4 to 8 blocks of 1024 threads
@@ -44,6 +46,18 @@ from ..ops.train import FlatAdamW
 # runs, the full width for the last buckets of a step.
 NVLS_BLOCKS = 8
 PEER_OVERLAP_BLOCKS = 32
+
+
+def _bucket_callback(ddp, p):
+    """What a gradient sink calls when its parameter's gradient is complete.  Weak references: the parameter owns the sink."""
+    owner, param = weakref.ref(ddp), weakref.ref(p)
+
+    def done():
+        d, q = owner(), param()
+        if d is not None and q is not None:
+            d._on_grad(q)
+
+    return done
 
 
 class _Bucket:
@@ -104,13 +118,16 @@ class DataParallel:
         g = group.symm_empty((total,), dtype=dtype)
         self.flat_grad = g[0] if isinstance(g, list) else g
         self.flat_grad.zero_()
+        self._sinks = []
         for p, o in zip(order, offs):
             self.flat_param[o:o + p.numel()].copy_(p.data.reshape(-1))
             p.data = self.flat_param[o:o + p.numel()].view_as(p.data)
             p.grad = self.flat_grad[o:o + p.numel()].view_as(p.data)
-            # layers that can accumulate straight into the flat buffer (oneccl_b200.ops.nn.linear) use this
-            # instead of handing autograd a gradient to add; the callback does the bucket accounting
-            p._grad_sink = (p.grad, self._on_grad)
+            # operators that can write straight into the flat buffer (oneccl_b200.ops.nn) use this instead of
+            # handing autograd a gradient to add; the callback does the bucket accounting
+            sink = native().GradSink(p.grad, _bucket_callback(self, p))
+            p._grad_sink = sink
+            self._sinks.append((p, sink, sink.clear_before_accumulation(p)))
 
         # ---- buckets: ranges of the flat gradient, cut every `cap` elements inside the matrices and
         # inside the rest (a parameter may span several buckets; starts stay 16-byte aligned)
@@ -144,10 +161,23 @@ class DataParallel:
 
     # ---- per step -------------------------------------------------------------------
     def zero_grad(self):
+        self._arm()
+        self.flat_grad.zero_()
+        for _, sink, _ in self._sinks:
+            sink.fresh = False
+
+    def begin_step(self):
+        """``zero_grad`` for a step that ends with ``finish``: the buffer is not cleared, the first contribution to
+        every gradient overwrites it, and ``finish`` clears what received none.  Until then the buffer holds a
+        mixture of the last step's gradients and this one's."""
+        self._arm()
+        for _, sink, _ in self._sinks:
+            sink.fresh = True
+
+    def _arm(self):
         if self.record_timeline:
             self.t_step = torch.cuda.Event(enable_timing=True)
             self.t_step.record()
-        self.flat_grad.zero_()
         for b in self.buckets:
             b.pending = b.n_params
         self._unlaunched = len(self.buckets)
@@ -215,6 +245,10 @@ class DataParallel:
         if self.record_timeline:
             self.t_backward_end = torch.cuda.Event(enable_timing=True)
             self.t_backward_end.record()
+        for _, sink, _ in self._sinks:
+            if sink.fresh:
+                sink.grad.zero_()
+                sink.fresh = False
         late = [b for b in self.buckets if b.pending > 0]  # parameters that received no gradient this step
         for b in late:
             b.pending = 0
@@ -240,10 +274,11 @@ class DataParallel:
         for hk in self._hooks:
             hk.remove()
         self._hooks = []
-        for p in self.module.parameters():
-            if hasattr(p, "_grad_sink"):
-                del p._grad_sink
+        for p, sink, hook in self._sinks:
+            sink.remove_hook(p, hook)
+            del p._grad_sink
             p.grad = None
+        self._sinks = []
         if self.flat_grad is not None:
             torch.cuda.synchronize()
             self.group.symm_free(self.flat_grad)
@@ -263,7 +298,7 @@ class DataParallel:
 def train_step(ddp: DataParallel, opt: FlatAdamW, idx: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
     """One full data-parallel step: forward, backward with overlapped bucket
     allreduce, gradient clipping + AdamW.  Returns the (device) loss."""
-    ddp.zero_grad()
+    ddp.begin_step()
     loss = ddp(idx, targets)
     loss.backward()
     ddp.finish()

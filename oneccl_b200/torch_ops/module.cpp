@@ -2,6 +2,19 @@
 
 namespace cclx_ops {
 std::atomic<long long> launches{ 0 };
+std::atomic<int> GradSink::live{ 0 };
+
+SinkRef sink_of(const pybind11::object& param) {
+    if (GradSink::live.load(std::memory_order_relaxed) == 0 || param.is_none())
+        return nullptr;
+    static PyObject* name = PyUnicode_InternFromString("_grad_sink");
+    PyObject* s = PyObject_GetAttr(param.ptr(), name);
+    if (!s) {
+        PyErr_Clear();
+        return nullptr;
+    }
+    return pybind11::reinterpret_steal<pybind11::object>(s).cast<SinkRef>();
+}
 }
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -25,6 +38,22 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         return reinterpret_cast<uintptr_t>(s.stream());
     }, "handle of the current stream; the library's runtime follows its device");
     m.def("set_device", [](int dev) { set_device(dev); });
+    py::class_<GradSink, SinkRef>(m, "GradSink")
+        .def(py::init<Tensor, py::object>())
+        .def_readonly("grad", &GradSink::grad)
+        .def_readwrite("fresh", &GradSink::fresh)
+        // gradients that autograd accumulates itself are added in place: give them a clean buffer first
+        .def("clear_before_accumulation",
+             [](const SinkRef& s, const Tensor& param) {
+                 std::weak_ptr<GradSink> w = s;
+                 return param.register_hook([w](const Tensor& g) {
+                     if (const SinkRef s = w.lock(); s && s->fresh && g.defined()) {
+                         s->fresh = false;
+                         s->grad.zero_();
+                     }
+                 });
+             })
+        .def("remove_hook", [](const SinkRef&, const Tensor& param, unsigned h) { param.remove_hook(h); });
     bind_nn(m);
     bind_train(m);
     bind_gemm(m);

@@ -1,4 +1,9 @@
-// LayerNorm with the residual addition as an autograd function (kernels: csrc/gpu/nn_kernels.cu).
+// Layers of the decoder models as autograd functions (kernels: csrc/gpu/nn_kernels.cu, embedding_kernels.cu).
+//
+// Bias gradients are column sums of the gradient of a linear layer's output.  The kernel that produces that gradient sums
+// it on the way: LayerNorm's backward for the layer in front of a residual addition, GELU's for the first MLP layer, the
+// packing of the QKV gradient for the attention projection.  Such an operator takes the bias as an input whose value it
+// does not need and returns its gradient; `linear` is then called with defer_bias.
 #include "torch_ops.hpp"
 
 namespace cclx_ops {
@@ -10,16 +15,70 @@ using torch::autograd::variable_list;
 // [rows, D] form of a tensor whose last dimension is D
 Tensor rows_of(const Tensor& t, int64_t D) {
     Tensor r = t.dim() == 2 ? t : t.reshape({ -1, D });
-    return r.is_contiguous() ? r : r.contiguous();
+    r = r.is_contiguous() ? r : r.contiguous();
+    return aligned16(r) ? r : r.clone();
 }
 
 Tensor shaped(const Tensor& t, at::IntArrayRef shape) {
     return shape.size() == 2 ? t : t.view(shape);
 }
 
+// the sinks of an operator's parameters, kept with its autograd node
+struct Sinks : torch::CustomClassHolder {
+    std::vector<SinkRef> s;
+};
+
+void keep_sinks(AutogradContext* ctx, std::vector<SinkRef> s) {
+    for (const auto& x : s)
+        if (x) {
+            auto h = c10::make_intrusive<Sinks>();
+            h->s = std::move(s);
+            ctx->saved_data["sinks"] = c10::IValue::make_capsule(std::move(h));
+            return;
+        }
+}
+
+// Destination of a parameter's gradient: the sink's buffer, or a tensor to return to autograd.
+struct ParamGrad {
+    SinkRef sink;
+    Tensor out;
+    bool add = false;
+
+    ParamGrad(const SinkRef& s, const Tensor& like, at::IntArrayRef shape) : sink(s) {
+        if (s) {
+            out = s->grad;
+            add = s->add();
+        }
+        else
+            out = empty_on(like, shape, at::kBFloat16);
+    }
+    void* ptr() const {
+        return out.data_ptr();
+    }
+    void nothing() const { // no row contributes
+        if (!add)
+            out.zero_();
+    }
+    Tensor result() const {
+        return sink ? Tensor() : out;
+    }
+    void done() const {
+        if (sink)
+            sink->report();
+    }
+};
+
+std::vector<SinkRef> sinks_of(AutogradContext* ctx, size_t n) {
+    auto it = ctx->saved_data.find("sinks");
+    if (it == ctx->saved_data.end())
+        return std::vector<SinkRef>(n);
+    return c10::static_intrusive_pointer_cast<Sinks>(it->second.toCapsule())->s;
+}
+
 struct AddLayerNorm : torch::autograd::Function<AddLayerNorm> {
+    // res_bias: bias of the linear layer that produced `res`
     static variable_list forward(AutogradContext* ctx, const Tensor& x, const std::optional<Tensor>& res, const Tensor& weight,
-                                 const Tensor& bias, double eps) {
+                                 const Tensor& bias, double eps, const std::optional<Tensor>& res_bias, std::vector<SinkRef> sinks) {
         const int64_t D = x.size(-1);
         const Tensor x2 = rows_of(x, D);
         const int64_t rows = x2.size(0);
@@ -38,7 +97,8 @@ struct AddLayerNorm : torch::autograd::Function<AddLayerNorm> {
             check(cclx_layer_norm_fwd(x2.data_ptr(), nullptr, weight.data_ptr(), bias.data_ptr(), y.data_ptr(), nullptr,
                                       mean, mean + rows, rows, (int)D, (float)eps, st));
         launches += 1;
-        ctx->save_for_backward({ total, weight, stats });
+        ctx->save_for_backward({ total, weight, stats, res_bias ? *res_bias : Tensor() });
+        keep_sinks(ctx, std::move(sinks));
         ctx->set_materialize_grads(false); // an unused output costs no zero tensor
         if (res)
             return { shaped(y, x.sizes()), shaped(total, x.sizes()) };
@@ -52,26 +112,37 @@ struct AddLayerNorm : torch::autograd::Function<AddLayerNorm> {
         const bool has_res = grads.size() == 2; // as many as forward had outputs
         Tensor dsum = has_res ? grads[1] : Tensor();
         if (!grads[0].defined() && !dsum.defined())
-            return variable_list(5);
+            return variable_list(7);
         const Tensor dy = grads[0].defined() ? rows_of(grads[0], D) : at::zeros_like(total);
         if (dsum.defined())
             dsum = rows_of(dsum, D);
         void* st = stream_of(total);
         const Tensor dx = empty_on(total, total.sizes(), at::kBFloat16);
-        const Tensor dgamma = empty_on(total, weight.sizes(), at::kBFloat16), dbeta = empty_on(total, weight.sizes(), at::kBFloat16);
+        const auto sinks = sinks_of(ctx, 3);
+        const ParamGrad dg(sinks[0], total, weight.sizes()), db(sinks[1], total, weight.sizes());
+        std::optional<ParamGrad> dr;
+        if (saved[3].defined())
+            dr.emplace(sinks[2], total, weight.sizes());
         if (rows == 0) {
-            dgamma.zero_();
-            dbeta.zero_();
+            dg.nothing();
+            db.nothing();
+            if (dr)
+                dr->nothing();
         }
-        const Tensor ws = empty_on(total, { (int64_t)cclx_layer_norm_bwd_blocks(rows) * 2 * D }, at::kFloat);
+        const Tensor ws = empty_on(total, { (int64_t)cclx_layer_norm_bwd_blocks(rows) * (dr ? 3 : 2) * D }, at::kFloat);
         const float* mean = stats.data_ptr<float>();
         check(cclx_layer_norm_bwd_sums(dy.data_ptr(), total.data_ptr(), weight.data_ptr(), mean, mean + rows,
-                                       dsum.defined() ? dsum.data_ptr() : nullptr, dx.data_ptr(), dgamma.data_ptr(),
-                                       dbeta.data_ptr(), nullptr, 0, ws.data_ptr<float>(), rows, (int)D, st));
+                                       dsum.defined() ? dsum.data_ptr() : nullptr, dx.data_ptr(), dg.ptr(), db.ptr(),
+                                       dr ? dr->ptr() : nullptr, (dg.add ? 1 : 0) | (db.add ? 2 : 0) | (dr && dr->add ? 4 : 0),
+                                       ws.data_ptr<float>(), rows, (int)D, st));
         launches += 2;
+        dg.done();
+        db.done();
+        if (dr)
+            dr->done();
         const auto shape = grads[0].defined() ? grads[0].sizes() : grads[1].sizes();
         const Tensor d = shaped(dx, shape);
-        return { d, has_res ? d : Tensor(), dgamma, dbeta, Tensor() };
+        return { d, has_res ? d : Tensor(), dg.result(), db.result(), Tensor(), dr ? dr->result() : Tensor(), Tensor() };
     }
 };
 
@@ -89,24 +160,261 @@ bool layer_norm_ok(const Tensor& x, const std::optional<Tensor>& res, const Tens
            ln_param_ok(w, D) && ln_param_ok(b, D);
 }
 
+Tensor tensor_of(const pybind11::object& o) {
+    return o.cast<Tensor>();
+}
+std::optional<Tensor> maybe_tensor(const pybind11::object& o) {
+    return o.is_none() ? std::optional<Tensor>() : std::optional<Tensor>(o.cast<Tensor>());
+}
+
 // (LayerNorm(x + res), x + res), or None where the kernels do not take the call
-pybind11::object add_layer_norm(const Tensor& x, const std::optional<Tensor>& res, const Tensor& w, const Tensor& b, double eps) {
+pybind11::object add_layer_norm(const Tensor& x, const std::optional<Tensor>& res, const pybind11::object& w_,
+                                const pybind11::object& b_, double eps, const pybind11::object& res_bias_) {
+    const Tensor w = tensor_of(w_), b = tensor_of(b_);
     if (!layer_norm_ok(x, res, w, b))
         return pybind11::none();
+    const auto res_bias = maybe_tensor(res_bias_);
+    std::vector<SinkRef> sinks{ sink_of(w_), sink_of(b_), sink_of(res_bias_) };
     variable_list out;
     {
         pybind11::gil_scoped_release nogil;
-        out = AddLayerNorm::apply(x, res, w, b, eps);
+        out = AddLayerNorm::apply(x, res, w, b, eps, res_bias, std::move(sinks));
     }
     if (res)
         return pybind11::make_tuple(out[0], out[1]);
     return pybind11::cast(out[0]);
 }
 
+// bias gradient: column sums of a gradient of [rows, N]
+void column_sums(const Tensor& dy, const ParamGrad& out) {
+    const int64_t rows = dy.size(0), N = dy.size(1);
+    if (rows == 0)
+        return out.nothing();
+    const Tensor ws = empty_on(dy, { (int64_t)cclx_map_colsum_workspace(rows, (int)N) }, at::kFloat);
+    check(cclx_colsum(dy.data_ptr(), out.ptr(), out.add, ws.data_ptr<float>(), rows, (int)N, stream_of(dy)));
+    launches += 2;
+}
+
+// cuBLAS products with the weight gradient accumulated straight into its sink.
+struct Linear : torch::autograd::Function<Linear> {
+    // bias_grad: computed here (else another operator returns it); report: this is the weight's last contribution
+    static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const std::optional<Tensor>& bias,
+                                 bool bias_grad, bool report, std::vector<SinkRef> sinks) {
+        const Tensor x2 = x.dim() == 2 ? x : x.reshape({ -1, x.size(-1) });
+        ctx->save_for_backward({ x2, weight });
+        ctx->saved_data["flags"] = (int64_t)((bias && bias_grad ? 1 : 0) | (report ? 2 : 0));
+        ctx->saved_data["shape"] = x.sizes().vec();
+        keep_sinks(ctx, std::move(sinks));
+        const Tensor y = bias ? at::addmm(*bias, x2, weight.t()) : x2.mm(weight.t());
+        if (x.dim() == 2)
+            return { y };
+        auto shape = x.sizes().vec();
+        shape.back() = weight.size(0);
+        return { y.view(shape) };
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        const Tensor &x2 = saved[0], &weight = saved[1];
+        const auto sinks = sinks_of(ctx, 2);
+        const int64_t flags = ctx->saved_data["flags"].toInt();
+        const Tensor dy = rows_of(grads[0], grads[0].size(-1));
+        Tensor dx, dw, db;
+        if (ctx->needs_input_grad(0))
+            dx = dy.mm(weight).view(ctx->saved_data["shape"].toIntVector());
+        if (sinks[0]) {
+            if (sinks[0]->add())
+                sinks[0]->grad.addmm_(dy.t(), x2);
+            else
+                at::mm_out(sinks[0]->grad, dy.t(), x2);
+        }
+        else if (ctx->needs_input_grad(1))
+            dw = dy.t().mm(x2);
+        if (flags & 1) {
+            const ParamGrad g(sinks[1], dy, { dy.size(1) });
+            column_sums(dy, g);
+            db = g.result();
+            g.done();
+        }
+        if (sinks[0] && flags & 2)
+            sinks[0]->report();
+        return { dx, dw, db, Tensor(), Tensor(), Tensor() };
+    }
+};
+
+bool bf16_cuda(const Tensor& t) {
+    return t.is_cuda() && t.scalar_type() == at::kBFloat16;
+}
+
+// None where the operator does not take the call
+pybind11::object linear(const Tensor& x, const pybind11::object& w_, const pybind11::object& b_, bool bias_grad, bool report) {
+    const Tensor w = tensor_of(w_);
+    const auto b = maybe_tensor(b_);
+    if (!bf16_cuda(x) || !bf16_cuda(w) || w.dim() != 2 || w.size(0) % 8 != 0 || (b && !bf16_cuda(*b)))
+        return pybind11::none();
+    std::vector<SinkRef> sinks{ sink_of(w_), sink_of(b_) };
+    pybind11::gil_scoped_release nogil;
+    Tensor y = Linear::apply(x, w, b, bias_grad, report, std::move(sinks))[0];
+    pybind11::gil_scoped_acquire gil;
+    return pybind11::cast(y);
+}
+
+// tanh-form GELU of a linear layer's output u = ... + bias; backward also returns the bias gradient
+struct BiasGelu : torch::autograd::Function<BiasGelu> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& u, const Tensor& bias, std::vector<SinkRef> sinks) {
+        const Tensor u2 = rows_of(u, u.size(-1));
+        const Tensor y = empty_on(u2, u2.sizes(), at::kBFloat16);
+        check(cclx_gelu_fwd(u2.data_ptr(), y.data_ptr(), u2.numel(), stream_of(u2)));
+        launches += 1;
+        ctx->save_for_backward({ u2, bias });
+        keep_sinks(ctx, std::move(sinks));
+        return { shaped(y, u.sizes()) };
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        const Tensor& u = saved[0];
+        const int64_t rows = u.size(0), N = u.size(1);
+        const Tensor dy = rows_of(grads[0], N), du = empty_on(u, u.sizes(), at::kBFloat16);
+        const ParamGrad g(sinks_of(ctx, 1)[0], u, saved[1].sizes());
+        if (rows == 0)
+            g.nothing();
+        const Tensor ws = empty_on(u, { (int64_t)cclx_map_colsum_workspace(rows, (int)N) }, at::kFloat);
+        check(cclx_gelu_bwd_colsum(dy.data_ptr(), u.data_ptr(), du.data_ptr(), g.ptr(), g.add, ws.data_ptr<float>(), rows, (int)N,
+                                   stream_of(u)));
+        launches += 2;
+        g.done();
+        return { shaped(du, grads[0].sizes()), g.result(), Tensor() };
+    }
+};
+
+Tensor bias_gelu(const Tensor& u, const pybind11::object& b_) {
+    std::vector<SinkRef> sinks{ sink_of(b_) };
+    const Tensor b = tensor_of(b_);
+    pybind11::gil_scoped_release nogil;
+    return BiasGelu::apply(u, b, std::move(sinks))[0];
+}
+
+// views of a packed QKV projection for the attention call; backward assembles the packed gradient in one pass that also
+// sums the bias gradient
+struct SplitQKV : torch::autograd::Function<SplitQKV> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& qkv, const std::optional<Tensor>& bias, int64_t n_head,
+                                 std::vector<SinkRef> sinks) {
+        const int64_t B = qkv.size(0), S = qkv.size(1), D = qkv.size(2) / 3, dh = D / n_head;
+        const Tensor parts = qkv.view({ B, S, 3, n_head, dh }).permute({ 2, 0, 3, 1, 4 }); // [3, B, H, S, dh] views
+        ctx->saved_data["heads"] = n_head;
+        ctx->saved_data["bias"] = bias.has_value();
+        keep_sinks(ctx, std::move(sinks));
+        return { parts[0], parts[1], parts[2] };
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list g) {
+        const bool bias = ctx->saved_data["bias"].toBool();
+        const int64_t B = g[0].size(0), H = g[0].size(1), S = g[0].size(2), dh = g[0].size(3), N = 3 * H * dh;
+        const Tensor out = empty_on(g[0], { B, S, N }, at::kBFloat16);
+        const void* src[3];
+        long long strides[9];
+        for (int p = 0; p < 3; p++) { // gradients are indexed [B, H, S, dh]
+            if (g[p].scalar_type() != at::kBFloat16 || g[p].stride(3) != 1 || g[p].stride(0) % 8 || g[p].stride(1) % 8 ||
+                g[p].stride(2) % 8 || !aligned16(g[p]))
+                g[p] = g[p].to(at::kBFloat16).contiguous().clone();
+            src[p] = g[p].data_ptr();
+            strides[3 * p] = g[p].stride(0);
+            strides[3 * p + 1] = g[p].stride(2);
+            strides[3 * p + 2] = g[p].stride(1);
+        }
+        // without a bias the sums go nowhere
+        const ParamGrad db(sinks_of(ctx, 1)[0], out, { N });
+        if (B * S == 0)
+            db.nothing();
+        const Tensor ws = empty_on(out, { (int64_t)cclx_map_colsum_workspace(B * S, (int)N) }, at::kFloat);
+        check(cclx_qkv_grad_colsum(src, strides, out.data_ptr(), db.ptr(), db.add, ws.data_ptr<float>(), (int)B, (int)S, (int)H,
+                                   (int)dh, stream_of(out)));
+        launches += 2;
+        db.done();
+        return { out, bias ? db.result() : Tensor(), Tensor(), Tensor() };
+    }
+};
+
+pybind11::object split_qkv(const Tensor& qkv, int64_t n_head, const pybind11::object& b_) {
+    if (!bf16_cuda(qkv) || qkv.dim() != 3 || !qkv.is_contiguous() || qkv.size(2) / 3 / n_head % 8 != 0)
+        return pybind11::none();
+    std::vector<SinkRef> sinks{ sink_of(b_) };
+    const auto b = maybe_tensor(b_);
+    variable_list out;
+    {
+        pybind11::gil_scoped_release nogil;
+        out = SplitQKV::apply(qkv, b, n_head, std::move(sinks));
+    }
+    return pybind11::make_tuple(out[0], out[1], out[2]);
+}
+
+// token embedding + position embedding of [B, S] ids
+struct Embed : torch::autograd::Function<Embed> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& idx, const Tensor& tokens, const Tensor& positions,
+                                 std::vector<SinkRef> sinks) {
+        const int64_t B = idx.size(0), S = idx.size(1), D = tokens.size(1);
+        const Tensor out = empty_on(tokens, { B, S, D }, at::kBFloat16);
+        check(cclx_embed_fwd(reinterpret_cast<const long long*>(idx.data_ptr<int64_t>()), tokens.data_ptr(), positions.data_ptr(),
+                             out.data_ptr(), B * S, (int)S, (int)tokens.size(0), (int)D, stream_of(tokens)));
+        launches += 1;
+        ctx->save_for_backward({ idx, tokens, positions });
+        keep_sinks(ctx, std::move(sinks));
+        return { out };
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        const Tensor &idx = saved[0], &tokens = saved[1], &positions = saved[2];
+        const int64_t D = tokens.size(1);
+        const Tensor dx = rows_of(grads[0], D);
+        const auto sinks = sinks_of(ctx, 2);
+        const ParamGrad gt(sinks[0], tokens, tokens.sizes()), gp(sinks[1], positions, positions.sizes());
+        if (!gt.add) // only the rows of tokens that occur are touched
+            gt.out.zero_();
+        check(cclx_embed_bwd(reinterpret_cast<const long long*>(idx.data_ptr<int64_t>()), dx.data_ptr(), gt.ptr(), gp.ptr(), gp.add,
+                             (int)idx.size(0), (int)idx.size(1), (int)tokens.size(0), (int)positions.size(0), (int)D,
+                             stream_of(dx)));
+        launches += 2;
+        gp.done();
+        gt.done();
+        return { Tensor(), gt.result(), gp.result(), Tensor() };
+    }
+};
+
+// None where the operator does not take the call
+pybind11::object embed(const Tensor& idx_, const pybind11::object& tokens_, const pybind11::object& positions_) {
+    const Tensor tokens = tensor_of(tokens_), positions = tensor_of(positions_);
+    if (!bf16_cuda(tokens) || !bf16_cuda(positions) || !idx_.is_cuda() || idx_.scalar_type() != at::kLong || idx_.dim() != 2 ||
+        idx_.numel() > cclx_embed_bwd_max_ids() || tokens.size(1) % 8 != 0 || positions.size(1) != tokens.size(1) ||
+        idx_.size(1) > positions.size(0) || idx_.numel() == 0 || !tokens.is_contiguous() || !positions.is_contiguous() ||
+        !aligned16(tokens) || !aligned16(positions))
+        return pybind11::none();
+    const Tensor idx = idx_.contiguous();
+    std::vector<SinkRef> sinks{ sink_of(tokens_), sink_of(positions_) };
+    pybind11::gil_scoped_release nogil;
+    const Tensor y = Embed::apply(idx, tokens, positions, std::move(sinks))[0];
+    pybind11::gil_scoped_acquire gil;
+    return pybind11::cast(y);
+}
+
+Tensor colsum(const Tensor& dy) {
+    const ParamGrad g(nullptr, dy, { dy.size(1) });
+    column_sums(dy, g);
+    return g.out;
+}
+
 } // namespace
 
 void bind_nn(pybind11::module_& m) {
-    m.def("add_layer_norm", &add_layer_norm);
+    m.def("layer_norm_ok", &layer_norm_ok);
+    m.def("add_layer_norm", &add_layer_norm, pybind11::arg("x"), pybind11::arg("res"), pybind11::arg("weight"),
+          pybind11::arg("bias"), pybind11::arg("eps"), pybind11::arg("res_bias") = pybind11::none());
+    m.def("linear", &linear);
+    m.def("bias_gelu", &bias_gelu);
+    m.def("split_qkv", &split_qkv);
+    m.def("embed", &embed);
+    m.def("colsum", &colsum);
 }
 
 } // namespace cclx_ops

@@ -23,6 +23,18 @@ int cclx_layer_norm_bwd_blocks(size_t rows);
 int cclx_layer_norm_bwd_sums(const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
                              const void* dres, void* dx, void* dgamma, void* dbeta, void* dxsum, int add,
                              float* workspace, size_t rows, int D, void* stream);
+size_t cclx_map_colsum_workspace(size_t rows, int N);
+int cclx_colsum(const void* x, void* out, int add, float* workspace, size_t rows, int N, void* stream);
+int cclx_gelu_fwd(const void* x, void* y, size_t n, void* stream);
+int cclx_gelu_bwd_colsum(const void* dy, const void* x, void* dx, void* colsum, int add, float* workspace, size_t rows, int N,
+                         void* stream);
+int cclx_qkv_grad_colsum(const void* const* src, const long long* strides, void* out, void* colsum, int add, float* workspace,
+                         int B, int S, int H, int dh, void* stream);
+int cclx_embed_fwd(const long long* idx, const void* tokens, const void* positions, void* out, size_t n, int S, int table_rows,
+                   int D, void* stream);
+int cclx_embed_bwd_max_ids();
+int cclx_embed_bwd(const long long* idx, const void* dx, void* token_grad, void* pos_grad, int add_pos, int B, int S,
+                   int token_rows, int pos_rows, int D, void* stream);
 int cclx_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int ctas, void* err_words,
                    void* stream);
 int cclx_gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int clusters,
@@ -78,6 +90,40 @@ inline bool aligned16(const Tensor& t) {
 inline Tensor empty_on(const Tensor& like, at::IntArrayRef sizes, at::ScalarType dtype) {
     return at::detail::empty_cuda(sizes, dtype, like.device(), std::nullopt);
 }
+
+// Where a parameter's gradient goes when its layer accumulates it itself: a view of DataParallel's flat gradient.  `fresh`
+// says that the buffer still holds the last step's gradient, so that the first contribution overwrites it (a product with
+// beta = 0 instead of clearing the buffer and reading it back).  `callback` (no argument) does the bucket accounting;
+// it must not keep the parameter alive, which owns this object.
+struct GradSink {
+    Tensor grad;
+    PyObject* callback;
+    bool fresh = false;
+    static std::atomic<int> live;
+
+    GradSink(Tensor g, pybind11::object cb) : grad(std::move(g)), callback(cb.release().ptr()) {
+        live++;
+    }
+    ~GradSink() {
+        live--;
+        if (Py_IsInitialized()) {
+            pybind11::gil_scoped_acquire gil;
+            Py_XDECREF(callback);
+        }
+    }
+    // whether a contribution is added (or overwrites); from then on they are
+    bool add() {
+        const bool a = !fresh;
+        fresh = false;
+        return a;
+    }
+    void report() {
+        pybind11::gil_scoped_acquire gil;
+        pybind11::reinterpret_borrow<pybind11::object>(callback)();
+    }
+};
+typedef std::shared_ptr<GradSink> SinkRef;
+SinkRef sink_of(const pybind11::object& param); // null without one
 
 void bind_nn(pybind11::module_& m);
 void bind_train(pybind11::module_& m);

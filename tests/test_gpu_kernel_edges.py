@@ -114,3 +114,85 @@ def test_flat_adamw_sizes(n, dtype, aligned, max_norm):
     torch.testing.assert_close(opt.master.double(), p, rtol=1e-5, atol=1e-5)
     torch.testing.assert_close(opt.v.double(), v, rtol=1e-5, atol=1e-9)
     assert torch.equal(model, opt.master.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("rows,N", [(1, 8), (7, 1032), (33, 1024), (2051, 4096), (70, 136)])
+def test_gelu_and_bias_gradient(rows, N):
+    from oneccl_b200.ops.nn import gelu
+
+    g = torch.Generator(device="cuda").manual_seed(rows + N)
+    u, b = _bf16(g, rows, N, scale=3).requires_grad_(True), _bf16(g, N).requires_grad_(True)
+    with torch.no_grad():
+        u[0, :6] = torch.tensor([0.0, 40.0, -40.0, 6.0, -6.0, 1e-4])
+    dy = _bf16(g, rows, N)
+    y = gelu(u, b)
+    du, db = torch.autograd.grad(y, [u, b], dy)
+    r = u.detach().float().requires_grad_(True)
+    yr = torch.nn.functional.gelu(r, approximate="tanh")
+    (dr,) = torch.autograd.grad(yr, r, dy.float())
+    torch.testing.assert_close(y.float(), yr, rtol=8e-3, atol=1e-6)
+    torch.testing.assert_close(du.float(), dr, rtol=8e-3, atol=1e-4)
+    torch.testing.assert_close(db.float(), dr.sum(0), rtol=1e-2, atol=2e-3 * rows ** 0.5)
+
+
+@pytest.mark.parametrize("B,S,H,dh", [(1, 1, 1, 8), (2, 37, 3, 64), (3, 130, 12, 72)])
+def test_split_qkv_bias_gradient(B, S, H, dh):
+    from oneccl_b200.ops.nn import split_qkv
+
+    g = torch.Generator(device="cuda").manual_seed(B + S)
+    qkv, b = _bf16(g, B, S, 3 * H * dh).requires_grad_(True), _bf16(g, 3 * H * dh).requires_grad_(True)
+    outs = split_qkv(qkv, H, b)
+    grads = [_bf16(g, B, H, S, dh), _bf16(g, B, S, H, dh).transpose(1, 2), _bf16(g, H, B, S, dh).transpose(0, 1)]
+    d, db = torch.autograd.grad(outs, [qkv, b], grads)
+    want = torch.stack([x.transpose(1, 2) for x in grads], 2).reshape(B, S, -1)
+    assert torch.equal(d, want)
+    torch.testing.assert_close(db.float(), want.float().sum((0, 1)), rtol=1e-2, atol=2e-3 * (B * S) ** 0.5)
+
+
+@pytest.mark.parametrize("B,S,table,D", [(1, 1, 1, 8), (3, 50, 9, 264), (2, 1100, 3, 256), (4, 256, 50000, 1024), (2, 8192, 700, 64)])
+def test_embedding_gradients(B, S, table, D):
+    """Many and few repetitions of a token (more than one list of positions), tables longer than the batch's positions."""
+    from oneccl_b200.ops.nn import embed
+
+    g = torch.Generator(device="cuda").manual_seed(B + S)
+    tok, pos = _bf16(g, table, D).requires_grad_(True), _bf16(g, S + 3, D).requires_grad_(True)
+    idx = torch.randint(0, table, (B, S), generator=g, device="cuda")
+    x = embed(idx, tok, pos)
+    assert torch.equal(x, tok[idx] + pos[:S])
+    dx = _bf16(g, B, S, D)
+    dt, dp = torch.autograd.grad(x, [tok, pos], dx)
+    rt = torch.zeros(table, D, device="cuda").index_add_(0, idx.flatten(), dx.float().view(-1, D))
+    count = torch.bincount(idx.flatten(), minlength=table).max().item()
+    torch.testing.assert_close(dt.float(), rt, rtol=1e-2, atol=4e-3 * count ** 0.5)
+    torch.testing.assert_close(dp[:S].float(), dx.float().sum(0), rtol=1e-2, atol=1e-2)
+    assert torch.count_nonzero(dp[S:]) == 0
+
+
+def test_step_that_overwrites_gradients_matches_cleared_ones():
+    """``begin_step`` leaves the last step's gradients in the buffer: a parameter without a gradient must end up zero, one
+    that autograd accumulates itself must not keep them, and a tied weight adds both parts."""
+    from oneccl_b200.models.gpt2 import GPT2, GPT2Config
+    from oneccl_b200.ops.device_group import DeviceGroup
+    from oneccl_b200.parallel.ddp import DataParallel
+
+    cfg = GPT2Config(2, 4, 256, 64, 1000)
+    torch.manual_seed(0)
+    model = GPT2(cfg).cuda().to(torch.bfloat16)
+    model.extra = torch.nn.Parameter(torch.ones(8, device="cuda", dtype=torch.bfloat16))
+    model.scale = torch.nn.Parameter(torch.ones(8, device="cuda", dtype=torch.bfloat16))
+    group = DeviceGroup.emulated(1, heap_bytes=64 << 20, staging_bytes=1 << 20)
+    ddp = DataParallel(model, group, bucket_mb=0.5)
+    idx, tgt = (torch.randint(0, cfg.vocab, (4, 64), device="cuda") for _ in range(2))
+    got = []
+    for start in (ddp.zero_grad, ddp.begin_step):
+        ddp.flat_grad.fill_(3.0)
+        start()
+        (ddp(idx, tgt) + model.scale.float().sum() * 0.5).backward()
+        ddp.finish()
+        torch.cuda.synchronize()
+        got.append([p.grad.clone() for p in model.parameters()])
+    for (n, _), a, b in zip(model.named_parameters(), *got):
+        torch.testing.assert_close(a, b, rtol=1e-2, atol=1e-4, msg=n)
+    assert torch.count_nonzero(model.extra.grad) == 0 and bool((model.scale.grad == 0.5).all())
+    ddp.close()
+    group.close()
