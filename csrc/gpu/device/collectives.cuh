@@ -25,6 +25,11 @@
 namespace cclx {
 namespace dev {
 
+template <int V>
+struct int_const {
+    static constexpr int value = V;
+};
+
 __device__ __forceinline__ size_t round_up16(size_t b) {
     return (b + 15) & ~(size_t)15;
 }
@@ -137,15 +142,40 @@ __global__ void __launch_bounds__(1024) allreduce_oneshot_kernel(const comm_dev*
     }
     if (peer_barrier(c, s, sig)) {
         const char* mine = c.staging[c.rank] + (size_t)s.gen * c.staging_bytes;
-        for (size_t i = lo + tid; i < hi; i += nt) {
-            A acc[N];
-            unpack16<T, A>(ld_cv16(mine + (i << 4)), acc);
-            for (int p = 1; p < c.world; p++)
-                accum16<T, A, Op>(ld_cv16(mine + (size_t)p * slot + (i << 4)), acc);
-            store_pack<Tout, A, N>(recv, i, count, vout, acc, a.scale, a.do_scale != 0);
-        }
+        // For 2, 4 and 8 ranks all slots of a pack are loaded before the first is added: a loop over a run-time number
+        // of ranks waits for one load at a time, eight round trips to the L2 in a kernel that has little else to do.
+        auto reduce = [&](auto wt) {
+            constexpr int WT = decltype(wt)::value;
+            for (size_t i = lo + tid; i < hi; i += nt) {
+                A acc[N];
+                if constexpr (WT > 0) {
+                    uint4 v[WT];
+#pragma unroll
+                    for (int p = 0; p < WT; p++)
+                        v[p] = ld_cv16(mine + (size_t)p * slot + (i << 4));
+                    unpack16<T, A>(v[0], acc);
+#pragma unroll
+                    for (int p = 1; p < WT; p++)
+                        accum16<T, A, Op>(v[p], acc);
+                }
+                else {
+                    unpack16<T, A>(ld_cv16(mine + (i << 4)), acc);
+                    for (int p = 1; p < c.world; p++)
+                        accum16<T, A, Op>(ld_cv16(mine + (size_t)p * slot + (i << 4)), acc);
+                }
+                store_pack<Tout, A, N>(recv, i, count, vout, acc, a.scale, a.do_scale != 0);
+            }
+        };
+        if (c.world == 8)
+            reduce(int_const<8>());
+        else if (c.world == 4)
+            reduce(int_const<4>());
+        else if (c.world == 2)
+            reduce(int_const<2>());
+        else
+            reduce(int_const<0>());
     }
-    sync_end(c, gridDim.x, 1, true);
+    sync_end(c, s, gridDim.x, 1, true);
 }
 
 // ---------------------------------------------------------------------------
@@ -255,7 +285,7 @@ __global__ void __launch_bounds__(1024) allreduce_twoshot_kernel(const comm_dev*
             }
         }
     }
-    sync_end(c, gridDim.x, 2, true);
+    sync_end(c, s, gridDim.x, 2, true);
 }
 
 // ---------------------------------------------------------------------------
@@ -436,7 +466,7 @@ __global__ void __launch_bounds__(1024) allreduce_pipelined_kernel(const comm_de
         if (j <= nchunks)
             ok = peer_barrier(c, s, sig);
     }
-    sync_end(c, gridDim.x, (uint32_t)(nchunks + 1), true);
+    sync_end(c, s, gridDim.x, (uint32_t)(nchunks + 1), true);
 }
 
 // ---------------------------------------------------------------------------
@@ -617,15 +647,17 @@ __global__ void __launch_bounds__(1024) allreduce_symm_kernel(const comm_dev* ta
                     st16(peer_out(c, a, p) + (i << 4), o);
                 }
             };
-            size_t i = mlo + lo + tid;
-            const size_t end = mlo + hi;
+            // the blocks of a rank walk its slice side by side, so that all of them work on the same DRAM pages
+            size_t i = mlo + (size_t)blockIdx.x * nt + tid;
+            const size_t end = mhi, step = (size_t)gridDim.x * nt;
             if (W == 8)
-                ar_p2p_loop<T, A, Op, N, 8>(c, a, i, end, nt, scale);
+                ar_p2p_loop<T, A, Op, N, 8>(c, a, i, end, step, scale);
             else if (W == 4)
-                ar_p2p_loop<T, A, Op, N, 4>(c, a, i, end, nt, scale);
+                ar_p2p_loop<T, A, Op, N, 4>(c, a, i, end, step, scale);
             else if (W == 2)
-                ar_p2p_loop<T, A, Op, N, 2>(c, a, i, end, nt, scale);
+                ar_p2p_loop<T, A, Op, N, 2>(c, a, i, end, step, scale);
             else {
+                const size_t nt = step;
                 for (; i + nt < end; i += 2 * nt) {
                     uint4 v0[MAX_RANKS], v1[MAX_RANKS];
                     for (int p = 0; p < W; p++) {
@@ -659,7 +691,7 @@ __global__ void __launch_bounds__(1024) allreduce_symm_kernel(const comm_dev* ta
     }
     // nobody reads a peer's input after the second barrier, so the next
     // operation on the stream may overwrite it
-    sync_end(c, gridDim.x, 2, false);
+    sync_end(c, s, gridDim.x, 2, false);
 }
 
 // ---------------------------------------------------------------------------
@@ -713,7 +745,7 @@ __global__ void __launch_bounds__(1024) reduce_scatter_kernel(const comm_dev* ta
             store_pack<Tout, A, N>(recv, i, rc, vout, acc, a.scale, a.do_scale != 0);
         }
     }
-    sync_end(c, gridDim.x, 1, true);
+    sync_end(c, s, gridDim.x, 1, true);
 }
 
 // ---------------------------------------------------------------------------
@@ -814,7 +846,7 @@ __global__ void __launch_bounds__(1024) reduce_scatter_pipelined_kernel(const co
         if (j < nchunks)
             ok = peer_barrier(c, s, sig);
     }
-    sync_end(c, gridDim.x, (uint32_t)nchunks, true);
+    sync_end(c, s, gridDim.x, (uint32_t)nchunks, true);
 }
 
 // reduce_scatter on symmetric send buffers: pull my block from every peer
@@ -900,7 +932,7 @@ __global__ void __launch_bounds__(1024) reduce_scatter_symm_kernel(const comm_de
         }
     }
     peer_barrier(c, s, sig); // peers may still read my send buffer until here
-    sync_end(c, gridDim.x, 2, false);
+    sync_end(c, s, gridDim.x, 2, false);
 }
 
 // ---------------------------------------------------------------------------
@@ -971,7 +1003,7 @@ __global__ void __launch_bounds__(1024) allgatherv_kernel(const comm_dev* tab, c
                 }
             }
         }
-        sync_end(c, gridDim.x, 1, true);
+        sync_end(c, s, gridDim.x, 1, true);
     }
     else {
         split_range((mybytes + 15) >> 4, gridDim.x, blockIdx.x, lo, hi);
@@ -991,7 +1023,7 @@ __global__ void __launch_bounds__(1024) allgatherv_kernel(const comm_dev* tab, c
                     block_copy<true>(recv + ra.sdispl[p] + l, c.staging[p] + gbase + l, h - l);
             }
         }
-        sync_end(c, gridDim.x, 1, true);
+        sync_end(c, s, gridDim.x, 1, true);
     }
 }
 
@@ -1047,7 +1079,7 @@ __global__ void __launch_bounds__(1024) allgather_symm_kernel(const comm_dev* ta
         }
     }
     peer_barrier(c, s, sig);
-    sync_end(c, gridDim.x, 2, false);
+    sync_end(c, s, gridDim.x, 2, false);
 }
 
 // ---------------------------------------------------------------------------
@@ -1159,7 +1191,7 @@ static __global__ void __launch_bounds__(1024) alltoallv_kernel(const comm_dev* 
         if (!again)
             break;
     }
-    sync_end(c, gridDim.x, rounds, rounds);
+    sync_end(c, s, gridDim.x, rounds, rounds);
 }
 
 // alltoall with equal blocks into a symmetric recv buffer: every rank stores block q of its send
@@ -1193,7 +1225,7 @@ static __global__ void __launch_bounds__(1024) alltoall_symm_kernel(const comm_d
         }
     }
     peer_barrier(c, s, sig);
-    sync_end(c, gridDim.x, 2, false);
+    sync_end(c, s, gridDim.x, 2, false);
 }
 
 // ---------------------------------------------------------------------------
@@ -1230,7 +1262,7 @@ static __global__ void __launch_bounds__(1024) broadcast_kernel(const comm_dev* 
         if (c.rank != a.root && h > l)
             block_copy<true>(recv + l, c.staging[c.rank] + gbase + l, h - l);
     }
-    sync_end(c, gridDim.x, 1, true);
+    sync_end(c, s, gridDim.x, 1, true);
 }
 
 // ---------------------------------------------------------------------------
@@ -1277,7 +1309,7 @@ __global__ void __launch_bounds__(1024) reduce_kernel(const comm_dev* tab, coll_
             store_pack<Tout, A, N>(recv, i, count, vout, acc, a.scale, a.do_scale != 0);
         }
     }
-    sync_end(c, gridDim.x, 1, true);
+    sync_end(c, s, gridDim.x, 1, true);
 }
 
 // barrier only
@@ -1285,7 +1317,7 @@ static __global__ void __launch_bounds__(64) barrier_kernel(const comm_dev* tab,
     CCLX_KERNEL_PROLOGUE();
     const uint32_t sig = kernel_signature(14, a, c);
     peer_barrier(c, s, sig);
-    sync_end(c, gridDim.x, 1, false);
+    sync_end(c, s, gridDim.x, 1, false);
 }
 
 // ---------------------------------------------------------------------------

@@ -118,17 +118,16 @@ __device__ __forceinline__ void sync_begin(const comm_dev& c, block_sync& s) {
 // Called by every block exactly once at the end of a kernel.  The last block of
 // this rank to finish publishes the new epoch / generation for the next kernel.
 // `nblocks` is the number of blocks of this rank (gridDim.x), `nbarriers` the
-// number of peer_barrier calls every block of this kernel makes.
-__device__ __forceinline__ void sync_end(const comm_dev& c, uint32_t nblocks, uint32_t nbarriers,
+// number of peer_barrier calls every block of this kernel makes.  The new values follow from what
+// the block read at its start, and only the next kernel on the stream reads them: no fence and no
+// further load stands between the last data and the end of the kernel (2.5 us of a 12 us small allreduce).
+__device__ __forceinline__ void sync_end(const comm_dev& c, const block_sync& s, uint32_t nblocks, uint32_t nbarriers,
                                          uint32_t advance_gen) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence();
-        uint32_t done = atomicAdd(c.state + STATE_DONE, 1u);
-        if (done == nblocks - 1) {
-            c.state[STATE_EPOCH] += nbarriers;
-            c.state[STATE_GEN] += advance_gen;
-            __threadfence();
+        if (nblocks == 1 || atomicAdd(c.state + STATE_DONE, 1u) == nblocks - 1) {
+            c.state[STATE_EPOCH] = s.epoch + nbarriers;
+            c.state[STATE_GEN] = s.gen + advance_gen;
             c.state[STATE_DONE] = 0;
         }
     }
@@ -181,9 +180,7 @@ __device__ __forceinline__ bool wait_flag_sys(const comm_dev& c, const uint32_t*
 // with ST_ARG_MISMATCH before any data is touched.  The slot is chosen by the barrier's epoch, so a
 // peer that is already in its next kernel writes another slot.
 __device__ __forceinline__ bool peer_barrier(const comm_dev& c, block_sync& s, uint32_t sig = 0) {
-    __shared__ int bar_fail;
-    if (threadIdx.x == 0)
-        bar_fail = 0;
+    int fail = 0;
     __syncthreads();
     s.used++;
     const uint32_t target = s.epoch + s.used;
@@ -197,17 +194,16 @@ __device__ __forceinline__ bool peer_barrier(const comm_dev& c, block_sync& s, u
         // block's earlier writes (made visible to this thread by bar.sync) before the flag
         st_release_sys(c.flags[p] + blockIdx.x * MAX_RANKS + c.rank, target);
         if (!wait_flag_sys(c, c.flags[c.rank] + blockIdx.x * MAX_RANKS + p, target, p, ST_BARRIER_TIMEOUT))
-            bar_fail = 1;
+            fail = 1;
         else if (check) {
             const uint32_t theirs = ld_volatile_u32(c.p2p_flags[c.rank] + slot + p);
             if (theirs != sig) {
                 report(c, ST_ARG_MISMATCH, p, theirs);
-                bar_fail = 1;
+                fail = 1;
             }
         }
     }
-    __syncthreads();
-    if (bar_fail)
+    if (__syncthreads_or(fail))
         s.ok = false;
     return s.ok;
 }

@@ -65,16 +65,19 @@ void device_comm::build_tables() {
     const int entries = emulated_ ? world_ : 1;
     const heap_regions& R = heap_.regions();
 
-    CUDA_CHECK(cudaMalloc((void**)&state_dev_, entries * dev::STATE_WORDS * sizeof(uint32_t)));
-    CUDA_CHECK(cudaMemset(state_dev_, 0, entries * dev::STATE_WORDS * sizeof(uint32_t)));
-    CUDA_CHECK(cudaMalloc((void**)&p2p_seq_dev_, entries * dev::P2P_SEQ_WORDS * sizeof(uint32_t)));
-    CUDA_CHECK(cudaMemset(p2p_seq_dev_, 0, entries * dev::P2P_SEQ_WORDS * sizeof(uint32_t)));
-    const size_t status_words = (size_t)entries * 8 + 8;
-    CUDA_CHECK(cudaHostAlloc((void**)&status_host_, status_words * sizeof(uint32_t), cudaHostAllocMapped));
+    // one device and one pinned allocation: state words, point-to-point counters and (emulation) argument tables;
+    // status words and the tables' host side
+    const size_t words = (size_t)entries * (dev::STATE_WORDS + dev::P2P_SEQ_WORDS);
+    const size_t emu_bytes = emulated_ ? EMU_SLOTS * EMU_SLOT_BYTES : 0, words_bytes = (words * sizeof(uint32_t) + 255) / 256 * 256;
+    CUDA_CHECK(cudaMalloc((void**)&state_dev_, words_bytes + emu_bytes));
+    CUDA_CHECK(cudaMemset(state_dev_, 0, words_bytes));
+    p2p_seq_dev_ = state_dev_ + entries * dev::STATE_WORDS;
+    emu_dev_ = (char*)state_dev_ + words_bytes;
+    const size_t status_words = (size_t)entries * 8 + 8, status_bytes = (status_words * sizeof(uint32_t) + 255) / 256 * 256;
+    CUDA_CHECK(cudaHostAlloc((void**)&status_host_, status_bytes + emu_bytes, cudaHostAllocMapped));
     std::memset(status_host_, 0, status_words * sizeof(uint32_t));
+    emu_host_ = (char*)status_host_ + status_bytes;
     CUDA_CHECK(cudaHostGetDevicePointer((void**)&status_devptr_, status_host_, 0));
-    CUDA_CHECK(cudaMalloc((void**)&emu_args_dev_, dev::MAX_RANKS * sizeof(dev::rank_args)));
-    CUDA_CHECK(cudaMalloc((void**)&emu_ops_dev_, dev::MAX_RANKS * sizeof(dev::p2p_ops)));
     device_id_ = devid;
 
     table_host_.assign(entries, dev::comm_dev{});
@@ -138,14 +141,34 @@ void device_comm::destroy() {
     cudaFree(table_dev_);
     table_dev_ = nullptr;
     cudaFree(state_dev_);
-    cudaFree(p2p_seq_dev_);
-    cudaFree(emu_args_dev_);
-    cudaFree(emu_ops_dev_);
+    emu_dev_ = emu_host_ = nullptr;
     cudaFreeHost(status_host_);
     state_dev_ = p2p_seq_dev_ = nullptr;
     status_host_ = nullptr;
-    emu_args_dev_ = nullptr;
     heap_.destroy();
+}
+
+const void* device_comm::emu_table(int kind, const void* data, size_t bytes, cudaStream_t st) {
+    CCL_THROW_IF_NOT(emulated_ && bytes <= EMU_SLOT_BYTES, "argument table of ", bytes, " bytes");
+    cudaStreamCaptureStatus capturing;
+    CUDA_CHECK(cudaStreamIsCapturing(st, &capturing));
+    CCL_THROW_IF_NOT(capturing == cudaStreamCaptureStatusNone, "launches of several emulated ranks cannot be captured");
+    std::lock_guard<std::mutex> g(emu_mu_);
+    emu_last& l = emu_last_[kind];
+    if (l.slot >= 0 && l.bytes == bytes && l.stream == st && std::memcmp(emu_host_ + l.slot * EMU_SLOT_BYTES, data, bytes) == 0)
+        return emu_dev_ + l.slot * EMU_SLOT_BYTES;
+    const int slot = emu_next_++ % EMU_SLOTS;
+    if (slot == 0 && emu_next_ > 1) { // earlier launches may still read their tables
+        CUDA_CHECK(cudaDeviceSynchronize());
+        for (auto& x : emu_last_)
+            x = emu_last();
+    }
+    std::memcpy(emu_host_ + slot * EMU_SLOT_BYTES, data, bytes);
+    CUDA_CHECK(cudaMemcpyAsync(emu_dev_ + slot * EMU_SLOT_BYTES, emu_host_ + slot * EMU_SLOT_BYTES, bytes, cudaMemcpyHostToDevice, st));
+    l.slot = slot;
+    l.bytes = bytes;
+    l.stream = st;
+    return emu_dev_ + slot * EMU_SLOT_BYTES;
 }
 
 int device_comm::max_blocks() const {

@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -64,8 +65,11 @@ public:
     int sm_count() const { return sm_count_; }
     int max_blocks() const; // per rank, keeps every block co-resident
     int threads() const { return threads_; }
-    dev::rank_args* emu_args_dev() const { return emu_args_dev_; }
-    dev::p2p_ops* emu_ops_dev() const { return emu_ops_dev_; }
+    // Emulation: the per-rank argument table of a launch in device memory.  `kind` names the table's layout.  A table equal
+    // to the last one of its kind on this stream is still there; another is copied from a pinned ring, in stream order.
+    // The host waits only when the ring comes round.
+    enum { EMU_COLL = 0, EMU_P2P = 1, EMU_MOE = 2, EMU_KINDS = 3 };
+    const void* emu_table(int kind, const void* data, size_t bytes, cudaStream_t st);
     int device_id() const { return device_id_; }
     size_t staging_bytes() const { return heap_.regions().staging_bytes; }
 
@@ -141,8 +145,18 @@ private:
     uint32_t* p2p_seq_dev_ = nullptr;
     uint32_t* status_host_ = nullptr; // pinned + mapped: per rank 8 words, then abort word
     uint32_t* status_devptr_ = nullptr;
-    dev::rank_args* emu_args_dev_ = nullptr;
-    dev::p2p_ops* emu_ops_dev_ = nullptr;
+    static constexpr int EMU_SLOTS = 32;
+    static constexpr size_t EMU_SLOT_BYTES = dev::MAX_RANKS * (sizeof(dev::rank_args) > sizeof(dev::p2p_ops) ? sizeof(dev::rank_args)
+                                                                                                             : sizeof(dev::p2p_ops));
+    char* emu_dev_ = nullptr; // EMU_SLOTS tables, part of the allocation at state_dev_
+    char* emu_host_ = nullptr; // pinned, the same layout, part of the allocation at status_host_
+    int emu_next_ = 0;
+    struct emu_last {
+        int slot = -1;
+        size_t bytes = 0;
+        cudaStream_t stream = nullptr;
+    } emu_last_[EMU_KINDS];
+    std::mutex emu_mu_;
     int device_id_ = 0;
     int sm_count_ = 0;
     int threads_ = 512;

@@ -179,16 +179,12 @@ inline void fill_registered(const device_comm& dc, dev::coll_args& a, const zc_v
     a.flags |= recv_side ? dev::CF_REG_OUT : dev::CF_REG_IN;
 }
 
-// Fill the mode-dependent part of coll_args.  In emulation mode the per-rank
-// table is uploaded to the device (the stream is drained first because an
-// earlier launch may still read the previous table).
+// Fill the mode-dependent part of coll_args.  In emulation mode the per-rank table goes to the device.
 inline void prepare_args(device_comm& dc, dev::coll_args& a, const dev::rank_args* ra, cudaStream_t st) {
     a.sig_skew = dc.test_sig_skew;
     if (dc.emulated()) {
-        CUDA_CHECK(cudaStreamSynchronize(st));
-        CUDA_CHECK(cudaMemcpy(dc.emu_args_dev(), ra, dc.world() * sizeof(dev::rank_args), cudaMemcpyHostToDevice));
         a.emu = 1;
-        a.emu_tab = dc.emu_args_dev();
+        a.emu_tab = (const dev::rank_args*)dc.emu_table(device_comm::EMU_COLL, ra, dc.world() * sizeof(dev::rank_args), st);
         a.r0 = ra[0];
     }
     else {

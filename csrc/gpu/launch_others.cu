@@ -446,9 +446,7 @@ void launch_sendrecv(device_comm& dc, const dev::p2p_ops* ops, cudaStream_t st) 
     dc.check_status();
     const dev::p2p_ops* tab = nullptr;
     if (dc.emulated()) {
-        CUDA_CHECK(cudaStreamSynchronize(st));
-        CUDA_CHECK(cudaMemcpy(dc.emu_ops_dev(), ops, entries * sizeof(dev::p2p_ops), cudaMemcpyHostToDevice));
-        tab = dc.emu_ops_dev();
+        tab = (const dev::p2p_ops*)dc.emu_table(device_comm::EMU_P2P, ops, entries * sizeof(dev::p2p_ops), st);
     }
     const int emu = dc.emulated() ? 1 : 0;
     // Blocks wait for the peer's blocks, so all blocks of a launch must be resident at once: the lanes of an

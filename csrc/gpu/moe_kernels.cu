@@ -107,6 +107,66 @@ namespace {
 constexpr int ROUTE_MAX_EXPERTS = 64;
 constexpr int ROUTE_MAX_TOPK = 8;
 
+// Top-k of one token's logits: ids, softmax weights over the chosen logits.  Ties go to the lower expert index (as
+// torch.topk on a sorted scan would).  `pick(s, e)` is told every choice.  E: a bound of the number of experts for which
+// the row is read once into registers, 0 for any number.
+template <int E, class F>
+__device__ __forceinline__ void route_token(const float* __restrict__ row, int n_experts, int topk, long long* __restrict__ idx,
+                                            float* __restrict__ wts, F&& pick) {
+    unsigned long long taken = 0; // a bit per expert
+    int best[ROUTE_MAX_TOPK];
+    float val[ROUTE_MAX_TOPK];
+    float v[E > 0 ? E : 1];
+    if constexpr (E > 0) {
+#pragma unroll
+        for (int e = 0; e < E; e++)
+            if (e < n_experts)
+                v[e] = row[e];
+    }
+#pragma unroll
+    for (int s = 0; s < ROUTE_MAX_TOPK; s++) {
+        if (s < topk) {
+            int be = -1;
+            float bv = 0.f;
+            auto look = [&](int e, float x) {
+                if (!(taken >> e & 1) && (be < 0 || x > bv)) {
+                    be = e;
+                    bv = x;
+                }
+            };
+            if constexpr (E > 0) {
+#pragma unroll
+                for (int e = 0; e < E; e++)
+                    if (e < n_experts)
+                        look(e, v[e]);
+            }
+            else {
+                for (int e = 0; e < n_experts; e++)
+                    look(e, row[e]);
+            }
+            taken |= 1ull << be;
+            best[s] = be;
+            val[s] = bv;
+        }
+    }
+    float sum = 0.f;
+    const float vmax = val[0]; // the first pick is the maximum
+#pragma unroll
+    for (int s = 0; s < ROUTE_MAX_TOPK; s++)
+        if (s < topk) {
+            val[s] = __expf(val[s] - vmax);
+            sum += val[s];
+        }
+#pragma unroll
+    for (int s = 0; s < ROUTE_MAX_TOPK; s++)
+        if (s < topk) {
+            idx[s] = best[s];
+            wts[s] = val[s] / sum;
+            pick(s, best[s]);
+        }
+}
+
+template <int E>
 __global__ void __launch_bounds__(256)
     route_topk_kernel(const float* __restrict__ logits, int n_tokens, int n_experts, int topk, long long* __restrict__ idx,
                       float* __restrict__ wts, unsigned long long* __restrict__ counts) {
@@ -115,43 +175,59 @@ __global__ void __launch_bounds__(256)
         hist[e] = 0;
     __syncthreads();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n_tokens) {
-        const float* row = logits + (size_t)t * n_experts;
-        int best[ROUTE_MAX_TOPK];
-        float val[ROUTE_MAX_TOPK];
-        for (int s = 0; s < topk; s++) {
-            // largest logit not taken yet; ties go to the lower expert index (as torch.topk on a sorted scan would)
-            int be = -1;
-            float bv = 0.f;
-            for (int e = 0; e < n_experts; e++) {
-                bool taken = false;
-                for (int q = 0; q < s; q++)
-                    taken |= best[q] == e;
-                const float v = row[e];
-                if (!taken && (be < 0 || v > bv)) {
-                    be = e;
-                    bv = v;
-                }
-            }
-            best[s] = be;
-            val[s] = bv;
-        }
-        float sum = 0.f;
-        const float vmax = val[0]; // the first pick is the maximum
-        for (int s = 0; s < topk; s++) {
-            val[s] = __expf(val[s] - vmax);
-            sum += val[s];
-        }
-        for (int s = 0; s < topk; s++) {
-            idx[(size_t)t * topk + s] = best[s];
-            wts[(size_t)t * topk + s] = val[s] / sum;
-            atomicAdd(&hist[best[s]], 1u);
-        }
-    }
+    if (t < n_tokens)
+        route_token<E>(logits + (size_t)t * n_experts, n_experts, topk, idx + (size_t)t * topk, wts + (size_t)t * topk,
+                       [&](int, int e) { atomicAdd(&hist[e], 1u); });
     __syncthreads();
     for (int e = threadIdx.x; e < n_experts; e += blockDim.x)
         if (hist[e])
             atomicAdd(&counts[e], (unsigned long long)hist[e]);
+}
+
+// The whole routing of a batch of up to ROUTE_ONE_BLOCK items in one block: selection, counts, offsets and placement with
+// the counters in shared memory.  Latency is what it costs: 1024 tokens 4 us instead of two fills and two kernels (10 us).
+constexpr int ROUTE_ONE_BLOCK = 8192;
+
+template <int E>
+__global__ void __launch_bounds__(1024)
+    route_one_block_kernel(const float* __restrict__ logits, int n_tokens, int n_experts, int topk, long long* __restrict__ idx,
+                           float* __restrict__ wts, unsigned long long* __restrict__ counts, long long* __restrict__ order,
+                           long long* __restrict__ pos) {
+    __shared__ unsigned int count[ROUTE_MAX_EXPERTS], offs[ROUTE_MAX_EXPERTS];
+    __shared__ unsigned short ticket[ROUTE_ONE_BLOCK];
+    __shared__ unsigned char expert[ROUTE_ONE_BLOCK];
+    for (int e = threadIdx.x; e < n_experts; e += blockDim.x)
+        count[e] = 0;
+    __syncthreads();
+    for (int t = threadIdx.x; t < n_tokens; t += blockDim.x)
+        route_token<E>(logits + (size_t)t * n_experts, n_experts, topk, idx + (size_t)t * topk, wts + (size_t)t * topk,
+                       [&](int s, int e) {
+                        // lanes that chose the same expert draw their tickets together
+                        const unsigned peers = __match_any_sync(__activemask(), e);
+                        const int lead = __ffs(peers) - 1, lane = threadIdx.x & 31;
+                        unsigned base = 0;
+                        if (lane == lead)
+                            base = atomicAdd(&count[e], (unsigned)__popc(peers));
+                        base = __shfl_sync(peers, base, lead);
+                        ticket[t * topk + s] = (unsigned short)(base + __popc(peers & ((1u << lane) - 1)));
+                        expert[t * topk + s] = (unsigned char)e;
+                    });
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned acc = 0;
+        for (int e = 0; e < n_experts; e++) {
+            offs[e] = acc;
+            acc += count[e];
+        }
+    }
+    if (threadIdx.x < n_experts)
+        counts[threadIdx.x] = count[threadIdx.x];
+    __syncthreads();
+    for (int i = threadIdx.x; i < n_tokens * topk; i += blockDim.x) {
+        const unsigned p = offs[expert[i]] + ticket[i];
+        order[p] = i;
+        pos[i] = p;
+    }
 }
 
 // cursor[e] starts at zero; item i = token * topk + slot lands at offset(expert) + ticket.  Tickets are drawn in
@@ -193,7 +269,8 @@ __global__ void __launch_bounds__(256)
 } // namespace
 
 // logits [n_tokens, n_experts] fp32 -> idx [n_tokens, topk] (int64), wts [n_tokens, topk] (fp32),
-// counts [n_experts] (int64), order / pos [n_tokens * topk] (int64).  scratch: n_experts 32-bit words.
+// counts [n_experts] (int64), order / pos [n_tokens * topk] (int64).  scratch: n_experts 32-bit words; directly behind
+// `counts` it is cleared together with them.
 CCLX_API int cclx_moe_route(const float* logits, int n_tokens, int n_experts, int topk, long long* idx, float* wts,
                             long long* counts, long long* order, long long* pos, void* scratch, void* stream) {
     return cclx::capi::guard([&] {
@@ -202,12 +279,24 @@ CCLX_API int cclx_moe_route(const float* logits, int n_tokens, int n_experts, in
         CCL_THROW_IF_NOT(topk >= 1 && topk <= ROUTE_MAX_TOPK && topk <= n_experts, "top-k must be between 1 and min(",
                          ROUTE_MAX_TOPK, ", experts)");
         cudaStream_t st = (cudaStream_t)stream;
-        CUDA_CHECK(cudaMemsetAsync(counts, 0, sizeof(long long) * n_experts, st));
-        CUDA_CHECK(cudaMemsetAsync(scratch, 0, sizeof(unsigned int) * n_experts, st));
+        if (n_tokens > 0 && (size_t)n_tokens * topk <= ROUTE_ONE_BLOCK) {
+            auto kernel = n_experts <= 8 ? route_one_block_kernel<8> : n_experts <= 16 ? route_one_block_kernel<16> : route_one_block_kernel<0>;
+            const int threads = std::min(1024, (n_tokens + 31) / 32 * 32); // at least a warp; a thread per token
+            kernel<<<1, std::max(threads, 64), 0, st>>>(logits, n_tokens, n_experts, topk, idx, wts, (unsigned long long*)counts, order,
+                                                        pos);
+            CUDA_CHECK(cudaGetLastError());
+            return;
+        }
+        if (scratch == (void*)(counts + n_experts))
+            CUDA_CHECK(cudaMemsetAsync(counts, 0, (sizeof(long long) + sizeof(unsigned int)) * n_experts, st));
+        else {
+            CUDA_CHECK(cudaMemsetAsync(counts, 0, sizeof(long long) * n_experts, st));
+            CUDA_CHECK(cudaMemsetAsync(scratch, 0, sizeof(unsigned int) * n_experts, st));
+        }
         if (n_tokens == 0)
             return;
-        route_topk_kernel<<<(n_tokens + 255) / 256, 256, 0, st>>>(logits, n_tokens, n_experts, topk, idx, wts,
-                                                                  (unsigned long long*)counts);
+        auto topk_kernel = n_experts <= 8 ? route_topk_kernel<8> : n_experts <= 16 ? route_topk_kernel<16> : route_topk_kernel<0>;
+        topk_kernel<<<(n_tokens + 255) / 256, 256, 0, st>>>(logits, n_tokens, n_experts, topk, idx, wts, (unsigned long long*)counts);
         CUDA_CHECK(cudaGetLastError());
         const size_t n_items = (size_t)n_tokens * topk;
         route_place_kernel<<<(unsigned)((n_items + 255) / 256), 256, 0, st>>>(
@@ -270,63 +359,80 @@ __global__ void __launch_bounds__(512) moe_dispatch_kernel(const comm_dev* tab, 
     block_sync s;
     sync_begin(c, s);
     const int W = c.world;
-    __shared__ int s_dst[MAX_RANKS], s_pre[MAX_RANKS + 1], s_over;
+    __shared__ int s_cnt[MAX_RANKS * MAX_RANKS], s_own[MAX_RANKS], s_dst[MAX_RANKS], s_pre[MAX_RANKS + 1], s_over;
     // my counts into every rank's table, slot of this block
     const size_t blk_words = (size_t)blockIdx.x * W * W;
     for (int i = threadIdx.x; i < W * W; i += blockDim.x) {
         const int p = i / W, e = i % W;
+        const int v = (int)ra.send_counts[e];
         int* t = reinterpret_cast<int*>(c.heap[p] + a.cnt_off) + blk_words;
-        t[c.rank * W + e] = (int)ra.send_counts[e];
+        t[c.rank * W + e] = v;
+        if (p == 0)
+            s_own[e] = v;
     }
     bool ok = peer_barrier(c, s);
-    if (threadIdx.x == 0) {
-        const int* t = reinterpret_cast<const int*>(c.heap[c.rank] + a.cnt_off) + blk_words;
-        int over = 0, pre = 0, recv = 0;
-        for (int e = 0; e < W; e++) {
-            int off = 0, tot = 0;
-            for (int q = 0; q < W; q++) {
-                const int v = __ldcv(t + q * W + e);
-                if (q < c.rank)
-                    off += v;
-                tot += v;
-            }
-            s_dst[e] = off;
-            s_pre[e] = pre;
-            pre += (int)ra.send_counts[e];
-            over |= tot > (long long)a.cap_rows ? 1 : 0;
-            if (e == c.rank)
-                recv = tot;
+    // The table is read by all threads at once and worked on in shared memory: one thread that walked it in global memory
+    // waited W * W times for the L2, some 40 us for eight ranks, in every block.
+    for (int i = threadIdx.x; i < W * W; i += blockDim.x)
+        s_cnt[i] = __ldcv(reinterpret_cast<const int*>(c.heap[c.rank] + a.cnt_off) + blk_words + i);
+    if (threadIdx.x == 0)
+        s_over = 0;
+    __syncthreads();
+    if (threadIdx.x < W) {
+        const int e = threadIdx.x;
+        int off = 0, tot = 0, pre = 0;
+        for (int q = 0; q < W; q++) {
+            const int v = s_cnt[q * W + e];
+            off += q < c.rank ? v : 0;
+            tot += v;
+            pre += q < e ? s_own[q] : 0;
         }
-        s_pre[W] = pre;
-        s_over = over;
+        s_dst[e] = off;
+        s_pre[e] = pre;
+        if (e == W - 1)
+            s_pre[W] = pre + s_own[e];
+        if (tot > (long long)a.cap_rows)
+            s_over = 1;
         if (blockIdx.x == 0) {
-            for (int e = 0; e < W; e++) {
-                ra.meta[e] = s_dst[e];
-                ra.meta[W + e] = s_pre[e];
-            }
-            ra.meta[2 * W] = recv;
-            ra.meta[2 * W + 1] = over;
+            ra.meta[e] = off;
+            ra.meta[W + e] = pre;
+            if (e == c.rank)
+                ra.meta[2 * W] = tot;
         }
     }
     __syncthreads();
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        ra.meta[2 * W + 1] = s_over;
     if (ok && !s_over) {
-        // one warp per row
+        // one warp per row, eight packs per lane in flight; the index of the warp's next row is fetched meanwhile
         const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
         const size_t warp = (size_t)blockIdx.x * wpb + (threadIdx.x >> 5), nwarps = (size_t)gridDim.x * wpb;
         const int packs = a.hidden / 8;
+        long long item = warp < a.n_items ? ra.order[warp] : 0;
         for (size_t i = warp; i < a.n_items; i += nwarps) {
+            const uint4* src = reinterpret_cast<const uint4*>(ra.x + (size_t)((unsigned)item / (unsigned)a.topk) * a.hidden);
+            if (i + nwarps < a.n_items)
+                item = ra.order[i + nwarps];
             int e = 0;
             while (e + 1 < W && (long long)i >= s_pre[e + 1])
                 e++;
             const size_t row = (size_t)s_dst[e] + (i - (size_t)s_pre[e]);
-            const uint4* src = reinterpret_cast<const uint4*>(ra.x + (size_t)(ra.order[i] / a.topk) * a.hidden);
             char* dst = c.heap[e] + a.buf_off + row * (size_t)a.hidden * 2;
-            for (int k = lane; k < packs; k += 32)
-                st16(dst + (size_t)k * 16, src[k]);
+            for (int k0 = lane; k0 < packs; k0 += 256) {
+                uint4 v[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    if (k0 + k * 32 < packs)
+                        v[k] = src[k0 + k * 32];
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    if (k0 + k * 32 < packs)
+                        st16(dst + (size_t)(k0 + k * 32) * 16, v[k]);
+            }
         }
     }
     peer_barrier(c, s);
-    sync_end(c, gridDim.x, 2, false);
+    sync_end(c, s, gridDim.x, 2, false);
 }
 
 __global__ void __launch_bounds__(512) moe_combine_kernel(const comm_dev* tab, moe_args a) {
@@ -343,32 +449,73 @@ __global__ void __launch_bounds__(512) moe_combine_kernel(const comm_dev* tab, m
         const size_t warp = (size_t)blockIdx.x * wpb + (threadIdx.x >> 5), nwarps = (size_t)gridDim.x * wpb;
         const int packs = a.hidden / 8;
         const size_t tokens = a.n_items / a.topk;
+        // Lane sl of a warp works out where the row of slot sl lies (expert, place, weight: three dependent loads) for the
+        // warp's next token while the rows of this one are summed; four packs of two slots are in flight per lane.
+        const int topk = a.topk;
+        auto locate = [&](size_t t, int sl0, const char*& row, float& w) {
+            row = nullptr;
+            w = 0.f;
+            if (t < tokens && sl0 + lane < topk) {
+                const size_t f = t * topk + sl0 + lane;
+                const int e = (int)ra.expert[f];
+                const long long p = ra.pos[f];
+                w = ra.weight[f];
+                row = c.heap[e] + a.buf_off + (size_t)(ra.meta[e] + (p - ra.meta[W + e])) * (size_t)a.hidden * 2;
+            }
+        };
+        const char* next_row;
+        float next_w;
+        locate(warp, 0, next_row, next_w);
         for (size_t t = warp; t < tokens; t += nwarps) {
-            for (int k0 = lane; k0 < packs; k0 += 32) {
-                float acc[8] = { 0, 0, 0, 0, 0, 0, 0, 0 };
-                for (int sl = 0; sl < a.topk; sl++) {
-                    const size_t f = t * a.topk + sl;
-                    const int e = (int)ra.expert[f];
-                    const size_t row = (size_t)ra.meta[e] + ((size_t)ra.pos[f] - (size_t)ra.meta[W + e]);
-                    const float w = ra.weight[f];
-                    const uint4 v = ld_cv16(c.heap[e] + a.buf_off + row * (size_t)a.hidden * 2 + (size_t)k0 * 16);
-                    const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&v);
+            const char* my_row = next_row;
+            float my_w = next_w;
+            locate(t + nwarps, 0, next_row, next_w);
+            for (int k0 = lane; k0 < (packs + 31) / 32 * 32; k0 += 128) {
+                float acc[4][8] = {};
+                for (int sl = 0; sl < topk; sl += 2) {
+                    if (topk > 32 && sl % 32 == 0) // more slots than lanes
+                        locate(t, sl, my_row, my_w);
+                    uint4 v[2][4];
+                    float w[2];
 #pragma unroll
-                    for (int q = 0; q < 8; q++)
-                        acc[q] = fmaf(w, __bfloat162float(h[q]), acc[q]);
+                    for (int h = 0; h < 2; h++) {
+                        const int from = min(sl + h, topk - 1) & 31;
+                        const char* row = (const char*)__shfl_sync(0xffffffffu, (unsigned long long)my_row, from);
+                        w[h] = __shfl_sync(0xffffffffu, my_w, from);
+                        if (sl + h < topk)
+#pragma unroll
+                            for (int k = 0; k < 4; k++)
+                                if (k0 + k * 32 < packs)
+                                    v[h][k] = ld_cv16(row + (size_t)(k0 + k * 32) * 16);
+                    }
+#pragma unroll
+                    for (int h = 0; h < 2; h++)
+                        if (sl + h < topk)
+#pragma unroll
+                            for (int k = 0; k < 4; k++)
+                                if (k0 + k * 32 < packs) {
+                                    const __nv_bfloat16* b = reinterpret_cast<const __nv_bfloat16*>(&v[h][k]);
+#pragma unroll
+                                    for (int q = 0; q < 8; q++)
+                                        acc[k][q] = fmaf(w[h], __bfloat162float(b[q]), acc[k][q]);
+                                }
                 }
-                uint4 o;
-                __nv_bfloat16* oh = reinterpret_cast<__nv_bfloat16*>(&o);
 #pragma unroll
-                for (int q = 0; q < 8; q++)
-                    oh[q] = __float2bfloat16_rn(acc[q]);
-                reinterpret_cast<uint4*>(ra.out + t * a.hidden)[k0] = o;
+                for (int k = 0; k < 4; k++)
+                    if (k0 + k * 32 < packs) {
+                        uint4 o;
+                        __nv_bfloat16* oh = reinterpret_cast<__nv_bfloat16*>(&o);
+#pragma unroll
+                        for (int q = 0; q < 8; q++)
+                            oh[q] = __float2bfloat16_rn(acc[k][q]);
+                        reinterpret_cast<uint4*>(ra.out + t * a.hidden)[k0 + k * 32] = o;
+                    }
             }
         }
     }
     // nobody may overwrite its output rows (the next layer's FFN) before every reader is done
     peer_barrier(c, s);
-    sync_end(c, gridDim.x, 2, false);
+    sync_end(c, s, gridDim.x, 2, false);
 }
 
 void launch_moe(gpu::device_comm& dc, bool dispatch, moe_args& a, const moe_rank_args* ra, int blocks,
@@ -378,10 +525,9 @@ void launch_moe(gpu::device_comm& dc, bool dispatch, moe_args& a, const moe_rank
     a.r0 = ra[0];
     if (dc.emulated()) {
         static_assert(sizeof(moe_rank_args) <= sizeof(dev::rank_args), "argument block too large");
-        CUDA_CHECK(cudaStreamSynchronize(st));
-        CUDA_CHECK(cudaMemcpy(dc.emu_args_dev(), ra, dc.world() * sizeof(moe_rank_args), cudaMemcpyHostToDevice));
         a.emu = 1;
-        a.emu_tab = reinterpret_cast<const moe_rank_args*>(dc.emu_args_dev());
+        a.emu_tab = (const moe_rank_args*)dc.emu_table(dispatch ? gpu::device_comm::EMU_COLL : gpu::device_comm::EMU_MOE, ra,
+                                                       dc.world() * sizeof(moe_rank_args), st);
         const comm_dev* tab = dc.table();
         void* argv[] = { (void*)&tab, (void*)&a };
         dim3 grid(blocks, dc.world());

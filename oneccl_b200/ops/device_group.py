@@ -193,13 +193,9 @@ class DeviceGroup:
     def allreduce(self, send, recv=None, op="sum", algo="auto", blocks=0, scale: Optional[float] = None, stream=None):
         recv = send if recv is None else recv
         s, r = self._lists(send, recv)
-        for a, b in zip(s, r):
-            assert a.is_contiguous() and b.is_contiguous() and a.numel() == b.numel()
-        rc = self._lib.cclx_dc_allreduce(
-            self._h, self._ptrs(s), self._ptrs(r), s[0].numel(), torch_to_ccl(s[0].dtype), torch_to_ccl(r[0].dtype),
-            reduce_op_code(op), GPU_ALGO[algo], blocks, 1.0 if scale is None else float(scale),
-            0 if scale is None else 1, _stream_ptr(stream))
-        self._finish(rc)
+        if stream is not None:
+            stream = _stream_ptr(stream)
+        native().dc_allreduce(self._h.value, s, r, reduce_op_code(op), GPU_ALGO[algo], blocks, scale, stream)
         return recv
 
     def allreduce_fused(self, tensors, op="sum", scale: Optional[float] = None, stream=None):

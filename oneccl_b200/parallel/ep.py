@@ -17,8 +17,10 @@ import torch
 from .. import _lib
 from ..ops.device_group import DeviceGroup, _stream_ptr
 from ..ops.gemm import gemm_bf16
+from ..torch_ops import native
 
 launches = 0
+_ROUTE_ONE_BLOCK = 8192  # items (token, slot) up to which one block does the whole routing
 
 
 def gather_rows(x: torch.Tensor, src_row: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -46,7 +48,7 @@ def combine_rows(y: torch.Tensor, pos: torch.Tensor, w: torch.Tensor, out: torch
 
 def _per_entry(group: DeviceGroup, t):
     """Real mode takes one tensor, emulation a list with one tensor per rank."""
-    return list(t) if group.emulated_mode else [t]
+    return [t] if isinstance(t, torch.Tensor) else t
 
 
 def fused_dispatch(group: DeviceGroup, x, order, send_counts, meta, recv_buf, cnt_table, topk: int, blocks: int = 0):
@@ -56,10 +58,8 @@ def fused_dispatch(group: DeviceGroup, x, order, send_counts, meta, recv_buf, cn
     offsets, the number of rows this rank's expert got (``meta[2 * world]``) and an overflow flag."""
     global launches
     xs, orders, counts, metas = (_per_entry(group, v) for v in (x, order, send_counts, meta))
-    rb, ct = _per_entry(group, recv_buf)[0], _per_entry(group, cnt_table)[0]
-    _lib.check(_lib.load().cclx_moe_dispatch(
-        group.handle, group._ptrs(xs), group._ptrs(orders), group._ptrs(counts), group._ptrs(metas),
-        orders[0].numel(), topk, xs[0].shape[1], rb.data_ptr(), rb.shape[0], ct.data_ptr(), blocks, _stream_ptr()))
+    native().moe_dispatch(group.handle.value, xs, orders, counts, metas, _per_entry(group, recv_buf)[0],
+                          _per_entry(group, cnt_table)[0], topk, blocks)
     launches += 1
 
 
@@ -69,33 +69,20 @@ def fused_combine(group: DeviceGroup, expert, pos, weight, out, meta, expert_out
     in the order ``fused_dispatch`` delivered them."""
     global launches
     es, ps, ws, outs, metas = (_per_entry(group, v) for v in (expert, pos, weight, out, meta))
-    eo = _per_entry(group, expert_out)[0]
-    _lib.check(_lib.load().cclx_moe_combine_peer(
-        group.handle, group._ptrs(es), group._ptrs(ps), group._ptrs(ws), group._ptrs(outs), group._ptrs(metas),
-        es[0].numel(), topk, outs[0].shape[1], eo.data_ptr(), blocks, _stream_ptr()))
+    native().moe_combine(group.handle.value, es, ps, ws, outs, metas, _per_entry(group, expert_out)[0], topk, blocks)
     launches += 1
 
 
 def route_device(logits: torch.Tensor, topk: int):
-    """Top-k routing in two kernels: expert ids [T, k] (int64), softmax weights over the chosen logits [T, k]
+    """Top-k routing in one kernel (small batches) or two: expert ids [T, k] (int64), softmax weights over the chosen logits [T, k]
     (fp32), items per expert [E] (int64), a permutation ``order`` of the T * k (token, slot) items that groups
     them by expert, and its inverse ``pos``.  What ``torch.topk`` + ``softmax`` + ``bincount`` + ``argsort`` +
     a scatter compute, without the sort (the order inside an expert's group is arbitrary)."""
     global launches
     assert logits.is_cuda and logits.dim() == 2
-    lg = logits.float().contiguous()
-    T, E = lg.shape
-    dev = lg.device
-    idx = torch.empty((T, topk), dtype=torch.int64, device=dev)
-    wts = torch.empty((T, topk), dtype=torch.float32, device=dev)
-    counts = torch.empty((E,), dtype=torch.int64, device=dev)
-    order = torch.empty((T * topk,), dtype=torch.int64, device=dev)
-    pos = torch.empty((T * topk,), dtype=torch.int64, device=dev)
-    scratch = torch.empty((E,), dtype=torch.int32, device=dev)
-    _lib.check(_lib.load().cclx_moe_route(lg.data_ptr(), T, E, topk, idx.data_ptr(), wts.data_ptr(), counts.data_ptr(),
-                                          order.data_ptr(), pos.data_ptr(), scratch.data_ptr(), _stream_ptr()))
-    launches += 2
-    return idx, wts, counts, order, pos
+    out = native().moe_route(logits, topk)
+    launches += 1 if logits.shape[0] * topk <= _ROUTE_ONE_BLOCK else 2
+    return out
 
 
 class ExpertParallelMoE:

@@ -1,0 +1,96 @@
+// Host side of the small calls on a device group and of the expert-parallel steps: tensors to pointer tables without a
+// Python loop over them (kernels: csrc/gpu/launch_allreduce.cu, moe_kernels.cu).
+#include "torch_ops.hpp"
+
+namespace cclx_ops {
+namespace {
+
+typedef std::vector<Tensor> tensors;
+
+int ccl_dtype(at::ScalarType t) {
+    switch (t) {
+        case at::kChar: return 0;
+        case at::kByte:
+        case at::kBool: return 1;
+        case at::kShort: return 2;
+        case at::kUInt16: return 3;
+        case at::kInt: return 4;
+        case at::kUInt32: return 5;
+        case at::kLong: return 6;
+        case at::kUInt64: return 7;
+        case at::kHalf: return 8;
+        case at::kFloat: return 9;
+        case at::kDouble: return 10;
+        case at::kBFloat16: return 11;
+        default: throw pybind11::type_error(std::string(c10::toString(t)) + " has no ccl datatype");
+    }
+}
+
+template <class T>
+std::vector<T*> pointers(const tensors& ts) {
+    std::vector<T*> p;
+    p.reserve(ts.size());
+    for (const auto& t : ts)
+        p.push_back(reinterpret_cast<T*>(t.data_ptr()));
+    return p;
+}
+
+// one tensor per entry: this rank's, or one per emulated rank
+void allreduce(uintptr_t group, const tensors& send, const tensors& recv, int op, int algo, int blocks, std::optional<double> scale,
+               std::optional<uintptr_t> stream) {
+    for (size_t i = 0; i < send.size(); i++)
+        if (!send[i].is_contiguous() || !recv[i].is_contiguous() || send[i].numel() != recv[i].numel()) {
+            PyErr_SetString(PyExc_AssertionError, "allreduce takes contiguous tensors of one size");
+            throw pybind11::error_already_set();
+        }
+    void* st = stream ? reinterpret_cast<void*>(*stream) : stream_of(send[0]);
+    const auto s = pointers<const void>(send);
+    const auto r = pointers<void>(recv);
+    check(cclx_dc_allreduce(reinterpret_cast<void*>(group), s.data(), r.data(), send[0].numel(), ccl_dtype(send[0].scalar_type()),
+                            ccl_dtype(recv[0].scalar_type()), op, algo, blocks, scale ? (float)*scale : 1.0f, scale ? 1 : 0, st));
+}
+
+// expert ids [T, k], weights [T, k], items per expert [E], grouping permutation and its inverse [T * k]
+pybind11::tuple route(const Tensor& logits_, int64_t topk) {
+    const Tensor logits = logits_.scalar_type() == at::kFloat && logits_.is_contiguous() ? logits_ : logits_.to(at::kFloat).contiguous();
+    const int64_t T = logits.size(0), E = logits.size(1);
+    const Tensor idx = empty_on(logits, { T, topk }, at::kLong), wts = empty_on(logits, { T, topk }, at::kFloat);
+    const Tensor counts = empty_on(logits, { E + (E + 1) / 2 }, at::kLong); // the placement cursors stand behind the counts
+    const Tensor order = empty_on(logits, { T * topk }, at::kLong), pos = empty_on(logits, { T * topk }, at::kLong);
+    long long* c = reinterpret_cast<long long*>(counts.data_ptr<int64_t>());
+    check(cclx_moe_route(logits.data_ptr<float>(), (int)T, (int)E, (int)topk, reinterpret_cast<long long*>(idx.data_ptr<int64_t>()),
+                         wts.data_ptr<float>(), c, reinterpret_cast<long long*>(order.data_ptr<int64_t>()),
+                         reinterpret_cast<long long*>(pos.data_ptr<int64_t>()), c + E, stream_of(logits)));
+    return pybind11::make_tuple(idx, wts, counts.narrow(0, 0, E), order, pos);
+}
+
+void dispatch(uintptr_t group, const tensors& x, const tensors& order, const tensors& counts, const tensors& meta, const Tensor& recv,
+              const Tensor& table, int topk, int blocks) {
+    const auto px = pointers<const void>(x);
+    const auto po = pointers<const long long>(order), pc = pointers<const long long>(counts);
+    const auto pm = pointers<int>(meta);
+    check(cclx_moe_dispatch(reinterpret_cast<void*>(group), px.data(), po.data(), pc.data(), pm.data(), order[0].numel(), topk,
+                            (int)x[0].size(1), recv.data_ptr(), recv.size(0), table.data_ptr(), blocks, stream_of(recv)));
+}
+
+void combine(uintptr_t group, const tensors& expert, const tensors& pos, const tensors& weight, const tensors& out, const tensors& meta,
+             const Tensor& expert_out, int topk, int blocks) {
+    const auto pe = pointers<const long long>(expert), pp = pointers<const long long>(pos);
+    const auto pw = pointers<const float>(weight);
+    const auto po = pointers<void>(out);
+    const auto pm = pointers<int>(meta);
+    check(cclx_moe_combine_peer(reinterpret_cast<void*>(group), pe.data(), pp.data(), pw.data(), po.data(), pm.data(),
+                                expert[0].numel(), topk, (int)out[0].size(1), expert_out.data_ptr(), blocks,
+                                stream_of(expert_out)));
+}
+
+} // namespace
+
+void bind_coll(pybind11::module_& m) {
+    m.def("dc_allreduce", &allreduce);
+    m.def("moe_route", &route);
+    m.def("moe_dispatch", &dispatch);
+    m.def("moe_combine", &combine);
+}
+
+} // namespace cclx_ops

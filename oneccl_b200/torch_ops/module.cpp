@@ -57,4 +57,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     bind_nn(m);
     bind_train(m);
     bind_gemm(m);
+    bind_coll(m);
 }

@@ -23,6 +23,16 @@ int cclx_layer_norm_bwd_blocks(size_t rows);
 int cclx_layer_norm_bwd_sums(const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
                              const void* dres, void* dx, void* dgamma, void* dbeta, void* dxsum, int add,
                              float* workspace, size_t rows, int D, void* stream);
+int cclx_dc_allreduce(void* h, const void* const* send, void* const* recv, size_t count, int dt_in, int dt_out, int op, int algo,
+                      int blocks, float scale, int do_scale, void* stream);
+int cclx_moe_route(const float* logits, int n_tokens, int n_experts, int topk, long long* idx, float* wts, long long* counts,
+                   long long* order, long long* pos, void* scratch, void* stream);
+int cclx_moe_dispatch(void* h, const void* const* x, const long long* const* order, const long long* const* send_counts,
+                      int* const* meta, size_t n_items, int topk, int hidden, const void* recv_buf, size_t cap_rows,
+                      const void* cnt_table, int blocks, void* stream);
+int cclx_moe_combine_peer(void* h, const long long* const* expert, const long long* const* pos, const float* const* weight,
+                          void* const* out, int* const* meta, size_t n_items, int topk, int hidden, const void* expert_out,
+                          int blocks, void* stream);
 size_t cclx_map_colsum_workspace(size_t rows, int N);
 int cclx_colsum(const void* x, void* out, int add, float* workspace, size_t rows, int N, void* stream);
 int cclx_gelu_fwd(const void* x, void* y, size_t n, void* stream);
@@ -128,5 +138,6 @@ SinkRef sink_of(const pybind11::object& param); // null without one
 void bind_nn(pybind11::module_& m);
 void bind_train(pybind11::module_& m);
 void bind_gemm(pybind11::module_& m);
+void bind_coll(pybind11::module_& m);
 
 } // namespace cclx_ops

@@ -196,3 +196,60 @@ def test_step_that_overwrites_gradients_matches_cleared_ones():
     assert torch.count_nonzero(model.extra.grad) == 0 and bool((model.scale.grad == 0.5).all())
     ddp.close()
     group.close()
+
+
+@pytest.mark.parametrize("W", [2, 4])
+@pytest.mark.parametrize("T,H,k", [(1, 8, 1), (3, 264, 2), (65, 1032, 2), (40, 4096, 2), (5000, 64, 2)])
+def test_moe_dispatch_and_combine_shapes(W, T, H, k):
+    """Rows shorter and longer than one batch of loads, more and fewer tokens than warps, routing in one block and in two
+    kernels; repeated so that changed and unchanged argument tables follow one another."""
+    from oneccl_b200.ops.device_group import DeviceGroup
+    from oneccl_b200.parallel.ep import fused_combine, fused_dispatch, route_device
+
+    g = torch.Generator(device="cuda").manual_seed(T + H)
+    cap = T * k * W
+    group = DeviceGroup.emulated(W, heap_bytes=cap * H * 2 + (40 << 20), staging_bytes=1 << 20)
+    recv = group.symm_empty((cap, H), dtype=torch.bfloat16)
+    table = group.symm_empty((256 * W * W,), dtype=torch.int32)
+    meta = [torch.zeros(2 * W + 2, dtype=torch.int32, device="cuda") for _ in range(W)]
+    for _ in range(2):
+        x = [_bf16(g, T, H) for _ in range(W)]
+        logits = [torch.randn(T, W, generator=g, device="cuda") for _ in range(W)]
+        out = [torch.empty_like(t) for t in x]
+        idx, wts, counts, order, pos = zip(*(route_device(lg, k) for lg in logits))
+        for r in range(W):
+            ref_w, ref_i = torch.topk(logits[r], k, dim=-1)
+            assert torch.equal(idx[r], ref_i) and torch.equal(counts[r], torch.bincount(ref_i.flatten(), minlength=W))
+            torch.testing.assert_close(wts[r], torch.softmax(ref_w, -1), rtol=1e-5, atol=1e-6)
+            assert torch.equal(order[r][pos[r]], torch.arange(T * k, device="cuda"))
+            assert bool((ref_i.flatten()[order[r]].diff() >= 0).all())
+        for again in range(2):
+            fused_dispatch(group, x, order, counts, meta, recv, table, k)
+            fused_combine(group, [i.view(-1) for i in idx], pos, [w.view(-1) for w in wts], out, meta, recv, k)
+        torch.cuda.synchronize()
+        group.check()
+        for r in range(W):
+            assert int(meta[r][2 * W]) == sum(int(c[r]) for c in counts) and int(meta[r][2 * W + 1]) == 0
+            torch.testing.assert_close(out[r].float(), x[r].float(), rtol=1e-2, atol=1e-2)
+    group.close()
+
+
+def test_emulated_argument_tables_wrap_around():
+    """More different argument tables than the ring holds, on two streams."""
+    from oneccl_b200.ops.device_group import DeviceGroup
+
+    group = DeviceGroup.emulated(2, heap_bytes=40 << 20, staging_bytes=1 << 20)
+    xs = [[torch.full((100 + i,), float(r + i), device="cuda") for r in range(2)] for i in range(150)]
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    for i, pair in enumerate(xs):
+        s = side if i % 50 > 40 else torch.cuda.current_stream()
+        if i and (i % 50 > 40) != ((i - 1) % 50 > 40):
+            side.wait_stream(torch.cuda.current_stream())
+            torch.cuda.current_stream().wait_stream(side)
+        group.allreduce(pair, pair, stream=s)
+    torch.cuda.synchronize()
+    group.check()
+    for i, pair in enumerate(xs):
+        assert all(bool((t == 2 * i + 1).all()) for t in pair), i
+    group.close()
