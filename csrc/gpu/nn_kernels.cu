@@ -485,7 +485,7 @@ struct qkv_map {
     };
     __device__ __forceinline__ input load(size_t r, int p) const {
         const int head = p / ppr, part = head / H, h = head - part * H;
-        const size_t b = r / S, s = r - b * S;
+        const unsigned b = (unsigned)r / (unsigned)S, s = (unsigned)r - b * (unsigned)S; // 64-bit divisions cost more than the copy
         const __nv_bfloat16* q = part == 0 ? src[0] : part == 1 ? src[1] : src[2];
         const long long o = part == 0 ? b * sb[0] + s * ss[0] + h * sh[0]
                             : part == 1 ? b * sb[1] + s * ss[1] + h * sh[1]
@@ -664,6 +664,7 @@ CCLX_API int cclx_qkv_grad_colsum(const void* const* src, const long long* strid
         CCL_THROW_IF_NOT(dh % 8 == 0, "head size must be a multiple of 8");
         if (B == 0 || S == 0)
             return;
+        CCL_THROW_IF_NOT((long long)B * S < (1ll << 31), "too many rows: ", B, " x ", S);
         qkv_map f;
         for (int p = 0; p < 3; p++) {
             f.src[p] = (const __nv_bfloat16*)src[p];
