@@ -8,6 +8,7 @@
 #include "core/env.hpp"
 #include "core/log.hpp"
 #include "gpu/cuda_driver.hpp"
+#include "gpu/device_info.hpp"
 #include "gpu/device_comm.hpp"
 #include "gpu/fused_gemm.hpp"
 
@@ -322,9 +323,7 @@ CCLX_API int cclx_gemm_bf16_2sm(const void* A, const void* B, void* C, int M, in
 CCLX_API int cclx_gemm_bf16_rows(const void* A, const void* B, void* C, int M, int N, int K, int epilogue,
                                  const void* rows_dev, void* err_words, void* stream) {
     return capi::guard([&] {
-        int dev = 0, sms = 0;
-        CUDA_CHECK(cudaGetDevice(&dev));
-        CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        const int sms = device_sms();
         if (gemm_small_preferred(M, N, K, sms))
             gemm_bf16_small(A, B, C, M, N, K, epilogue, (uint32_t*)err_words, (cudaStream_t)stream, (const int*)rows_dev);
         else

@@ -8,6 +8,7 @@
 #include "core/env.hpp"
 #include "core/log.hpp"
 #include "gpu/cuda_driver.hpp"
+#include "gpu/device_info.hpp"
 #include "gpu/device_comm.hpp"
 #include "gpu/fused_gemm.hpp"
 
@@ -81,10 +82,7 @@ void launch(const dev::comm_dev* tab, const fused_params& P, int bn, int ctas, i
 }
 
 int sm_count() {
-    int dev = 0, n = 0;
-    CUDA_CHECK(cudaGetDevice(&dev));
-    CUDA_CHECK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
-    return n;
+    return device_sms();
 }
 
 } // namespace

@@ -280,9 +280,7 @@ void gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, i
     P.epilogue = epilogue;
     P.rows = rows_dev;
     P.timeout_ns = (unsigned long long)env_data::get().wait_timeout_ms * 1000000ull;
-    int dev = 0, sms = 0;
-    CUDA_CHECK(cudaGetDevice(&dev));
-    CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int sms = device_sms();
     const int tiles = ((M + 255) / 256) * ((N + G2_BN - 1) / G2_BN);
     int nc = clusters > 0 ? clusters : sms / 2;
     nc = std::max(1, std::min(nc, tiles));

@@ -322,9 +322,7 @@ bool gemm_small_preferred(int M, int N, int K, int sms) {
 void gemm_bf16_small(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, uint32_t* err, cudaStream_t st,
                      const int* rows_dev) {
     CCL_THROW_IF_NOT(M > 0 && N > 0 && K > 0 && N % 8 == 0 && K % 8 == 0, "unsupported GEMM shape ", M, "x", N, "x", K);
-    int dev = 0, sms = 0;
-    CUDA_CHECK(cudaGetDevice(&dev));
-    CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int sms = device_sms();
     const small_plan plan = plan_small(M, N, K, sms);
     gemm_small_params P;
     std::memset(&P, 0, sizeof(P));

@@ -11,6 +11,7 @@
 #include <utility>
 
 #include "gpu/cuda_driver.hpp"
+#include "gpu/device_info.hpp"
 
 namespace cclx {
 namespace gpu {

@@ -16,6 +16,9 @@
 #include "capi/capi_common.hpp"
 #include "core/log.hpp"
 #include "gpu/cuda_driver.hpp"
+#include "gpu/launch_util.cuh"
+
+using namespace cclx;
 
 namespace {
 
@@ -62,10 +65,7 @@ __global__ void __launch_bounds__(256) combine_rows_kernel(const __nv_bfloat16* 
 }
 
 int blocks_for(size_t rows) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    size_t cap = (size_t)sms * 8;
+    size_t cap = (size_t)gpu::device_sms() * 8;
     return (int)(rows < cap ? (rows ? rows : 1) : cap);
 }
 
@@ -196,9 +196,11 @@ __global__ void __launch_bounds__(1024)
     __shared__ unsigned int count[ROUTE_MAX_EXPERTS], offs[ROUTE_MAX_EXPERTS];
     __shared__ unsigned short ticket[ROUTE_ONE_BLOCK];
     __shared__ unsigned char expert[ROUTE_ONE_BLOCK];
+    gpu::pdl_trigger();
     for (int e = threadIdx.x; e < n_experts; e += blockDim.x)
         count[e] = 0;
     __syncthreads();
+    gpu::pdl_wait(); // launched while the kernel in front still runs
     for (int t = threadIdx.x; t < n_tokens; t += blockDim.x)
         route_token<E>(logits + (size_t)t * n_experts, n_experts, topk, idx + (size_t)t * topk, wts + (size_t)t * topk,
                        [&](int s, int e) {
@@ -282,9 +284,8 @@ CCLX_API int cclx_moe_route(const float* logits, int n_tokens, int n_experts, in
         if (n_tokens > 0 && (size_t)n_tokens * topk <= ROUTE_ONE_BLOCK) {
             auto kernel = n_experts <= 8 ? route_one_block_kernel<8> : n_experts <= 16 ? route_one_block_kernel<16> : route_one_block_kernel<0>;
             const int threads = std::min(1024, (n_tokens + 31) / 32 * 32); // at least a warp; a thread per token
-            kernel<<<1, std::max(threads, 64), 0, st>>>(logits, n_tokens, n_experts, topk, idx, wts, (unsigned long long*)counts, order,
-                                                        pos);
-            CUDA_CHECK(cudaGetLastError());
+            gpu::launch_dependent(kernel, dim3(1), dim3(std::max(threads, 64)), 0, st, logits, n_tokens, n_experts, topk, idx, wts,
+                                  (unsigned long long*)counts, order, pos);
             return;
         }
         if (scratch == (void*)(counts + n_experts))

@@ -500,13 +500,6 @@ struct qkv_map {
     }
 };
 
-int sm_count_now() {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
-}
-
 } // namespace
 
 // ---- C entry points -----------------------------------------------------------------------------
@@ -519,7 +512,7 @@ CCLX_API int cclx_layer_norm_fwd(const void* x, const void* res, const void* w, 
         if (rows == 0)
             return;
         // four warps per block; up to 24 warps per SM, after which warps take several rows
-        const int blocks = (int)std::min<size_t>((rows + 3) / 4, (size_t)sm_count_now() * 6);
+        const int blocks = (int)std::min<size_t>((rows + 3) / 4, (size_t)device_sms() * 6);
         cudaStream_t st = (cudaStream_t)stream;
 #define LN_FWD(V)                                                                                                     \
     case V:                                                                                                           \
@@ -543,7 +536,7 @@ CCLX_API int cclx_layer_norm_fwd(const void* x, const void* res, const void* w, 
 
 // rows of the backward workspace: an upper bound of the blocks that any width launches
 CCLX_API int cclx_layer_norm_bwd_blocks(size_t rows) {
-    return (int)std::min<size_t>(rows, (size_t)sm_count_now() * LN_BWD_BLOCKS);
+    return (int)std::min<size_t>(rows, (size_t)device_sms() * LN_BWD_BLOCKS);
 }
 
 namespace {
@@ -555,7 +548,7 @@ int launch_ln_bwd(const void* dy, const void* x, const void* w, const float* mea
     const size_t ring = (size_t)LN_BWD_STAGES * 3 * R * threads * 16;
     const size_t smem = std::max(ring + (size_t)2 * groups * 2 * R * 8 * 4, groups > 1 ? (size_t)groups * D * 4 : 0);
     const size_t want = (rows + (size_t)groups * R - 1) / ((size_t)groups * R);
-    const int blocks = (int)std::min<size_t>(want, (size_t)sm_count_now() * LN_BWD_BLOCKS);
+    const int blocks = (int)std::min<size_t>(want, (size_t)device_sms() * LN_BWD_BLOCKS);
     allow_smem<ln_bwd_kernel<R, COLSUM>>((size_t)LN_BWD_STAGES * 3 * R * 256 * 16 + 2048);
     ln_bwd_kernel<R, COLSUM><<<blocks, threads, smem, st>>>((const uint4*)dy, (const uint4*)x, (const uint4*)w, mean, rstd,
                                                             (const uint4*)dres, (uint4*)dx, workspace, rows, packs, tpr,
@@ -578,7 +571,7 @@ CCLX_API int cclx_layer_norm_bwd_sums(const void* dy, const void* x, const void*
         cudaStream_t st = (cudaStream_t)stream;
         // Two rows per step halve the barriers; with too few rows to give every SM several steps, one row at a time
         // spreads them over the chip instead (64 rows of 1024: 32 blocks, not 16).
-        const bool wide = rows >= (size_t)sm_count_now() * 16;
+        const bool wide = rows >= (size_t)device_sms() * 16;
         int n;
         if (dxsum)
             n = wide ? launch_ln_bwd<LN_BWD_ROWS, true>(dy, x, w, mean, rstd, dres, dx, workspace, rows, D, st)
@@ -602,7 +595,7 @@ namespace {
 int map_rows_per_block(size_t rows, int packs) {
     // about six blocks of 128 threads per SM, between 8 and 64 rows each: fewer rows would spend more on partial sums
     const size_t cols = (packs + 127) / 128;
-    const size_t per = rows * cols / ((size_t)sm_count_now() * 6);
+    const size_t per = rows * cols / ((size_t)device_sms() * 6);
     return (int)std::min<size_t>(64, std::max<size_t>(8, (per + 3) / 4 * 4));
 }
 

@@ -600,13 +600,6 @@ __global__ void __launch_bounds__(128)
         x[i] = __float2bfloat16_rn(0.f);
 }
 
-int sm_count_now() {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
-}
-
 constexpr size_t XENT_SMEM = 226 * 1024; // shared memory of an SM that blocks can have, reserved parts aside
 
 template <int T>
@@ -616,7 +609,7 @@ void launch_xent_stream(__nv_bfloat16* logits, const long long* targets, float* 
     const size_t smem = (size_t)ppt * T * 16;
     allow_smem<xent_stream_kernel<T>>(XENT_SMEM);
     const int per_sm = std::max(1, std::min((int)(XENT_SMEM / (smem + 1536)), T == 1024 ? 1 : 1024 / T));
-    const int blocks = (int)std::min<size_t>(rows, (size_t)sm_count_now() * per_sm);
+    const int blocks = (int)std::min<size_t>(rows, (size_t)device_sms() * per_sm);
     xent_stream_kernel<T><<<blocks, T, smem, st>>>(logits, targets, loss_rows, rows, vocab, ld, grad_scale, pad_cols, ppt);
 }
 
