@@ -119,6 +119,7 @@ class DataParallel:
         self.flat_grad = g[0] if isinstance(g, list) else g
         self.flat_grad.zero_()
         self._sinks = []
+        self._grad_stream = native().GradStream(dev.index if dev.index is not None else torch.cuda.current_device())
         for p, o in zip(order, offs):
             self.flat_param[o:o + p.numel()].copy_(p.data.reshape(-1))
             p.data = self.flat_param[o:o + p.numel()].view_as(p.data)
@@ -164,17 +165,19 @@ class DataParallel:
         self._arm()
         self.flat_grad.zero_()
         for _, sink, _ in self._sinks:
-            sink.fresh = False
+            sink.end_step()
 
     def begin_step(self):
         """``zero_grad`` for a step that ends with ``finish``: the buffer is not cleared, the first contribution to
         every gradient overwrites it, and ``finish`` clears what received none.  Until then the buffer holds a
-        mixture of the last step's gradients and this one's."""
+        mixture of the last step's gradients and this one's, and weight gradients may still be on their way on a
+        stream of their own."""
         self._arm()
         for _, sink, _ in self._sinks:
-            sink.fresh = True
+            sink.begin_step(self._grad_stream)
 
     def _arm(self):
+        self._grad_stream.finish()  # of a step that never came to its end
         if self.record_timeline:
             self.t_step = torch.cuda.Event(enable_timing=True)
             self.t_step.record()
@@ -190,6 +193,8 @@ class DataParallel:
         ev = torch.cuda.Event(enable_timing=timing)
         ev.record()
         self.comm_stream.wait_event(ev)
+        if self.world > 1:
+            self._grad_stream.join(self.comm_stream.cuda_stream, self.comm_stream.device_index)
         seg = self.flat_grad[bs[0].start:bs[-1].end]
         with torch.cuda.stream(self.comm_stream):
             t0 = t1 = None
@@ -248,12 +253,13 @@ class DataParallel:
         for _, sink, _ in self._sinks:
             if sink.fresh:
                 sink.grad.zero_()
-                sink.fresh = False
+            sink.end_step()
         late = [b for b in self.buckets if b.pending > 0]  # parameters that received no gradient this step
         for b in late:
             b.pending = 0
         self._launch_ready(late)
         torch.cuda.current_stream().wait_stream(self.comm_stream)
+        self._grad_stream.finish()
         self._armed = False
 
     def timeline(self):

@@ -38,19 +38,35 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         return reinterpret_cast<uintptr_t>(s.stream());
     }, "handle of the current stream; the library's runtime follows its device");
     m.def("set_device", [](int dev) { set_device(dev); });
+    py::class_<GradStream, GradStreamRef>(m, "GradStream")
+        .def(py::init<int>())
+        .def("join", [](GradStream& g, uintptr_t stream, int dev) {
+            g.join(at::cuda::getStreamFromExternal(reinterpret_cast<cudaStream_t>(stream), (c10::DeviceIndex)dev));
+        })
+        .def("finish", &GradStream::finish);
     py::class_<GradSink, SinkRef>(m, "GradSink")
         .def(py::init<Tensor, py::object>())
         .def_readonly("grad", &GradSink::grad)
         .def_readwrite("fresh", &GradSink::fresh)
+        .def("begin_step", [](GradSink& s, const GradStreamRef& beside) {
+            s.fresh = true;
+            s.on_side = false;
+            s.beside = beside;
+        })
+        // whether the parameter received a gradient since begin_step
+        .def("end_step", [](GradSink& s) {
+            const bool got = !s.fresh;
+            s.fresh = s.on_side = false;
+            s.beside = nullptr;
+            return got;
+        })
         // gradients that autograd accumulates itself are added in place: give them a clean buffer first
         .def("clear_before_accumulation",
              [](const SinkRef& s, const Tensor& param) {
                  std::weak_ptr<GradSink> w = s;
                  return param.register_hook([w](const Tensor& g) {
-                     if (const SinkRef s = w.lock(); s && s->fresh && g.defined()) {
-                         s->fresh = false;
+                     if (const SinkRef s = w.lock(); s && g.defined() && !s->add())
                          s->grad.zero_();
-                     }
                  });
              })
         .def("remove_hook", [](const SinkRef&, const Tensor& param, unsigned h) { param.remove_hook(h); });

@@ -195,7 +195,7 @@ void column_sums(const Tensor& dy, const ParamGrad& out) {
     launches += 2;
 }
 
-// cuBLAS products with the weight gradient accumulated straight into its sink.
+// cuBLAS products with the weight gradient accumulated straight into its sink, if possible beside the rest of backward.
 struct Linear : torch::autograd::Function<Linear> {
     // bias_grad: computed here (else another operator returns it); report: this is the weight's last contribution
     static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const std::optional<Tensor>& bias,
@@ -220,13 +220,27 @@ struct Linear : torch::autograd::Function<Linear> {
         const int64_t flags = ctx->saved_data["flags"].toInt();
         const Tensor dy = rows_of(grads[0], grads[0].size(-1));
         Tensor dx, dw, db;
+        const bool beside = sinks[0] && sinks[0]->beside;
+        at::cuda::CUDAEvent ready; // dy is there
+        if (beside)
+            ready.record(at::cuda::getCurrentCUDAStream(dy.get_device()));
         if (ctx->needs_input_grad(0))
             dx = dy.mm(weight).view(ctx->saved_data["shape"].toIntVector());
         if (sinks[0]) {
-            if (sinks[0]->add())
-                sinks[0]->grad.addmm_(dy.t(), x2);
+            GradSink& s = *sinks[0];
+            const bool add = beside && s.on_side ? s.take() : s.add();
+            auto product = [&] {
+                if (add)
+                    s.grad.addmm_(dy.t(), x2);
+                else
+                    at::mm_out(s.grad, dy.t(), x2);
+            };
+            if (beside) {
+                s.beside->launch(ready, product, dy, x2);
+                s.on_side = true;
+            }
             else
-                at::mm_out(sinks[0]->grad, dy.t(), x2);
+                product();
         }
         else if (ctx->needs_input_grad(1))
             dw = dy.t().mm(x2);

@@ -5,11 +5,15 @@
 // ctypes, LayerNorm forward + backward took 125 to 190 us of host time around 42 us of kernels.
 #pragma once
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
 
 #include <atomic>
+#include <deque>
+#include <mutex>
 #include <optional>
 #include <stdexcept>
 #include <string>
@@ -101,6 +105,60 @@ inline Tensor empty_on(const Tensor& like, at::IntArrayRef sizes, at::ScalarType
     return at::detail::empty_cuda(sizes, dtype, like.device(), std::nullopt);
 }
 
+// A stream of their own for weight gradients that go to sinks: nothing else in backward waits for them, products of a few
+// hundred tokens leave most SMs idle, and a long product's last wave some.  One per DataParallel.
+//
+// The operands of a product must outlive it, but the allocator knows them as memory of the current stream: the last DEPTH
+// products' operands are kept, and the current stream waits for the oldest product before its operands go.
+class GradStream {
+public:
+    explicit GradStream(int dev) : stream_(at::cuda::getStreamFromPool(false, (c10::DeviceIndex)dev)) {}
+
+    // runs `product` there once what the current stream has done up to `ready` is done
+    template <class F>
+    void launch(at::cuda::CUDAEvent& ready, F&& product, const Tensor& a, const Tensor& b) {
+        const auto current = at::cuda::getCurrentCUDAStream(a.get_device());
+        std::lock_guard<std::mutex> g(mu_);
+        ready.block(stream_);
+        {
+            at::cuda::CUDAStreamGuard guard(stream_);
+            product();
+        }
+        held_.emplace_back();
+        held_.back().done.record(stream_);
+        held_.back().a = a;
+        held_.back().b = b;
+        if (held_.size() > DEPTH) {
+            held_.front().done.block(current);
+            held_.pop_front();
+        }
+    }
+    // `s` waits for everything launched since the last finish()
+    void join(at::cuda::CUDAStream s) {
+        std::lock_guard<std::mutex> g(mu_);
+        if (!held_.empty())
+            held_.back().done.block(s);
+    }
+    // the same for the current stream, at the end of a step
+    void finish() {
+        std::lock_guard<std::mutex> g(mu_);
+        if (!held_.empty())
+            held_.back().done.block(at::cuda::getCurrentCUDAStream(stream_.device_index()));
+        held_.clear();
+    }
+
+private:
+    static constexpr size_t DEPTH = 8; // two transformer blocks
+    struct entry {
+        at::cuda::CUDAEvent done;
+        Tensor a, b;
+    };
+    at::cuda::CUDAStream stream_;
+    std::deque<entry> held_;
+    std::mutex mu_;
+};
+typedef std::shared_ptr<GradStream> GradStreamRef;
+
 // Where a parameter's gradient goes when its layer accumulates it itself: a view of DataParallel's flat gradient.  `fresh`
 // says that the buffer still holds the last step's gradient, so that the first contribution overwrites it (a product with
 // beta = 0 instead of clearing the buffer and reading it back).  `callback` (no argument) does the bucket accounting;
@@ -109,6 +167,8 @@ struct GradSink {
     Tensor grad;
     PyObject* callback;
     bool fresh = false;
+    GradStreamRef beside; // set during a step that ends by finishing it: weight gradients may run there
+    bool on_side = false; // the last contribution did
     static std::atomic<int> live;
 
     GradSink(Tensor g, pybind11::object cb) : grad(std::move(g)), callback(cb.release().ptr()) {
@@ -121,8 +181,14 @@ struct GradSink {
             Py_XDECREF(callback);
         }
     }
-    // whether a contribution is added (or overwrites); from then on they are
+    // whether a contribution is added (or overwrites); from then on they are.  The current stream may write afterwards.
     bool add() {
+        if (on_side && beside)
+            beside->join(at::cuda::getCurrentCUDAStream(grad.get_device()));
+        on_side = false;
+        return take();
+    }
+    bool take() {
         const bool a = !fresh;
         fresh = false;
         return a;
