@@ -116,12 +116,19 @@ __device__ __forceinline__ void route_token(const float* __restrict__ row, int n
     unsigned long long taken = 0; // a bit per expert
     int best[ROUTE_MAX_TOPK];
     float val[ROUTE_MAX_TOPK];
-    float v[E > 0 ? E : 1];
+    __align__(16) float v[E > 0 ? E : 1];
     if constexpr (E > 0) {
+        if (n_experts == E && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
 #pragma unroll
-        for (int e = 0; e < E; e++)
-            if (e < n_experts)
-                v[e] = row[e];
+            for (int e = 0; e < E; e += 4)
+                *reinterpret_cast<float4*>(v + e) = *reinterpret_cast<const float4*>(row + e);
+        }
+        else {
+#pragma unroll
+            for (int e = 0; e < E; e++)
+                if (e < n_experts)
+                    v[e] = row[e];
+        }
     }
 #pragma unroll
     for (int s = 0; s < ROUTE_MAX_TOPK; s++) {
@@ -204,16 +211,9 @@ __global__ void __launch_bounds__(1024)
     for (int t = threadIdx.x; t < n_tokens; t += blockDim.x)
         route_token<E>(logits + (size_t)t * n_experts, n_experts, topk, idx + (size_t)t * topk, wts + (size_t)t * topk,
                        [&](int s, int e) {
-                        // lanes that chose the same expert draw their tickets together
-                        const unsigned peers = __match_any_sync(__activemask(), e);
-                        const int lead = __ffs(peers) - 1, lane = threadIdx.x & 31;
-                        unsigned base = 0;
-                        if (lane == lead)
-                            base = atomicAdd(&count[e], (unsigned)__popc(peers));
-                        base = __shfl_sync(peers, base, lead);
-                        ticket[t * topk + s] = (unsigned short)(base + __popc(peers & ((1u << lane) - 1)));
-                        expert[t * topk + s] = (unsigned char)e;
-                    });
+                           ticket[t * topk + s] = (unsigned short)atomicAdd(&count[e], 1u);
+                           expert[t * topk + s] = (unsigned char)e;
+                       });
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned acc = 0;
@@ -271,8 +271,8 @@ __global__ void __launch_bounds__(256)
 } // namespace
 
 // logits [n_tokens, n_experts] fp32 -> idx [n_tokens, topk] (int64), wts [n_tokens, topk] (fp32),
-// counts [n_experts] (int64), order / pos [n_tokens * topk] (int64).  scratch: n_experts 32-bit words; directly behind
-// `counts` it is cleared together with them.
+// counts [n_experts] (int64), order / pos [n_tokens * topk] (int64).  scratch: n_experts 32-bit words; behind
+// `counts` (at most one word between) it is cleared together with them.
 CCLX_API int cclx_moe_route(const float* logits, int n_tokens, int n_experts, int topk, long long* idx, float* wts,
                             long long* counts, long long* order, long long* pos, void* scratch, void* stream) {
     return cclx::capi::guard([&] {
@@ -288,8 +288,9 @@ CCLX_API int cclx_moe_route(const float* logits, int n_tokens, int n_experts, in
                                   (unsigned long long*)counts, order, pos);
             return;
         }
-        if (scratch == (void*)(counts + n_experts))
-            CUDA_CHECK(cudaMemsetAsync(counts, 0, (sizeof(long long) + sizeof(unsigned int)) * n_experts, st));
+        const ptrdiff_t gap = (const char*)scratch - (const char*)(counts + n_experts);
+        if (gap >= 0 && gap <= 8)
+            CUDA_CHECK(cudaMemsetAsync(counts, 0, (sizeof(long long) + sizeof(unsigned int)) * n_experts + gap, st));
         else {
             CUDA_CHECK(cudaMemsetAsync(counts, 0, sizeof(long long) * n_experts, st));
             CUDA_CHECK(cudaMemsetAsync(scratch, 0, sizeof(unsigned int) * n_experts, st));
@@ -353,6 +354,28 @@ struct moe_args {
     size_t cnt_off; // heap offset of the int32 table [blocks][W][W]
 };
 
+// The pieces of rows that a warp takes: warp, warp + nwarps, ... of row-major (row, piece) pairs, without a division per step.
+struct piece_walk {
+    size_t row;
+    int piece, pieces;
+    unsigned step_rows;
+    int step_pieces;
+    __device__ __forceinline__ piece_walk(unsigned warp, unsigned nwarps, int n) : pieces(n) {
+        row = warp / n;
+        piece = warp % n;
+        step_rows = nwarps / n;
+        step_pieces = nwarps % n;
+    }
+    __device__ __forceinline__ void next() {
+        row += step_rows;
+        piece += step_pieces;
+        if (piece >= pieces) {
+            piece -= pieces;
+            row++;
+        }
+    }
+};
+
 __global__ void __launch_bounds__(512) moe_dispatch_kernel(const comm_dev* tab, moe_args a) {
     const int er = a.emu ? (int)blockIdx.y : 0;
     const comm_dev& c = tab[er];
@@ -405,31 +428,35 @@ __global__ void __launch_bounds__(512) moe_dispatch_kernel(const comm_dev* tab, 
     if (blockIdx.x == 0 && threadIdx.x == 0)
         ra.meta[2 * W + 1] = s_over;
     if (ok && !s_over) {
-        // one warp per row, eight packs per lane in flight; the index of the warp's next row is fetched meanwhile
+        // A warp moves up to 256 packs of a row at a time, eight per lane in flight, and fetches the index of its next row
+        // meanwhile.  Pieces instead of rows: 2048 rows among 288 warps are 8 rounds for 7.1 rows each, their halves 15 for
+        // 14.2 (the last barrier waited 8 us for the slowest of 50).
         const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-        const size_t warp = (size_t)blockIdx.x * wpb + (threadIdx.x >> 5), nwarps = (size_t)gridDim.x * wpb;
+        const unsigned warp = blockIdx.x * wpb + (threadIdx.x >> 5), nwarps = gridDim.x * wpb;
         const int packs = a.hidden / 8;
-        long long item = warp < a.n_items ? ra.order[warp] : 0;
-        for (size_t i = warp; i < a.n_items; i += nwarps) {
+        piece_walk w(warp, nwarps, (packs + 255) / 256);
+        long long item = w.row < a.n_items ? ra.order[w.row] : 0;
+        while (w.row < a.n_items) {
+            const size_t i = w.row;
+            const int first = w.piece * 256 + lane;
             const uint4* src = reinterpret_cast<const uint4*>(ra.x + (size_t)((unsigned)item / (unsigned)a.topk) * a.hidden);
-            if (i + nwarps < a.n_items)
-                item = ra.order[i + nwarps];
+            w.next();
+            if (w.row < a.n_items)
+                item = ra.order[w.row];
             int e = 0;
             while (e + 1 < W && (long long)i >= s_pre[e + 1])
                 e++;
             const size_t row = (size_t)s_dst[e] + (i - (size_t)s_pre[e]);
             char* dst = c.heap[e] + a.buf_off + row * (size_t)a.hidden * 2;
-            for (int k0 = lane; k0 < packs; k0 += 256) {
-                uint4 v[8];
+            uint4 v[8];
 #pragma unroll
-                for (int k = 0; k < 8; k++)
-                    if (k0 + k * 32 < packs)
-                        v[k] = src[k0 + k * 32];
+            for (int k = 0; k < 8; k++)
+                if (first + k * 32 < packs)
+                    v[k] = src[first + k * 32];
 #pragma unroll
-                for (int k = 0; k < 8; k++)
-                    if (k0 + k * 32 < packs)
-                        st16(dst + (size_t)(k0 + k * 32) * 16, v[k]);
-            }
+            for (int k = 0; k < 8; k++)
+                if (first + k * 32 < packs)
+                    st16(dst + (size_t)(first + k * 32) * 16, v[k]);
         }
     }
     peer_barrier(c, s);

@@ -54,14 +54,17 @@ void allreduce(uintptr_t group, const tensors& send, const tensors& recv, int op
 pybind11::tuple route(const Tensor& logits_, int64_t topk) {
     const Tensor logits = logits_.scalar_type() == at::kFloat && logits_.is_contiguous() ? logits_ : logits_.to(at::kFloat).contiguous();
     const int64_t T = logits.size(0), E = logits.size(1);
-    const Tensor idx = empty_on(logits, { T, topk }, at::kLong), wts = empty_on(logits, { T, topk }, at::kFloat);
-    const Tensor counts = empty_on(logits, { E + (E + 1) / 2 }, at::kLong); // the placement cursors stand behind the counts
-    const Tensor order = empty_on(logits, { T * topk }, at::kLong), pos = empty_on(logits, { T * topk }, at::kLong);
-    long long* c = reinterpret_cast<long long*>(counts.data_ptr<int64_t>());
-    check(cclx_moe_route(logits.data_ptr<float>(), (int)T, (int)E, (int)topk, reinterpret_cast<long long*>(idx.data_ptr<int64_t>()),
-                         wts.data_ptr<float>(), c, reinterpret_cast<long long*>(order.data_ptr<int64_t>()),
-                         reinterpret_cast<long long*>(pos.data_ptr<int64_t>()), c + E, stream_of(logits)));
-    return pybind11::make_tuple(idx, wts, counts.narrow(0, 0, E), order, pos);
+    const int64_t n = T * topk, row = (E + 1) / 2 * 2; // 16-byte aligned parts: ids, order, places, weights, counts, cursors
+    const size_t w_at = 3 * 8 * n, c_at = w_at + (4 * n + 15) / 16 * 16;
+    const Tensor all = empty_on(logits, { (int64_t)c_at + 8 * row + 4 * E }, at::kByte);
+    char* base = static_cast<char*>(all.data_ptr());
+    long long* items = reinterpret_cast<long long*>(base);
+    long long* counts = reinterpret_cast<long long*>(base + c_at);
+    check(cclx_moe_route(logits.data_ptr<float>(), (int)T, (int)E, (int)topk, items, reinterpret_cast<float*>(base + w_at), counts,
+                         items + n, items + 2 * n, counts + row, stream_of(logits)));
+    return pybind11::make_tuple(part_of(all, 0, { T, topk }, at::kLong), part_of(all, w_at, { T, topk }, at::kFloat),
+                                part_of(all, c_at, { E }, at::kLong), part_of(all, 8 * n, { n }, at::kLong),
+                                part_of(all, 16 * n, { n }, at::kLong));
 }
 
 void dispatch(uintptr_t group, const tensors& x, const tensors& order, const tensors& counts, const tensors& meta, const Tensor& recv,

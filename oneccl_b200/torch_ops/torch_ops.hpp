@@ -68,6 +68,16 @@ namespace cclx_ops {
 
 using at::Tensor;
 
+// A contiguous tensor over bytes [offset, ...) of another's storage (offset a multiple of the element size), made without
+// the dispatcher: outputs of a small operator that are born together share one allocation.
+inline Tensor part_of(const Tensor& base, size_t offset, at::IntArrayRef sizes, at::ScalarType dtype) {
+    auto impl = c10::make_intrusive<c10::TensorImpl>(c10::Storage(base.storage()), c10::DispatchKeySet(c10::DispatchKey::CUDA),
+                                                     c10::scalarTypeToTypeMeta(dtype));
+    impl->set_storage_offset((int64_t)(offset / c10::elementSize(dtype)));
+    impl->set_sizes_contiguous(sizes);
+    return Tensor(std::move(impl));
+}
+
 // becomes oneccl_b200.CclError in Python
 struct ccl_error : std::runtime_error {
     using std::runtime_error::runtime_error;
