@@ -23,7 +23,7 @@ enum : uint32_t {
 };
 
 // words of comm_dev::state
-enum { STATE_EPOCH = 0, STATE_GEN = 1, STATE_DONE = 2, STATE_WORDS = 8 };
+enum { STATE_EPOCH = 0, STATE_GEN = 1, STATE_DONE = 2, STATE_LL = 3, STATE_WORDS = 8 };
 
 struct comm_dev {
     int rank;
@@ -36,15 +36,22 @@ struct comm_dev {
     uint32_t* mc_flags;
     uint32_t* p2p_flags[MAX_RANKS]; // point-to-point sequence words, peer-mapped
     uint32_t* aux[MAX_RANKS]; // auxiliary flag words (alltoallv round consensus, fused-GEMM tile flags), peer-mapped
+    char* ll[MAX_RANKS]; // packet areas of the small allreduce, peer-mapped: two generations of `world` slots each
     size_t heap_bytes;
     size_t staging_bytes; // one generation
-    uint32_t* state; // local device words: epoch, generation, finished-block counter
+    uint32_t* state; // local device words: epoch, generation, finished-block counter, packet sequence number
     uint32_t* p2p_seq; // local device words: per (direction, peer, lane) count of chunks moved so far
     volatile uint32_t* status; // host-mapped: [0] code, [1] block, [2] peer, [3] detail
     volatile uint32_t* abort_flag; // host-mapped, set by communicator abort
     unsigned long long timeout_ns;
 };
 
+
+// Small allreduce by packets (allreduce_packets_kernel): a slot holds one rank's message as 16-byte packets of 8 data
+// bytes each, and a header packet behind them.
+constexpr size_t LL_MAX_BYTES = 32u << 10; // largest message
+constexpr size_t LL_SLOT_BYTES = 2 * LL_MAX_BYTES + 256;
+constexpr size_t LL_HEADER = 2 * LL_MAX_BYTES; // offset of the header in a slot
 
 // point-to-point (see sendrecv_kernel): every ordered pair has P2P_LANES independent chains of chunks,
 // each with a ring of P2P_STAGES chunk buffers at the receiver and a pair of counters

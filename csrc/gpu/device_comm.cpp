@@ -65,18 +65,16 @@ void device_comm::build_tables() {
     const int entries = emulated_ ? world_ : 1;
     const heap_regions& R = heap_.regions();
 
-    // one device and one pinned allocation: state words, point-to-point counters and (emulation) argument tables;
-    // status words and the tables' host side
+    // one device allocation: state words, point-to-point counters and (emulation) argument tables
     const size_t words = (size_t)entries * (dev::STATE_WORDS + dev::P2P_SEQ_WORDS);
-    const size_t emu_bytes = emulated_ ? EMU_SLOTS * EMU_SLOT_BYTES : 0, words_bytes = (words * sizeof(uint32_t) + 255) / 256 * 256;
+    const size_t emu_bytes = emulated_ ? EMU_KINDS * emu_slot_bytes() : 0, words_bytes = (words * sizeof(uint32_t) + 255) / 256 * 256;
     CUDA_CHECK(cudaMalloc((void**)&state_dev_, words_bytes + emu_bytes));
     CUDA_CHECK(cudaMemset(state_dev_, 0, words_bytes));
     p2p_seq_dev_ = state_dev_ + entries * dev::STATE_WORDS;
     emu_dev_ = (char*)state_dev_ + words_bytes;
-    const size_t status_words = (size_t)entries * 8 + 8, status_bytes = (status_words * sizeof(uint32_t) + 255) / 256 * 256;
-    CUDA_CHECK(cudaHostAlloc((void**)&status_host_, status_bytes + emu_bytes, cudaHostAllocMapped));
+    const size_t status_words = (size_t)entries * 8 + 8;
+    CUDA_CHECK(cudaHostAlloc((void**)&status_host_, status_words * sizeof(uint32_t), cudaHostAllocMapped));
     std::memset(status_host_, 0, status_words * sizeof(uint32_t));
-    emu_host_ = (char*)status_host_ + status_bytes;
     CUDA_CHECK(cudaHostGetDevicePointer((void**)&status_devptr_, status_host_, 0));
     device_id_ = devid;
 
@@ -91,6 +89,7 @@ void device_comm::build_tables() {
             c.p2p_flags[p] = (uint32_t*)(b + R.p2p_flags_off);
             c.staging[p] = b + R.staging_off;
             c.aux[p] = (uint32_t*)(b + R.aux_flags_off);
+            c.ll[p] = b + R.ll_off;
             c.heap[p] = b;
         }
         c.mc_heap = heap_.mc_base();
@@ -141,7 +140,7 @@ void device_comm::destroy() {
     cudaFree(table_dev_);
     table_dev_ = nullptr;
     cudaFree(state_dev_);
-    emu_dev_ = emu_host_ = nullptr;
+    emu_dev_ = nullptr;
     cudaFreeHost(status_host_);
     state_dev_ = p2p_seq_dev_ = nullptr;
     status_host_ = nullptr;
@@ -149,26 +148,19 @@ void device_comm::destroy() {
 }
 
 const void* device_comm::emu_table(int kind, const void* data, size_t bytes, cudaStream_t st) {
-    CCL_THROW_IF_NOT(emulated_ && bytes <= EMU_SLOT_BYTES, "argument table of ", bytes, " bytes");
+    CCL_THROW_IF_NOT(emulated_ && bytes <= emu_slot_bytes(), "argument table of ", bytes, " bytes");
     cudaStreamCaptureStatus capturing;
     CUDA_CHECK(cudaStreamIsCapturing(st, &capturing));
     CCL_THROW_IF_NOT(capturing == cudaStreamCaptureStatusNone, "launches of several emulated ranks cannot be captured");
     std::lock_guard<std::mutex> g(emu_mu_);
-    emu_last& l = emu_last_[kind];
-    if (l.slot >= 0 && l.bytes == bytes && l.stream == st && std::memcmp(emu_host_ + l.slot * EMU_SLOT_BYTES, data, bytes) == 0)
-        return emu_dev_ + l.slot * EMU_SLOT_BYTES;
-    const int slot = emu_next_++ % EMU_SLOTS;
-    if (slot == 0 && emu_next_ > 1) { // earlier launches may still read their tables
-        CUDA_CHECK(cudaDeviceSynchronize());
-        for (auto& x : emu_last_)
-            x = emu_last();
+    char* dst = emu_dev_ + kind * emu_slot_bytes();
+    std::vector<char>& last = emu_last_[kind];
+    if (last.size() != bytes || emu_stream_[kind] != st || std::memcmp(last.data(), data, bytes) != 0) {
+        last.assign((const char*)data, (const char*)data + bytes);
+        emu_stream_[kind] = st;
+        CUDA_CHECK(cudaMemcpyAsync(dst, last.data(), bytes, cudaMemcpyHostToDevice, st));
     }
-    std::memcpy(emu_host_ + slot * EMU_SLOT_BYTES, data, bytes);
-    CUDA_CHECK(cudaMemcpyAsync(emu_dev_ + slot * EMU_SLOT_BYTES, emu_host_ + slot * EMU_SLOT_BYTES, bytes, cudaMemcpyHostToDevice, st));
-    l.slot = slot;
-    l.bytes = bytes;
-    l.stream = st;
-    return emu_dev_ + slot * EMU_SLOT_BYTES;
+    return dst;
 }
 
 int device_comm::max_blocks() const {

@@ -66,8 +66,8 @@ public:
     int max_blocks() const; // per rank, keeps every block co-resident
     int threads() const { return threads_; }
     // Emulation: the per-rank argument table of a launch in device memory.  `kind` names the table's layout.  A table equal
-    // to the last one of its kind on this stream is still there; another is copied from a pinned ring, in stream order.
-    // The host waits only when the ring comes round.
+    // to the last one of its kind is still there; another one is copied over it in stream order (operations of one
+    // communicator are ordered among themselves).  No host wait: the runtime takes a small pageable source at once.
     enum { EMU_COLL = 0, EMU_P2P = 1, EMU_MOE = 2, EMU_KINDS = 3 };
     const void* emu_table(int kind, const void* data, size_t bytes, cudaStream_t st);
     int device_id() const { return device_id_; }
@@ -145,17 +145,12 @@ private:
     uint32_t* p2p_seq_dev_ = nullptr;
     uint32_t* status_host_ = nullptr; // pinned + mapped: per rank 8 words, then abort word
     uint32_t* status_devptr_ = nullptr;
-    static constexpr int EMU_SLOTS = 32;
-    static constexpr size_t EMU_SLOT_BYTES = dev::MAX_RANKS * (sizeof(dev::rank_args) > sizeof(dev::p2p_ops) ? sizeof(dev::rank_args)
-                                                                                                             : sizeof(dev::p2p_ops));
-    char* emu_dev_ = nullptr; // EMU_SLOTS tables, part of the allocation at state_dev_
-    char* emu_host_ = nullptr; // pinned, the same layout, part of the allocation at status_host_
-    int emu_next_ = 0;
-    struct emu_last {
-        int slot = -1;
-        size_t bytes = 0;
-        cudaStream_t stream = nullptr;
-    } emu_last_[EMU_KINDS];
+    size_t emu_slot_bytes() const {
+        return (size_t)world_ * (sizeof(dev::rank_args) > sizeof(dev::p2p_ops) ? sizeof(dev::rank_args) : sizeof(dev::p2p_ops));
+    }
+    char* emu_dev_ = nullptr; // a table per kind, part of the allocation at state_dev_
+    std::vector<char> emu_last_[EMU_KINDS]; // what they hold
+    cudaStream_t emu_stream_[EMU_KINDS] = {}; // and in whose order it was written
     std::mutex emu_mu_;
     int device_id_ = 0;
     int sm_count_ = 0;

@@ -207,6 +207,16 @@ void launch_allreduce(device_comm& dc, const dev::rank_args* ra, size_t count, i
             a.count = count;
             a.flags = algo == ga_nvls_oneshot ? dev::CF_NVLS : 0;
             prepare_args(dc, a, ra, st);
+            // Packets carry their own flags but double the traffic: faster than data and a barrier up to LL_MAX_BYTES.
+            // The choice rests on values that are the same on every rank.
+            if (algo == ga_oneshot && bytes <= dev::LL_MAX_BYTES) {
+                const int blocks = pick_blocks(dc, (bytes + 7) / 8, 512, o.blocks);
+                dispatch_reduce_types(dt_in, dt_out, op, [&](auto tin, auto tout, auto opv) {
+                    launch_kernel(dc, dev::allreduce_packets_kernel<decltype(tin), decltype(tout), decltype(opv)>, blocks,
+                                  512, st, dc.table(), a);
+                });
+                return;
+            }
             const int blocks = pick_blocks(dc, slot / 16, 512, o.blocks); // one pack per thread: latency, not throughput, counts here
             dispatch_reduce_types(dt_in, dt_out, op, [&](auto tin, auto tout, auto opv) {
                 launch_kernel(dc, dev::allreduce_oneshot_kernel<decltype(tin), decltype(tout), decltype(opv)>, blocks,

@@ -36,14 +36,17 @@ heap_regions plan_regions(int world, size_t heap_bytes, size_t staging_bytes, si
     r.p2p_slot_bytes = dev::P2P_SLOT_BYTES;
     r.p2p_data_off = off;
     off += (size_t)world * r.p2p_slot_bytes;
+    r.ll_off = off;
+    const size_t ll_bytes = round_up(2 * (size_t)world * dev::LL_SLOT_BYTES, 1u << 20);
+    off += ll_bytes;
     off = round_up(off, 1u << 20);
     r.staging_off = off;
     r.staging_bytes = round_up(staging_bytes, 4096);
     off += 2 * r.staging_bytes;
     off = round_up(off, 1u << 20);
     r.user_off = off;
-    // the requested size covers flags, staging and the user part; the point-to-point slots come on top
-    r.total = round_up(std::max(off + (1u << 20), heap_bytes + (size_t)world * r.p2p_slot_bytes), granularity);
+    // the requested size covers flags, staging and the user part; the point-to-point and packet slots come on top
+    r.total = round_up(std::max(off + (1u << 20), heap_bytes + (size_t)world * r.p2p_slot_bytes + ll_bytes), granularity);
     return r;
 }
 

@@ -42,6 +42,7 @@ struct heap_regions {
     size_t aux_flags_bytes = 0;
     size_t p2p_data_off = 0;
     size_t p2p_slot_bytes = 0;
+    size_t ll_off = 0; // packets of the small allreduce
     size_t staging_off = 0;
     size_t staging_bytes = 0; // one generation
     size_t user_off = 0;

@@ -234,8 +234,8 @@ def test_moe_dispatch_and_combine_shapes(W, T, H, k):
     group.close()
 
 
-def test_emulated_argument_tables_wrap_around():
-    """More different argument tables than the ring holds, on two streams."""
+def test_emulated_argument_tables_follow_the_calls():
+    """Many different argument tables in a row, on two streams."""
     from oneccl_b200.ops.device_group import DeviceGroup
 
     group = DeviceGroup.emulated(2, heap_bytes=40 << 20, staging_bytes=1 << 20)
@@ -252,4 +252,45 @@ def test_emulated_argument_tables_wrap_around():
     group.check()
     for i, pair in enumerate(xs):
         assert all(bool((t == 2 * i + 1).all()) for t in pair), i
+    group.close()
+
+
+@pytest.mark.parametrize("W", [2, 3, 4, 8])
+@pytest.mark.parametrize("dtype,out_dtype", [(torch.float32, None), (torch.bfloat16, torch.float32), (torch.float32, torch.bfloat16),
+                                             (torch.int8, None), (torch.float64, None), (torch.int64, None)])
+def test_small_allreduce_packets(W, dtype, out_dtype):
+    """One element up to the largest message of the packet kernel and one more (which takes staging and a barrier),
+    remainders of a packet, unaligned buffers; alternating with other collectives."""
+    from oneccl_b200.ops.device_group import DeviceGroup
+
+    group = DeviceGroup.emulated(W, heap_bytes=40 << 20, staging_bytes=1 << 20)
+    group.set_timeout_ms(1000)
+    g = torch.Generator(device="cuda").manual_seed(W)
+    top = (32 << 10) // torch.empty((), dtype=dtype).element_size()
+    for n in (1, 2, 3, 7, 8, 1027, top - 1, top, top + 1):
+        for off in (0, 1):
+            x = [torch.randint(-8, 8, (n + off,), generator=g, device="cuda").to(dtype)[off:] for _ in range(W)]
+            y = [torch.zeros(n + off, dtype=out_dtype or dtype, device="cuda")[off:] for _ in range(W)]
+            group.allreduce(x, y, algo="oneshot")
+            if n == 8:
+                group.barrier()
+            want = sum(t.double() for t in x)
+            torch.cuda.synchronize()
+            group.check()
+            assert all(torch.equal(t.double(), want) for t in y), (n, off)
+    x = [torch.full((9,), float(r), device="cuda") for r in range(W)]
+    group.allreduce(x, x, scale=0.5)
+    torch.cuda.synchronize()
+    assert all(bool((t == W * (W - 1) / 4).all()) for t in x)
+    # a rank whose arguments differ
+    group.test_sig_skew(W - 1)
+    group.allreduce(x, x, algo="oneshot")
+    torch.cuda.synchronize()
+    assert {group.status(r) for r in range(W)} == {7}
+    group.test_sig_skew(-1)
+    group.clear_status()
+    x = [torch.ones(70, device="cuda") for _ in range(W)]
+    group.allreduce(x, x, algo="oneshot")
+    torch.cuda.synchronize()
+    assert all(bool((t == W).all()) for t in x)
     group.close()
