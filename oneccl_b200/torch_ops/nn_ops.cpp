@@ -6,6 +6,9 @@
 // does not need and returns its gradient; `linear` is then called with defer_bias.
 #include "torch_ops.hpp"
 
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+
 namespace cclx_ops {
 namespace {
 
@@ -16,6 +19,12 @@ using torch::autograd::variable_list;
 Tensor rows_of(const Tensor& t, int64_t D) {
     Tensor r = t.dim() == 2 ? t : t.reshape({ -1, D });
     r = r.is_contiguous() ? r : r.contiguous();
+    return aligned16(r) ? r : r.clone();
+}
+
+// the same elements contiguous and 16-byte aligned
+Tensor dense(const Tensor& t) {
+    const Tensor r = t.is_contiguous() ? t : t.contiguous();
     return aligned16(r) ? r : r.clone();
 }
 
@@ -44,13 +53,14 @@ struct ParamGrad {
     Tensor out;
     bool add = false;
 
-    ParamGrad(const SinkRef& s, const Tensor& like, at::IntArrayRef shape) : sink(s) {
+    // `room`: where the gradient goes if there is no sink (allocated if undefined)
+    ParamGrad(const SinkRef& s, const Tensor& like, at::IntArrayRef shape, Tensor room = Tensor()) : sink(s) {
         if (s) {
             out = s->grad;
             add = s->add();
         }
         else
-            out = empty_on(like, shape, at::kBFloat16);
+            out = room.defined() ? std::move(room) : empty_on(like, shape, at::kBFloat16);
     }
     void* ptr() const {
         return out.data_ptr();
@@ -75,63 +85,55 @@ std::vector<SinkRef> sinks_of(AutogradContext* ctx, size_t n) {
     return c10::static_intrusive_pointer_cast<Sinks>(it->second.toCapsule())->s;
 }
 
-struct AddLayerNorm : torch::autograd::Function<AddLayerNorm> {
-    // res_bias: bias of the linear layer that produced `res`
-    static variable_list forward(AutogradContext* ctx, const Tensor& x, const std::optional<Tensor>& res, const Tensor& weight,
-                                 const Tensor& bias, double eps, const std::optional<Tensor>& res_bias, std::vector<SinkRef> sinks) {
-        const int64_t D = x.size(-1);
-        const Tensor x2 = rows_of(x, D);
-        const int64_t rows = x2.size(0);
-        void* st = stream_of(x2);
-        const Tensor y = empty_on(x2, x2.sizes(), at::kBFloat16);
-        const Tensor stats = empty_on(x2, { 2, rows }, at::kFloat); // mean, 1 / standard deviation
-        float* mean = stats.data_ptr<float>();
-        Tensor total = x2;
-        if (res) {
-            const Tensor r2 = rows_of(*res, D);
-            total = empty_on(x2, x2.sizes(), at::kBFloat16);
-            check(cclx_layer_norm_fwd(x2.data_ptr(), r2.data_ptr(), weight.data_ptr(), bias.data_ptr(), y.data_ptr(),
-                                      total.data_ptr(), mean, mean + rows, rows, (int)D, (float)eps, st));
-        }
-        else
-            check(cclx_layer_norm_fwd(x2.data_ptr(), nullptr, weight.data_ptr(), bias.data_ptr(), y.data_ptr(), nullptr,
-                                      mean, mean + rows, rows, (int)D, (float)eps, st));
-        launches += 1;
-        ctx->save_for_backward({ total, weight, stats, res_bias ? *res_bias : Tensor() });
-        keep_sinks(ctx, std::move(sinks));
-        ctx->set_materialize_grads(false); // an unused output costs no zero tensor
-        if (res)
-            return { shaped(y, x.sizes()), shaped(total, x.sizes()) };
-        return { shaped(y, x.sizes()) };
-    }
+// Written as a plain autograd node: the wrapper of torch::autograd::Function costs several microseconds each way.
+struct AddLayerNormBackward : torch::autograd::Node {
+    torch::autograd::SavedVariable total, weight;
+    Tensor stats; // mean, 1 / standard deviation
+    std::vector<SinkRef> sinks;
+    bool has_res = false, has_res_bias = false;
 
-    static variable_list backward(AutogradContext* ctx, variable_list grads) {
-        const auto saved = ctx->get_saved_variables();
-        const Tensor &total = saved[0], &weight = saved[1], &stats = saved[2];
-        const int64_t rows = total.size(0), D = total.size(1);
-        const bool has_res = grads.size() == 2; // as many as forward had outputs
+    std::string name() const override {
+        return "AddLayerNormBackward";
+    }
+    void release_variables() override {
+        std::lock_guard<std::mutex> g(mutex_);
+        total.reset_data();
+        weight.reset_data();
+        stats.reset();
+    }
+    // gradients of x, the residual, gamma, beta and the bias of the linear layer that produced the residual
+    variable_list apply(variable_list&& grads) override {
+        std::lock_guard<std::mutex> g(mutex_);
         Tensor dsum = has_res ? grads[1] : Tensor();
         if (!grads[0].defined() && !dsum.defined())
-            return variable_list(7);
-        const Tensor dy = grads[0].defined() ? rows_of(grads[0], D) : at::zeros_like(total);
+            return variable_list(5);
+        at::AutoDispatchBelowADInplaceOrView below;
+        const Tensor t = total.unpack(shared_from_this()), w = weight.unpack();
+        TORCH_CHECK(stats.defined(), "LayerNorm's saved tensors have been freed: backward ran through the graph a second time");
+        const auto shape = t.sizes();
+        const int64_t D = shape.back(), rows = t.numel() / std::max<int64_t>(D, 1);
+        const Tensor dy = grads[0].defined() ? dense(grads[0]) : at::zeros_like(t);
         if (dsum.defined())
-            dsum = rows_of(dsum, D);
-        void* st = stream_of(total);
-        const Tensor dx = empty_on(total, total.sizes(), at::kBFloat16);
-        const auto sinks = sinks_of(ctx, 3);
-        const ParamGrad dg(sinks[0], total, weight.sizes()), db(sinks[1], total, weight.sizes());
+            dsum = dense(dsum);
+        void* st = stream_of(t);
+        const Tensor dx = empty_on(t, shape, at::kBFloat16);
+        const int64_t wide[] = { D };
+        const bool own = !sinks[0] && !sinks[1];
+        const Tensor both = own ? empty_on(t, { 2 * D }, at::kBFloat16) : Tensor(); // gamma's and beta's gradients are born together
+        const ParamGrad dg(sinks[0], t, wide, own ? part_of(both, 0, wide, at::kBFloat16) : Tensor());
+        const ParamGrad db(sinks[1], t, wide, own ? part_of(both, 2 * D, wide, at::kBFloat16) : Tensor());
         std::optional<ParamGrad> dr;
-        if (saved[3].defined())
-            dr.emplace(sinks[2], total, weight.sizes());
+        if (has_res_bias)
+            dr.emplace(sinks[2], t, wide);
         if (rows == 0) {
             dg.nothing();
             db.nothing();
             if (dr)
                 dr->nothing();
         }
-        const Tensor ws = empty_on(total, { (int64_t)cclx_layer_norm_bwd_blocks(rows) * (dr ? 3 : 2) * D }, at::kFloat);
+        const Tensor ws = empty_on(t, { (int64_t)cclx_layer_norm_bwd_blocks(rows) * (dr ? 3 : 2) * D }, at::kFloat);
         const float* mean = stats.data_ptr<float>();
-        check(cclx_layer_norm_bwd_sums(dy.data_ptr(), total.data_ptr(), weight.data_ptr(), mean, mean + rows,
+        check(cclx_layer_norm_bwd_sums(dy.data_ptr(), t.data_ptr(), w.data_ptr(), mean, mean + rows,
                                        dsum.defined() ? dsum.data_ptr() : nullptr, dx.data_ptr(), dg.ptr(), db.ptr(),
                                        dr ? dr->ptr() : nullptr, (dg.add ? 1 : 0) | (db.add ? 2 : 0) | (dr && dr->add ? 4 : 0),
                                        ws.data_ptr<float>(), rows, (int)D, st));
@@ -140,11 +142,49 @@ struct AddLayerNorm : torch::autograd::Function<AddLayerNorm> {
         db.done();
         if (dr)
             dr->done();
-        const auto shape = grads[0].defined() ? grads[0].sizes() : grads[1].sizes();
-        const Tensor d = shaped(dx, shape);
-        return { d, has_res ? d : Tensor(), dg.result(), db.result(), Tensor(), dr ? dr->result() : Tensor(), Tensor() };
+        return { dx, has_res ? dx : Tensor(), dg.result(), db.result(), dr ? dr->result() : Tensor() };
     }
 };
+
+// {LayerNorm(x + res), x + res}; res_bias: bias of the linear layer that produced `res`
+variable_list add_layer_norm_fwd(const Tensor& x, const std::optional<Tensor>& res, const Tensor& weight, const Tensor& bias,
+                                 double eps, const std::optional<Tensor>& res_bias, std::vector<SinkRef> sinks) {
+    const Tensor none;
+    const Tensor &r = res ? *res : none, &rb = res_bias ? *res_bias : none;
+    const bool grad = torch::autograd::compute_requires_grad(x, r, weight, bias, rb);
+    Tensor xd, y, total, stats;
+    {
+        at::AutoDispatchBelowADInplaceOrView below;
+        xd = dense(x);
+        const int64_t D = xd.size(-1), rows = xd.numel() / D;
+        void* st = stream_of(xd);
+        y = empty_on(xd, xd.sizes(), at::kBFloat16);
+        stats = empty_on(xd, { 2, rows }, at::kFloat);
+        float* mean = stats.data_ptr<float>();
+        const Tensor rd = res ? dense(r) : none;
+        if (res)
+            total = empty_on(xd, xd.sizes(), at::kBFloat16);
+        check(cclx_layer_norm_fwd(xd.data_ptr(), res ? rd.data_ptr() : nullptr, weight.data_ptr(), bias.data_ptr(), y.data_ptr(),
+                                  res ? total.data_ptr() : nullptr, mean, mean + rows, rows, (int)D, (float)eps, st));
+        launches += 1;
+    }
+    if (grad) {
+        std::shared_ptr<AddLayerNormBackward> node(new AddLayerNormBackward(), torch::autograd::deleteNode);
+        node->set_next_edges(torch::autograd::collect_next_edges(x, r, weight, bias, rb));
+        node->stats = stats;
+        node->sinks = std::move(sinks);
+        node->has_res = res.has_value();
+        node->has_res_bias = res_bias.has_value();
+        torch::autograd::set_history(y, node);
+        if (res)
+            torch::autograd::set_history(total, node);
+        node->total = res ? torch::autograd::SavedVariable(total, true) : torch::autograd::SavedVariable(xd, false);
+        node->weight = torch::autograd::SavedVariable(weight, false);
+    }
+    if (res)
+        return { y, total };
+    return { y };
+}
 
 bool ln_param_ok(const Tensor& p, int64_t D) {
     return p.scalar_type() == at::kBFloat16 && p.is_cuda() && p.numel() == D && p.is_contiguous() && aligned16(p);
@@ -178,7 +218,7 @@ pybind11::object add_layer_norm(const Tensor& x, const std::optional<Tensor>& re
     variable_list out;
     {
         pybind11::gil_scoped_release nogil;
-        out = AddLayerNorm::apply(x, res, w, b, eps, res_bias, std::move(sinks));
+        out = add_layer_norm_fwd(x, res, w, b, eps, res_bias, std::move(sinks));
     }
     if (res)
         return pybind11::make_tuple(out[0], out[1]);

@@ -1,44 +1,61 @@
 // Mean softmax cross-entropy whose logits become their own gradient (kernels: csrc/gpu/train_kernels.cu).
 #include "torch_ops.hpp"
 
+#include <torch/csrc/autograd/functions/utils.h>
+
 namespace cclx_ops {
 namespace {
 
-using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
-struct SoftmaxXent : torch::autograd::Function<SoftmaxXent> {
-    static variable_list forward(AutogradContext* ctx, const Tensor& logits, const Tensor& targets, int64_t vocab, bool scale) {
-        const int64_t rows = logits.size(0), cols = logits.size(1);
+struct SoftmaxXentBackward : torch::autograd::Node {
+    Tensor grad; // the logits' memory, which holds their gradient
+    bool scale = false;
+
+    std::string name() const override {
+        return "SoftmaxXentBackward";
+    }
+    void release_variables() override {
+        std::lock_guard<std::mutex> g(mutex_);
+        grad.reset();
+    }
+    variable_list apply(variable_list&& grads) override {
+        std::lock_guard<std::mutex> g(mutex_);
+        if (!grads[0].defined())
+            return { Tensor() };
+        TORCH_CHECK(grad.defined(), "the logits' gradient has been freed: backward ran through the graph a second time");
+        // the stored gradient assumes d(loss) = 1; scale only when the caller scaled the loss
+        return { scale ? grad * grads[0].to(grad.scalar_type()) : grad };
+    }
+};
+
+Tensor softmax_xent(const Tensor& logits, const Tensor& targets_, int64_t vocab, bool scale) {
+    TORCH_CHECK(logits.is_cuda() && targets_.is_cuda(), "the fused cross-entropy takes CUDA tensors");
+    pybind11::gil_scoped_release nogil;
+    const Tensor targets = targets_.is_contiguous() ? targets_ : targets_.contiguous();
+    const int64_t rows = logits.size(0), cols = logits.size(1);
+    Tensor mean;
+    if (rows == 0) // the mean of nothing
+        mean = at::full({}, std::numeric_limits<float>::quiet_NaN(), logits.options().dtype(at::kFloat).requires_grad(false));
+    else {
+        void* st = stream_of(logits);
+        const Tensor losses = empty_on(logits, { rows }, at::kFloat);
+        mean = empty_on(logits, {}, at::kFloat);
         // autograd is not told about the in-place write: the producer of `logits` (a matmul) does not need its output
         // for its own backward
-        ctx->save_for_backward({ logits });
-        ctx->saved_data["scale"] = scale;
-        if (rows == 0) // the mean of nothing
-            return { at::full({}, std::numeric_limits<float>::quiet_NaN(), logits.options().dtype(at::kFloat)) };
-        void* st = stream_of(logits);
-        const Tensor losses = empty_on(logits, { rows }, at::kFloat), mean = empty_on(logits, {}, at::kFloat);
         check(cclx_softmax_xent_mean(logits.data_ptr(), reinterpret_cast<const long long*>(targets.data_ptr<int64_t>()),
                                      losses.data_ptr<float>(), mean.data_ptr<float>(), rows, (int)vocab, logits.stride(0),
                                      1.0f / (float)rows, (int)(cols - vocab), st));
         launches += 2;
-        return { mean };
     }
-
-    static variable_list backward(AutogradContext* ctx, variable_list grads) {
-        Tensor g = ctx->get_saved_variables()[0];
-        // the stored gradient assumes d(loss) = 1; scale only when the caller scaled the loss
-        if (grads[0].defined() && ctx->saved_data["scale"].toBool())
-            g = g * grads[0].to(g.scalar_type());
-        return { g, Tensor(), Tensor(), Tensor() };
+    if (torch::autograd::compute_requires_grad(logits)) {
+        std::shared_ptr<SoftmaxXentBackward> node(new SoftmaxXentBackward(), torch::autograd::deleteNode);
+        node->set_next_edges(torch::autograd::collect_next_edges(logits));
+        node->grad = logits.detach();
+        node->scale = scale;
+        torch::autograd::set_history(mean, node);
     }
-};
-
-Tensor softmax_xent(const Tensor& logits, const Tensor& targets, int64_t vocab, bool scale) {
-    TORCH_CHECK(logits.is_cuda() && targets.is_cuda(), "the fused cross-entropy takes CUDA tensors");
-    const Tensor t = targets.is_contiguous() ? targets : targets.contiguous();
-    pybind11::gil_scoped_release nogil;
-    return SoftmaxXent::apply(logits, t, vocab, scale)[0];
+    return mean;
 }
 
 // one step of the flat AdamW: clipping norm (max_norm > 0) and update
