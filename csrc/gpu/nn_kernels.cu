@@ -560,10 +560,11 @@ int launch_ln_bwd(const void* dy, const void* x, const void* w, const float* mea
 
 // workspace: fp32 [cclx_layer_norm_bwd_blocks(rows) * (dxsum ? 3 : 2) * D].  dres may be null.  dxsum (optional): column
 // sums of dx, the bias gradient of the linear layer whose output the residual addition took.  `add`: bits 0 to 2
-// say which of dgamma, dbeta and dxsum are added to what the outputs hold.
+// say which of dgamma, dbeta and dxsum are added to what the outputs hold.  `defer` (optional) receives the number of
+// partial rows in `workspace` instead: the caller sums them with cclx_partial_sums, on another stream for instance.
 CCLX_API int cclx_layer_norm_bwd_sums(const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
                                       const void* dres, void* dx, void* dgamma, void* dbeta, void* dxsum, int add,
-                                      float* workspace, size_t rows, int D, void* stream) {
+                                      float* workspace, size_t rows, int D, int* defer, void* stream) {
     return cclx::capi::guard([&] {
         CCL_THROW_IF_NOT(D % 8 == 0 && D >= 8 && D <= 2048, "fused LayerNorm supports multiples of 8 up to 2048 columns");
         if (rows == 0)
@@ -579,6 +580,10 @@ CCLX_API int cclx_layer_norm_bwd_sums(const void* dy, const void* x, const void*
         else
             n = wide ? launch_ln_bwd<LN_BWD_ROWS, false>(dy, x, w, mean, rstd, dres, dx, workspace, rows, D, st)
                      : launch_ln_bwd<1, false>(dy, x, w, mean, rstd, dres, dx, workspace, rows, D, st);
+        if (defer) {
+            *defer = n;
+            return;
+        }
         partial_outs o{ { (__nv_bfloat16*)dgamma, (__nv_bfloat16*)dbeta, (__nv_bfloat16*)dxsum }, add };
         launch_dependent(partial_rows_sum_kernel, dim3((D + 31) / 32, dxsum ? 3 : 2), dim3(256), 0, st,
                               (const float*)workspace, n, D, o);
@@ -588,7 +593,7 @@ CCLX_API int cclx_layer_norm_bwd_sums(const void* dy, const void* x, const void*
 CCLX_API int cclx_layer_norm_bwd(const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
                                  const void* dres, void* dx, void* dgamma, void* dbeta, float* workspace, size_t rows, int D,
                                  void* stream) {
-    return cclx_layer_norm_bwd_sums(dy, x, w, mean, rstd, dres, dx, dgamma, dbeta, nullptr, 0, workspace, rows, D, stream);
+    return cclx_layer_norm_bwd_sums(dy, x, w, mean, rstd, dres, dx, dgamma, dbeta, nullptr, 0, workspace, rows, D, nullptr, stream);
 }
 
 namespace {
@@ -600,16 +605,32 @@ int map_rows_per_block(size_t rows, int packs) {
 }
 
 template <class F>
-void launch_map_colsum(const F& f, size_t rows, int packs, void* colsum, int add, float* workspace, cudaStream_t st) {
+void launch_map_colsum(const F& f, size_t rows, int packs, void* colsum, int add, float* workspace, int* defer, cudaStream_t st) {
     const int rpb = map_rows_per_block(rows, packs);
     const int n = (int)((rows + rpb - 1) / rpb);
     map_colsum_kernel<F><<<dim3((packs + 127) / 128, n), 128, 0, st>>>(f, rows, packs, rpb, workspace);
     CUDA_CHECK(cudaGetLastError());
+    if (defer) {
+        *defer = n;
+        return;
+    }
     partial_outs o{ { (__nv_bfloat16*)colsum, nullptr, nullptr }, add };
     launch_dependent(partial_rows_sum_kernel, dim3((packs * 8 + 31) / 32, 1), dim3(256), 0, st, (const float*)workspace, n,
                      packs * 8, o);
 }
 } // namespace
+
+// The sums that an entry point deferred: `n` partial rows of `outputs` (1 to 3) times `cols` floats; bit i of `add`: add to
+// what output i holds.
+CCLX_API int cclx_partial_sums(const float* workspace, int n, int cols, int outputs, void* out0, void* out1, void* out2, int add,
+                               void* stream) {
+    return cclx::capi::guard([&] {
+        CCL_THROW_IF_NOT(outputs >= 1 && outputs <= 3, "one to three outputs");
+        partial_outs o{ { (__nv_bfloat16*)out0, (__nv_bfloat16*)out1, (__nv_bfloat16*)out2 }, add };
+        partial_rows_sum_kernel<<<dim3((cols + 31) / 32, outputs), 256, 0, (cudaStream_t)stream>>>(workspace, n, cols, o);
+        CUDA_CHECK(cudaGetLastError());
+    });
+}
 
 // floats of workspace that the entry points below need for a result of [rows, N]
 CCLX_API size_t cclx_map_colsum_workspace(size_t rows, int N) {
@@ -623,7 +644,7 @@ CCLX_API int cclx_colsum(const void* x, void* out, int add, float* workspace, si
         CCL_THROW_IF_NOT(N % 8 == 0, "column count must be a multiple of 8");
         if (rows == 0 || N == 0)
             return;
-        launch_map_colsum(sum_map{ (const uint4*)x, N / 8 }, rows, N / 8, out, add, workspace, (cudaStream_t)stream);
+        launch_map_colsum(sum_map{ (const uint4*)x, N / 8 }, rows, N / 8, out, add, workspace, nullptr, (cudaStream_t)stream);
     });
 }
 
@@ -639,20 +660,20 @@ CCLX_API int cclx_gelu_fwd(const void* x, void* y, size_t n, void* stream) {
 
 // dx = dy * gelu'(x) over [rows, N], and its column sums (added to what `colsum` holds if `add`)
 CCLX_API int cclx_gelu_bwd_colsum(const void* dy, const void* x, void* dx, void* colsum, int add, float* workspace, size_t rows,
-                                  int N, void* stream) {
+                                  int N, int* defer, void* stream) {
     return cclx::capi::guard([&] {
         CCL_THROW_IF_NOT(N % 8 == 0, "the fused GELU takes whole 16-byte packs");
         if (rows == 0)
             return;
         gelu_bwd_map f{ (const uint4*)dy, (const uint4*)x, (uint4*)dx, N / 8 };
-        launch_map_colsum(f, rows, N / 8, colsum, add, workspace, (cudaStream_t)stream);
+        launch_map_colsum(f, rows, N / 8, colsum, add, workspace, defer, (cudaStream_t)stream);
     });
 }
 
 // packed QKV gradient out [B, S, 3, H, dh] from three [B, H, S, dh]-indexed gradients with 9 element strides (b, s, h per
 // part), and its column sums
 CCLX_API int cclx_qkv_grad_colsum(const void* const* src, const long long* strides, void* out, void* colsum, int add,
-                                  float* workspace, int B, int S, int H, int dh, void* stream) {
+                                  float* workspace, int B, int S, int H, int dh, int* defer, void* stream) {
     return cclx::capi::guard([&] {
         CCL_THROW_IF_NOT(dh % 8 == 0, "head size must be a multiple of 8");
         if (B == 0 || S == 0)
@@ -671,6 +692,6 @@ CCLX_API int cclx_qkv_grad_colsum(const void* const* src, const long long* strid
         f.S = S;
         f.H = H;
         f.ppr = dh / 8;
-        launch_map_colsum(f, (size_t)B * S, 3 * H * dh / 8, colsum, add, workspace, (cudaStream_t)stream);
+        launch_map_colsum(f, (size_t)B * S, 3 * H * dh / 8, colsum, add, workspace, defer, (cudaStream_t)stream);
     });
 }

@@ -53,11 +53,13 @@ struct ParamGrad {
     Tensor out;
     bool add = false;
 
+    // `beside`: it will be written on the sink's stream of gradients, not on the current stream.
     // `room`: where the gradient goes if there is no sink (allocated if undefined)
-    ParamGrad(const SinkRef& s, const Tensor& like, at::IntArrayRef shape, Tensor room = Tensor()) : sink(s) {
+    ParamGrad(const SinkRef& s, const Tensor& like, at::IntArrayRef shape, bool beside = false, Tensor room = Tensor()) : sink(s) {
         if (s) {
             out = s->grad;
-            add = s->add();
+            add = beside && s->on_side ? s->take() : s->add();
+            s->on_side = beside;
         }
         else
             out = room.defined() ? std::move(room) : empty_on(like, shape, at::kBFloat16);
@@ -77,6 +79,38 @@ struct ParamGrad {
             sink->report();
     }
 };
+
+// Runs `f(defer)`, which launches a kernel that leaves partial sums in `ws` and adds them up unless it can leave their number
+// in *defer; then they are added up beside the rest of backward.
+template <class F>
+void with_sums(const GradStreamRef& beside, const Tensor& ws, int cols, std::initializer_list<const ParamGrad*> outs, F&& f) {
+    int n = 0;
+    f(beside ? &n : nullptr);
+    launches += 2;
+    if (!beside || n == 0)
+        return;
+    void* o[3] = {};
+    int k = 0, add = 0;
+    for (const ParamGrad* p : outs) {
+        add |= (p->add ? 1 : 0) << k;
+        o[k++] = p->ptr();
+    }
+    at::cuda::CUDAEvent ready;
+    ready.record(at::cuda::getCurrentCUDAStream(ws.get_device()));
+    beside->launch(
+        ready, [&] { check(cclx_partial_sums(ws.data_ptr<float>(), n, cols, k, o[0], o[1], o[2], add, stream_of(ws))); }, ws, ws);
+}
+
+// the stream of gradients that all of these sinks allow, or none
+GradStreamRef beside_of(std::initializer_list<SinkRef> sinks) {
+    GradStreamRef b;
+    for (const SinkRef& s : sinks) {
+        if (!s || !s->beside || (b && b != s->beside))
+            return nullptr;
+        b = s->beside;
+    }
+    return b;
+}
 
 std::vector<SinkRef> sinks_of(AutogradContext* ctx, size_t n) {
     auto it = ctx->saved_data.find("sinks");
@@ -119,12 +153,13 @@ struct AddLayerNormBackward : torch::autograd::Node {
         const Tensor dx = empty_on(t, shape, at::kBFloat16);
         const int64_t wide[] = { D };
         const bool own = !sinks[0] && !sinks[1];
+        const GradStreamRef beside = has_res_bias ? beside_of({ sinks[0], sinks[1], sinks[2] }) : beside_of({ sinks[0], sinks[1] });
         const Tensor both = own ? empty_on(t, { 2 * D }, at::kBFloat16) : Tensor(); // gamma's and beta's gradients are born together
-        const ParamGrad dg(sinks[0], t, wide, own ? part_of(both, 0, wide, at::kBFloat16) : Tensor());
-        const ParamGrad db(sinks[1], t, wide, own ? part_of(both, 2 * D, wide, at::kBFloat16) : Tensor());
+        const ParamGrad dg(sinks[0], t, wide, (bool)beside, own ? part_of(both, 0, wide, at::kBFloat16) : Tensor());
+        const ParamGrad db(sinks[1], t, wide, (bool)beside, own ? part_of(both, 2 * D, wide, at::kBFloat16) : Tensor());
         std::optional<ParamGrad> dr;
         if (has_res_bias)
-            dr.emplace(sinks[2], t, wide);
+            dr.emplace(sinks[2], t, wide, (bool)beside);
         if (rows == 0) {
             dg.nothing();
             db.nothing();
@@ -133,11 +168,17 @@ struct AddLayerNormBackward : torch::autograd::Node {
         }
         const Tensor ws = empty_on(t, { (int64_t)cclx_layer_norm_bwd_blocks(rows) * (dr ? 3 : 2) * D }, at::kFloat);
         const float* mean = stats.data_ptr<float>();
-        check(cclx_layer_norm_bwd_sums(dy.data_ptr(), t.data_ptr(), w.data_ptr(), mean, mean + rows,
-                                       dsum.defined() ? dsum.data_ptr() : nullptr, dx.data_ptr(), dg.ptr(), db.ptr(),
-                                       dr ? dr->ptr() : nullptr, (dg.add ? 1 : 0) | (db.add ? 2 : 0) | (dr && dr->add ? 4 : 0),
-                                       ws.data_ptr<float>(), rows, (int)D, st));
-        launches += 2;
+        auto run = [&](int* defer) {
+            check(cclx_layer_norm_bwd_sums(dy.data_ptr(), t.data_ptr(), w.data_ptr(), mean, mean + rows,
+                                           dsum.defined() ? dsum.data_ptr() : nullptr, dx.data_ptr(), dg.ptr(), db.ptr(),
+                                           dr ? dr->ptr() : nullptr,
+                                           (dg.add ? 1 : 0) | (db.add ? 2 : 0) | (dr && dr->add ? 4 : 0), ws.data_ptr<float>(), rows,
+                                           (int)D, defer, st));
+        };
+        if (dr)
+            with_sums(beside, ws, (int)D, { &dg, &db, &*dr }, run);
+        else
+            with_sums(beside, ws, (int)D, { &dg, &db }, run);
         dg.done();
         db.done();
         if (dr)
@@ -330,13 +371,16 @@ struct BiasGelu : torch::autograd::Function<BiasGelu> {
         const Tensor& u = saved[0];
         const int64_t rows = u.size(0), N = u.size(1);
         const Tensor dy = rows_of(grads[0], N), du = empty_on(u, u.sizes(), at::kBFloat16);
-        const ParamGrad g(sinks_of(ctx, 1)[0], u, saved[1].sizes());
+        const SinkRef sink = sinks_of(ctx, 1)[0];
+        const GradStreamRef beside = beside_of({ sink });
+        const ParamGrad g(sink, u, saved[1].sizes(), (bool)beside);
         if (rows == 0)
             g.nothing();
         const Tensor ws = empty_on(u, { (int64_t)cclx_map_colsum_workspace(rows, (int)N) }, at::kFloat);
-        check(cclx_gelu_bwd_colsum(dy.data_ptr(), u.data_ptr(), du.data_ptr(), g.ptr(), g.add, ws.data_ptr<float>(), rows, (int)N,
-                                   stream_of(u)));
-        launches += 2;
+        with_sums(beside, ws, (int)N, { &g }, [&](int* defer) {
+            check(cclx_gelu_bwd_colsum(dy.data_ptr(), u.data_ptr(), du.data_ptr(), g.ptr(), g.add, ws.data_ptr<float>(), rows, (int)N,
+                                       defer, stream_of(u)));
+        });
         g.done();
         return { shaped(du, grads[0].sizes()), g.result(), Tensor() };
     }
@@ -378,13 +422,16 @@ struct SplitQKV : torch::autograd::Function<SplitQKV> {
             strides[3 * p + 2] = g[p].stride(1);
         }
         // without a bias the sums go nowhere
-        const ParamGrad db(sinks_of(ctx, 1)[0], out, { N });
+        const SinkRef sink = sinks_of(ctx, 1)[0];
+        const GradStreamRef beside = beside_of({ sink });
+        const ParamGrad db(sink, out, { N }, (bool)beside);
         if (B * S == 0)
             db.nothing();
         const Tensor ws = empty_on(out, { (int64_t)cclx_map_colsum_workspace(B * S, (int)N) }, at::kFloat);
-        check(cclx_qkv_grad_colsum(src, strides, out.data_ptr(), db.ptr(), db.add, ws.data_ptr<float>(), (int)B, (int)S, (int)H,
-                                   (int)dh, stream_of(out)));
-        launches += 2;
+        with_sums(beside, ws, (int)N, { &db }, [&](int* defer) {
+            check(cclx_qkv_grad_colsum(src, strides, out.data_ptr(), db.ptr(), db.add, ws.data_ptr<float>(), (int)B, (int)S, (int)H,
+                                       (int)dh, defer, stream_of(out)));
+        });
         db.done();
         return { out, bias ? db.result() : Tensor(), Tensor(), Tensor() };
     }

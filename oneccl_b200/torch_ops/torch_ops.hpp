@@ -26,7 +26,7 @@ int cclx_layer_norm_fwd(const void* x, const void* res, const void* w, const voi
 int cclx_layer_norm_bwd_blocks(size_t rows);
 int cclx_layer_norm_bwd_sums(const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
                              const void* dres, void* dx, void* dgamma, void* dbeta, void* dxsum, int add,
-                             float* workspace, size_t rows, int D, void* stream);
+                             float* workspace, size_t rows, int D, int* defer, void* stream);
 int cclx_dc_allreduce(void* h, const void* const* send, void* const* recv, size_t count, int dt_in, int dt_out, int op, int algo,
                       int blocks, float scale, int do_scale, void* stream);
 int cclx_moe_route(const float* logits, int n_tokens, int n_experts, int topk, long long* idx, float* wts, long long* counts,
@@ -41,9 +41,10 @@ size_t cclx_map_colsum_workspace(size_t rows, int N);
 int cclx_colsum(const void* x, void* out, int add, float* workspace, size_t rows, int N, void* stream);
 int cclx_gelu_fwd(const void* x, void* y, size_t n, void* stream);
 int cclx_gelu_bwd_colsum(const void* dy, const void* x, void* dx, void* colsum, int add, float* workspace, size_t rows, int N,
-                         void* stream);
+                         int* defer, void* stream);
 int cclx_qkv_grad_colsum(const void* const* src, const long long* strides, void* out, void* colsum, int add, float* workspace,
-                         int B, int S, int H, int dh, void* stream);
+                         int B, int S, int H, int dh, int* defer, void* stream);
+int cclx_partial_sums(const float* workspace, int n, int cols, int outputs, void* out0, void* out1, void* out2, int add, void* stream);
 int cclx_embed_fwd(const long long* idx, const void* tokens, const void* positions, void* out, size_t n, int S, int table_rows,
                    int D, void* stream);
 int cclx_embed_bwd_max_ids();
@@ -118,8 +119,9 @@ inline Tensor empty_on(const Tensor& like, at::IntArrayRef sizes, at::ScalarType
 // A stream of their own for weight gradients that go to sinks: nothing else in backward waits for them, products of a few
 // hundred tokens leave most SMs idle, and a long product's last wave some.  One per DataParallel.
 //
-// The operands of a product must outlive it, but the allocator knows them as memory of the current stream: the last DEPTH
-// products' operands are kept, and the current stream waits for the oldest product before its operands go.
+// The operands of a product must outlive it, but the allocator knows them as memory of the current stream: the operands of
+// the last DEPTH launches are kept, and the current stream waits for the oldest before its operands go.  The final sums of
+// bias, gamma and beta gradients run there as well.
 class GradStream {
 public:
     explicit GradStream(int dev) : stream_(at::cuda::getStreamFromPool(false, (c10::DeviceIndex)dev)) {}
@@ -158,7 +160,7 @@ public:
     }
 
 private:
-    static constexpr size_t DEPTH = 8; // two transformer blocks
+    static constexpr size_t DEPTH = 16; // two transformer blocks
     struct entry {
         at::cuda::CUDAEvent done;
         Tensor a, b;
