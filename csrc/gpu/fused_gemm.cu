@@ -96,7 +96,7 @@ void gemm_bf16_plain(const void* A, const void* B, void* C, int M, int N, int K,
         gemm_bf16_small(A, B, C, M, N, K, epilogue, err, st);
         return;
     }
-    if (ctas >= 0 && env_data::get().gemm_2sm && M >= 256 && N >= 128) {
+    if (ctas >= 0 && env_data::get().gemm_2sm && (M >= 256 || (ctas == 0 && M > 128)) && N >= 128) {
         gemm_bf16_2sm(A, B, C, M, N, K, epilogue, ctas / 2, err, st);
         return;
     }

@@ -308,15 +308,17 @@ small_plan plan_small(int M, int N, int K, int sms) {
 
 } // namespace
 
-// Whether the kernel above is expected to be faster than CTA pairs on 256 x 256 tiles (560 cycles per step of 64 and
-// round of tiles while the chip is partly idle, 20000 for start and output): up to 128 rows always, beyond that when
-// the pairs would leave much of the chip idle.
+// Whether the kernel above is expected to be faster than CTA pairs on 256 x 256 tiles: up to 128 rows always, beyond that
+// when the pairs would leave much of the chip idle.  In time the estimate above comes out as 1.25 times its cycles and 4600 for
+// the launch; the pairs take 560 cycles per step of 64 and round of tiles and 14500 for launch, start and output.  The
+// line this draws at 4096 x 4096 lies between 512 rows (23 us here, 30 us with pairs) and 768 (33 and 31), at 7168 x 2048
+// between 200 rows (16.6 and 17.2) and 384 (20 and 18), at 4096 x 14336 between 512 (55 and 78) and 768 (80 and 78).
 bool gemm_small_preferred(int M, int N, int K, int sms) {
     if (M <= 128)
         return true;
     const int tiles = ((M + 255) / 256) * ((N + 255) / 256), pairs = sms / 2, kb = (K + GEMM_BK - 1) / GEMM_BK;
     const int rounds = (tiles + pairs - 1) / pairs;
-    return plan_small(M, N, K, sms).cycles < 0.9 * ((double)rounds * kb * 560 + 20000);
+    return plan_small(M, N, K, sms).cycles * 1.25 + 4600 < (double)rounds * kb * 560 + 14500;
 }
 
 void gemm_bf16_small(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, uint32_t* err, cudaStream_t st,
