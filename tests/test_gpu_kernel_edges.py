@@ -135,6 +135,24 @@ def test_gelu_and_bias_gradient(rows, N):
     torch.testing.assert_close(db.float(), dr.sum(0), rtol=1e-2, atol=2e-3 * rows ** 0.5)
 
 
+def test_gelu_of_every_value():
+    """Forward: the bits of the stock tanh form for all bf16 inputs (infinities, NaN and huge values too), so that a model gives
+    the same activations with either.  Backward: its value within the rounding to bf16 of the product, which two orders of the
+    fp32 operations can change by one unit in the last place (2^-7 of the value)."""
+    from oneccl_b200.ops.nn import gelu
+
+    x = torch.arange(65536, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.bfloat16).view(64, 1024)
+    want = torch.nn.functional.gelu(x, approximate="tanh")
+    u, b = x.clone().requires_grad_(True), torch.zeros(1024, device="cuda", dtype=torch.bfloat16)
+    y = gelu(u, b)
+    same = (y.view(torch.int16) == want.view(torch.int16)) | (y.isnan() & want.isnan())
+    assert bool(same.all()), x[~same][:8].tolist()
+    r = x.clone().requires_grad_(True)
+    dy = torch.full_like(x, 1.25)
+    (dx,), (dr,) = torch.autograd.grad(y, u, dy), torch.autograd.grad(torch.nn.functional.gelu(r, approximate="tanh"), r, dy)
+    torch.testing.assert_close(dx.float(), dr.float(), rtol=2.0**-7, atol=0, equal_nan=True)
+
+
 @pytest.mark.parametrize("B,S,H,dh", [(1, 1, 1, 8), (2, 37, 3, 64), (3, 130, 12, 72)])
 def test_split_qkv_bias_gradient(B, S, H, dh):
     from oneccl_b200.ops.nn import split_qkv
