@@ -431,21 +431,30 @@ __device__ __forceinline__ float pick8(const uint4& u, int at) {
     return __uint_as_float(at & 1 ? w & 0xffff0000u : w << 16);
 }
 
-// Running maximum and sum of exponentials below it: one more pack.  The maximum rarely moves after the first packs.
+// Running maximum and sum of exponentials below it: one more pack.  The maximum rarely moves after the first packs.  Before the
+// first number above -inf the sum is 0, or NaN from NaN logits, and is kept.  A share of a row may hold nothing but the type's
+// lowest value (a mask), whose product with log2(e) overflows: below -1e38 exponents are taken from there and come out as 0,
+// which is their part of any row that has a larger logit.
+__device__ __forceinline__ float rescaled(float s, float m, float to) {
+    return m == -INFINITY ? s : s * ex2((m - to) * LOG2E);
+}
+__device__ __forceinline__ float shift_of(float m) {
+    return -fmaxf(m, -1e38f) * LOG2E;
+}
 __device__ __forceinline__ void online8(const uint4& u, float& m, float& shift, float& s) {
     const float pm = max8(u);
     if (pm > m) {
-        s = m == -INFINITY ? 0.f : s * ex2((m - pm) * LOG2E);
+        s = rescaled(s, m, pm);
         m = pm;
-        shift = -m * LOG2E;
+        shift = shift_of(m);
     }
     s += exp_sum8(u, shift);
 }
 __device__ __forceinline__ void online1(float x, float& m, float& shift, float& s) {
     if (x > m) {
-        s = m == -INFINITY ? 0.f : s * ex2((m - x) * LOG2E);
+        s = rescaled(s, m, x);
         m = x;
-        shift = -m * LOG2E;
+        shift = shift_of(m);
     }
     s += ex2(fmaf(x, LOG2E, shift));
 }
@@ -501,13 +510,13 @@ __global__ void __launch_bounds__(T, T == 1024 ? 1 : 1024 / T)
         if (tail < vocab)
             online1(xt, m, shift, s);
         const float wm = warp_max(m);
-        const float ws = warp_sum(m == -INFINITY ? 0.f : s * ex2((m - wm) * LOG2E));
+        const float ws = warp_sum(rescaled(s, m, wm));
         if (lane == 0)
             part[buf][warp] = make_float2(wm, ws);
         __syncthreads();
         const float2 p = lane < T / 32 ? part[buf][lane] : make_float2(-INFINITY, 0.f);
         const float mx = warp_max(p.x);
-        const float sum = warp_sum(p.x == -INFINITY ? 0.f : p.y * ex2((p.x - mx) * LOG2E));
+        const float sum = warp_sum(rescaled(p.y, p.x, mx));
         const bool ignore = tgt < 0 || tgt >= vocab;
         const float inv = ignore ? 0.f : grad_scale / sum, hit = ignore ? 0.f : grad_scale;
         shift = -mx * LOG2E;

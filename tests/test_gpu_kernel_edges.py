@@ -69,6 +69,35 @@ def test_softmax_xent_row_lengths(rows, vocab, pad):
     assert not pad or torch.count_nonzero(got[:, vocab:]) == 0
 
 
+@pytest.mark.parametrize("vocab", [1000, 8199, 16391, 50257, 106503, 106504])  # every kernel, a tail of less than a pack
+def test_softmax_xent_masked_and_invalid_logits(vocab):
+    """Logits masked with the type's lowest value (long runs of them, so that a thread's first packs or whole share of a row hold
+    nothing else), and a NaN among masked logits, which must reach loss and gradient of its row and of no other."""
+    from oneccl_b200.ops.train import softmax_cross_entropy
+
+    g = torch.Generator(device="cuda").manual_seed(vocab)
+    low, cols = torch.finfo(torch.bfloat16).min, (vocab + 7) // 8 * 8
+    logits = _bf16(g, 8, cols, scale=3)
+    logits[0, : vocab - 9] = low
+    logits[1, 5 : vocab - 2] = low
+    logits[3, :vocab] = torch.where(torch.arange(vocab, device="cuda") % 5 == 0, 1.0, low)
+    logits[4, : vocab - 1] = float("-inf")
+    logits[4, 40:48] = float("nan")
+    logits[5, : vocab - 1] = float("-inf")
+    tgt = torch.full((8,), vocab - 1, device="cuda")
+    tgt[3] = vocab // 5 * 5 - 5
+    ref = logits[:, :vocab].float().requires_grad_(True)
+    per_row = torch.nn.functional.cross_entropy(ref, tgt, reduction="none")
+    (want,) = torch.autograd.grad(per_row.sum(), ref)
+    for r in range(8):
+        x = logits[r : r + 1].clone().requires_grad_(True)
+        loss = softmax_cross_entropy(x, tgt[r : r + 1], vocab)
+        (got,) = torch.autograd.grad(loss, x)
+        # fp32 sums of up to 106504 terms; the gradient is rounded to bf16 once
+        torch.testing.assert_close(loss, per_row[r], rtol=1e-4, atol=1e-4, equal_nan=True, msg=f"row {r}")
+        torch.testing.assert_close(got[0, :vocab].float(), want[r], rtol=1e-2, atol=1e-6, equal_nan=True, msg=f"row {r}")
+
+
 @pytest.mark.parametrize("M", [1, 15, 16, 17, 32, 33, 64, 65, 128, 129, 257, 700])  # tile widths 16 ... 256, one or more tiles
 @pytest.mark.parametrize("N,K", [(8, 8), (128, 64), (136, 264), (1024, 512), (1000, 2056), (4096, 1024)])  # 1 to 8 parts of K
 @pytest.mark.parametrize("rows", [None, 0.4])
