@@ -609,10 +609,11 @@ CCLX_API int cclx_layer_norm_bwd(const void* dy, const void* x, const void* w, c
 
 namespace {
 int map_rows_per_block(size_t rows, int packs) {
-    // about six blocks of 128 threads per SM, between 8 and 64 rows each: fewer rows would spend more on partial sums
+    // about six blocks of 128 threads per SM, between 8 and 64 rows each: fewer rows would spend more on partial sums.  More
+    // only where the grid has no room for so many blocks (over 65535 of them).
     const size_t cols = (packs + 127) / 128;
     const size_t per = rows * cols / ((size_t)device_sms() * 6);
-    return (int)std::min<size_t>(64, std::max<size_t>(8, (per + 3) / 4 * 4));
+    return (int)std::max<size_t>(std::min<size_t>(64, std::max<size_t>(8, (per + 3) / 4 * 4)), (rows + 65534) / 65535);
 }
 
 template <class F>

@@ -182,6 +182,20 @@ def test_gelu_of_every_value():
     torch.testing.assert_close(dx.float(), dr.float(), rtol=2.0**-7, atol=0, equal_nan=True)
 
 
+@pytest.mark.parametrize("rows,N", [(1, 8), (9, 1032), (65535 * 64, 8), (65535 * 64 + 1, 8), (9_000_001, 8)])
+def test_column_sums_of_many_rows(rows, N):
+    """Up to and beyond the rows for which a block's 64 rows fill the grid's second dimension."""
+    from oneccl_b200.ops.nn import colsum, gelu
+
+    x = torch.randint(-1, 2, (rows, N), device="cuda", dtype=torch.int8).to(torch.bfloat16)
+    x[rows // 2 :, 0] = 0  # sums of whole numbers: exact in fp32, rounded once
+    want = x.float().sum(0, dtype=torch.float64).to(torch.bfloat16)
+    assert torch.equal(colsum(x), want)
+    u, b = torch.zeros_like(x).requires_grad_(True), torch.zeros(N, device="cuda", dtype=torch.bfloat16).requires_grad_(True)
+    du, db = torch.autograd.grad(gelu(u, b), [u, b], x * 2)  # the slope at 0 is one half
+    assert torch.equal(du, x) and torch.equal(db, want)
+
+
 @pytest.mark.parametrize("B,S,H,dh", [(1, 1, 1, 8), (2, 37, 3, 64), (3, 130, 12, 72)])
 def test_split_qkv_bias_gradient(B, S, H, dh):
     from oneccl_b200.ops.nn import split_qkv
