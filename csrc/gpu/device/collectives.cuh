@@ -186,7 +186,9 @@ __global__ void __launch_bounds__(1024) allreduce_oneshot_kernel(const comm_dev*
 //
 // The packet areas are used by nothing else and alternate between two generations.  Call n + 2 may overwrite a packet of
 // call n because a rank finishes call n + 1 only with every peer's packets of it, which a peer sends after its call n.
-// The header packet carries the argument signature: a peer that disagrees ends the kernel with ST_ARG_MISMATCH.
+// The header packet carries the argument signature: a peer that disagrees ends the kernel with ST_ARG_MISMATCH, before
+// anything is stored (in place that would destroy the input).  The packet with its flag inside is the layout known from
+// low-latency protocols of collective libraries (hence LL).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint4 ld_packet(const char* p) {
     uint4 v;
@@ -244,9 +246,7 @@ __global__ void __launch_bounds__(512) allreduce_packets_kernel(const comm_dev* 
     if (blockIdx.x == 0 && threadIdx.x < (unsigned)W)
         st_packet(c.ll[threadIdx.x] + mine + LL_HEADER, sig, 0, seq);
     __syncthreads();
-    bool checked = threadIdx.x >= (unsigned)W || threadIdx.x == (unsigned)rank;
-    auto check = [&] { // the peer's arguments, after this thread's own packets are on their way
-        checked = true;
+    auto check_peer = [&] { // the arguments of peer threadIdx.x
         uint4 h;
         if (wait_packet(c, in + (size_t)threadIdx.x * LL_SLOT_BYTES + LL_HEADER, seq, threadIdx.x, &failed, h) && h.x != sig) {
             report(c, ST_ARG_MISMATCH, threadIdx.x, h.x);
@@ -255,10 +255,12 @@ __global__ void __launch_bounds__(512) allreduce_packets_kernel(const comm_dev* 
     };
     auto exchange = [&](auto wt) {
         constexpr int WT = decltype(wt)::value;
-        for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < packets; i += gridDim.x * blockDim.x) {
-            const size_t e0 = (size_t)i * N;
+        bool checked = false;
+        unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+        do { // every thread of the block makes the first round
+            const size_t e0 = (size_t)i * N, at = (size_t)i * 16;
+            const bool mine_to_do = i < packets, whole = e0 + N <= count;
             uint2 raw = make_uint2(0, 0);
-            const bool whole = e0 + N <= count;
             if (whole && ((uintptr_t)(send + e0) & 7) == 0)
                 raw = *reinterpret_cast<const uint2*>(send + e0);
             else {
@@ -268,14 +270,15 @@ __global__ void __launch_bounds__(512) allreduce_packets_kernel(const comm_dev* 
                     if (e0 + k < count)
                         t[k] = send[e0 + k];
             }
-            const size_t at = (size_t)i * 16;
-            const int n = WT > 0 ? WT : W;
+            if (mine_to_do) {
+                const int n = WT > 0 ? WT : W;
 #pragma unroll
-            for (int p = 0; p < n; p++)
-                if (p != rank)
-                    st_packet(c.ll[p] + mine + at, raw.x, raw.y, seq);
-            if (!checked)
-                check();
+                for (int p = 0; p < n; p++)
+                    if (p != rank)
+                        st_packet(c.ll[p] + mine + at, raw.x, raw.y, seq);
+            }
+            if (!checked && threadIdx.x < (unsigned)W && threadIdx.x != (unsigned)rank)
+                check_peer(); // after this thread's own packets are on their way
             A acc[N];
             auto add = [&](int p, const uint4& v) {
                 const uint2 d = p == rank ? raw : make_uint2(v.x, v.z);
@@ -291,7 +294,7 @@ __global__ void __launch_bounds__(512) allreduce_packets_kernel(const comm_dev* 
                 uint4 v[WT];
 #pragma unroll
                 for (int p = 0; p < WT; p++)
-                    v[p] = ld_packet(in + (size_t)p * LL_SLOT_BYTES + at);
+                    v[p] = mine_to_do ? ld_packet(in + (size_t)p * LL_SLOT_BYTES + at) : make_uint4(0, seq, 0, seq);
 #pragma unroll
                 for (int p = 0; p < WT; p++)
                     if (ok && p != rank && (v[p].y != seq || v[p].w != seq))
@@ -303,10 +306,15 @@ __global__ void __launch_bounds__(512) allreduce_packets_kernel(const comm_dev* 
             else {
                 for (int p = 0; p < W; p++) {
                     uint4 v = make_uint4(0, 0, 0, 0);
-                    if (ok && p != rank)
+                    if (mine_to_do && ok && p != rank)
                         ok = wait_packet(c, in + (size_t)p * LL_SLOT_BYTES + at, seq, p, &failed, v);
                     add(p, v);
                 }
+            }
+            if (!checked) { // nothing is stored before all arguments of all peers have been compared
+                checked = true;
+                if (__syncthreads_or(!ok || failed))
+                    break;
             }
             if (!ok || failed)
                 break;
@@ -318,9 +326,8 @@ __global__ void __launch_bounds__(512) allreduce_packets_kernel(const comm_dev* 
                     if (e0 + k < count)
                         recv[e0 + k] = from_acc<Tout, A>(a.do_scale ? apply_scale<A>(acc[k], a.scale) : acc[k]);
             }
-        }
-        if (!checked)
-            check();
+            i += gridDim.x * blockDim.x;
+        } while (i < packets);
     };
     if (W == 8)
         exchange(int_const<8>());

@@ -355,3 +355,27 @@ def test_small_allreduce_packets(W, dtype, out_dtype):
     torch.cuda.synchronize()
     assert all(bool((t == W).all()) for t in x)
     group.close()
+
+
+@pytest.mark.parametrize("W", [2, 3, 8])
+@pytest.mark.parametrize("n,blocks", [(1, 0), (700, 0), (8192, 0), (8192, 1)])  # fewer packets than ranks, many blocks, many rounds of one
+def test_small_allreduce_mismatch_leaves_the_buffers(W, n, blocks):
+    """A rank whose arguments differ ends the call before anything is stored: in place the inputs are still there."""
+    from oneccl_b200.ops.device_group import DeviceGroup
+
+    group = DeviceGroup.emulated(W, heap_bytes=40 << 20, staging_bytes=1 << 20)
+    group.set_timeout_ms(1000)
+    for skewed in (0, W - 1):
+        x = [torch.full((n,), float(r + 1), device="cuda") for r in range(W)]
+        group.test_sig_skew(skewed)
+        group.allreduce(x, x, algo="oneshot", blocks=blocks)
+        torch.cuda.synchronize()
+        assert {group.status(r) for r in range(W)} == {7}
+        assert all(bool((t == r + 1).all()) for r, t in enumerate(x))
+        group.test_sig_skew(-1)
+        group.clear_status()
+        group.allreduce(x, x, algo="oneshot", blocks=blocks)
+        torch.cuda.synchronize()
+        group.check()
+        assert all(bool((t == W * (W + 1) / 2).all()) for t in x)
+    group.close()
