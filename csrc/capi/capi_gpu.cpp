@@ -90,7 +90,8 @@ CCLX_API int cclx_dc_clear_status(void* h) {
 CCLX_API int cclx_dc_abort(void* h) {
     return capi::guard([&] { ((device_comm*)h)->abort(); });
 }
-// test hook: the next collectives of emulated rank `rank` (-1: none) carry a falsified argument signature
+// test hook: the next collectives of emulated rank `rank` (-1: none) carry a falsified argument signature; -2 - rank: the rank
+// calls a barrier where the others call a small allreduce
 CCLX_API int cclx_dc_test_sig_skew(void* h, int rank) {
     return capi::guard([&] { ((device_comm*)h)->test_sig_skew = rank + 1; });
 }

@@ -190,26 +190,26 @@ __global__ void __launch_bounds__(1024) allreduce_oneshot_kernel(const comm_dev*
 // anything is stored (in place that would destroy the input).  The packet with its flag inside is the layout known from
 // low-latency protocols of collective libraries (hence LL).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint4 ld_packet(const char* p) {
-    uint4 v;
-    asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_packet(char* p, uint32_t lo, uint32_t hi, uint32_t seq) {
-    asm volatile("st.volatile.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(lo), "r"(seq), "r"(hi), "r"(seq) : "memory");
-}
-
-// Polls packet `p` of `peer` until both halves carry `seq`; false after the time limit, an abort or a failure elsewhere in
-// the block (status recorded).
+// Polls packet `p` of `peer` until both halves carry `seq`; false after the time limit, an abort, a failure elsewhere in
+// the block or when the peer is in another kernel, seen twice as in wait_flag_sys (status recorded).
 __device__ __forceinline__ bool wait_packet(const comm_dev& c, const char* p, uint32_t seq, int peer, volatile int* failed, uint4& v) {
     unsigned long long t0 = 0;
+    bool elsewhere = false;
     for (uint32_t it = 0;; it++) {
         v = ld_packet(p);
         if (v.y == seq && v.w == seq)
             return true;
-        if ((it & 0xff) == 0xff) {
+        if ((it & 0x3ff) == 0x3ff) {
             if (*failed)
                 return false;
+            if (peer_in_barrier(c, peer)) {
+                if (elsewhere) {
+                    report(c, ST_ARG_MISMATCH, peer, seq);
+                    *failed = 1;
+                    return false;
+                }
+                elsewhere = true;
+            }
             const unsigned long long now = globaltimer_ns();
             if (t0 == 0)
                 t0 = now;
@@ -243,6 +243,13 @@ __global__ void __launch_bounds__(512) allreduce_packets_kernel(const comm_dev* 
     const size_t mine = gen + (size_t)rank * LL_SLOT_BYTES;
     const char* in = c.ll[rank] + gen;
     const uint32_t sig = kernel_signature(15, a, c);
+    if (a.sig_skew == -1 - rank) { // test hook: this emulated rank has called a barrier
+        block_sync s;
+        sync_begin(c, s);
+        peer_barrier(c, s, kernel_signature(14, a, c));
+        sync_end(c, s, gridDim.x, 1, false);
+        return;
+    }
     if (blockIdx.x == 0 && threadIdx.x < (unsigned)W)
         st_packet(c.ll[threadIdx.x] + mine + LL_HEADER, sig, 0, seq);
     __syncthreads();

@@ -143,16 +143,49 @@ __device__ __forceinline__ void report(const comm_dev& c, uint32_t code, uint32_
     }
 }
 
+// 16-byte packets that carry the sequence number of a small allreduce in two of their words (allreduce_packets_kernel)
+__device__ __forceinline__ uint4 ld_packet(const char* p) {
+    uint4 v;
+    asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_packet(char* p, uint32_t lo, uint32_t hi, uint32_t seq) {
+    asm volatile("st.volatile.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(lo), "r"(seq), "r"(hi), "r"(seq) : "memory");
+}
+
+// Ranks that called different collectives meet in none.  Every kernel but the small allreduce starts with a barrier, where
+// signatures are compared; the small allreduce has packets instead, so each kind looks for the other while it waits.
+// Is `peer` in the small allreduce that this rank has not called?  Its header is there then.
+__device__ __forceinline__ bool peer_in_packets(const comm_dev& c, int peer) {
+    const uint32_t seq = ld_volatile_u32(c.state + STATE_LL) + 1;
+    const uint4 h = ld_packet(c.ll[c.rank] + ((size_t)(seq & 1) * c.world + peer) * LL_SLOT_BYTES + LL_HEADER);
+    return h.y == seq && h.w == seq;
+}
+// Is `peer` in a barrier that this rank has not come to?  The flag for this rank's first block is raised then.
+__device__ __forceinline__ bool peer_in_barrier(const comm_dev& c, int peer) {
+    return (int32_t)(ld_acquire_sys(c.flags[c.rank] + peer) - ld_volatile_u32(c.state + STATE_EPOCH)) > 0;
+}
+
 // Spin until *p reaches `target` (wrap-safe), the abort flag is raised or the
 // time limit passes.  Returns false on timeout/abort after recording the status.
+// A barrier's wait also ends when the peer is in a small allreduce.  Seen twice, with a thousand looks at the flag in
+// between: a peer that has left the barrier and is in the call after it raised its flag before.
 __device__ __forceinline__ bool wait_flag_sys(const comm_dev& c, const uint32_t* p, uint32_t target,
                                               uint32_t peer, uint32_t code) {
     unsigned long long t0 = 0;
+    bool elsewhere = false;
     for (uint32_t it = 0;; it++) {
         uint32_t v = ld_acquire_sys(p);
         if ((int32_t)(v - target) >= 0)
             return true;
         if ((it & 0x3ff) == 0x3ff) {
+            if (code == ST_BARRIER_TIMEOUT && peer_in_packets(c, peer)) {
+                if (elsewhere) {
+                    report(c, ST_ARG_MISMATCH, peer, target);
+                    return false;
+                }
+                elsewhere = true;
+            }
             unsigned long long now = globaltimer_ns();
             if (t0 == 0)
                 t0 = now;

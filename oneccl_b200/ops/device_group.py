@@ -112,7 +112,8 @@ class DeviceGroup:
 
     def test_sig_skew(self, rank: int):
         """Test hook: falsify the argument signature that emulated rank `rank` presents in the next
-        collectives (-1 switches it off), to exercise the cross-rank argument check on one GPU."""
+        collectives (-1 switches it off), to exercise the cross-rank argument check on one GPU.  ``-2 - r``: in small
+        allreduces emulated rank ``r`` calls a barrier instead."""
         _lib.check(self._lib.cclx_dc_test_sig_skew(self._h, rank))
 
     def algo_hits(self, coll: str, algo: str) -> int:

@@ -379,3 +379,28 @@ def test_small_allreduce_mismatch_leaves_the_buffers(W, n, blocks):
         group.check()
         assert all(bool((t == W * (W + 1) / 2).all()) for t in x)
     group.close()
+
+
+@pytest.mark.parametrize("W", [2, 3, 8])
+@pytest.mark.parametrize("n", [1, 8192])
+def test_small_allreduce_against_a_barrier_is_reported(W, n):
+    """One rank is in a barrier, the others in a small allreduce: both sides end with an argument mismatch, long before the time
+    limit, and nothing is stored."""
+    import time
+
+    from oneccl_b200.ops.device_group import DeviceGroup
+
+    group = DeviceGroup.emulated(W, heap_bytes=40 << 20, staging_bytes=1 << 20)
+    x = [torch.full((n,), float(r + 1), device="cuda") for r in range(W)]
+    group.allreduce(x, [torch.empty_like(t) for t in x], algo="oneshot")
+    group.barrier()
+    torch.cuda.synchronize()
+    group.set_timeout_ms(5000)
+    group.test_sig_skew(-2 - (W - 1))
+    t0 = time.perf_counter()
+    group.allreduce(x, x, algo="oneshot")
+    torch.cuda.synchronize()
+    assert time.perf_counter() - t0 < 1.0
+    assert {group.status(r) for r in range(W)} == {7}
+    assert all(bool((t == r + 1).all()) for r, t in enumerate(x))
+    group.close()
