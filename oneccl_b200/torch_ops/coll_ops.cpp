@@ -1,5 +1,6 @@
 // Host side of the small calls on a device group and of the expert-parallel steps: tensors to pointer tables without a
-// Python loop over them (kernels: csrc/gpu/launch_allreduce.cu, moe_kernels.cu).
+// Python loop over them (kernels: csrc/gpu/launch_allreduce.cu, moe_kernels.cu).  A launch into a full queue waits for the GPU:
+// other Python threads run meanwhile.
 #include "torch_ops.hpp"
 
 namespace cclx_ops {
@@ -46,8 +47,10 @@ void allreduce(uintptr_t group, const tensors& send, const tensors& recv, int op
     void* st = stream ? reinterpret_cast<void*>(*stream) : stream_of(send[0]);
     const auto s = pointers<const void>(send);
     const auto r = pointers<void>(recv);
-    check(cclx_dc_allreduce(reinterpret_cast<void*>(group), s.data(), r.data(), send[0].numel(), ccl_dtype(send[0].scalar_type()),
-                            ccl_dtype(recv[0].scalar_type()), op, algo, blocks, scale ? (float)*scale : 1.0f, scale ? 1 : 0, st));
+    const int dt_in = ccl_dtype(send[0].scalar_type()), dt_out = ccl_dtype(recv[0].scalar_type());
+    pybind11::gil_scoped_release nogil;
+    check(cclx_dc_allreduce(reinterpret_cast<void*>(group), s.data(), r.data(), send[0].numel(), dt_in, dt_out, op, algo, blocks,
+                            scale ? (float)*scale : 1.0f, scale ? 1 : 0, st));
 }
 
 // expert ids [T, k], weights [T, k], items per expert [E], grouping permutation and its inverse [T * k]
@@ -60,8 +63,11 @@ pybind11::tuple route(const Tensor& logits_, int64_t topk) {
     char* base = static_cast<char*>(all.data_ptr());
     long long* items = reinterpret_cast<long long*>(base);
     long long* counts = reinterpret_cast<long long*>(base + c_at);
-    check(cclx_moe_route(logits.data_ptr<float>(), (int)T, (int)E, (int)topk, items, reinterpret_cast<float*>(base + w_at), counts,
-                         items + n, items + 2 * n, counts + row, stream_of(logits)));
+    {
+        pybind11::gil_scoped_release nogil;
+        check(cclx_moe_route(logits.data_ptr<float>(), (int)T, (int)E, (int)topk, items, reinterpret_cast<float*>(base + w_at),
+                             counts, items + n, items + 2 * n, counts + row, stream_of(logits)));
+    }
     return pybind11::make_tuple(part_of(all, 0, { T, topk }, at::kLong), part_of(all, w_at, { T, topk }, at::kFloat),
                                 part_of(all, c_at, { E }, at::kLong), part_of(all, 8 * n, { n }, at::kLong),
                                 part_of(all, 16 * n, { n }, at::kLong));
@@ -72,6 +78,7 @@ void dispatch(uintptr_t group, const tensors& x, const tensors& order, const ten
     const auto px = pointers<const void>(x);
     const auto po = pointers<const long long>(order), pc = pointers<const long long>(counts);
     const auto pm = pointers<int>(meta);
+    pybind11::gil_scoped_release nogil;
     check(cclx_moe_dispatch(reinterpret_cast<void*>(group), px.data(), po.data(), pc.data(), pm.data(), order[0].numel(), topk,
                             (int)x[0].size(1), recv.data_ptr(), recv.size(0), table.data_ptr(), blocks, stream_of(recv)));
 }
@@ -82,6 +89,7 @@ void combine(uintptr_t group, const tensors& expert, const tensors& pos, const t
     const auto pw = pointers<const float>(weight);
     const auto po = pointers<void>(out);
     const auto pm = pointers<int>(meta);
+    pybind11::gil_scoped_release nogil;
     check(cclx_moe_combine_peer(reinterpret_cast<void*>(group), pe.data(), pp.data(), pw.data(), po.data(), pm.data(),
                                 expert[0].numel(), topk, (int)out[0].size(1), expert_out.data_ptr(), blocks,
                                 stream_of(expert_out)));

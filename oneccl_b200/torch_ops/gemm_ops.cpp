@@ -7,6 +7,7 @@ namespace {
 // kernel: 0 = the library decides, 1 = one CTA per tile, 2 = CTA pairs
 Tensor gemm_bf16(const Tensor& a_, const Tensor& w_, const std::optional<Tensor>& out_, int64_t epilogue, int64_t ctas, int64_t kernel,
                  const std::optional<Tensor>& rows, const Tensor& err) {
+    pybind11::gil_scoped_release nogil;
     const Tensor a = a_.is_contiguous() ? a_ : a_.contiguous(), w = w_.is_contiguous() ? w_ : w_.contiguous();
     const int M = (int)a.size(0), K = (int)a.size(1), N = (int)w.size(0);
     const Tensor out = out_ ? *out_ : empty_on(a, { M, N }, at::kBFloat16);

@@ -62,6 +62,7 @@ Tensor softmax_xent(const Tensor& logits, const Tensor& targets_, int64_t vocab,
 void adamw_step(const Tensor& master, const Tensor& grad, const Tensor& m, const Tensor& v, const std::optional<Tensor>& model,
                 int64_t n_decay, double lr, double beta1, double beta2, double eps, double weight_decay, int64_t step,
                 double grad_scale, double max_norm, const Tensor& norm, const Tensor& counter, const std::optional<Tensor>& step_dev) {
+    pybind11::gil_scoped_release nogil;
     const int dt = grad.scalar_type() == at::kBFloat16 ? 11 : grad.scalar_type() == at::kFloat ? 9 : -1;
     void* st = stream_of(master);
     const bool clip = max_norm > 0;

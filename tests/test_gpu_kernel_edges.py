@@ -404,3 +404,63 @@ def test_small_allreduce_against_a_barrier_is_reported(W, n):
     assert {group.status(r) for r in range(W)} == {7}
     assert all(bool((t == r + 1).all()) for r, t in enumerate(x))
     group.close()
+
+
+@pytest.mark.parametrize("call", ["allreduce", "route", "dispatch", "combine", "gemm", "adamw", "layer_norm", "xent"])
+def test_launch_into_a_full_queue_leaves_other_threads_running(call):
+    """The stream is busy for half a second and more calls are issued than its queue holds, so that one of them has to wait.  A
+    thread that only ticks must not stand still for as long."""
+    import threading
+    import time
+
+    from oneccl_b200.ops.device_group import DeviceGroup
+    from oneccl_b200.ops.gemm import gemm_bf16
+    from oneccl_b200.ops.nn import add_layer_norm
+    from oneccl_b200.ops.train import FlatAdamW, softmax_cross_entropy
+    from oneccl_b200.parallel.ep import fused_combine, fused_dispatch, route_device
+
+    g = torch.Generator(device="cuda").manual_seed(0)
+    group = DeviceGroup.emulated(2, heap_bytes=40 << 20, staging_bytes=1 << 20)
+    x = [_bf16(g, 16, 64) for _ in range(2)]
+    logits = [torch.randn(16, 2, generator=g, device="cuda") for _ in range(2)]
+    idx, wts, counts, order, pos = zip(*(route_device(t, 1) for t in logits))
+    idx, wts = [i.view(-1) for i in idx], [w.view(-1) for w in wts]
+    meta, out = [torch.zeros(6, dtype=torch.int32, device="cuda") for _ in range(2)], [torch.empty_like(t) for t in x]
+    recv, table = group.symm_empty((32, 64), dtype=torch.bfloat16), group.symm_empty((1024,), dtype=torch.int32)
+    w, b = _bf16(g, 256), _bf16(g, 256)
+    h, opt, tgt = _bf16(g, 16, 256), FlatAdamW(_bf16(g, 1024), 512), torch.zeros(16, dtype=torch.int64, device="cuda")
+    fused_dispatch(group, x, order, counts, meta, recv, table, 1)
+    calls = {
+        "allreduce": lambda: group.allreduce(x, out), "route": lambda: route_device(logits[0], 1),
+        "dispatch": lambda: fused_dispatch(group, x, order, counts, meta, recv, table, 1),
+        "combine": lambda: fused_combine(group, idx, pos, wts, out, meta, recv, 1),
+        "gemm": lambda: gemm_bf16(h, h, out=None), "adamw": lambda: opt.step(opt_grad),
+        "layer_norm": lambda: add_layer_norm(h, h, w, b), "xent": lambda: softmax_cross_entropy(h, tgt),
+    }
+    opt_grad = _bf16(g, 1024)
+    for _ in range(3):
+        calls[call]()
+    torch.cuda.synchronize()
+    ticks, stop = [], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            ticks.append(time.perf_counter())
+            time.sleep(0.002)
+
+    ticker = threading.Thread(target=tick)
+    ticker.start()
+    busy = torch.cuda.Event()
+    torch.cuda._sleep(1_000_000_000)  # half a second at the highest clock
+    busy.record()
+    n = 0
+    while not busy.query() and n < 20000:
+        calls[call]()
+        n += 1
+    stop.set()
+    ticker.join()
+    torch.cuda.synchronize()
+    group.check()
+    group.close()
+    gap = max(b - a for a, b in zip(ticks, ticks[1:]))
+    assert gap < 0.2, f"{gap:.3f} s without a tick, {n} calls"
