@@ -61,12 +61,17 @@ def linear(x, weight, bias, defer_bias: bool = False, last_use: bool = True):
     if bias is None and getattr(weight, "_grad_sink", None) is None:
         return F.linear(x, weight)
     y = native().linear(x, weight, bias, not defer_bias, last_use)
-    return F.linear(x, weight, bias) if y is None else y
+    if y is None:  # the operator that consumes the output returns a deferred bias gradient in any case
+        return F.linear(x, weight, bias.detach() if defer_bias and bias is not None else bias)
+    return y
 
 
 def gelu(u, bias):
     """tanh-form GELU of ``u``, the output of a ``linear(..., bias, defer_bias=True)``."""
-    return native().bias_gelu(u, bias)
+    y = native().bias_gelu(u, bias)
+    if y is None:  # adds nothing, but hands the bias its gradient
+        return F.gelu(u + (bias - bias.detach()).to(u.dtype), approximate="tanh")
+    return y
 
 
 def split_qkv(qkv: torch.Tensor, n_head: int, bias=None):

@@ -227,6 +227,15 @@ variable_list add_layer_norm_fwd(const Tensor& x, const std::optional<Tensor>& r
     return { y };
 }
 
+bool bf16_cuda(const Tensor& t) {
+    return t.is_cuda() && t.scalar_type() == at::kBFloat16;
+}
+
+// whether the kernels can write the gradient of bias `b` of a layer with `n` outputs, beside `x`
+bool bias_ok(const Tensor& b, const Tensor& x, int64_t n) {
+    return bf16_cuda(b) && b.device() == x.device() && b.dim() == 1 && b.size(0) == n;
+}
+
 bool ln_param_ok(const Tensor& p, int64_t D) {
     return p.scalar_type() == at::kBFloat16 && p.is_cuda() && p.numel() == D && p.is_contiguous() && aligned16(p);
 }
@@ -255,6 +264,8 @@ pybind11::object add_layer_norm(const Tensor& x, const std::optional<Tensor>& re
     if (!layer_norm_ok(x, res, w, b))
         return pybind11::none();
     const auto res_bias = maybe_tensor(res_bias_);
+    if (res_bias && (!res || !bias_ok(*res_bias, x, x.size(-1))))
+        return pybind11::none();
     std::vector<SinkRef> sinks{ sink_of(w_), sink_of(b_), sink_of(res_bias_) };
     variable_list out;
     {
@@ -337,15 +348,11 @@ struct Linear : torch::autograd::Function<Linear> {
     }
 };
 
-bool bf16_cuda(const Tensor& t) {
-    return t.is_cuda() && t.scalar_type() == at::kBFloat16;
-}
-
 // None where the operator does not take the call
 pybind11::object linear(const Tensor& x, const pybind11::object& w_, const pybind11::object& b_, bool bias_grad, bool report) {
     const Tensor w = tensor_of(w_);
     const auto b = maybe_tensor(b_);
-    if (!bf16_cuda(x) || !bf16_cuda(w) || w.dim() != 2 || w.size(0) % 8 != 0 || (b && !bf16_cuda(*b)))
+    if (!bf16_cuda(x) || !bf16_cuda(w) || w.dim() != 2 || w.size(0) % 8 != 0 || (b && !bias_ok(*b, x, w.size(0))))
         return pybind11::none();
     std::vector<SinkRef> sinks{ sink_of(w_), sink_of(b_) };
     pybind11::gil_scoped_release nogil;
@@ -386,11 +393,16 @@ struct BiasGelu : torch::autograd::Function<BiasGelu> {
     }
 };
 
-Tensor bias_gelu(const Tensor& u, const pybind11::object& b_) {
-    std::vector<SinkRef> sinks{ sink_of(b_) };
+// None where the operator does not take the call
+pybind11::object bias_gelu(const Tensor& u, const pybind11::object& b_) {
     const Tensor b = tensor_of(b_);
+    if (!bf16_cuda(u) || u.dim() < 1 || u.size(-1) == 0 || u.size(-1) % 8 != 0 || !bias_ok(b, u, u.size(-1)))
+        return pybind11::none();
+    std::vector<SinkRef> sinks{ sink_of(b_) };
     pybind11::gil_scoped_release nogil;
-    return BiasGelu::apply(u, b, std::move(sinks))[0];
+    Tensor y = BiasGelu::apply(u, b, std::move(sinks))[0];
+    pybind11::gil_scoped_acquire gil;
+    return pybind11::cast(y);
 }
 
 // views of a packed QKV projection for the attention call; backward assembles the packed gradient in one pass that also
@@ -440,8 +452,10 @@ struct SplitQKV : torch::autograd::Function<SplitQKV> {
 pybind11::object split_qkv(const Tensor& qkv, int64_t n_head, const pybind11::object& b_) {
     if (!bf16_cuda(qkv) || qkv.dim() != 3 || !qkv.is_contiguous() || qkv.size(2) / 3 / n_head % 8 != 0)
         return pybind11::none();
-    std::vector<SinkRef> sinks{ sink_of(b_) };
     const auto b = maybe_tensor(b_);
+    if (b && !bias_ok(*b, qkv, qkv.size(2)))
+        return pybind11::none();
+    std::vector<SinkRef> sinks{ sink_of(b_) };
     variable_list out;
     {
         pybind11::gil_scoped_release nogil;
