@@ -46,9 +46,23 @@ def combine_rows(y: torch.Tensor, pos: torch.Tensor, w: torch.Tensor, out: torch
     return out
 
 
-def _per_entry(group: DeviceGroup, t):
-    """Real mode takes one tensor, emulation a list with one tensor per rank."""
-    return [t] if isinstance(t, torch.Tensor) else t
+def _per_entry(group: DeviceGroup, t, dims: int):
+    """Real mode takes one tensor (of ``dims`` dimensions), emulation one per rank: a list, or a tensor that stacks them.  A single
+    emulated rank may pass a bare tensor."""
+    if not isinstance(t, torch.Tensor):
+        ts = t
+    elif group.emulated_mode and (group.world > 1 or t.dim() > dims and t.shape[0] == 1):
+        ts = list(t)
+    else:
+        ts = [t]
+    if len(ts) != group.n_entries:
+        raise ValueError(f"{len(ts)} tensors for {group.n_entries} ranks")
+    return ts
+
+
+def _symmetric(t, dims: int):
+    """A symmetric allocation as ``symm_empty`` returns it (emulation: one tensor per rank, of which the first stands for all)."""
+    return t if isinstance(t, torch.Tensor) and t.dim() <= dims else t[0]
 
 
 def fused_dispatch(group: DeviceGroup, x, order, send_counts, meta, recv_buf, cnt_table, topk: int, blocks: int = 0):
@@ -57,9 +71,10 @@ def fused_dispatch(group: DeviceGroup, x, order, send_counts, meta, recv_buf, cn
     (int32, >= 256 * world**2) are symmetric allocations; ``meta`` (int32 [2 * world + 2]) receives the row
     offsets, the number of rows this rank's expert got (``meta[2 * world]``) and an overflow flag."""
     global launches
-    xs, orders, counts, metas = (_per_entry(group, v) for v in (x, order, send_counts, meta))
-    native().moe_dispatch(group.handle.value, xs, orders, counts, metas, _per_entry(group, recv_buf)[0],
-                          _per_entry(group, cnt_table)[0], topk, blocks)
+    xs = _per_entry(group, x, 2)
+    orders, counts, metas = (_per_entry(group, v, 1) for v in (order, send_counts, meta))
+    native().moe_dispatch(group.handle.value, xs, orders, counts, metas, _symmetric(recv_buf, 2),
+                          _symmetric(cnt_table, 1), topk, blocks)
     launches += 1
 
 
@@ -68,8 +83,9 @@ def fused_combine(group: DeviceGroup, expert, pos, weight, out, meta, expert_out
     peer loads.  ``expert_out`` is the symmetric [cap, hidden] bf16 buffer every expert wrote its rows to,
     in the order ``fused_dispatch`` delivered them."""
     global launches
-    es, ps, ws, outs, metas = (_per_entry(group, v) for v in (expert, pos, weight, out, meta))
-    native().moe_combine(group.handle.value, es, ps, ws, outs, metas, _per_entry(group, expert_out)[0], topk, blocks)
+    es, ps, ws, metas = (_per_entry(group, v, 1) for v in (expert, pos, weight, meta))
+    native().moe_combine(group.handle.value, es, ps, ws, _per_entry(group, out, 2), metas, _symmetric(expert_out, 2), topk,
+                         blocks)
     launches += 1
 
 
