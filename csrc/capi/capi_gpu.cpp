@@ -44,8 +44,13 @@ CCLX_API int cclx_cuda_device_count() {
 // The library carries its own (static) CUDA runtime, whose notion of the
 // current device is per thread and independent of the caller's runtime: the
 // bindings call this before every launch with the caller's current device.
+// Asked of the runtime each time and not remembered by callers: groups, collectives and other threads' work set it too.
 CCLX_API int cclx_set_device(int dev) {
-    return capi::guard([&] { CUDA_CHECK(cudaSetDevice(dev)); });
+    return capi::guard([&] {
+        int now = -1;
+        if (cudaGetDevice(&now) != cudaSuccess || now != dev)
+            CUDA_CHECK(cudaSetDevice(dev));
+    });
 }
 
 // ---- emulated group (all ranks on the current device) ---------------------------

@@ -92,11 +92,7 @@ inline void check(int rc) {
 // The library has its own CUDA runtime, whose current device is per thread as well: it follows the device of the call
 // (autograd runs backward on threads of its own).
 inline void set_device(int dev) {
-    thread_local int current = -1;
-    if (current != dev) {
-        check(cclx_set_device(dev));
-        current = dev;
-    }
+    check(cclx_set_device(dev));
 }
 
 inline void* stream_of(const Tensor& t) {

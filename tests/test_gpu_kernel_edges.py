@@ -464,3 +464,21 @@ def test_launch_into_a_full_queue_leaves_other_threads_running(call):
     group.close()
     gap = max(b - a for a, b in zip(ticks, ticks[1:]))
     assert gap < 0.2, f"{gap:.3f} s without a tick, {n} calls"
+
+
+def test_operators_follow_their_tensors_device():
+    """Other code of the library may have set another device on this thread since the last operator."""
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs 2 GPUs")
+    from oneccl_b200 import _lib
+    from oneccl_b200.ops.gemm import gemm_bf16
+    from oneccl_b200.ops.nn import layer_norm
+
+    for dev in (0, 1):
+        with torch.cuda.device(dev):
+            a, w = torch.ones(8, 256, device="cuda", dtype=torch.bfloat16), torch.ones(256, 256, device="cuda", dtype=torch.bfloat16)
+            for other in (None, 1 - dev):
+                if other is not None:
+                    _lib.load().cclx_set_device(other)
+                assert bool((gemm_bf16(a, w, check=True) == 256).all())
+                assert bool((layer_norm(a, w[0], w[0]) == 1).all())
