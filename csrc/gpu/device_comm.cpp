@@ -154,12 +154,7 @@ const void* device_comm::emu_table(int kind, const void* data, size_t bytes, cud
     CCL_THROW_IF_NOT(capturing == cudaStreamCaptureStatusNone, "launches of several emulated ranks cannot be captured");
     std::lock_guard<std::mutex> g(emu_mu_);
     char* dst = emu_dev_ + kind * emu_slot_bytes();
-    std::vector<char>& last = emu_last_[kind];
-    if (last.size() != bytes || emu_stream_[kind] != st || std::memcmp(last.data(), data, bytes) != 0) {
-        last.assign((const char*)data, (const char*)data + bytes);
-        emu_stream_[kind] = st;
-        CUDA_CHECK(cudaMemcpyAsync(dst, last.data(), bytes, cudaMemcpyHostToDevice, st));
-    }
+    emu_held_[kind].put(data, bytes, st, [&] { CUDA_CHECK(cudaMemcpyAsync(dst, data, bytes, cudaMemcpyHostToDevice, st)); });
     return dst;
 }
 

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "core/types.hpp"
+#include "gpu/arg_table.hpp"
 #include "gpu/device/coll_args.hpp"
 #include "gpu/device/layout.hpp"
 #include "gpu/symm_heap.hpp"
@@ -65,10 +66,10 @@ public:
     int sm_count() const { return sm_count_; }
     int max_blocks() const; // per rank, keeps every block co-resident
     int threads() const { return threads_; }
-    // Emulation: the per-rank argument table of a launch in device memory.  `kind` names the table's layout.  A table equal
+    // Emulation: the per-rank argument table of a launch in device memory, one per `kind` of call.  A table equal
     // to the last one of its kind is still there; another one is copied over it in stream order (operations of one
     // communicator are ordered among themselves).  No host wait: the runtime takes a small pageable source at once.
-    enum { EMU_COLL = 0, EMU_P2P = 1, EMU_MOE = 2, EMU_KINDS = 3 };
+    enum { EMU_COLL, EMU_P2P, EMU_DISPATCH, EMU_COMBINE, EMU_KINDS };
     const void* emu_table(int kind, const void* data, size_t bytes, cudaStream_t st);
     int device_id() const { return device_id_; }
     size_t staging_bytes() const { return heap_.regions().staging_bytes; }
@@ -149,8 +150,7 @@ private:
         return (size_t)world_ * (sizeof(dev::rank_args) > sizeof(dev::p2p_ops) ? sizeof(dev::rank_args) : sizeof(dev::p2p_ops));
     }
     char* emu_dev_ = nullptr; // a table per kind, part of the allocation at state_dev_
-    std::vector<char> emu_last_[EMU_KINDS]; // what they hold
-    cudaStream_t emu_stream_[EMU_KINDS] = {}; // and in whose order it was written
+    arg_table emu_held_[EMU_KINDS]; // what they hold
     std::mutex emu_mu_;
     int device_id_ = 0;
     int sm_count_ = 0;

@@ -554,7 +554,7 @@ void launch_moe(gpu::device_comm& dc, bool dispatch, moe_args& a, const moe_rank
     if (dc.emulated()) {
         static_assert(sizeof(moe_rank_args) <= sizeof(dev::rank_args), "argument block too large");
         a.emu = 1;
-        a.emu_tab = (const moe_rank_args*)dc.emu_table(dispatch ? gpu::device_comm::EMU_COLL : gpu::device_comm::EMU_MOE, ra,
+        a.emu_tab = (const moe_rank_args*)dc.emu_table(dispatch ? gpu::device_comm::EMU_DISPATCH : gpu::device_comm::EMU_COMBINE, ra,
                                                        dc.world() * sizeof(moe_rank_args), st);
         const comm_dev* tab = dc.table();
         void* argv[] = { (void*)&tab, (void*)&a };
