@@ -487,9 +487,10 @@ struct Embed : torch::autograd::Function<Embed> {
         const ParamGrad gt(sinks[0], tokens, tokens.sizes()), gp(sinks[1], positions, positions.sizes());
         if (!gt.add) // only the rows of tokens that occur are touched
             gt.out.zero_();
+        const Tensor ws = empty_on(dx, { idx.numel() }, at::kByte);
         check(cclx_embed_bwd(reinterpret_cast<const long long*>(idx.data_ptr<int64_t>()), dx.data_ptr(), gt.ptr(), gp.ptr(), gp.add,
                              (int)idx.size(0), (int)idx.size(1), (int)tokens.size(0), (int)positions.size(0), (int)D,
-                             stream_of(dx)));
+                             ws.data_ptr(), stream_of(dx)));
         launches += 2;
         gp.done();
         gt.done();

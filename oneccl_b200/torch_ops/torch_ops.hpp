@@ -49,7 +49,7 @@ int cclx_embed_fwd(const long long* idx, const void* tokens, const void* positio
                    int D, void* stream);
 int cclx_embed_bwd_max_ids();
 int cclx_embed_bwd(const long long* idx, const void* dx, void* token_grad, void* pos_grad, int add_pos, int B, int S,
-                   int token_rows, int pos_rows, int D, void* stream);
+                   int token_rows, int pos_rows, int D, void* workspace, void* stream);
 int cclx_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int ctas, void* err_words,
                    void* stream);
 int cclx_gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int clusters,

@@ -482,3 +482,48 @@ def test_operators_follow_their_tensors_device():
                     _lib.load().cclx_set_device(other)
                 assert bool((gemm_bf16(a, w, check=True) == 256).all())
                 assert bool((layer_norm(a, w[0], w[0]) == 1).all())
+
+
+@pytest.mark.parametrize("D", [8, 1032, 2056])
+@pytest.mark.parametrize("counts", [(64,), (65,), (63, 64, 65), (128, 129, 1, 700, 65), (16384,), (8191, 8193), (65,) * 252, (1,) * 100])
+def test_embedding_gradients_of_frequent_tokens(counts, D):
+    """Tokens around the length of a warp's list, all positions one token, many frequent tokens; ids outside the table among
+    them.  Gradients are whole numbers: the sum is exact in fp32 and rounded once."""
+    from oneccl_b200.ops.nn import embed
+
+    g = torch.Generator(device="cuda").manual_seed(len(counts) + D)
+    ids = torch.cat([torch.full((c,), 3 * t + 1) for t, c in enumerate(counts)])
+    table = 3 * len(counts) + 2
+    if ids.numel() < 16384:
+        ids = torch.cat([ids, torch.full((3,), table + 5)])  # gradient rows that nobody takes
+    idx = ids[torch.randperm(ids.numel(), generator=torch.Generator().manual_seed(1))].cuda()[None]
+    tok, pos = _bf16(g, table, D).requires_grad_(True), _bf16(g, idx.numel(), D).requires_grad_(True)
+    dx = torch.randint(-3, 4, (1, idx.numel(), D), generator=g, device="cuda").to(torch.bfloat16)
+    want = torch.zeros(table + 6, D, device="cuda", dtype=torch.float64).index_add_(0, idx[0], dx[0].double())[:table]
+    for _ in range(2):
+        dt, dp = torch.autograd.grad(embed(idx, tok, pos), [tok, pos], dx)
+        assert torch.equal(dt, want.to(torch.bfloat16))
+        assert torch.equal(dp, dx[0])
+
+
+def test_embedding_gradient_of_a_padded_batch_takes_no_longer():
+    """Nine of ten positions hold the padding token: the time stays near that of a batch of different tokens."""
+    from oneccl_b200.ops.nn import embed
+
+    g = torch.Generator(device="cuda").manual_seed(0)
+    tok, pos = _bf16(g, 50304, 1024).requires_grad_(True), _bf16(g, 1024, 1024).requires_grad_(True)
+    dx, times = _bf16(g, 8, 1024, 1024), []
+    for padded in (0.0, 0.9):
+        idx = torch.randint(0, 50304, (8, 1024), generator=g, device="cuda")
+        idx[torch.rand(8, 1024, generator=g, device="cuda") < padded] = 0
+        y = embed(idx, tok, pos)
+        best = 1e9
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            torch.autograd.grad(y, [tok, pos], dx, retain_graph=True)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        times.append(best)
+    assert times[1] < 4 * times[0] + 0.1, times  # ms; one warp for all of them took 45 times as long
