@@ -401,29 +401,24 @@ __global__ void __launch_bounds__(128) map_colsum_kernel(F f, size_t rows, int p
     out[1] = make_float4(s[4], s[5], s[6], s[7]);
 }
 
-// Gaussian error linear unit, tanh form: 0.5 x (1 + tanh(u)), u = sqrt(2 / pi) (x + 0.044715 x^3).
+// Gaussian error linear unit, tanh form: 0.5 x (1 + tanh(u)) = x g with g = 1 / (1 + exp(-2 u)), u = sqrt(2 / pi) (x + 0.044715 x^3).
 //
-// tanh(u) = 2 / (1 + exp(-2 u)) - 1 is rounded to fp32 before the 1 is added back.  x / (1 + exp(-2 u)) would be the same
-// product with one rounding less, and nearer to the true value below x = -3, but there other bf16 values than the operator
-// of the same name in the framework around it gives: a handful of activations per layer, from which every later one of
-// the sequence rounds differently (1.3 % in the gradients of a 24-layer step).  In this form all 65536 bf16 inputs give
-// that operator's bits, and an infinite or huge negative x its NaN or zero, at the same 23 us for 8192 x 4096 values
-// (tanhf: 31 us).
-__device__ __forceinline__ float gelu_tanh(float x) {
+// g is rounded where tanh(u) = 2 g - 1 is rounded to fp32 before the 1 is added back.  Without that the result is nearer to the
+// true value below x = -3, but there other bf16 values than the operator of the same name in the framework around it gives: a
+// handful of activations per layer, from which every later one of the sequence rounds differently (1 % in the gradients of
+// a 24-layer step).  With it all 65536 bf16 inputs give that operator's bits, and an infinite or huge negative x its
+// NaN or zero, in the same 20 us for 8192 x 4096 values (tanhf: 31 us).
+__device__ __forceinline__ float gelu_gate(float x) {
     constexpr float C = -2.f * 0.7978845608028654f * 1.4426950408889634f; // -2 sqrt(2 / pi) log2(e)
-    float e;
-    const float t = C * x * fmaf(0.044715f * x, x, 1.f);
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t));
-    return __fdividef(2.f, 1.f + fminf(e, 1e37f)) - 1.f; // within __fdividef's range
+    float e, g;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(C * x * fmaf(0.044715f * x, x, 1.f)));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(g) : "f"(1.f + e));
+    return (g - 0.5f) + 0.5f;
 }
-__device__ __forceinline__ float gelu(float x) {
-    return 0.5f * x * (1.f + gelu_tanh(x));
-}
-// its derivative 0.5 (1 + tanh(u)) + 0.5 x (1 - tanh(u)^2) u'
-__device__ __forceinline__ float gelu_slope(float x) {
-    const float th = gelu_tanh(x);
-    const float du = 0.7978845608028654f * (1.f + 3.f * 0.044715f * (x * x));
-    return 0.5f * (1.f + th) + 0.5f * x * (1.f - th * th) * du;
+__device__ __forceinline__ float gelu_slope(float x) { // g + 2 x g (1 - g) u'
+    constexpr float K = 2.f * 0.7978845608028654f;
+    const float g = gelu_gate(x);
+    return fmaf(x * g * (1.f - g), fmaf(K * 3.f * 0.044715f, x * x, K), g);
 }
 
 __global__ void __launch_bounds__(256) gelu_fwd_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, size_t packs) {
@@ -440,7 +435,7 @@ __global__ void __launch_bounds__(256) gelu_fwd_kernel(const uint4* __restrict__
             unpack8(u[k], v);
 #pragma unroll
             for (int e = 0; e < 8; e++)
-                v[e] = gelu(v[e]);
+                v[e] *= gelu_gate(v[e]);
             y[i0 + k * 256] = pack8(v);
         }
 }
