@@ -192,6 +192,7 @@ variable_list add_layer_norm_fwd(const Tensor& x, const std::optional<Tensor>& r
                                  double eps, const std::optional<Tensor>& res_bias, std::vector<SinkRef> sinks) {
     const Tensor none;
     const Tensor &r = res ? *res : none, &rb = res_bias ? *res_bias : none;
+    no_tangent("the fused LayerNorm", { x, r, weight, bias, rb });
     const bool grad = torch::autograd::compute_requires_grad(x, r, weight, bias, rb);
     Tensor xd, y, total, stats;
     {

@@ -13,6 +13,8 @@
 
 #include <atomic>
 #include <deque>
+#include <functional>
+#include <initializer_list>
 #include <mutex>
 #include <optional>
 #include <stdexcept>
@@ -99,6 +101,12 @@ inline void* stream_of(const Tensor& t) {
     const int dev = t.get_device();
     set_device(dev);
     return at::cuda::getCurrentCUDAStream(dev).stream();
+}
+
+// Operators written as plain autograd nodes have backward alone: a tangent must not get lost in them.
+inline void no_tangent(const char* op, std::initializer_list<std::reference_wrapper<const Tensor>> inputs) {
+    for (const Tensor& t : inputs)
+        TORCH_CHECK_NOT_IMPLEMENTED(!t.defined() || !t._fw_grad(0).defined(), "forward-mode differentiation is not implemented for ", op);
 }
 
 extern std::atomic<long long> launches; // kernels of the library launched through this module

@@ -31,6 +31,7 @@ struct SoftmaxXentBackward : torch::autograd::Node {
 
 Tensor softmax_xent(const Tensor& logits, const Tensor& targets_, int64_t vocab, bool scale) {
     TORCH_CHECK(logits.is_cuda() && targets_.is_cuda(), "the fused cross-entropy takes CUDA tensors");
+    no_tangent("the fused cross-entropy", { logits });
     pybind11::gil_scoped_release nogil;
     const Tensor targets = targets_.is_contiguous() ? targets_ : targets_.contiguous();
     const int64_t rows = logits.size(0), cols = logits.size(1);

@@ -527,3 +527,24 @@ def test_embedding_gradient_of_a_padded_batch_takes_no_longer():
             best = min(best, a.elapsed_time(b))
         times.append(best)
     assert times[1] < 4 * times[0] + 0.1, times  # ms; one warp for all of them took 45 times as long
+
+
+def test_tangents_are_not_lost():
+    """The fused operators have no forward-mode derivative and say so."""
+    import torch.autograd.forward_ad as fwAD
+
+    from oneccl_b200.ops import nn as K
+    from oneccl_b200.ops.train import softmax_cross_entropy
+
+    g = torch.Generator(device="cuda").manual_seed(0)
+    x, w, b = _bf16(g, 8, 256), _bf16(g, 256), _bf16(g, 256)
+    idx = torch.zeros(1, 8, dtype=torch.int64, device="cuda")
+    with fwAD.dual_level():
+        dual = fwAD.make_dual(x, torch.ones_like(x))
+        dual_w = fwAD.make_dual(w, torch.ones_like(w))
+        for f in (lambda: K.layer_norm(dual, w, b), lambda: K.add_layer_norm(x, dual, w, b), lambda: K.layer_norm(x, dual_w, b),
+                  lambda: K.layer_norm(x, w, dual_w), lambda: K.add_layer_norm(x, x, w, b, res_bias=dual_w),
+                  lambda: softmax_cross_entropy(dual, idx[0]), lambda: K.linear(dual, x[:8], b[:8]), lambda: K.gelu(dual, b),
+                  lambda: K.split_qkv(_bf16(g, 1, 8, 24), 1, dual_w[:24]), lambda: K.embed(idx, dual, x)):
+            with pytest.raises(RuntimeError, match="(?i)forward|jvp"):
+                f()
