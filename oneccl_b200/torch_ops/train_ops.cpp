@@ -10,6 +10,7 @@ using torch::autograd::variable_list;
 
 struct SoftmaxXentBackward : torch::autograd::Node {
     Tensor grad; // the logits' memory, which holds their gradient
+    int64_t version = 0; // of the logits: the kernel's write is not counted, any later one is
     bool scale = false;
 
     std::string name() const override {
@@ -24,6 +25,9 @@ struct SoftmaxXentBackward : torch::autograd::Node {
         if (!grads[0].defined())
             return { Tensor() };
         TORCH_CHECK(grad.defined(), "the logits' gradient has been freed: backward ran through the graph a second time");
+        TORCH_CHECK((int64_t)grad._version() == version,
+                    "one of the variables needed for gradient computation has been modified by an inplace operation: the logits hold "
+                    "their gradient after the fused cross-entropy");
         // the stored gradient assumes d(loss) = 1; scale only when the caller scaled the loss
         return { scale ? grad * grads[0].to(grad.scalar_type()) : grad };
     }
@@ -53,6 +57,7 @@ Tensor softmax_xent(const Tensor& logits, const Tensor& targets_, int64_t vocab,
         std::shared_ptr<SoftmaxXentBackward> node(new SoftmaxXentBackward(), torch::autograd::deleteNode);
         node->set_next_edges(torch::autograd::collect_next_edges(logits));
         node->grad = logits.detach();
+        node->version = (int64_t)logits._version();
         node->scale = scale;
         torch::autograd::set_history(mean, node);
     }

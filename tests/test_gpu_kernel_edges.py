@@ -548,3 +548,19 @@ def test_tangents_are_not_lost():
                   lambda: K.split_qkv(_bf16(g, 1, 8, 24), 1, dual_w[:24]), lambda: K.embed(idx, dual, x)):
             with pytest.raises(RuntimeError, match="(?i)forward|jvp"):
                 f()
+
+
+def test_softmax_xent_notices_modified_logits():
+    from oneccl_b200.ops.train import softmax_cross_entropy
+
+    g = torch.Generator(device="cuda").manual_seed(0)
+    tgt = torch.zeros(8, dtype=torch.int64, device="cuda")
+    x = _bf16(g, 8, 64).requires_grad_(True)
+    loss = softmax_cross_entropy(x, tgt)
+    with torch.no_grad():
+        x.zero_()
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        loss.backward()
+    y = x * 1.0  # the output of another operator, used by itself
+    softmax_cross_entropy(y, tgt).backward()
+    torch.testing.assert_close(x.grad.float().sum(1), torch.zeros(8, device="cuda"), rtol=0, atol=64 * 2.0**-12)
