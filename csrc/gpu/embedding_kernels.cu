@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <mutex>
 
 #include "capi/capi_common.hpp"
 #include "core/log.hpp"
@@ -18,18 +19,36 @@ using namespace cclx::gpu;
 
 namespace {
 
+// Word in mapped host memory that a kernel sets when it meets an id outside the table.  The host looks at it without waiting, so
+// an error is reported by a later call.
+int* bad_id_word() {
+    static std::once_flag once;
+    static int* word = nullptr;
+    std::call_once(once, [] {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed; // an allocation is allowed beside this thread's capture
+        CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode));
+        const cudaError_t e = cudaHostAlloc((void**)&word, 64, cudaHostAllocMapped | cudaHostAllocPortable);
+        CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode));
+        CUDA_CHECK(e);
+        *word = 0;
+    });
+    return word;
+}
+
 // out[i] = tokens[idx[i]] + positions[i % S]; one thread per 16-byte pack
 __global__ void __launch_bounds__(128) embed_fwd_kernel(const long long* __restrict__ idx, const uint4* __restrict__ tokens,
                                                         const uint4* __restrict__ positions, uint4* __restrict__ out, size_t n,
-                                                        int S, int table_rows, int packs) {
+                                                        int S, int table_rows, int packs, volatile int* bad_id) {
     const size_t i = (size_t)blockIdx.x * 128 + threadIdx.x;
     const size_t row = i / packs;
     if (row >= n)
         return;
     const int p = (int)(i - row * packs);
     f32x2 a[4], b[4];
-    // an id outside the table reads nothing and makes its row NaN
+    // an id outside the table reads nothing, makes its row NaN and is reported
     const bool ok = (unsigned long long)idx[row] < (unsigned long long)table_rows;
+    if (!ok && p == 0)
+        *bad_id = 1;
     unpack4x2(ok ? tokens[(size_t)idx[row] * packs + p] : make_uint4(~0u, ~0u, ~0u, ~0u), a);
     unpack4x2(positions[(row % S) * packs + p], b);
 #pragma unroll
@@ -266,6 +285,13 @@ __global__ void __launch_bounds__(EMBED_POS_THREADS)
 
 } // namespace
 
+// Whether a cclx_embed_fwd that has run met an id outside its table; clears the answer.
+CCLX_API int cclx_embed_bad_id() {
+    int bad = 0;
+    const int rc = cclx::capi::guard([&] { bad = __atomic_exchange_n(bad_id_word(), 0, __ATOMIC_RELAXED); });
+    return rc == 0 ? bad : 0;
+}
+
 // out[b, s, :] = tokens[idx[b, s], :] + positions[s, :]; bf16, D a multiple of 8
 CCLX_API int cclx_embed_fwd(const long long* idx, const void* tokens, const void* positions, void* out, size_t n, int S,
                             int table_rows, int D, void* stream) {
@@ -275,7 +301,7 @@ CCLX_API int cclx_embed_fwd(const long long* idx, const void* tokens, const void
         if (total == 0)
             return;
         embed_fwd_kernel<<<(unsigned)((total + 127) / 128), 128, 0, (cudaStream_t)stream>>>(
-            idx, (const uint4*)tokens, (const uint4*)positions, (uint4*)out, n, S, table_rows, D / 8);
+            idx, (const uint4*)tokens, (const uint4*)positions, (uint4*)out, n, S, table_rows, D / 8, bad_id_word());
         CUDA_CHECK(cudaGetLastError());
     });
 }

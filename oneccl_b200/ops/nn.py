@@ -86,7 +86,10 @@ def split_qkv(qkv: torch.Tensor, n_head: int, bias=None):
 
 
 def embed(idx, tokens, positions):
-    """tokens[idx] + positions[: S] for ids [B, S]."""
+    """tokens[idx] + positions[: S] for ids [B, S].  An id outside the table makes its row NaN; as the GPU finds out, a later
+    ``embed``, its backward or ``GraphedTrainStep`` call raises the IndexError."""
+    if idx.dim() == 2 and idx.shape[1] > positions.shape[0]:
+        raise IndexError(f"{idx.shape[1]} positions, but a table of {positions.shape[0]}")
     x = native().embed(idx, tokens, positions)
     if x is None:
         return F.embedding(idx, tokens) + positions[: idx.shape[1]]

@@ -357,6 +357,7 @@ class GraphedTrainStep:
         torch.cuda.synchronize()
 
     def __call__(self, idx: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
+        native().embed_check()  # of an earlier replay
         self.idx.copy_(idx, non_blocking=True)
         self.targets.copy_(targets, non_blocking=True)
         self.graph.replay()

@@ -465,6 +465,11 @@ pybind11::object split_qkv(const Tensor& qkv, int64_t n_head, const pybind11::ob
     return pybind11::make_tuple(out[0], out[1], out[2]);
 }
 
+// An id outside the table is found by the kernel: its row is NaN, and the next call on any thread reports it.
+void embed_check() {
+    TORCH_CHECK_INDEX(!cclx_embed_bad_id(), "an earlier embedding was given a token id outside its table");
+}
+
 // token embedding + position embedding of [B, S] ids
 struct Embed : torch::autograd::Function<Embed> {
     static variable_list forward(AutogradContext* ctx, const Tensor& idx, const Tensor& tokens, const Tensor& positions,
@@ -480,6 +485,7 @@ struct Embed : torch::autograd::Function<Embed> {
     }
 
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        embed_check();
         const auto saved = ctx->get_saved_variables();
         const Tensor &idx = saved[0], &tokens = saved[1], &positions = saved[2];
         const int64_t D = tokens.size(1);
@@ -507,6 +513,7 @@ pybind11::object embed(const Tensor& idx_, const pybind11::object& tokens_, cons
         idx_.size(1) > positions.size(0) || idx_.numel() == 0 || !tokens.is_contiguous() || !positions.is_contiguous() ||
         !aligned16(tokens) || !aligned16(positions))
         return pybind11::none();
+    embed_check();
     const Tensor idx = idx_.contiguous();
     std::vector<SinkRef> sinks{ sink_of(tokens_), sink_of(positions_) };
     pybind11::gil_scoped_release nogil;
@@ -531,6 +538,7 @@ void bind_nn(pybind11::module_& m) {
     m.def("bias_gelu", &bias_gelu);
     m.def("split_qkv", &split_qkv);
     m.def("embed", &embed);
+    m.def("embed_check", &embed_check);
     m.def("colsum", &colsum);
 }
 

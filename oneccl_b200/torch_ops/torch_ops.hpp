@@ -49,6 +49,7 @@ int cclx_qkv_grad_colsum(const void* const* src, const long long* strides, void*
 int cclx_partial_sums(const float* workspace, int n, int cols, int outputs, void* out0, void* out1, void* out2, int add, void* stream);
 int cclx_embed_fwd(const long long* idx, const void* tokens, const void* positions, void* out, size_t n, int S, int table_rows,
                    int D, void* stream);
+int cclx_embed_bad_id();
 int cclx_embed_bwd_max_ids();
 int cclx_embed_bwd(const long long* idx, const void* dx, void* token_grad, void* pos_grad, int add_pos, int B, int S,
                    int token_rows, int pos_rows, int D, void* workspace, void* stream);

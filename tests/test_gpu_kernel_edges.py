@@ -487,19 +487,17 @@ def test_operators_follow_their_tensors_device():
 @pytest.mark.parametrize("D", [8, 1032, 2056])
 @pytest.mark.parametrize("counts", [(64,), (65,), (63, 64, 65), (128, 129, 1, 700, 65), (16384,), (8191, 8193), (65,) * 252, (1,) * 100])
 def test_embedding_gradients_of_frequent_tokens(counts, D):
-    """Tokens around the length of a warp's list, all positions one token, many frequent tokens; ids outside the table among
-    them.  Gradients are whole numbers: the sum is exact in fp32 and rounded once."""
+    """Tokens around the length of a warp's list, all positions one token, many frequent tokens.  Gradients are whole numbers: the
+    sum is exact in fp32 and rounded once."""
     from oneccl_b200.ops.nn import embed
 
     g = torch.Generator(device="cuda").manual_seed(len(counts) + D)
     ids = torch.cat([torch.full((c,), 3 * t + 1) for t, c in enumerate(counts)])
     table = 3 * len(counts) + 2
-    if ids.numel() < 16384:
-        ids = torch.cat([ids, torch.full((3,), table + 5)])  # gradient rows that nobody takes
     idx = ids[torch.randperm(ids.numel(), generator=torch.Generator().manual_seed(1))].cuda()[None]
     tok, pos = _bf16(g, table, D).requires_grad_(True), _bf16(g, idx.numel(), D).requires_grad_(True)
     dx = torch.randint(-3, 4, (1, idx.numel(), D), generator=g, device="cuda").to(torch.bfloat16)
-    want = torch.zeros(table + 6, D, device="cuda", dtype=torch.float64).index_add_(0, idx[0], dx[0].double())[:table]
+    want = torch.zeros(table, D, device="cuda", dtype=torch.float64).index_add_(0, idx[0], dx[0].double())
     for _ in range(2):
         dt, dp = torch.autograd.grad(embed(idx, tok, pos), [tok, pos], dx)
         assert torch.equal(dt, want.to(torch.bfloat16))
@@ -564,3 +562,44 @@ def test_softmax_xent_notices_modified_logits():
     y = x * 1.0  # the output of another operator, used by itself
     softmax_cross_entropy(y, tgt).backward()
     torch.testing.assert_close(x.grad.float().sum(1), torch.zeros(8, device="cuda"), rtol=0, atol=64 * 2.0**-12)
+
+
+def test_token_ids_outside_the_table_are_reported():
+    """In the call, and in a replayed step: the row is NaN, the next call raises once, and then all is as before."""
+    from oneccl_b200.models.gpt2 import GPT2, GPT2Config
+    from oneccl_b200.ops.device_group import DeviceGroup
+    from oneccl_b200.ops.nn import embed
+    from oneccl_b200.parallel.ddp import DataParallel, GraphedTrainStep
+
+    g = torch.Generator(device="cuda").manual_seed(0)
+    tok, pos = _bf16(g, 10, 64), _bf16(g, 4, 64)
+    for bad in (10, -1, 1 << 40):
+        idx = torch.tensor([[0, 9, 3, 3]], device="cuda")
+        idx[0, 2] = bad
+        x = embed(idx, tok, pos)
+        torch.cuda.synchronize()
+        assert bool(x[0, 2].isnan().all()) and torch.equal(x[0, [0, 1, 3]], tok[[0, 9, 3]] + pos[[0, 1, 3]])
+        with pytest.raises(IndexError, match="outside its table"):
+            embed(idx.clamp(0, 9), tok, pos)
+        embed(idx.clamp(0, 9), tok, pos)
+    tok.requires_grad_(True)
+    x = embed(torch.tensor([[10]], device="cuda"), tok, pos)
+    torch.cuda.synchronize()
+    with pytest.raises(IndexError, match="outside its table"):
+        x.sum().backward()
+    with pytest.raises(IndexError, match="5 positions"):
+        embed(torch.zeros(1, 5, dtype=torch.int64, device="cuda"), tok, pos)
+
+    cfg = GPT2Config(1, 4, 256, 16, 1000)
+    group = DeviceGroup.emulated(1, heap_bytes=64 << 20, staging_bytes=1 << 20)
+    ddp = DataParallel(GPT2(cfg).cuda().to(torch.bfloat16), group)
+    idx = torch.zeros(2, 16, dtype=torch.int64, device="cuda")
+    step = GraphedTrainStep(ddp, ddp.make_optimizer(device_step=True), idx, idx)
+    step(idx, idx)
+    step(idx + 5000, idx)
+    torch.cuda.synchronize()
+    with pytest.raises(IndexError, match="outside its table"):
+        step(idx, idx)
+    del step
+    ddp.close()
+    group.close()
