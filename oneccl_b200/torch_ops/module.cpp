@@ -43,7 +43,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         .def("join", [](GradStream& g, uintptr_t stream, int dev) {
             g.join(at::cuda::getStreamFromExternal(reinterpret_cast<cudaStream_t>(stream), (c10::DeviceIndex)dev));
         })
-        .def("finish", &GradStream::finish);
+        .def("finish", &GradStream::finish)
+        .def_property_readonly("handle", &GradStream::handle);
     py::class_<GradSink, SinkRef>(m, "GradSink")
         .def(py::init<Tensor, py::object>())
         .def_readonly("grad", &GradSink::grad)

@@ -124,9 +124,9 @@ inline Tensor empty_on(const Tensor& like, at::IntArrayRef sizes, at::ScalarType
 // A stream of their own for weight gradients that go to sinks: nothing else in backward waits for them, products of a few
 // hundred tokens leave most SMs idle, and a long product's last wave some.  One per DataParallel.
 //
-// The operands of a product must outlive it, but the allocator knows them as memory of the current stream: the operands of
-// the last DEPTH launches are kept, and the current stream waits for the oldest before its operands go.  The final sums of
-// bias, gamma and beta gradients run there as well.
+// The operands of a product must outlive it, but the allocator knows them as memory of the stream that is current at the launch:
+// the operands of the last DEPTH launches are kept, and their stream waits for the oldest before its operands go, whichever
+// stream is current by then.  The final sums of bias, gamma and beta gradients run there as well.
 class GradStream {
 public:
     explicit GradStream(int dev) : stream_(at::cuda::getStreamFromPool(false, (c10::DeviceIndex)dev)) {}
@@ -141,12 +141,10 @@ public:
             at::cuda::CUDAStreamGuard guard(stream_);
             product();
         }
-        held_.emplace_back();
+        held_.push_back({ {}, a, b, current });
         held_.back().done.record(stream_);
-        held_.back().a = a;
-        held_.back().b = b;
         if (held_.size() > DEPTH) {
-            held_.front().done.block(current);
+            held_.front().done.block(held_.front().home);
             held_.pop_front();
         }
     }
@@ -156,12 +154,19 @@ public:
         if (!held_.empty())
             held_.back().done.block(s);
     }
-    // the same for the current stream, at the end of a step
+    // the same for the current stream and those that the operands belong to, at the end of a step
     void finish() {
         std::lock_guard<std::mutex> g(mu_);
+        const auto current = at::cuda::getCurrentCUDAStream(stream_.device_index());
         if (!held_.empty())
-            held_.back().done.block(at::cuda::getCurrentCUDAStream(stream_.device_index()));
+            held_.back().done.block(current);
+        for (size_t i = 0; i < held_.size(); i++)
+            if (held_[i].home != current && (i == 0 || held_[i].home != held_[i - 1].home))
+                held_.back().done.block(held_[i].home);
         held_.clear();
+    }
+    uintptr_t handle() const {
+        return reinterpret_cast<uintptr_t>(stream_.stream());
     }
 
 private:
@@ -169,6 +174,7 @@ private:
     struct entry {
         at::cuda::CUDAEvent done;
         Tensor a, b;
+        at::cuda::CUDAStream home;
     };
     at::cuda::CUDAStream stream_;
     std::deque<entry> held_;

@@ -603,3 +603,38 @@ def test_token_ids_outside_the_table_are_reported():
     del step
     ddp.close()
     group.close()
+
+
+def test_gradient_stream_keeps_operands_until_their_stream_has_waited():
+    """Backward on one stream, ``finish`` on another: the memory of the operands belongs to the first, which has to wait for the
+    gradient stream before it may use it again."""
+    from oneccl_b200.models.gpt2 import GPT2, GPT2Config
+    from oneccl_b200.ops.device_group import DeviceGroup
+    from oneccl_b200.parallel.ddp import DataParallel
+
+    cfg = GPT2Config(1, 4, 256, 64, 1000)
+    group = DeviceGroup.emulated(1, heap_bytes=64 << 20, staging_bytes=1 << 20)
+    ddp = DataParallel(GPT2(cfg).cuda().to(torch.bfloat16), group)
+    idx, tgt = (torch.randint(0, cfg.vocab, (4, 64), device="cuda") for _ in range(2))
+    home, slow = torch.cuda.Stream(), torch.cuda.ExternalStream(ddp._grad_stream.handle)
+    for busy in (False, True):
+        torch.cuda.synchronize()
+        with torch.cuda.stream(home):
+            ddp.begin_step()
+            loss = ddp(idx, tgt)
+            if busy:
+                with torch.cuda.stream(slow):
+                    torch.cuda._sleep(400_000_000)  # 0.2 s at the highest clock
+            loss.backward()
+        del loss
+        ddp.finish()
+        after = home.record_event()
+        done = slow.record_event()
+        if busy:
+            import time
+
+            time.sleep(0.05)
+            assert not done.query() and not after.query()
+    torch.cuda.synchronize()
+    ddp.close()
+    group.close()
