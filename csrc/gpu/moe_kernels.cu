@@ -271,8 +271,8 @@ __global__ void __launch_bounds__(256)
 } // namespace
 
 // logits [n_tokens, n_experts] fp32 -> idx [n_tokens, topk] (int64), wts [n_tokens, topk] (fp32),
-// counts [n_experts] (int64), order / pos [n_tokens * topk] (int64).  scratch: n_experts 32-bit words; behind
-// `counts` (at most one word between) it is cleared together with them.
+// counts [n_experts] (int64), order / pos [n_tokens * topk] (int64).  scratch: n_experts 32-bit words; right
+// behind `counts` it is cleared together with them.
 CCLX_API int cclx_moe_route(const float* logits, int n_tokens, int n_experts, int topk, long long* idx, float* wts,
                             long long* counts, long long* order, long long* pos, void* scratch, void* stream) {
     return cclx::capi::guard([&] {
@@ -288,9 +288,8 @@ CCLX_API int cclx_moe_route(const float* logits, int n_tokens, int n_experts, in
                                   (unsigned long long*)counts, order, pos);
             return;
         }
-        const ptrdiff_t gap = (const char*)scratch - (const char*)(counts + n_experts);
-        if (gap >= 0 && gap <= 8)
-            CUDA_CHECK(cudaMemsetAsync(counts, 0, (sizeof(long long) + sizeof(unsigned int)) * n_experts + gap, st));
+        if (scratch == (void*)(counts + n_experts))
+            CUDA_CHECK(cudaMemsetAsync(counts, 0, (sizeof(long long) + sizeof(unsigned int)) * n_experts, st));
         else {
             CUDA_CHECK(cudaMemsetAsync(counts, 0, sizeof(long long) * n_experts, st));
             CUDA_CHECK(cudaMemsetAsync(scratch, 0, sizeof(unsigned int) * n_experts, st));

@@ -57,20 +57,20 @@ void allreduce(uintptr_t group, const tensors& send, const tensors& recv, int op
 pybind11::tuple route(const Tensor& logits_, int64_t topk) {
     const Tensor logits = logits_.scalar_type() == at::kFloat && logits_.is_contiguous() ? logits_ : logits_.to(at::kFloat).contiguous();
     const int64_t T = logits.size(0), E = logits.size(1);
-    const int64_t n = T * topk, row = (E + 1) / 2 * 2; // 16-byte aligned parts: ids, order, places, weights, counts, cursors
-    const size_t w_at = 3 * 8 * n, c_at = w_at + (4 * n + 15) / 16 * 16;
-    const Tensor all = empty_on(logits, { (int64_t)c_at + 8 * row + 4 * E }, at::kByte);
+    // 16-byte aligned parts: ids, order, places, weights, counts; the cursors lie right behind the counts
+    const int64_t n = T * topk;
+    const size_t items = ((size_t)n * 8 + 15) / 16 * 16, w_at = 3 * items, c_at = w_at + ((size_t)n * 4 + 15) / 16 * 16;
+    const Tensor all = empty_on(logits, { (int64_t)c_at + 12 * E }, at::kByte);
     char* base = static_cast<char*>(all.data_ptr());
-    long long* items = reinterpret_cast<long long*>(base);
-    long long* counts = reinterpret_cast<long long*>(base + c_at);
+    auto longs = [&](size_t at) { return reinterpret_cast<long long*>(base + at); };
     {
         pybind11::gil_scoped_release nogil;
-        check(cclx_moe_route(logits.data_ptr<float>(), (int)T, (int)E, (int)topk, items, reinterpret_cast<float*>(base + w_at),
-                             counts, items + n, items + 2 * n, counts + row, stream_of(logits)));
+        check(cclx_moe_route(logits.data_ptr<float>(), (int)T, (int)E, (int)topk, longs(0), reinterpret_cast<float*>(base + w_at),
+                             longs(c_at), longs(items), longs(2 * items), longs(c_at) + E, stream_of(logits)));
     }
     return pybind11::make_tuple(part_of(all, 0, { T, topk }, at::kLong), part_of(all, w_at, { T, topk }, at::kFloat),
-                                part_of(all, c_at, { E }, at::kLong), part_of(all, 8 * n, { n }, at::kLong),
-                                part_of(all, 16 * n, { n }, at::kLong));
+                                part_of(all, c_at, { E }, at::kLong), part_of(all, items, { n }, at::kLong),
+                                part_of(all, 2 * items, { n }, at::kLong));
 }
 
 void dispatch(uintptr_t group, const tensors& x, const tensors& order, const tensors& counts, const tensors& meta, const Tensor& recv,

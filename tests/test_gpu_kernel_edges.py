@@ -638,3 +638,26 @@ def test_gradient_stream_keeps_operands_until_their_stream_has_waited():
     torch.cuda.synchronize()
     ddp.close()
     group.close()
+
+
+@pytest.mark.parametrize("T,E,k", [(3, 3, 1), (5000, 5, 2), (4097, 63, 3)])
+def test_routing_outputs_are_aligned_and_nothing_else_is_written(T, E, k):
+    """One block and two kernels, odd numbers of items and experts.  The C entry with another value between counts and scratch."""
+    from oneccl_b200 import _lib
+    from oneccl_b200.parallel.ep import route_device
+
+    g = torch.Generator(device="cuda").manual_seed(T)
+    logits = torch.randn(T, E, generator=g, device="cuda")
+    outs = route_device(logits, k)
+    assert all(t.data_ptr() % 16 == 0 for t in outs)
+    ref = torch.topk(logits, k, dim=-1).indices
+    assert torch.equal(outs[0], ref) and torch.equal(outs[2], torch.bincount(ref.flatten(), minlength=E))
+    assert torch.equal(outs[3][outs[4]], torch.arange(T * k, device="cuda"))
+    for between in (0, 1, 2):
+        tail = torch.full((E + between + E,), 77, dtype=torch.int64, device="cuda")
+        idx, order, pos = (torch.empty(T * k, dtype=torch.int64, device="cuda") for _ in range(3))
+        wts = torch.empty(T * k, device="cuda")
+        _lib.check(_lib.load().cclx_moe_route(logits.data_ptr(), T, E, k, idx.data_ptr(), wts.data_ptr(), tail.data_ptr(), order.data_ptr(),
+                                              pos.data_ptr(), tail[E + between:].data_ptr(), torch.cuda.current_stream().cuda_stream))
+        assert torch.equal(tail[:E], outs[2]) and bool((tail[E:E + between] == 77).all())
+        assert torch.equal(order[pos], torch.arange(T * k, device="cuda"))
