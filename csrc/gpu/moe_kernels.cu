@@ -270,6 +270,11 @@ __global__ void __launch_bounds__(256)
 }
 } // namespace
 
+// items (token, slot) up to which one block does the whole routing
+CCLX_API int cclx_moe_route_one_block() {
+    return ROUTE_ONE_BLOCK;
+}
+
 // logits [n_tokens, n_experts] fp32 -> idx [n_tokens, topk] (int64), wts [n_tokens, topk] (fp32),
 // counts [n_experts] (int64), order / pos [n_tokens * topk] (int64).  scratch: n_experts 32-bit words; right
 // behind `counts` it is cleared together with them.

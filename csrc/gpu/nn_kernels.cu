@@ -596,12 +596,6 @@ CCLX_API int cclx_layer_norm_bwd_sums(const void* dy, const void* x, const void*
     });
 }
 
-CCLX_API int cclx_layer_norm_bwd(const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
-                                 const void* dres, void* dx, void* dgamma, void* dbeta, float* workspace, size_t rows, int D,
-                                 void* stream) {
-    return cclx_layer_norm_bwd_sums(dy, x, w, mean, rstd, dres, dx, dgamma, dbeta, nullptr, 0, workspace, rows, D, nullptr, stream);
-}
-
 namespace {
 int map_rows_per_block(size_t rows, int packs) {
     // about six blocks of 128 threads per SM, between 8 and 64 rows each: fewer rows would spend more on partial sums.  More

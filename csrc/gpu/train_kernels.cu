@@ -78,8 +78,6 @@ template <class T>
 __global__ void __launch_bounds__(512) sq_norm_partial_kernel(const T* g, size_t n, float* partial, int* step_dev,
                                                               unsigned* counter, float* out) {
     constexpr size_t N = 16 / sizeof(T);
-    if (!counter)
-        pdl_trigger();
     if (step_dev && blockIdx.x == 0 && threadIdx.x == 0)
         *step_dev += 1; // read by the optimizer kernel behind this one
     const size_t nv = ((((uintptr_t)g) & 15) == 0) ? n / N : 0;
@@ -717,33 +715,15 @@ CCLX_API int cclx_sq_norm(const void* g, size_t n, int dt, float* out, float* pa
     });
 }
 
-// `step_dev` (optional): device word holding the step number.  When given, the launch first adds one to
-// it and the update takes its bias corrections from it instead of `step`, so that the same launch
-// sequence can be replayed from a CUDA graph.
-CCLX_API int cclx_adamw_flat(float* master, const void* grad, int grad_dt, float* m, float* v, void* model_bf16,
-                             size_t n, size_t n_decay, float lr, float beta1, float beta2, float eps,
-                             float weight_decay, int step, float grad_scale, float max_norm, const float* sq_norm,
-                             int* step_dev, void* stream) {
-    return cclx::capi::guard([&] {
-        if (n == 0)
-            return;
-        if (step_dev) {
-            bump_step_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(step_dev);
-            CUDA_CHECK(cudaGetLastError());
-        }
-        launch_adamw_any(master, grad, grad_dt, m, v, model_bf16, n,
-                         make_adamw_args(n_decay, lr, beta1, beta2, eps, weight_decay, step, grad_scale, max_norm), sq_norm,
-                         step_dev, (cudaStream_t)stream);
-    });
-}
-
 // floats of scratch that cclx_adamw_step needs for its norm
 CCLX_API size_t cclx_adamw_step_scratch(size_t n, int grad_dt) {
     return sq_norm_pieces(n, grad_dt);
 }
 
 // The whole optimizer step: squared norm of the gradient into sq_norm[0] (max_norm > 0; `counter`: a zero word that is
-// zero again afterwards, one per stream of calls), the step word, and the update clipped by that norm.
+// zero again afterwards, one per stream of calls), the step word, and the update clipped by that norm.  step_dev (optional):
+// device word holding the step number; it is advanced first and the bias corrections are taken from it instead of `step`, so
+// that the launches can be replayed from a CUDA graph.
 CCLX_API int cclx_adamw_step(float* master, const void* grad, int grad_dt, float* m, float* v, void* model_bf16, size_t n,
                              size_t n_decay, float lr, float beta1, float beta2, float eps, float weight_decay, int step,
                              float grad_scale, float max_norm, float* sq_norm, float* scratch, unsigned* counter,

@@ -48,7 +48,6 @@ def _proto(lib):
         "cclx_dc_symm_free": (i, [vp, sz]),
         "cclx_dc_heap_base": (vp, [vp, i]),
         "cclx_dc_mc_base": (vp, [vp]),
-        "cclx_dc_allreduce": (i, [vp, pp, pp, sz, i, i, i, i, i, f, i, vp]),
         "cclx_dc_reduce_scatter": (i, [vp, pp, pp, sz, i, i, i, i, i, f, i, vp]),
         "cclx_dc_reduce": (i, [vp, pp, pp, sz, i, i, i, i, i, f, i, vp]),
         "cclx_dc_allgatherv": (i, [vp, pp, pp, psz, psz, i, i, vp]),
@@ -64,9 +63,6 @@ def _proto(lib):
         "cclx_dc_allreduce_fused": (i, [vp, pp, pp, psz, i, i, i, f, i, vp]),
         "cclx_dc_fused_batches": (C.c_ulonglong, [vp]),
         "cclx_transpose_blocks": (i, [vp, vp, i, i, sz, vp]),
-        "cclx_gemm_bf16": (i, [vp, vp, vp, i, i, i, i, i, vp, vp]),
-        "cclx_gemm_bf16_2sm": (i, [vp, vp, vp, i, i, i, i, i, vp, vp]),
-        "cclx_gemm_bf16_rows": (i, [vp, vp, vp, i, i, i, i, vp, vp, vp]),
         "cclx_fused_plan_create": (vp, [vp, i, i, i, i, i, i, i]),
         "cclx_fused_plan_destroy": (i, [vp]),
         "cclx_fused_plan_x_shard": (vp, [vp, i]),

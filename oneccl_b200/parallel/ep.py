@@ -20,7 +20,6 @@ from ..ops.gemm import gemm_bf16
 from ..torch_ops import native
 
 launches = 0
-_ROUTE_ONE_BLOCK = 8192  # items (token, slot) up to which one block does the whole routing
 
 
 def gather_rows(x: torch.Tensor, src_row: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -97,7 +96,7 @@ def route_device(logits: torch.Tensor, topk: int):
     global launches
     assert logits.is_cuda and logits.dim() == 2
     out = native().moe_route(logits, topk)
-    launches += 1 if logits.shape[0] * topk <= _ROUTE_ONE_BLOCK else 2
+    launches += 1 if logits.shape[0] * topk <= native().route_one_block else 2
     return out
 
 

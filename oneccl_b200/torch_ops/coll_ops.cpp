@@ -100,6 +100,7 @@ void combine(uintptr_t group, const tensors& expert, const tensors& pos, const t
 void bind_coll(pybind11::module_& m) {
     m.def("dc_allreduce", &allreduce);
     m.def("moe_route", &route);
+    m.attr("route_one_block") = cclx_moe_route_one_block();
     m.def("moe_dispatch", &dispatch);
     m.def("moe_combine", &combine);
 }

@@ -31,6 +31,7 @@ int cclx_layer_norm_bwd_sums(const void* dy, const void* x, const void* w, const
                              float* workspace, size_t rows, int D, int* defer, void* stream);
 int cclx_dc_allreduce(void* h, const void* const* send, void* const* recv, size_t count, int dt_in, int dt_out, int op, int algo,
                       int blocks, float scale, int do_scale, void* stream);
+int cclx_moe_route_one_block();
 int cclx_moe_route(const float* logits, int n_tokens, int n_experts, int topk, long long* idx, float* wts, long long* counts,
                    long long* order, long long* pos, void* scratch, void* stream);
 int cclx_moe_dispatch(void* h, const void* const* x, const long long* const* order, const long long* const* send_counts,
