@@ -44,12 +44,15 @@ CCLX_API int cclx_cuda_device_count() {
 // The library carries its own (static) CUDA runtime, whose notion of the
 // current device is per thread and independent of the caller's runtime: the
 // bindings call this before every launch with the caller's current device.
-// Asked of the runtime each time and not remembered by callers: groups, collectives and other threads' work set it too.
+// Asked of the runtime each time and not remembered by callers: groups and collectives set it too.  A thread's first call makes
+// the device's context current whatever the runtime answers: other libraries on the thread (cuBLAS) look for one.
 CCLX_API int cclx_set_device(int dev) {
     return capi::guard([&] {
+        static thread_local bool current = false;
         int now = -1;
-        if (cudaGetDevice(&now) != cudaSuccess || now != dev)
+        if (!current || cudaGetDevice(&now) != cudaSuccess || now != dev)
             CUDA_CHECK(cudaSetDevice(dev));
+        current = true;
     });
 }
 

@@ -751,3 +751,31 @@ def test_training_step_against_an_fp32_step():
     assert max(off.values()) < 0.025, max(off.items(), key=lambda x: x[1])
     ddp.close()
     group.close()
+
+
+def test_operators_make_a_context_current_on_new_threads():
+    """The first kernel of a thread is the library's; a cuBLAS product behind it must find a context (torch warns if not)."""
+    import subprocess
+    import sys
+
+    code = """
+import threading, warnings, torch
+warnings.simplefilter("error")
+from oneccl_b200.ops.gemm import gemm_bf16
+a = torch.ones(64, 64, device="cuda", dtype=torch.bfloat16)
+bad = []
+def run():
+    try:
+        gemm_bf16(a, a)
+        torch.mm(a, a)
+    except Exception as e:
+        bad.append(repr(e))
+for _ in range(2):
+    t = threading.Thread(target=run)
+    t.start()
+    t.join()
+torch.cuda.synchronize()
+assert not bad, bad
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True)
+    assert r.returncode == 0 and "no current CUDA context" not in r.stderr, r.stderr[-2000:]
