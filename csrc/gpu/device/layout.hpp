@@ -19,7 +19,7 @@ enum : uint32_t {
     ST_MBAR_TIMEOUT = 4,
     ST_BAD_ARGS = 5,
     ST_NOT_FINITE = 6, // debug scan found NaN / Inf in a reduction result (CCL_CUDA_CHECK_NAN)
-    ST_ARG_MISMATCH = 7 // a zero-copy collective was called with a different buffer kind, offset or count on a peer
+    ST_ARG_MISMATCH = 7 // a peer called another collective, or this one with another buffer kind, offset or count
 };
 
 // words of comm_dev::state
@@ -47,7 +47,7 @@ struct comm_dev {
 };
 
 
-// Small allreduce by packets (allreduce_packets_kernel): a slot holds one rank's message as 16-byte packets of 8 data
+// Small allreduce by packets (allreduce_packets_kernel; LL: low latency): a slot holds one rank's message as 16-byte packets of 8 data
 // bytes each, and a header packet behind them.
 constexpr size_t LL_MAX_BYTES = 32u << 10; // largest message
 constexpr size_t LL_SLOT_BYTES = 2 * LL_MAX_BYTES + 256;

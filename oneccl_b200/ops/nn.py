@@ -4,9 +4,9 @@
 * ``layer_norm`` / ``add_layer_norm``: LayerNorm whose backward produces the input gradient and the
   weight / bias gradients from one read of the activations; the ``add_`` form also performs the residual
   addition in front of it (and adds the residual branch's gradient inside the backward kernel);
-* ``linear``: cuBLAS matmuls with the bias gradient taken by a two-stage column sum;
+* ``linear``: cuBLAS matmuls, with the bias gradient by a column sum or left to the next operator;
 * ``split_qkv``: views of a packed QKV projection for the attention call, whose backward assembles the
-  packed gradient with one strided copy kernel instead of a concatenation;
+  packed gradient and sums it over the rows in one pass;
 * ``gelu``: tanh-form GELU; ``embed``: token plus position embedding.
 
 The kernel that produces the gradient of a linear layer's output can sum the bias gradient on the way.  ``linear(...,

@@ -317,7 +317,7 @@ class GraphedTrainStep:
 
     The optimizer must keep its step number on the device (``make_optimizer(device_step=True)``).
     Capture needs the lazily created state of the libraries involved (cuBLAS workspaces, autograd
-    buffers, the column-sum counters) to exist already, so two eager steps run first on a side
+    buffers, kernel attributes) to exist already, so two eager steps run first on a side
     stream; parameters and optimizer state are put back afterwards, so constructing this object does
     not train.  ``__call__`` copies the batch into the graph's static input tensors (the copies are
     ordinary stream work, pinned host tensors are fine), replays the graph and returns the static
