@@ -8,7 +8,6 @@
 #include "core/env.hpp"
 #include "core/log.hpp"
 #include "gpu/cuda_driver.hpp"
-#include "gpu/device_info.hpp"
 #include "gpu/device_comm.hpp"
 #include "gpu/fused_gemm.hpp"
 
@@ -324,7 +323,10 @@ CCLX_API int cclx_gemm_bf16(const void* A, const void* B, void* C, int M, int N,
 CCLX_API int cclx_gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int clusters,
                                 void* err_words, void* stream) {
     return capi::guard(
-        [&] { gemm_bf16_2sm(A, B, C, M, N, K, epilogue, clusters, (uint32_t*)err_words, (cudaStream_t)stream); });
+        [&] {
+            const int pairs = clusters == 0 && M > 0 && N > 0 && K > 0 ? choose_gemm(M, N, K, false).pairs : 1;
+            gemm_bf16_2sm(A, B, C, M, N, K, epilogue, clusters, (uint32_t*)err_words, (cudaStream_t)stream, nullptr, pairs);
+        });
 }
 
 // The same product over the first min(M, *rows_dev) rows of A: the count is read on the device, so a kernel in
@@ -332,11 +334,12 @@ CCLX_API int cclx_gemm_bf16_2sm(const void* A, const void* B, void* C, int M, in
 CCLX_API int cclx_gemm_bf16_rows(const void* A, const void* B, void* C, int M, int N, int K, int epilogue,
                                  const void* rows_dev, void* err_words, void* stream) {
     return capi::guard([&] {
-        const int sms = device_sms();
-        if (gemm_small_preferred(M, N, K, sms))
-            gemm_bf16_small(A, B, C, M, N, K, epilogue, (uint32_t*)err_words, (cudaStream_t)stream, (const int*)rows_dev);
+        const gemm_choice choice = choose_gemm(M, N, K, true);
+        if (choice.small)
+            gemm_bf16_small(A, B, C, M, N, K, epilogue, (uint32_t*)err_words, (cudaStream_t)stream, (const int*)rows_dev, choice);
         else
-            gemm_bf16_2sm(A, B, C, M, N, K, epilogue, 0, (uint32_t*)err_words, (cudaStream_t)stream, (const int*)rows_dev);
+            gemm_bf16_2sm(A, B, C, M, N, K, epilogue, 0, (uint32_t*)err_words, (cudaStream_t)stream, (const int*)rows_dev,
+                          choice.pairs);
     });
 }
 

@@ -92,12 +92,13 @@ void gemm_bf16_plain(const void* A, const void* B, void* C, int M, int N, int K,
     CCL_THROW_IF_NOT(M > 0 && N > 0 && K > 0 && N % 8 == 0 && K % 8 == 0, "unsupported GEMM shape ", M, "x", N, "x", K);
     // Without a grid asked for: the K-splitting kernel where it is expected to be faster (few rows, small C), else CTA
     // pairs (two-SM MMA).  A negative `ctas` forces the single-CTA kernel, CCL_CUDA_GEMM_2SM=0 turns the pairs off.
-    if (ctas == 0 && gemm_small_preferred(M, N, K, sm_count())) {
-        gemm_bf16_small(A, B, C, M, N, K, epilogue, err, st);
+    const gemm_choice choice = ctas == 0 ? choose_gemm(M, N, K, false) : gemm_choice{};
+    if (choice.small) {
+        gemm_bf16_small(A, B, C, M, N, K, epilogue, err, st, nullptr, choice);
         return;
     }
     if (ctas >= 0 && env_data::get().gemm_2sm && (M >= 256 || (ctas == 0 && M > 128)) && N >= 128) {
-        gemm_bf16_2sm(A, B, C, M, N, K, epilogue, ctas / 2, err, st);
+        gemm_bf16_2sm(A, B, C, M, N, K, epilogue, ctas / 2, err, st, nullptr, choice.pairs);
         return;
     }
     if (ctas < 0)

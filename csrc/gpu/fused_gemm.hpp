@@ -15,14 +15,24 @@ class device_comm;
 void gemm_bf16_plain(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int ctas,
                      uint32_t* err, cudaStream_t st);
 
-// the same product on CTA pairs (tcgen05.mma.cta_group::2, 256 x 256 tiles); `clusters` 0 = one pair per two SMs
-void gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int clusters,
-                   uint32_t* err, cudaStream_t st, const int* rows_dev = nullptr);
+// which of the two kernels below is expected to be the faster one, and in which form
+struct gemm_choice {
+    bool small; // the second
+    int tn, splits; // of the second: rows of A per tile, parts of K
+    int pairs; // of the first: per cluster
+    double us; // estimate of the second
+};
+gemm_choice choose_gemm(int M, int N, int K, bool rows_on_device);
 
-// the same product cut along K over clusters of CTAs, for few rows or a small C; and whether it is the faster choice
+// the same product on CTA pairs (tcgen05.mma.cta_group::2, 256 x 256 tiles); `clusters` 0: as many clusters as the device takes, of
+// `pairs` pairs each
+void gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int clusters,
+                   uint32_t* err, cudaStream_t st, const int* rows_dev = nullptr, int pairs = 1);
+double gemm_2sm_estimate(int M, int N, int K, int pairs); // us
+
+// the same product cut along K over clusters of CTAs, for few rows or a small C
 void gemm_bf16_small(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, uint32_t* err, cudaStream_t st,
-                     const int* rows_dev = nullptr);
-bool gemm_small_preferred(int M, int N, int K, int sms);
+                     const int* rows_dev, const gemm_choice& plan);
 
 struct fused_plan; // opaque
 

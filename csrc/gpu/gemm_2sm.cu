@@ -13,6 +13,7 @@
 // Every mbarrier wait is bounded; the cluster barriers at start and end are reached on every path.
 // The reference library has no GEMM: this kernel serves the tensor-parallel and expert-parallel layers.
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 
 #include "core/env.hpp"
@@ -67,8 +68,10 @@ __device__ __forceinline__ void g2_tile(int t, int tiles_m, int tiles_n, int gro
     ni = grp * group + in % width;
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
-    gemm2sm_kernel(const __grid_constant__ gemm2_params P) {
+// PAIRS: CTA pairs per cluster.  With two, the tiles of a last, less than half full round are cut along K between the pairs of a
+// cluster, which add their halves through distributed shared memory.
+template <int PAIRS>
+__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm2sm_kernel(const __grid_constant__ gemm2_params P) {
     using namespace sm100;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -84,9 +87,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     volatile int* abort_flag = (volatile int*)(tmem_holder + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t cr = cluster_ctarank(); // 0 = leader
+    const uint32_t rank = cluster_ctarank(), pair = rank >> 1, cr = rank & 1; // cr 0: leader of its pair
     const bool leader = cr == 0;
-    const int n_clusters = gridDim.x >> 1, cluster = blockIdx.x >> 1;
+    const int n_clusters = gridDim.x / (2 * PAIRS), cluster = blockIdx.x / (2 * PAIRS);
+    const int n_pairs = n_clusters * PAIRS, me = cluster * PAIRS + (int)pair;
     const int KB = (P.K + GEMM_BK - 1) / GEMM_BK;
     const unsigned long long limit = P.timeout_ns;
 
@@ -109,7 +113,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
         tc_fence_before_sync();
     }
     __syncthreads();
-    cluster_sync_all(); // the peer's barriers exist before anything is signalled across the pair
+    cluster_sync_all(); // the peers' barriers exist before anything is signalled across the pair
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_holder;
     pdl_trigger(); // the next kernel's blocks may take the SMs that this one's leave
@@ -119,14 +123,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     const int M = P.rows ? max(0, min(P.M, *P.rows)) : P.M;
     const int tiles_m = (M + 255) / 256, tiles_n = (P.N + G2_BN - 1) / G2_BN;
     const int total_tiles = tiles_m * tiles_n;
+    // tiles [whole, total_tiles) are cut in two, one per cluster
+    static_assert(PAIRS == 1 || PAIRS == 2, "a tile is cut in two at most");
+    const int left = PAIRS > 1 && KB > 1 ? total_tiles % n_pairs : 0;
+    const int whole = left <= n_clusters ? total_tiles - left : total_tiles;
+    const bool cut = whole + cluster < total_tiles; // the same in all CTAs of the cluster
+    const int mine = me < whole ? (whole - me + n_pairs - 1) / n_pairs : 0; // uncut tiles of this pair
+    auto tile_of = [&](int n) { return n < mine ? me + n * n_pairs : whole + cluster; };
+    auto k_first = [&](int n) { return n < mine ? 0 : KB * (int)pair / PAIRS; };
+    auto k_last = [&](int n) { return n < mine ? KB : KB * ((int)pair + 1) / PAIRS; };
+    const int items = mine + (cut ? 1 : 0);
 
     if (warp == 0) {
         if (lane == 0) {
             uint32_t it = 0;
-            for (int t = cluster; t < total_tiles && !*abort_flag; t += n_clusters) {
+            for (int n = 0; n < items && !*abort_flag; n++) {
                 int mi, ni;
-                g2_tile(t, tiles_m, tiles_n, P.group_n, mi, ni);
-                for (int kb = 0; kb < KB; kb++, it++) {
+                g2_tile(tile_of(n), tiles_m, tiles_n, P.group_n, mi, ni);
+                const int k1 = k_last(n);
+                for (int kb = k_first(n); kb < k1; kb++, it++) {
                     const uint32_t st = it % G2_STAGES, ph = (it / G2_STAGES) & 1;
                     if (!mbar_wait(&empty[st], ph ^ 1, abort_flag, limit)) {
                         g2_fail(P, abort_flag, GE_MBAR_TIMEOUT, 2);
@@ -150,9 +165,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     else if (warp == 1) {
         if (lane == 0 && leader) {
             constexpr uint32_t idesc = make_idesc_bf16(256, G2_BN);
-            uint32_t it = 0, tc = 0;
-            for (int t = cluster; t < total_tiles && !*abort_flag; t += n_clusters, tc++) {
-                const uint32_t acc = tc & 1, aph = (tc >> 1) & 1;
+            const uint16_t both = (uint16_t)(3u << (2 * pair));
+            uint32_t it = 0;
+            for (int n = 0; n < items && !*abort_flag; n++) {
+                const uint32_t acc = n & 1, aph = (n >> 1) & 1;
                 if (!mbar_wait(&tempty[acc], aph ^ 1, abort_flag, limit)) {
                     g2_fail(P, abort_flag, GE_MBAR_TIMEOUT, 3);
                     break;
@@ -160,7 +176,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
                 tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + acc * G2_BN;
                 bool bad = false;
-                for (int kb = 0; kb < KB; kb++, it++) {
+                const int k0 = k_first(n), k1 = k_last(n);
+                for (int kb = k0; kb < k1; kb++, it++) {
                     const uint32_t st = it % G2_STAGES, ph = (it / G2_STAGES) & 1;
                     if (!mbar_wait(&full[st], ph, abort_flag, limit)) {
                         g2_fail(P, abort_flag, GE_MBAR_TIMEOUT, 4);
@@ -173,31 +190,70 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 #pragma unroll
                     for (int k = 0; k < GEMM_BK / GEMM_UMMA_K; k++)
                         umma_bf16_2sm(d_tmem, make_smem_desc_sw128(a_addr + k * GEMM_UMMA_K * 2),
-                                      make_smem_desc_sw128(b_addr + k * GEMM_UMMA_K * 2), idesc, (kb | k) != 0 ? 1u : 0u);
-                    umma_commit_2sm(&empty[st], 3); // both CTAs may refill the stage once these MMAs have read it
+                                      make_smem_desc_sw128(b_addr + k * GEMM_UMMA_K * 2), idesc, (kb != k0 || k != 0) ? 1u : 0u);
+                    umma_commit_2sm(&empty[st], both); // both CTAs may refill the stage once these MMAs have read it
                 }
                 if (bad)
                     break;
-                umma_commit_2sm(&tfull[acc], 3); // accumulator complete in both CTAs
+                umma_commit_2sm(&tfull[acc], both); // accumulator complete in both CTAs
             }
         }
         __syncwarp();
     }
-    else {
-        const int q = warp & 3; // TMEM lane quarter this warp may read
-        uint8_t* stage = sEpi + (warp - 2) * 32 * GEMM_EPI_ROW_BYTES;
+    const int q = warp & 3; // TMEM lane quarter this warp may read
+    uint8_t* stage = sEpi + (q * 32) * GEMM_EPI_ROW_BYTES;
+    // 64 columns of one row per lane: activation, bf16, and through shared memory to coalesced stores
+    auto emit = [&](const uint32_t (&r0)[32], const uint32_t (&r1)[32], int row0, int col0) {
+        uint32_t packed[32];
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            float a0 = __uint_as_float(r0[2 * i]), a1 = __uint_as_float(r0[2 * i + 1]);
+            float b0 = __uint_as_float(r1[2 * i]), b1 = __uint_as_float(r1[2 * i + 1]);
+            if (P.epilogue == EPI_SILU) {
+                a0 = silu_f(a0);
+                a1 = silu_f(a1);
+                b0 = silu_f(b0);
+                b1 = silu_f(b1);
+            }
+            __nv_bfloat162 lo = __floats2bfloat162_rn(a0, a1);
+            __nv_bfloat162 hi = __floats2bfloat162_rn(b0, b1);
+            packed[i] = *reinterpret_cast<uint32_t*>(&lo);
+            packed[16 + i] = *reinterpret_cast<uint32_t*>(&hi);
+        }
+        uint8_t* myrow = stage + lane * GEMM_EPI_ROW_BYTES;
+#pragma unroll
+        for (int v = 0; v < 8; v++)
+            *reinterpret_cast<uint4*>(myrow + v * 16) =
+                make_uint4(packed[4 * v], packed[4 * v + 1], packed[4 * v + 2], packed[4 * v + 3]);
+        __syncwarp();
+        const int gcol = col0 + (lane & 7) * 8;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int rr = i * 4 + (lane >> 3);
+            const int grow = row0 + rr;
+            if (grow < M && gcol < P.N) {
+                uint4 v = *reinterpret_cast<const uint4*>(stage + rr * GEMM_EPI_ROW_BYTES + (lane & 7) * 16);
+                *reinterpret_cast<uint4*>(P.C + (size_t)grow * P.N + gcol) = v;
+            }
+        }
+        __syncwarp();
+    };
+    bool good = warp >= 2;
+    if (warp >= 2) {
         const uint32_t tempty_leader = smem_u32(&tempty[0]) & PEER_BIT_MASK;
-        uint32_t tc = 0;
-        for (int t = cluster; t < total_tiles && !*abort_flag; t += n_clusters, tc++) {
-            int mi, ni;
-            g2_tile(t, tiles_m, tiles_n, P.group_n, mi, ni);
-            const uint32_t acc = tc & 1, aph = (tc >> 1) & 1;
+        for (int n = 0; n < items && !*abort_flag; n++) {
+            const uint32_t acc = n & 1, aph = (n >> 1) & 1;
             if (!mbar_wait(&tfull[acc], aph, abort_flag, limit)) {
                 if (lane == 0)
                     g2_fail(P, abort_flag, GE_MBAR_TIMEOUT, 5);
+                good = false;
                 break;
             }
             tc_fence_after_sync();
+            if (n == mine) // the cut tile
+                break;
+            int mi, ni;
+            g2_tile(tile_of(n), tiles_m, tiles_n, P.group_n, mi, ni);
             const int row0 = mi * 256 + (int)cr * G2_HALF + q * 32;
 #pragma unroll 1
             for (int c = 0; c < G2_BN / GEMM_EPI_COLS; c++) {
@@ -213,39 +269,54 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
                     if (lane == 0)
                         mbar_arrive_cluster(tempty_leader + acc * 8);
                 }
-                uint32_t packed[32];
+                emit(r0, r1, row0, ni * G2_BN + c * GEMM_EPI_COLS);
+            }
+        }
+    }
+    if constexpr (PAIRS > 1) {
+        if (cut) {
+            // Pair p finishes columns [128 p, 128 p + 128) of the tile: the other pair's half sums of them arrive in the ring, which
+            // nobody uses any more, as packs of four columns per row.  The sum of two halves does not depend on their order.
+            const uint32_t acc = mine & 1;
+            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * G2_BN;
+            const uint32_t here = smem_u32(smem) + (uint32_t)(q * 32 + lane) * 16;
+            cluster_sync_all();
+            if (warp >= 2 && good) {
+                const uint32_t there = map_to_cta(here, rank ^ 2);
+#pragma unroll 1
+                for (int c = 0; c < G2_BN / 2; c += 32) {
+                    uint32_t r[32];
+                    tmem_ld_32x32(taddr + (pair ^ 1) * (G2_BN / 2) + c, r);
+                    tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    float a0 = __uint_as_float(r0[2 * i]), a1 = __uint_as_float(r0[2 * i + 1]);
-                    float b0 = __uint_as_float(r1[2 * i]), b1 = __uint_as_float(r1[2 * i + 1]);
-                    if (P.epilogue == EPI_SILU) {
-                        a0 = silu_f(a0);
-                        a1 = silu_f(a1);
-                        b0 = silu_f(b0);
-                        b1 = silu_f(b1);
-                    }
-                    __nv_bfloat162 lo = __floats2bfloat162_rn(a0, a1);
-                    __nv_bfloat162 hi = __floats2bfloat162_rn(b0, b1);
-                    packed[i] = *reinterpret_cast<uint32_t*>(&lo);
-                    packed[16 + i] = *reinterpret_cast<uint32_t*>(&hi);
+                    for (int i = 0; i < 32; i += 4)
+                        st_cluster_v4(there + (uint32_t)(c + i) / 4 * G2_HALF * 16, r[i], r[i + 1], r[i + 2], r[i + 3]);
                 }
-                uint8_t* myrow = stage + lane * GEMM_EPI_ROW_BYTES;
+            }
+            cluster_sync_all();
+            if (warp >= 2 && good && !*abort_flag) {
+                int mi, ni;
+                g2_tile(whole + cluster, tiles_m, tiles_n, P.group_n, mi, ni);
+#pragma unroll 1
+                for (int c = 0; c < G2_BN / 2; c += GEMM_EPI_COLS) {
+                    uint32_t r[2][32];
+                    tmem_ld_32x32(taddr + pair * (G2_BN / 2) + c, r[0]);
+                    tmem_ld_32x32(taddr + pair * (G2_BN / 2) + c + 32, r[1]);
+                    tmem_ld_wait();
 #pragma unroll
-                for (int v = 0; v < 8; v++)
-                    *reinterpret_cast<uint4*>(myrow + v * 16) =
-                        make_uint4(packed[4 * v], packed[4 * v + 1], packed[4 * v + 2], packed[4 * v + 3]);
-                __syncwarp();
-                const int gcol = ni * G2_BN + c * GEMM_EPI_COLS + (lane & 7) * 8;
+                    for (int h = 0; h < 2; h++)
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const int rr = i * 4 + (lane >> 3);
-                    const int grow = row0 + rr;
-                    if (grow < M && gcol < P.N) {
-                        uint4 v = *reinterpret_cast<const uint4*>(stage + rr * GEMM_EPI_ROW_BYTES + (lane & 7) * 16);
-                        *reinterpret_cast<uint4*>(P.C + (size_t)grow * P.N + gcol) = v;
-                    }
+                        for (int i = 0; i < 32; i += 4) {
+                            float v[4];
+                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                         : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                                         : "r"(here + (uint32_t)(c + 32 * h + i) / 4 * G2_HALF * 16));
+#pragma unroll
+                            for (int k = 0; k < 4; k++)
+                                r[h][i + k] = __float_as_uint(__uint_as_float(r[h][i + k]) + v[k]);
+                        }
+                    emit(r[0], r[1], mi * 256 + (int)cr * G2_HALF + q * 32, ni * G2_BN + (int)pair * (G2_BN / 2) + c);
                 }
-                __syncwarp();
             }
         }
     }
@@ -260,14 +331,76 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     }
 }
 
+// clusters of `PAIRS` CTA pairs that fit the device
+template <int PAIRS>
+int most_clusters() {
+    allow_smem<gemm2sm_kernel<PAIRS>>(G2_SMEM);
+    static std::atomic<int> known[64];
+    int dev = 0;
+    CUDA_CHECK(cudaGetDevice(&dev));
+    int n = dev < 64 ? known[dev].load(std::memory_order_relaxed) : 0;
+    if (n == 0) {
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute attr{};
+        cfg.gridDim = dim3(2 * PAIRS);
+        cfg.blockDim = dim3(GEMM_THREADS);
+        cfg.dynamicSmemBytes = G2_SMEM;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = 2 * PAIRS;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        CUDA_CHECK(cudaOccupancyMaxActiveClusters(&n, gemm2sm_kernel<PAIRS>, &cfg));
+        n = std::max(n, 1);
+        if (dev < 64)
+            known[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+// Expected time in us: 5.6 for launch, start and output, 0.335 per step of 64 and round of tiles, 15 % more where the rows of a
+// box begin between the 32-byte sectors; a cut tile takes half a round and 1.7 for the exchange.  4096 x 4096 with 512 rows, 32
+// tiles: 26.3 us uncut, 19.1 cut; with 1024 rows, 64 tiles for 74 pairs, nothing is cut.  Clusters of four leave some SMs out, so
+// products of many rounds keep the pairs.
+double estimate(int M, int N, int K, int pairs) {
+    const double step = (K % 16 ? 1.15 : 1.0) * 0.335 * ((K + GEMM_BK - 1) / GEMM_BK);
+    const long long tiles = (long long)((M + 255) / 256) * ((N + G2_BN - 1) / G2_BN);
+    if (pairs == 1) {
+        const int most = device_sms() / 2;
+        return 5.6 + (tiles + most - 1) / most * step;
+    }
+    const long long clusters = std::min<long long>(most_clusters<2>(), tiles), left = tiles % (2 * clusters);
+    const bool cut = left > 0 && left <= clusters;
+    return 5.8 + (tiles / (2 * clusters) + (cut ? 0.5 : left > 0 ? 1.0 : 0.0)) * step + (cut ? 1.7 : 0);
+}
+
+template <int PAIRS>
+void launch_2sm(const gemm2_params& P, int clusters, cudaStream_t st) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(2 * PAIRS * clusters);
+    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.dynamicSmemBytes = G2_SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2]{};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2 * PAIRS;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm2sm_kernel<PAIRS>, P));
+}
+
 } // namespace
 
 CUtensorMap make_bf16_kmajor_map(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
 
 void gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int clusters,
-                   uint32_t* err, cudaStream_t st, const int* rows_dev) {
+                   uint32_t* err, cudaStream_t st, const int* rows_dev, int pairs) {
     CCL_THROW_IF_NOT(M > 0 && N > 0 && K > 0 && N % 8 == 0 && K % 8 == 0, "unsupported GEMM shape ", M, "x", N, "x", K);
-    allow_smem<gemm2sm_kernel>(G2_SMEM);
+    allow_smem<gemm2sm_kernel<1>>(G2_SMEM);
+    allow_smem<gemm2sm_kernel<2>>(G2_SMEM);
     gemm2_params P;
     std::memset(&P, 0, sizeof(P));
     P.tmA = make_bf16_kmajor_map(A, M, K, G2_HALF);
@@ -280,16 +413,19 @@ void gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, i
     P.epilogue = epilogue;
     P.rows = rows_dev;
     P.timeout_ns = (unsigned long long)env_data::get().wait_timeout_ms * 1000000ull;
-    const int sms = device_sms();
-    const int tiles = ((M + 255) / 256) * ((N + G2_BN - 1) / G2_BN);
-    int nc = clusters > 0 ? clusters : sms / 2;
-    nc = std::max(1, std::min(nc, tiles));
     const int tiles_n = (N + G2_BN - 1) / G2_BN;
     const int most = (int)std::min<size_t>(std::max<size_t>(G2_GROUP_BYTES / ((size_t)G2_BN * K * 2), 4), 32);
     const int groups = (tiles_n + most - 1) / most;
     P.group_n = (tiles_n + groups - 1) / groups; // groups of about the same width
-    // the cluster shape is a compile-time attribute of the kernel; the grid must be a multiple of it
-    launch_dependent(gemm2sm_kernel, dim3(2 * nc), dim3(GEMM_THREADS), G2_SMEM, st, P);
+    const int tiles = ((M + 255) / 256) * tiles_n;
+    if (clusters == 0 && pairs == 2)
+        launch_2sm<2>(P, std::min(most_clusters<2>(), tiles), st);
+    else
+        launch_2sm<1>(P, std::max(1, std::min(clusters > 0 ? clusters : device_sms() / 2, tiles)), st);
+}
+
+double gemm_2sm_estimate(int M, int N, int K, int pairs) {
+    return estimate(M, N, K, pairs);
 }
 
 } // namespace gpu

@@ -7,10 +7,14 @@
 // TN / S columns from the partial sums the others stored into its shared memory (fixed order, fp32), applies the
 // activation and writes bf16.  No workspace, no second kernel, no atomics.
 //
-// What bounds it: with few rows the bytes of B.  Two CTAs per SM with 72 to 96 KB of loads in flight each are more than
-// the memory needs (24 x 14336 x 4096: 117 MB in 23.8 us = 4.9 TB/s; one 128 x 256 tile per CTA on 56 of 148 SMs
-// took 81 us).
+// What bounds it: with few rows the bytes of B, with few tiles the time of a step.  K is cut 1 to 8 times, in whatever way fills the
+// SMs once (1 x 1272 x 11552: 18.0 us on 40 CTAs, 11.2 on 80; 512 x 1024 x 4096: 15.5 us with 4 x 128 columns, 11.8 with 4 x 64).  A
+// ring takes half of an SM's shared memory, 24 x 14336 x 4096: 117 MB in 23.6 us = 5.0 TB/s; only tiles of 128 rows that are
+// alone on their SM gain from the whole of it (73 x 5632 x 10232, K cut in 3: 42.7 us, now 29.1).  The next kernel is not let in
+// early: its CTAs took the room that this one's clusters need (a call after another 6 % slower).
 #include <algorithm>
+#include <atomic>
+#include <cmath>
 #include <cstring>
 
 #include "core/env.hpp"
@@ -35,21 +39,29 @@ struct gemm_small_params {
     __nv_bfloat16* C;
     uint32_t* err;
     int M, N, K, epilogue;
-    int splits; // CTAs per cluster: 1, 2, 4 or 8
+    int splits; // CTAs per cluster: 1 to 8
+    uint32_t inv_splits; // 65536 / splits, rounded up
+    int pitch; // units of four columns that a CTA finishes, at most
     unsigned long long timeout_ns;
     const int* rows; // optional device word: only the first min(M, *rows) rows of A are multiplied
 };
 
-template <int TN>
+// Stages of the ring are a constant of the kernel: with a number known at launch alone the loops took 0.3 us of a 6 us product
+// longer.  Four leave room for two CTAs per SM; more of them slow the loads from memory down (2 x 6176 x 5432: 15.7 us with 4,
+// 16.2 with 6), but for 128 rows, where a CTA that is alone on its SM takes the whole of it.
+constexpr int GS_STAGES_ALONE = 6;
+
+template <int TN, int STAGES>
 struct gs_layout {
-    static constexpr int STAGES = TN == 128 ? 3 : 4;
     static constexpr int B_STAGE = GS_BN * GEMM_BK * 2;
     static constexpr int A_STAGE = TN * GEMM_BK * 2;
-    static constexpr int RING = STAGES * (A_STAGE + B_STAGE); // also holds the 128 x TN partial sums afterwards
-    static constexpr int TOTAL = 1024 + RING + 128;
+    static constexpr int STAGE = A_STAGE + B_STAGE;
     static constexpr int TMEM_COLS = TN < 32 ? 32 : TN;
-    static constexpr int BLOCKS = TN == 256 ? 1 : 2; // per SM
-    static_assert(GS_BN * TN * 4 <= RING, "the partial sums must fit the ring");
+    static constexpr int BLOCKS = TN == 256 || STAGES > 4 ? 1 : 2; // per SM
+    static constexpr int UNITS = TN / 4; // of four columns: what the CTAs of a cluster share out
+    static constexpr int TOTAL = 1024 + STAGES * STAGE + 128;
+    // the ring also holds the partial sums afterwards: a source's units for one CTA, rounded up, times up to 8 sources
+    static_assert((UNITS + 7) * GS_BN * 16 <= STAGES * STAGE, "the partial sums must fit the ring");
 };
 
 __device__ __forceinline__ void gs_fail(const gemm_small_params& P, volatile int* abort_flag, uint32_t detail) {
@@ -84,40 +96,42 @@ __device__ __forceinline__ void gs_store(const gemm_small_params& P, int M, int 
         *reinterpret_cast<__nv_bfloat162*>(dst + P.N) = odd ? __floats2bfloat162_rn(g1, k1) : __floats2bfloat162_rn(k1, g1);
 }
 
-// adds the S partial sums of this CTA's columns in order and stores the result; one thread per row of B
-template <int S>
-__device__ __forceinline__ void gs_reduce(const gemm_small_params& P, int M, uint32_t part, int cols, int tok, int n0, int row) {
-#pragma unroll 2
-    for (int c = 0; c < cols && tok + c < M; c += 4) {
-        float v[S][4];
+// adds the S partial sums of this CTA's units of four columns in order and stores the result; one thread per row of B
+__device__ __forceinline__ void gs_reduce(const gemm_small_params& P, int S, int M, uint32_t part, int pitch, int units, int tok,
+                                          int n0, int row) {
+    const uint32_t step = (uint32_t)pitch * GS_BN * 16;
+    for (int u = 0; u < units && tok + 4 * u < M; u++, part += GS_BN * 16) {
+        float v[8][4];
 #pragma unroll
-        for (int s = 0; s < S; s++)
-            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                         : "=f"(v[s][0]), "=f"(v[s][1]), "=f"(v[s][2]), "=f"(v[s][3])
-                         : "r"(part + (uint32_t)(s * cols + c) * GS_BN * 4));
+        for (int s = 0; s < 8; s++)
+            if (s < S)
+                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                             : "=f"(v[s][0]), "=f"(v[s][1]), "=f"(v[s][2]), "=f"(v[s][3])
+                             : "r"(part + s * step));
 #pragma unroll
-        for (int s = 1; s < S; s++)
+        for (int s = 1; s < 8; s++)
+            if (s < S)
 #pragma unroll
-            for (int k = 0; k < 4; k++)
-                v[0][k] += v[s][k];
-        gs_store(P, M, tok + c, n0, row, v[0]);
+                for (int k = 0; k < 4; k++)
+                    v[0][k] += v[s][k];
+        gs_store(P, M, tok + 4 * u, n0, row, v[0]);
     }
 }
 
-template <int TN>
-__global__ void __launch_bounds__(GEMM_THREADS, gs_layout<TN>::BLOCKS)
+template <int TN, int STAGES>
+__global__ void __launch_bounds__(GEMM_THREADS, gs_layout<TN, STAGES>::BLOCKS)
     gemm_small_kernel(const __grid_constant__ gemm_small_params P) {
     using namespace sm100;
-    typedef gs_layout<TN> L;
+    typedef gs_layout<TN, STAGES> L;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* sB = smem;
-    uint8_t* sA = smem + L::STAGES * L::B_STAGE;
-    uint64_t* bars = (uint64_t*)(smem + L::RING);
+    uint8_t* sA = smem + STAGES * L::B_STAGE;
+    uint64_t* bars = (uint64_t*)(smem + STAGES * L::STAGE);
     uint64_t* full = bars;
-    uint64_t* empty = bars + L::STAGES;
-    uint64_t* tfull = bars + 2 * L::STAGES;
-    uint32_t* tmem_holder = (uint32_t*)(bars + 2 * L::STAGES + 1);
+    uint64_t* empty = bars + STAGES;
+    uint64_t* tfull = bars + 2 * STAGES;
+    uint32_t* tmem_holder = (uint32_t*)(bars + 2 * STAGES + 1);
     volatile int* abort_flag = (volatile int*)(tmem_holder + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -129,7 +143,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, gs_layout<TN>::BLOCKS)
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
-        for (int i = 0; i < L::STAGES; i++) {
+        for (int i = 0; i < STAGES; i++) {
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], 1);
         }
@@ -147,35 +161,41 @@ __global__ void __launch_bounds__(GEMM_THREADS, gs_layout<TN>::BLOCKS)
     const uint32_t tmem = *tmem_holder;
     pdl_wait(); // everything above overlaps the end of the kernel in front
     const int M = P.rows ? max(0, min(P.M, *P.rows)) : P.M;
-    const bool live = tok0 < M; // the same in all CTAs of the cluster
+    if (tok0 >= M) { // no rows: the same in all CTAs of the cluster
+        if (warp == 2)
+            tmem_dealloc(tmem, L::TMEM_COLS);
+        return;
+    }
 
-    if (warp == 0 && live) {
+    if (warp == 0) {
         if (lane == 0) {
-            uint32_t it = 0;
+            uint32_t it = 0, st = 0, ph = 0;
             for (int kb = kb0; kb < kb1; kb++, it++) {
-                const uint32_t st = it % L::STAGES, ph = (it / L::STAGES) & 1;
                 if (!mbar_wait(&empty[st], ph ^ 1, abort_flag, limit)) {
                     gs_fail(P, abort_flag, 2);
                     break;
                 }
-                mbar_expect_tx(&full[st], L::A_STAGE + L::B_STAGE);
+                mbar_expect_tx(&full[st], L::STAGE);
                 tma_load_2d(sB + st * L::B_STAGE, &P.tmB, kb * GEMM_BK, n0, &full[st]);
                 tma_load_2d(sA + st * L::A_STAGE, &P.tmA, kb * GEMM_BK, tok0, &full[st]);
+                if (++st == STAGES) {
+                    st = 0;
+                    ph ^= 1;
+                }
             }
             // copies still in flight land before the ring is used for anything else
-            const uint32_t first = it > (uint32_t)L::STAGES ? it - L::STAGES : 0;
+            const uint32_t first = it > (uint32_t)STAGES ? it - STAGES : 0;
             for (uint32_t i = first; i < it; i++)
-                mbar_wait(&full[i % L::STAGES], (i / L::STAGES) & 1, abort_flag, limit);
+                mbar_wait(&full[i % STAGES], (i / STAGES) & 1, abort_flag, limit);
         }
         __syncwarp();
     }
-    else if (warp == 1 && live) {
+    else if (warp == 1) {
         if (lane == 0) {
             constexpr uint32_t idesc = make_idesc_bf16(GS_BN, TN);
-            uint32_t it = 0;
+            uint32_t st = 0, ph = 0;
             bool ok = true;
-            for (int kb = kb0; kb < kb1; kb++, it++) {
-                const uint32_t st = it % L::STAGES, ph = (it / L::STAGES) & 1;
+            for (int kb = kb0; kb < kb1; kb++) {
                 if (!mbar_wait(&full[st], ph, abort_flag, limit)) {
                     gs_fail(P, abort_flag, 4);
                     ok = false;
@@ -186,16 +206,20 @@ __global__ void __launch_bounds__(GEMM_THREADS, gs_layout<TN>::BLOCKS)
 #pragma unroll
                 for (int k = 0; k < GEMM_BK / GEMM_UMMA_K; k++)
                     umma_bf16(tmem, make_smem_desc_sw128(b_addr + k * GEMM_UMMA_K * 2),
-                              make_smem_desc_sw128(a_addr + k * GEMM_UMMA_K * 2), idesc, (it | k) != 0 ? 1u : 0u);
+                              make_smem_desc_sw128(a_addr + k * GEMM_UMMA_K * 2), idesc, (kb != kb0 || k != 0) ? 1u : 0u);
                 umma_commit(&empty[st]);
+                if (++st == STAGES) {
+                    st = 0;
+                    ph ^= 1;
+                }
             }
             if (ok)
                 umma_commit(tfull);
         }
         __syncwarp();
     }
-    bool good = live;
-    if (warp >= 2 && live) {
+    bool good = true;
+    if (warp >= 2) {
         good = mbar_wait(tfull, 0, abort_flag, limit);
         if (!good && lane == 0)
             gs_fail(P, abort_flag, 5);
@@ -206,14 +230,17 @@ __global__ void __launch_bounds__(GEMM_THREADS, gs_layout<TN>::BLOCKS)
         cluster_sync_all();
     else
         __syncthreads();
-    const int cols = TN / S; // columns (rows of A) this CTA finishes: a power of two, at least 4
+    // The units of four columns are shared out among the cluster's CTAs: CTA s finishes units [UNITS s / S, UNITS (s + 1) / S).
+    // Both numbers are small, so a multiplication divides by S exactly.
+    auto first_unit = [&](uint32_t s) { return (uint32_t)L::UNITS * s * P.inv_splits >> 16; };
+    const int pitch = P.pitch;
     const int q = warp & 3; // quarter of the tensor memory's lanes this warp may read
     const int row = q * 32 + lane;
     if (warp >= 2 && good) {
-        // Partial sums travel as [source][4 columns][row] packs of four floats: a warp stores 512 contiguous bytes,
+        // Partial sums travel as [source][unit][row] packs of four floats: a warp stores 512 contiguous bytes,
         // and the reader's lanes take consecutive rows.  An undivided K needs no exchange.
-        const uint32_t base = smem_u32(smem) + (uint32_t)(split * cols * GS_BN + row * 4) * 4;
-        const int shift = __ffs(cols) - 1;
+        const uint32_t base = smem_u32(smem) + (uint32_t)(split * pitch * GS_BN + row) * 16;
+        uint32_t owner = 0, end = first_unit(1), dst = S > 1 ? map_to_cta(base, 0) : 0; // of the next unit
         constexpr int CH = TN < 32 ? 16 : 32;
 #pragma unroll 1
         for (int c0 = 0; c0 < TN; c0 += CH) {
@@ -231,8 +258,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, gs_layout<TN>::BLOCKS)
                     gs_store(P, M, tok0 + c0 + i, n0, row, v);
                 }
                 else {
-                    const uint32_t owner = (uint32_t)(c0 + i) >> shift, c = (uint32_t)(c0 + i) & (cols - 1);
-                    st_cluster_v4(map_to_cta(base + c * GS_BN * 4, owner), r[i], r[i + 1], r[i + 2], r[i + 3]);
+                    if ((uint32_t)(c0 + i) / 4 == end) {
+                        owner++;
+                        end = first_unit(owner + 1);
+                        dst = map_to_cta(base, owner);
+                    }
+                    st_cluster_v4(dst, r[i], r[i + 1], r[i + 2], r[i + 3]);
+                    dst += GS_BN * 16;
                 }
             }
         }
@@ -242,14 +274,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, gs_layout<TN>::BLOCKS)
         cluster_sync_all();
     else
         __syncthreads();
-    if (S > 1 && warp >= 2 && live && !*abort_flag) {
+    if (S > 1 && warp >= 2 && !*abort_flag) {
         const uint32_t part = smem_u32(smem) + row * 16;
-        if (S == 2)
-            gs_reduce<2>(P, M, part, cols, tok0 + split * cols, n0, row);
-        else if (S == 4)
-            gs_reduce<4>(P, M, part, cols, tok0 + split * cols, n0, row);
-        else
-            gs_reduce<8>(P, M, part, cols, tok0 + split * cols, n0, row);
+        const int u0 = first_unit(split), units = first_unit(split + 1) - u0, tok = tok0 + 4 * u0;
+        gs_reduce(P, S, M, part, pitch, units, tok, n0, row);
     }
     if (warp == 2) { // all reads of the accumulator lie in front of the last barrier
         tc_fence_after_sync();
@@ -257,13 +285,44 @@ __global__ void __launch_bounds__(GEMM_THREADS, gs_layout<TN>::BLOCKS)
     }
 }
 
-template <int TN>
+// clusters of `splits` CTAs that run at the same time with one CTA per SM: fewer than SMs / splits, since a cluster
+// stays within a group of SMs
+int resident_clusters(int splits) {
+    static std::atomic<int> known[64][9];
+    if (splits == 1)
+        return device_sms();
+    int dev = 0;
+    CUDA_CHECK(cudaGetDevice(&dev));
+    int n = dev < 64 ? known[dev][splits].load(std::memory_order_relaxed) : 0;
+    if (n == 0) {
+        typedef gs_layout<128, GS_STAGES_ALONE> L;
+        allow_smem<gemm_small_kernel<128, GS_STAGES_ALONE>>(L::TOTAL);
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(splits);
+        cfg.blockDim = dim3(GEMM_THREADS);
+        cfg.dynamicSmemBytes = L::TOTAL;
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = splits;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        CUDA_CHECK(cudaOccupancyMaxActiveClusters(&n, gemm_small_kernel<128, GS_STAGES_ALONE>, &cfg));
+        n = std::max(n, 1);
+        if (dev < 64)
+            known[dev][splits].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+template <int TN, int STAGES>
 void launch_small(const gemm_small_params& P, int tiles_n, int tiles_m, cudaStream_t st) {
-    allow_smem<gemm_small_kernel<TN>>(gs_layout<TN>::TOTAL);
+    typedef gs_layout<TN, STAGES> L;
+    allow_smem<gemm_small_kernel<TN, STAGES>>(L::TOTAL);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(tiles_n * P.splits, tiles_m);
     cfg.blockDim = dim3(GEMM_THREADS);
-    cfg.dynamicSmemBytes = gs_layout<TN>::TOTAL;
+    cfg.dynamicSmemBytes = L::TOTAL;
     cfg.stream = st;
     cudaLaunchAttribute attr[2]{};
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -273,59 +332,92 @@ void launch_small(const gemm_small_params& P, int tiles_n, int tiles_m, cudaStre
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_small_kernel<TN>, P));
+    CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_small_kernel<TN, STAGES>, P));
 }
 
-struct small_plan {
-    int tn, splits;
-    double cycles; // estimate
+// What a product costs with tiles of TN rows of A, in us: `fixed` from launch to output, `exchange` if K is cut, a step of 64
+// of K with one CTA on an SM or with two, another round of resident CTAs, the factor on the steps where K is no multiple
+// of 16, so that the rows of a box begin between the 32-byte sectors, and a round of CTAs that find no rows.  Fitted to 8200 times
+// of 420 products of 1 to 700 rows, 520 to 14000 columns and K of 520 to 14300, then moved a little to where they choose best: the
+// chosen plan takes 2 to 3 % longer than the best one, 3 to 5 % where the device alone knows the rows; the rule this replaces
+// (1, 2, 4 or 8 parts, estimated cycles) 9 %.
+struct small_cost {
+    int tn;
+    double fixed, exchange, alone, two, round, ragged, idle;
 };
+constexpr small_cost SMALL_COSTS[] = {
+    { 16, 3.23, 0.80, 0.274, 0.396, 2.0, 1.06, 0.6 },  { 32, 3.75, 0.72, 0.286, 0.430, 3.3, 1.12, 0.7 },
+    { 64, 4.68, 0.71, 0.275, 0.432, 4.1, 1.18, 0.6 },  { 128, 6.75, 0.72, 0.303, 0.609, 7.0, 1.14, 0.6 },
+    { 256, 10.56, 0.3, 0.385, 0.385, 10.5, 1.40, 0.8 },
+};
+constexpr double SMALL_BYTES_PER_US = 6.3e6; // of B, from memory
+constexpr double SMALL_L2_BYTES = 64e6; // of B that a second row of tiles still finds in the L2
 
-// The split with the lowest estimate.  Measured on the pieces: a step of 64 takes a CTA's (16 + TN / 8) KB from the L2
-// at 64 bytes per cycle and SM, whichever CTAs share the SM; start, exchange and output cost 4000 cycles and 32 per
-// column (2048 x 1024 x 1 row 5 us, 128 rows 7 us, 256 rows 10 us), once for all CTAs that are resident together.
-small_plan plan_small(int M, int N, int K, int sms) {
-    const int kb = (K + GEMM_BK - 1) / GEMM_BK;
-    small_plan best{ 16, 1, 1e30 };
-    for (int tn = 16; tn <= 256; tn *= 2) {
-        const int tiles = (N + GS_BN - 1) / GS_BN * ((M + tn - 1) / tn);
-        const int resident = tn == 256 ? sms : 2 * sms;
-        for (int s = 1; s <= std::min(8, tn / 4) && (s == 1 || kb / s >= 2); s *= 2) {
-            const int ctas = tiles * s;
-            if (tn == 256 && s > 1 && ctas > sms * 7 / 8) // clusters of one CTA per SM leave some SMs without one
-                break;
-            // CTAs that share an SM even out; one per SM runs in whole rounds
-            const double load = tn == 256 ? (ctas + sms - 1) / sms : std::max(1.0, (double)ctas / sms);
-            const double cycles = load * ((kb + s - 1) / s) * (256 + 2 * tn) + (ctas + resident - 1) / resident * (4000.0 + 32 * tn);
-            if (cycles < 0.98 * best.cycles) // a finer cut has to gain something
-                best = { tn, s, cycles };
-        }
-        if (tn >= M)
+// The cheapest tiles and split of K for `rows` expected rows of the M that the grid covers.
+void plan_small(int M, int rows, int N, int K, gemm_choice& best) {
+    const int kb = (K + GEMM_BK - 1) / GEMM_BK, across = (N + GS_BN - 1) / GS_BN;
+    int resident[9];
+    for (int s = 1; s <= 8; s++)
+        resident[s] = resident_clusters(s);
+    best.us = 1e30;
+    for (const small_cost& c : SMALL_COSTS) {
+        if (c.tn >= 4 * std::max(rows, 16)) // mostly padding
             break;
+        const int down = (rows + c.tn - 1) / c.tn;
+        const long long tiles = (long long)across * down, launched = (long long)across * ((M + c.tn - 1) / c.tn);
+        const double bytes = (double)N * K * 2;
+        const double stream = (bytes > SMALL_L2_BYTES ? bytes * down : bytes) / SMALL_BYTES_PER_US;
+        for (int s = 1; s <= std::min(8, c.tn / 4) && (s == 1 || kb / s >= 2); s++) {
+            // clusters that run at the same time, with one CTA per SM and with the most
+            const long long one = resident[s], most = c.tn == 256 ? one : 2 * one;
+            if (s > 2 && launched > most) // a second round of wide clusters waits for whole groups of SMs
+                break;
+            const long long rounds = (tiles + most - 1) / most, idle = (launched + most - 1) / most - rounds;
+            const double steps = (double)rounds * ((kb + s - 1) / s) * (tiles <= one ? c.alone : c.two) * (K % 16 ? c.ragged : 1.0);
+            // both limits are felt where they are close: the fourth root of the sum of the fourth powers
+            const double s2 = steps * steps, m2 = stream * stream;
+            const double us = c.fixed + (s > 1 ? c.exchange : 0) + std::sqrt(std::sqrt(s2 * s2 + m2 * m2)) + c.round * (rounds - 1) +
+                              c.idle * idle;
+            if (us < best.us) {
+                best.tn = c.tn;
+                best.splits = s;
+                best.us = us;
+            }
+        }
     }
-    return best;
 }
 
 } // namespace
 
-// Whether the kernel above is expected to be faster than CTA pairs on 256 x 256 tiles: up to 128 rows always, beyond that
-// when the pairs would leave much of the chip idle.  In time the estimate above comes out as 1.25 times its cycles and 4600 for
-// the launch; the pairs take 560 cycles per step of 64 and round of tiles and 14500 for launch, start and output.  The
-// line this draws at 4096 x 4096 lies between 512 rows (23 us here, 30 us with pairs) and 768 (33 and 31), at 7168 x 2048
-// between 200 rows (16.6 and 17.2) and 384 (20 and 18), at 4096 x 14336 between 512 (55 and 78) and 768 (80 and 78).
-bool gemm_small_preferred(int M, int N, int K, int sms) {
-    if (M <= 128)
-        return true;
-    const int tiles = ((M + 255) / 256) * ((N + 255) / 256), pairs = sms / 2, kb = (K + GEMM_BK - 1) / GEMM_BK;
-    const int rounds = (tiles + pairs - 1) / pairs;
-    return plan_small(M, N, K, sms).cycles * 1.25 + 4600 < (double)rounds * kb * 560 + 14500;
+// Up to 128 rows this kernel, beyond that by the estimates.  The line this draws at 4096 x 4096 lies between 256 rows (17.2 us here,
+// 18.5 with pairs) and 512 (22.6 and 19.1), at 1024 x 4096 between 1024 rows (16.2 and 17.8) and 2048 (21.9 and 18.8).  A row count
+// that only the device knows lies somewhere below M: half of it is taken.  The answer depends on the sizes and the kind of device
+// alone and takes 2 us to work out, half a small product: each thread keeps its latest ones.
+gemm_choice choose_gemm(int M, int N, int K, bool rows_on_device) {
+    struct entry {
+        int dev = -1, M, N, K;
+        bool rows;
+        gemm_choice c;
+    };
+    static thread_local entry known[64];
+    int dev = 0;
+    CUDA_CHECK(cudaGetDevice(&dev));
+    entry& e = known[((unsigned)M * 31 + (unsigned)N * 17 + (unsigned)K * 5 + rows_on_device) / 8 % 64];
+    if (e.dev == dev && e.M == M && e.N == N && e.K == K && e.rows == rows_on_device)
+        return e.c;
+    const int rows = rows_on_device ? (M + 1) / 2 : M;
+    gemm_choice c;
+    plan_small(M, rows, N, K, c);
+    const double one = gemm_2sm_estimate(rows, N, K, 1), two = gemm_2sm_estimate(rows, N, K, 2);
+    c.pairs = two < one ? 2 : 1;
+    c.small = rows <= 128 || c.us < std::min(one, two);
+    e = { dev, M, N, K, rows_on_device, c };
+    return c;
 }
 
 void gemm_bf16_small(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, uint32_t* err, cudaStream_t st,
-                     const int* rows_dev) {
+                     const int* rows_dev, const gemm_choice& plan) {
     CCL_THROW_IF_NOT(M > 0 && N > 0 && K > 0 && N % 8 == 0 && K % 8 == 0, "unsupported GEMM shape ", M, "x", N, "x", K);
-    const int sms = device_sms();
-    const small_plan plan = plan_small(M, N, K, sms);
     gemm_small_params P;
     std::memset(&P, 0, sizeof(P));
     P.tmA = make_bf16_kmajor_map(A, M, K, plan.tn);
@@ -337,15 +429,22 @@ void gemm_bf16_small(const void* A, const void* B, void* C, int M, int N, int K,
     P.K = K;
     P.epilogue = epilogue;
     P.splits = plan.splits;
+    P.inv_splits = (65536u + plan.splits - 1) / plan.splits;
+    P.pitch = (plan.tn / 4 + plan.splits - 1) / plan.splits;
     P.rows = rows_dev;
     P.timeout_ns = (unsigned long long)env_data::get().wait_timeout_ms * 1000000ull;
     const int tiles_n = (N + GS_BN - 1) / GS_BN, tiles_m = (M + plan.tn - 1) / plan.tn;
     switch (plan.tn) {
-        case 16: launch_small<16>(P, tiles_n, tiles_m, st); break;
-        case 32: launch_small<32>(P, tiles_n, tiles_m, st); break;
-        case 64: launch_small<64>(P, tiles_n, tiles_m, st); break;
-        case 128: launch_small<128>(P, tiles_n, tiles_m, st); break;
-        default: launch_small<256>(P, tiles_n, tiles_m, st); break;
+        case 16: launch_small<16, 4>(P, tiles_n, tiles_m, st); break;
+        case 32: launch_small<32, 4>(P, tiles_n, tiles_m, st); break;
+        case 64: launch_small<64, 4>(P, tiles_n, tiles_m, st); break;
+        case 128:
+            if ((long long)tiles_n * tiles_m <= resident_clusters(plan.splits))
+                launch_small<128, GS_STAGES_ALONE>(P, tiles_n, tiles_m, st);
+            else
+                launch_small<128, 3>(P, tiles_n, tiles_m, st);
+            break;
+        default: launch_small<256, 4>(P, tiles_n, tiles_m, st); break;
     }
 }
 

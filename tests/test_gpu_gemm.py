@@ -35,6 +35,32 @@ def test_gemm_plain(shape, kernel):
     _check(out, _ref(a, w), K)
 
 
+@pytest.mark.parametrize("rows", [False, True], ids=["all-rows", "rows-on-device"])
+@pytest.mark.parametrize("shape", [
+    (1, 8, 8), (3, 136, 2184), (1, 1272, 2568),  # one tile or few: K cut up to eight times, units of columns shared out unevenly
+    (17, 1000, 1544), (65, 2880, 712), (129, 520, 3208), (70, 2816, 2056),  # every tile width, K with a part of a step at the end
+    (257, 4104, 1096), (512, 4096, 64), (520, 2048, 1032), (300, 7432, 328),  # tiles cut between two pairs; K of one step; a last round
+    (2048, 1032, 1024), (1900, 5000, 136),  # more tiles than clusters: whole rounds, then cut or uncut ones
+])
+def test_gemm_plans(shape, rows):
+    """The sizes at which the split of K or of the last tiles can go wrong, rows beyond the count untouched."""
+    from oneccl_b200.ops.gemm import gemm_bf16
+
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(2)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    ref = a.double() @ w.double().t()
+    # one rounding of the result to bf16, K roundings of the fp32 sum (each of at most the sum of the magnitudes)
+    bound = ref.abs() * 2.0**-8 + K * 2.0**-23 * (a.double().abs() @ w.double().abs().t()) + 1e-30
+    for n in sorted({1, M // 2, M - 1, M} - {0}) if rows else [M]:
+        for kernel in ["auto"] if rows else ["auto", "2sm"]:
+            out = torch.full((M, N), 7.0, dtype=torch.bfloat16, device="cuda")
+            count = torch.tensor([n], dtype=torch.int32, device="cuda") if rows else None
+            gemm_bf16(a, w, out=out, check=True, kernel=kernel, rows=count)
+            assert ((out[:n].double() - ref[:n]).abs() <= bound[:n]).all(), (n, kernel)
+            assert (out[n:] == 7.0).all(), (n, kernel)
+
 @pytest.mark.parametrize("kernel", ["1sm", "2sm"])
 def test_gemm_silu_and_persistence(kernel):
     """More tiles than CTAs (each CTA loops, both TMEM accumulators are reused) + SiLU epilogue."""
