@@ -8,8 +8,10 @@
 // stays in the L2 while A streams past it once per group, so a group is as wide as a third of the L2 allows (8192 x
 // 14336 x 4096: 14 columns instead of 8 take 2 % off the time under the power cap).
 //
-// Roles per CTA (192 threads): warp 0 TMA producer, warp 1 MMA issuer (leader CTA only), warps 2-5
-// epilogue (TMEM -> registers -> bf16 -> padded shared-memory transpose -> coalesced stores).
+// Roles per CTA (576 threads): warp 0 TMA producer, warp 1 MMA issuer (leader CTA only), 16 epilogue warps (TMEM -> registers ->
+// bf16 -> whole 32-byte sectors of the lanes' own rows).  With four of them and a transpose through shared memory, which the
+// tensor cores and the copies keep busy, a tile's output took longer than 16 steps of K: 8192 x 4096 x 1024 with SiLU 59.1 us,
+// now 53.4 (without 52.1 and 50.2; 1076 x 5648 x 560 13.8 and 13.0; 8192 x 14336 x 4096 739 and 726 under the power cap).
 // Every mbarrier wait is bounded; the cluster barriers at start and end are reached on every path.
 // The reference library has no GEMM: this kernel serves the tensor-parallel and expert-parallel layers.
 #include <algorithm>
@@ -32,8 +34,10 @@ constexpr int G2_HALF = 128; // rows of A and rows of B staged per CTA
 constexpr int G2_STAGE_A = G2_HALF * GEMM_BK * 2;
 constexpr int G2_STAGE_B = G2_HALF * GEMM_BK * 2;
 constexpr int G2_RING = G2_STAGES * (G2_STAGE_A + G2_STAGE_B);
-constexpr int G2_EPI = 4 * 32 * GEMM_EPI_ROW_BYTES;
-constexpr int G2_SMEM = 1024 + G2_RING + G2_EPI + 256;
+constexpr int G2_EPI_WARPS = 16;
+constexpr int G2_PART = G2_BN / (G2_EPI_WARPS / 4); // columns of a tile that an epilogue warp drains
+constexpr int G2_THREADS = 64 + 32 * G2_EPI_WARPS;
+constexpr int G2_SMEM = 1024 + G2_RING + 256;
 constexpr size_t G2_GROUP_BYTES = 32u << 20; // of B per raster group
 
 struct gemm2_params {
@@ -43,6 +47,7 @@ struct gemm2_params {
     uint32_t* err;
     int M, N, K, epilogue;
     int group_n; // tile columns per raster group
+    int wide; // rows of C begin at 32-byte sectors
     unsigned long long timeout_ns;
     const int* rows; // optional device word: only the first min(M, *rows) rows of A are multiplied
 };
@@ -71,18 +76,17 @@ __device__ __forceinline__ void g2_tile(int t, int tiles_m, int tiles_n, int gro
 // PAIRS: CTA pairs per cluster.  With two, the tiles of a last, less than half full round are cut along K between the pairs of a
 // cluster, which add their halves through distributed shared memory.
 template <int PAIRS>
-__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm2sm_kernel(const __grid_constant__ gemm2_params P) {
+__global__ void __launch_bounds__(G2_THREADS, 1) gemm2sm_kernel(const __grid_constant__ gemm2_params P) {
     using namespace sm100;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* sA = smem;
     uint8_t* sB = smem + G2_STAGES * G2_STAGE_A;
-    uint8_t* sEpi = smem + G2_RING;
-    uint64_t* bars = (uint64_t*)(smem + G2_RING + G2_EPI);
+    uint64_t* bars = (uint64_t*)(smem + G2_RING);
     uint64_t* full = bars; // [STAGES]  used in the leader: bytes of both CTAs
     uint64_t* empty = bars + G2_STAGES; // [STAGES]  per CTA, signalled by the MMA commit
     uint64_t* tfull = bars + 2 * G2_STAGES; // [2] per CTA
-    uint64_t* tempty = bars + 2 * G2_STAGES + 2; // [2] used in the leader: 4 warps x 2 CTAs
+    uint64_t* tempty = bars + 2 * G2_STAGES + 2; // [2] used in the leader: the epilogue warps of both CTAs
     uint32_t* tmem_holder = (uint32_t*)(bars + 2 * G2_STAGES + 4);
     volatile int* abort_flag = (volatile int*)(tmem_holder + 1);
 
@@ -102,7 +106,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm2sm_kernel(const __grid_c
         }
         for (int i = 0; i < 2; i++) {
             mbar_init(&tfull[i], 1);
-            mbar_init(&tempty[i], 8);
+            mbar_init(&tempty[i], 2 * G2_EPI_WARPS);
         }
         mbar_fence_init();
         tma_prefetch_desc(&P.tmA);
@@ -201,42 +205,35 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm2sm_kernel(const __grid_c
         __syncwarp();
     }
     const int q = warp & 3; // TMEM lane quarter this warp may read
-    uint8_t* stage = sEpi + (q * 32) * GEMM_EPI_ROW_BYTES;
-    // 64 columns of one row per lane: activation, bf16, and through shared memory to coalesced stores
-    auto emit = [&](const uint32_t (&r0)[32], const uint32_t (&r1)[32], int row0, int col0) {
-        uint32_t packed[32];
+    const int part = (warp - 2) >> 2; // this warp's share of the columns
+    // 16 columns of a lane's own row: activation, bf16, a whole 32-byte sector
+    auto emit = [&](const uint32_t (&r)[16], int row, int col) {
+        uint32_t w[8];
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            float a0 = __uint_as_float(r0[2 * i]), a1 = __uint_as_float(r0[2 * i + 1]);
-            float b0 = __uint_as_float(r1[2 * i]), b1 = __uint_as_float(r1[2 * i + 1]);
+        for (int i = 0; i < 8; i++) {
+            float a0 = __uint_as_float(r[2 * i]), a1 = __uint_as_float(r[2 * i + 1]);
             if (P.epilogue == EPI_SILU) {
                 a0 = silu_f(a0);
                 a1 = silu_f(a1);
-                b0 = silu_f(b0);
-                b1 = silu_f(b1);
             }
-            __nv_bfloat162 lo = __floats2bfloat162_rn(a0, a1);
-            __nv_bfloat162 hi = __floats2bfloat162_rn(b0, b1);
-            packed[i] = *reinterpret_cast<uint32_t*>(&lo);
-            packed[16 + i] = *reinterpret_cast<uint32_t*>(&hi);
+            const __nv_bfloat162 h = __floats2bfloat162_rn(a0, a1);
+            w[i] = *reinterpret_cast<const uint32_t*>(&h);
         }
-        uint8_t* myrow = stage + lane * GEMM_EPI_ROW_BYTES;
-#pragma unroll
-        for (int v = 0; v < 8; v++)
-            *reinterpret_cast<uint4*>(myrow + v * 16) =
-                make_uint4(packed[4 * v], packed[4 * v + 1], packed[4 * v + 2], packed[4 * v + 3]);
-        __syncwarp();
-        const int gcol = col0 + (lane & 7) * 8;
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int rr = i * 4 + (lane >> 3);
-            const int grow = row0 + rr;
-            if (grow < M && gcol < P.N) {
-                uint4 v = *reinterpret_cast<const uint4*>(stage + rr * GEMM_EPI_ROW_BYTES + (lane & 7) * 16);
-                *reinterpret_cast<uint4*>(P.C + (size_t)grow * P.N + gcol) = v;
+        __nv_bfloat16* p = P.C + (size_t)row * P.N + col;
+        if (row < M) {
+            if (P.wide) {
+                if (col < P.N)
+                    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]),
+                                 "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                                 : "memory");
             }
+            else
+#pragma unroll
+                for (int h = 0; h < 8; h += 4)
+                    if (col + 2 * h < P.N)
+                        *reinterpret_cast<uint4*>(p + 2 * h) = make_uint4(w[h], w[h + 1], w[h + 2], w[h + 3]);
         }
-        __syncwarp();
+        __syncwarp(); // lanes part where rows or columns end
     };
     bool good = warp >= 2;
     if (warp >= 2) {
@@ -247,29 +244,31 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm2sm_kernel(const __grid_c
                 if (lane == 0)
                     g2_fail(P, abort_flag, GE_MBAR_TIMEOUT, 5);
                 good = false;
-                break;
             }
+            // a lane may see the flag of another role's failure and leave alone: the warp goes on together or not at all
+            good = __all_sync(0xffffffffu, good);
+            if (!good)
+                break;
             tc_fence_after_sync();
             if (n == mine) // the cut tile
                 break;
             int mi, ni;
             g2_tile(tile_of(n), tiles_m, tiles_n, P.group_n, mi, ni);
-            const int row0 = mi * 256 + (int)cr * G2_HALF + q * 32;
-#pragma unroll 1
-            for (int c = 0; c < G2_BN / GEMM_EPI_COLS; c++) {
-                uint32_t r0[32], r1[32];
-                const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * G2_BN + c * GEMM_EPI_COLS;
-                tmem_ld_32x32(taddr, r0);
-                tmem_ld_32x32(taddr + 32, r1);
+            const int row = mi * 256 + (int)cr * G2_HALF + q * 32 + lane, col0 = ni * G2_BN + part * G2_PART;
+            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * G2_BN + part * G2_PART;
+#pragma unroll
+            for (int c = 0; c < G2_PART; c += 16) {
+                uint32_t r[16];
+                tmem_ld_32x16(taddr + c, r);
                 tmem_ld_wait();
-                if (c == G2_BN / GEMM_EPI_COLS - 1) {
+                if (c == G2_PART - 16) {
                     // all reads of this accumulator are done: hand it back to the leader's MMA warp
                     tc_fence_before_sync();
                     __syncwarp();
                     if (lane == 0)
                         mbar_arrive_cluster(tempty_leader + acc * 8);
                 }
-                emit(r0, r1, row0, ni * G2_BN + c * GEMM_EPI_COLS);
+                emit(r, row, col0 + c);
             }
         }
     }
@@ -277,45 +276,44 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm2sm_kernel(const __grid_c
         if (cut) {
             // Pair p finishes columns [128 p, 128 p + 128) of the tile: the other pair's half sums of them arrive in the ring, which
             // nobody uses any more, as packs of four columns per row.  The sum of two halves does not depend on their order.
+            constexpr int HALF_PART = G2_PART / 2;
             const uint32_t acc = mine & 1;
-            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * G2_BN;
-            const uint32_t here = smem_u32(smem) + (uint32_t)(q * 32 + lane) * 16;
+            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * G2_BN + part * HALF_PART;
+            const uint32_t here = smem_u32(smem) + (uint32_t)(q * 32 + lane + part * (HALF_PART / 4) * G2_HALF) * 16;
             cluster_sync_all();
             if (warp >= 2 && good) {
                 const uint32_t there = map_to_cta(here, rank ^ 2);
-#pragma unroll 1
-                for (int c = 0; c < G2_BN / 2; c += 32) {
-                    uint32_t r[32];
-                    tmem_ld_32x32(taddr + (pair ^ 1) * (G2_BN / 2) + c, r);
+#pragma unroll
+                for (int c = 0; c < HALF_PART; c += 16) {
+                    uint32_t r[16];
+                    tmem_ld_32x16(taddr + (pair ^ 1) * (G2_BN / 2) + c, r);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4)
+                    for (int i = 0; i < 16; i += 4)
                         st_cluster_v4(there + (uint32_t)(c + i) / 4 * G2_HALF * 16, r[i], r[i + 1], r[i + 2], r[i + 3]);
                 }
             }
             cluster_sync_all();
-            if (warp >= 2 && good && !*abort_flag) {
+            if (warp >= 2 && good && !__any_sync(0xffffffffu, *abort_flag != 0)) {
                 int mi, ni;
                 g2_tile(whole + cluster, tiles_m, tiles_n, P.group_n, mi, ni);
-#pragma unroll 1
-                for (int c = 0; c < G2_BN / 2; c += GEMM_EPI_COLS) {
-                    uint32_t r[2][32];
-                    tmem_ld_32x32(taddr + pair * (G2_BN / 2) + c, r[0]);
-                    tmem_ld_32x32(taddr + pair * (G2_BN / 2) + c + 32, r[1]);
+#pragma unroll
+                for (int c = 0; c < HALF_PART; c += 16) {
+                    uint32_t r[16];
+                    tmem_ld_32x16(taddr + pair * (G2_BN / 2) + c, r);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int h = 0; h < 2; h++)
+                    for (int i = 0; i < 16; i += 4) {
+                        float v[4];
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                                     : "r"(here + (uint32_t)(c + i) / 4 * G2_HALF * 16));
 #pragma unroll
-                        for (int i = 0; i < 32; i += 4) {
-                            float v[4];
-                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                                         : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
-                                         : "r"(here + (uint32_t)(c + 32 * h + i) / 4 * G2_HALF * 16));
-#pragma unroll
-                            for (int k = 0; k < 4; k++)
-                                r[h][i + k] = __float_as_uint(__uint_as_float(r[h][i + k]) + v[k]);
-                        }
-                    emit(r[0], r[1], mi * 256 + (int)cr * G2_HALF + q * 32, ni * G2_BN + (int)pair * (G2_BN / 2) + c);
+                        for (int k = 0; k < 4; k++)
+                            r[i + k] = __float_as_uint(__uint_as_float(r[i + k]) + v[k]);
+                    }
+                    emit(r, mi * 256 + (int)cr * G2_HALF + q * 32 + lane,
+                         ni * G2_BN + (int)pair * (G2_BN / 2) + part * HALF_PART + c);
                 }
             }
         }
@@ -343,7 +341,7 @@ int most_clusters() {
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute attr{};
         cfg.gridDim = dim3(2 * PAIRS);
-        cfg.blockDim = dim3(GEMM_THREADS);
+        cfg.blockDim = dim3(G2_THREADS);
         cfg.dynamicSmemBytes = G2_SMEM;
         attr.id = cudaLaunchAttributeClusterDimension;
         attr.val.clusterDim.x = 2 * PAIRS;
@@ -378,7 +376,7 @@ template <int PAIRS>
 void launch_2sm(const gemm2_params& P, int clusters, cudaStream_t st) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(2 * PAIRS * clusters);
-    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.blockDim = dim3(G2_THREADS);
     cfg.dynamicSmemBytes = G2_SMEM;
     cfg.stream = st;
     cudaLaunchAttribute attr[2]{};
@@ -412,6 +410,7 @@ void gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, i
     P.K = K;
     P.epilogue = epilogue;
     P.rows = rows_dev;
+    P.wide = N % 16 == 0 && ((uintptr_t)C & 31) == 0;
     P.timeout_ns = (unsigned long long)env_data::get().wait_timeout_ms * 1000000ull;
     const int tiles_n = (N + G2_BN - 1) / G2_BN;
     const int most = (int)std::min<size_t>(std::max<size_t>(G2_GROUP_BYTES / ((size_t)G2_BN * K * 2), 4), 32);
