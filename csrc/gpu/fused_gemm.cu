@@ -36,6 +36,9 @@ CUtensorMap make_map(const void* base, uint64_t rows, uint64_t cols, uint32_t bo
 
 } // namespace
 
+CUtensorMap make_bf16_map(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+    return make_map(base, rows, cols, box_rows);
+}
 CUtensorMap make_bf16_kmajor_map(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
     return make_map(base, rows, cols, box_rows);
 }

@@ -15,6 +15,7 @@
 #include "gpu/async_copy.cuh"
 #include "gpu/cuda_driver.hpp"
 #include "gpu/f32x2.cuh"
+#include "gpu/gelu.cuh"
 #include "gpu/launch_util.cuh"
 
 using namespace cclx;
@@ -401,26 +402,6 @@ __global__ void __launch_bounds__(128) map_colsum_kernel(F f, size_t rows, int p
     out[1] = make_float4(s[4], s[5], s[6], s[7]);
 }
 
-// Gaussian error linear unit, tanh form: 0.5 x (1 + tanh(u)) = x g with g = 1 / (1 + exp(-2 u)), u = sqrt(2 / pi) (x + 0.044715 x^3).
-//
-// g is rounded where tanh(u) = 2 g - 1 is rounded to fp32 before the 1 is added back.  Without that the result is nearer to the
-// true value below x = -3, but there other bf16 values than the operator of the same name in the framework around it gives: a
-// handful of activations per layer, from which every later one of the sequence rounds differently (1 % in the gradients of
-// a 24-layer step).  With it all 65536 bf16 inputs give that operator's bits, and an infinite or huge negative x its
-// NaN or zero, in the same 20 us for 8192 x 4096 values (tanhf: 31 us).
-__device__ __forceinline__ float gelu_gate(float x) {
-    constexpr float C = -2.f * 0.7978845608028654f * 1.4426950408889634f; // -2 sqrt(2 / pi) log2(e)
-    float e, g;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(C * x * fmaf(0.044715f * x, x, 1.f)));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(g) : "f"(1.f + e));
-    return (g - 0.5f) + 0.5f;
-}
-__device__ __forceinline__ float gelu_slope(float x) { // g + 2 x g (1 - g) u'
-    constexpr float K = 2.f * 0.7978845608028654f;
-    const float g = gelu_gate(x);
-    return fmaf(x * g * (1.f - g), fmaf(K * 3.f * 0.044715f, x * x, K), g);
-}
-
 __global__ void __launch_bounds__(256) gelu_fwd_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, size_t packs) {
     const size_t i0 = (size_t)blockIdx.x * 512 + threadIdx.x;
     uint4 u[2];
@@ -431,12 +412,12 @@ __global__ void __launch_bounds__(256) gelu_fwd_kernel(const uint4* __restrict__
 #pragma unroll
     for (int k = 0; k < 2; k++)
         if (i0 + k * 256 < packs) {
-            float v[8];
-            unpack8(u[k], v);
+            f32x2 v[4];
+            unpack4x2(u[k], v);
 #pragma unroll
-            for (int e = 0; e < 8; e++)
-                v[e] *= gelu_gate(v[e]);
-            y[i0 + k * 256] = pack8(v);
+            for (int e = 0; e < 4; e++)
+                v[e] = mul2(v[e], gelu_gate(v[e]));
+            y[i0 + k * 256] = pack4x2(v);
         }
 }
 
@@ -467,13 +448,12 @@ struct gelu_bwd_map {
         return { dy[r * packs + p], x[r * packs + p] };
     }
     __device__ __forceinline__ void apply(const input& in, f32x2 (&v)[4]) const {
-        float a[8];
-        f32x2 g[4];
-        unpack8(in.x, a);
+        f32x2 a[4], g[4];
+        unpack4x2(in.x, a);
         unpack4x2(in.dy, g);
 #pragma unroll
         for (int e = 0; e < 4; e++)
-            v[e] = mul2(g[e], pair(gelu_slope(a[2 * e]), gelu_slope(a[2 * e + 1])));
+            v[e] = mul2(g[e], gelu_slope(a[e]));
     }
     __device__ __forceinline__ void store(size_t r, int p, const uint4& u) const {
         dx[r * packs + p] = u;

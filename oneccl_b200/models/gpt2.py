@@ -76,9 +76,7 @@ class Block(nn.Module):
         a = F.scaled_dot_product_attention(q, k, v, is_causal=True)
         attn = K.linear(a.transpose(1, 2).reshape(B, S, D), self.proj.weight, self.proj.bias, defer_bias=True)
         h, x = K.add_layer_norm(x, attn, self.ln2.weight, self.ln2.bias, self.ln2.eps, self.proj.bias)
-        u = K.linear(h, self.fc.weight, self.fc.bias, defer_bias=True)
-        delta = K.linear(K.gelu(u, self.fc.bias), self.fc2.weight, self.fc2.bias, defer_bias=True)
-        return x, delta, self.fc2.bias
+        return x, K.mlp(h, self.fc.weight, self.fc.bias, self.fc2.weight, self.fc2.bias), self.fc2.bias
 
     def fused_ok(self, x) -> bool:
         """Whether ``forward_fused`` takes activations like ``x``."""

@@ -7,7 +7,8 @@
 * ``linear``: cuBLAS matmuls, with the bias gradient by a column sum or left to the next operator;
 * ``split_qkv``: views of a packed QKV projection for the attention call, whose backward assembles the
   packed gradient and sums it over the rows in one pass;
-* ``gelu``: tanh-form GELU; ``embed``: token plus position embedding.
+* ``gelu``: tanh-form GELU; ``mlp``: two linear layers with a GELU between them, which runs inside the products
+  (``csrc/gpu/gemm_mlp.cu``); ``embed``: token plus position embedding.
 
 The kernel that produces the gradient of a linear layer's output can sum the bias gradient on the way.  ``linear(...,
 defer_bias=True)`` leaves it to the operator that consumes the output and is given the bias: ``add_layer_norm(...,
@@ -71,6 +72,15 @@ def gelu(u, bias):
     y = native().bias_gelu(u, bias)
     if y is None:  # adds nothing, but hands the bias its gradient
         return F.gelu(u + (bias - bias.detach()).to(u.dtype), approximate="tanh")
+    return y
+
+
+def mlp(x, w1, b1, w2, b2):
+    """``gelu(x @ w1.T + b1) @ w2.T + b2`` with the tanh-form GELU and its gradient inside the products where the batch is large
+    enough, else as ``linear``, ``gelu``, ``linear``.  ``b2``'s gradient is left to the operator that consumes the output."""
+    y = native().mlp(x, w1, b1, w2, b2)
+    if y is None:
+        return linear(gelu(linear(x, w1, b1, defer_bias=True), b1), w2, b2, defer_bias=True)
     return y
 
 

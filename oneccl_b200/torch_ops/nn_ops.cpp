@@ -288,6 +288,40 @@ void column_sums(const Tensor& dy, const ParamGrad& out) {
     launches += 2;
 }
 
+// Gradient of a linear layer's weight: into its sink, if possible beside the rest of backward, or to autograd (`out`).
+struct WeightGrad {
+    SinkRef sink;
+    bool beside;
+    at::cuda::CUDAEvent ready; // the gradient of the layer's output is there
+    Tensor out;
+
+    WeightGrad(const SinkRef& s, const Tensor& dy) : sink(s), beside(s && s->beside) {
+        if (beside)
+            ready.record(at::cuda::getCurrentCUDAStream(dy.get_device()));
+    }
+    void product(const Tensor& dy, const Tensor& x, bool needed) {
+        if (!sink) {
+            if (needed)
+                out = dy.t().mm(x);
+            return;
+        }
+        GradSink& s = *sink;
+        const bool add = beside && s.on_side ? s.take() : s.add();
+        auto f = [&] {
+            if (add)
+                s.grad.addmm_(dy.t(), x);
+            else
+                at::mm_out(s.grad, dy.t(), x);
+        };
+        if (beside) {
+            s.beside->launch(ready, f, dy, x);
+            s.on_side = true;
+        }
+        else
+            f();
+    }
+};
+
 // cuBLAS products with the weight gradient accumulated straight into its sink, if possible beside the rest of backward.
 struct Linear : torch::autograd::Function<Linear> {
     // bias_grad: computed here (else another operator returns it); report: this is the weight's last contribution
@@ -312,31 +346,11 @@ struct Linear : torch::autograd::Function<Linear> {
         const auto sinks = sinks_of(ctx, 2);
         const int64_t flags = ctx->saved_data["flags"].toInt();
         const Tensor dy = rows_of(grads[0], grads[0].size(-1));
-        Tensor dx, dw, db;
-        const bool beside = sinks[0] && sinks[0]->beside;
-        at::cuda::CUDAEvent ready; // dy is there
-        if (beside)
-            ready.record(at::cuda::getCurrentCUDAStream(dy.get_device()));
+        Tensor dx, db;
+        WeightGrad dw(sinks[0], dy);
         if (ctx->needs_input_grad(0))
             dx = dy.mm(weight).view(ctx->saved_data["shape"].toIntVector());
-        if (sinks[0]) {
-            GradSink& s = *sinks[0];
-            const bool add = beside && s.on_side ? s.take() : s.add();
-            auto product = [&] {
-                if (add)
-                    s.grad.addmm_(dy.t(), x2);
-                else
-                    at::mm_out(s.grad, dy.t(), x2);
-            };
-            if (beside) {
-                s.beside->launch(ready, product, dy, x2);
-                s.on_side = true;
-            }
-            else
-                product();
-        }
-        else if (ctx->needs_input_grad(1))
-            dw = dy.t().mm(x2);
+        dw.product(dy, x2, ctx->needs_input_grad(1));
         if (flags & 1) {
             const ParamGrad g(sinks[1], dy, { dy.size(1) });
             column_sums(dy, g);
@@ -345,7 +359,7 @@ struct Linear : torch::autograd::Function<Linear> {
         }
         if (sinks[0] && flags & 2)
             sinks[0]->report();
-        return { dx, dw, db, Tensor(), Tensor(), Tensor() };
+        return { dx, dw.out, db, Tensor(), Tensor(), Tensor() };
     }
 };
 
@@ -402,6 +416,82 @@ pybind11::object bias_gelu(const Tensor& u, const pybind11::object& b_) {
     std::vector<SinkRef> sinks{ sink_of(b_) };
     pybind11::gil_scoped_release nogil;
     Tensor y = BiasGelu::apply(u, b, std::move(sinks))[0];
+    pybind11::gil_scoped_acquire gil;
+    return pybind11::cast(y);
+}
+
+// gelu(x W1^T + b1) W2^T + b2 with the GELU and its gradient inside the products (csrc/gpu/gemm_mlp.cu).  b2's gradient is left to
+// the operator that consumes the output.
+struct Mlp : torch::autograd::Function<Mlp> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& w1, const Tensor& b1, const Tensor& w2,
+                                 const Tensor& b2, std::vector<SinkRef> sinks) {
+        const int64_t D = x.size(-1), N = w1.size(0);
+        const Tensor x2 = rows_of(x, D), w = dense(w1), b = dense(b1);
+        const Tensor u = empty_on(x2, { x2.size(0), N }, at::kBFloat16), g = empty_on(x2, { x2.size(0), N }, at::kBFloat16);
+        check(cclx_linear_gelu(x2.data_ptr(), w.data_ptr(), b.data_ptr(), u.data_ptr(), g.data_ptr(), (int)x2.size(0), (int)N, (int)D,
+                               stream_of(x2)));
+        launches += 1;
+        ctx->save_for_backward({ x2, w1, b1, w2, u, g });
+        ctx->saved_data["shape"] = x.sizes().vec();
+        keep_sinks(ctx, std::move(sinks));
+        const Tensor y = at::addmm(b2, g, w2.t());
+        auto shape = x.sizes().vec();
+        shape.back() = w2.size(0);
+        return { y.view(shape) };
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        const Tensor &x2 = saved[0], &w1 = saved[1], &w2 = saved[3], &u = saved[4], &g = saved[5];
+        const auto sinks = sinks_of(ctx, 3); // of w1, b1, w2
+        const int64_t rows = u.size(0), N = u.size(1), K = w2.size(0);
+        const Tensor dy = rows_of(grads[0], K), w = dense(w2);
+        WeightGrad d2(sinks[2], dy);
+        const Tensor du = empty_on(u, u.sizes(), at::kBFloat16);
+        const GradStreamRef beside = beside_of({ sinks[1] });
+        const ParamGrad db(sinks[1], u, saved[2].sizes(), (bool)beside);
+        const int n = cclx_linear_gelu_bwd_rows((int)rows);
+        const Tensor ws = empty_on(u, { n * N }, at::kFloat);
+        void* st = stream_of(u);
+        with_sums(beside, ws, (int)N, { &db }, [&](int* defer) {
+            check(cclx_linear_gelu_bwd(dy.data_ptr(), w.data_ptr(), u.data_ptr(), du.data_ptr(), ws.data_ptr<float>(), (int)rows, (int)N,
+                                       (int)K, st));
+            if (defer)
+                *defer = n;
+            else
+                check(cclx_partial_sums(ws.data_ptr<float>(), n, (int)N, 1, db.ptr(), nullptr, nullptr, db.add, st));
+        });
+        d2.product(dy, g, ctx->needs_input_grad(3));
+        db.done();
+        if (sinks[2])
+            sinks[2]->report();
+        WeightGrad d1(sinks[0], du);
+        Tensor dx;
+        if (ctx->needs_input_grad(0))
+            dx = du.mm(w1).view(ctx->saved_data["shape"].toIntVector());
+        d1.product(du, x2, ctx->needs_input_grad(1));
+        if (sinks[0])
+            sinks[0]->report();
+        return { dx, d1.out, db.result(), d2.out, Tensor(), Tensor() };
+    }
+};
+
+// None where the operator does not take the call, or products of their own are expected to be faster
+pybind11::object mlp(const Tensor& x, const pybind11::object& w1_, const pybind11::object& b1_, const pybind11::object& w2_,
+                     const pybind11::object& b2_) {
+    const Tensor w1 = tensor_of(w1_), b1 = tensor_of(b1_), w2 = tensor_of(w2_), b2 = tensor_of(b2_);
+    if (!bf16_cuda(x) || x.dim() < 1 || !bf16_cuda(w1) || !bf16_cuda(w2) || w1.dim() != 2 || w2.dim() != 2 ||
+        w1.device() != x.device() || w2.device() != x.device() || w1.size(1) != x.size(-1) || w2.size(1) != w1.size(0) ||
+        w1.size(0) % 8 != 0 || w1.size(1) % 8 != 0 || w2.size(0) % 8 != 0 || x.numel() == 0 || w1.numel() == 0 || w2.numel() == 0 ||
+        !bias_ok(b1, x, w1.size(0)) || !bias_ok(b2, x, w2.size(0)))
+        return pybind11::none();
+    const int64_t rows = x.numel() / x.size(-1);
+    if (rows * std::max(w1.size(0), w2.size(0)) >= (int64_t)1 << 31 ||
+        !cclx_mlp_preferred((int)rows, (int)w1.size(0)))
+        return pybind11::none();
+    std::vector<SinkRef> sinks{ sink_of(w1_), sink_of(b1_), sink_of(w2_) };
+    pybind11::gil_scoped_release nogil;
+    Tensor y = Mlp::apply(x, w1, b1, w2, b2, std::move(sinks))[0];
     pybind11::gil_scoped_acquire gil;
     return pybind11::cast(y);
 }
@@ -536,6 +626,7 @@ void bind_nn(pybind11::module_& m) {
           pybind11::arg("bias"), pybind11::arg("eps"), pybind11::arg("res_bias") = pybind11::none());
     m.def("linear", &linear);
     m.def("bias_gelu", &bias_gelu);
+    m.def("mlp", &mlp);
     m.def("split_qkv", &split_qkv);
     m.def("embed", &embed);
     m.def("embed_check", &embed_check);

@@ -145,3 +145,38 @@ def test_data_parallel_gradient_sinks_match_autograd():
         for (n, a), (_, b) in zip(plain.named_parameters(), wrapped.named_parameters()):
             torch.testing.assert_close(b.grad.float(), a.grad.float(), rtol=2e-2, atol=2e-3, msg=n)
     group.close()
+
+
+@pytest.mark.parametrize("shape", [(4608, 64, 1024, 136), (1999, 1032, 2056, 8), (2305, 768, 3072, 768), (3, 600, 264, 2200, 64)])
+def test_mlp(shape):
+    """Two linear layers with the GELU inside the products against the same chain of operators of their own, and both against
+    64 bits: partial tiles in every dimension, K of one step, several leading dimensions."""
+    from oneccl_b200.ops import nn as K
+    from oneccl_b200.torch_ops import native
+
+    lead, (D, N, O) = (shape[:-3], shape[-3:])
+    g = torch.Generator(device="cuda").manual_seed(3)
+
+    def make(*s, scale=1.0):
+        return (torch.randn(*s, generator=g, device="cuda") * scale).to(torch.bfloat16)
+
+    x, w1, b1, w2, b2 = make(*lead, D), make(N, D, scale=D**-0.5), make(N), make(O, N, scale=N**-0.5), make(O)
+    dy = make(*lead, O)
+    ins = [t.requires_grad_(True) for t in (x, w1, b1, w2)]
+
+    def chain():
+        return K.linear(K.gelu(K.linear(x, w1, b1, defer_bias=True), b1), w2, b2, defer_bias=True)
+
+    fused = native().mlp(x, w1, b1, w2, b2)
+    assert fused is not None
+    outs = []
+    for y in (fused, chain()):
+        outs.append((y.detach(), *torch.autograd.grad(y, ins, dy)))
+    xd, w1d, b1d, w2d = (t.detach().double().requires_grad_(True) for t in ins)
+    yd = torch.nn.functional.gelu(xd @ w1d.t() + b1d, approximate="tanh") @ w2d.t() + b2.double()
+    exact = (yd.detach(), *torch.autograd.grad(yd, (xd, w1d, b1d, w2d), dy.double()))
+    for a, b, e in zip(*outs, exact):
+        assert a.shape == b.shape == e.shape and a.dtype == b.dtype
+        off, ref = ((t.double() - e).norm() / e.norm() for t in (a, b))
+        # both round u, gelu(u), its gradient and every result to bf16 once (2^-9 each, 2^-8 with their sum): neither is further off
+        assert off <= 2.0**-7 and off <= 1.05 * ref + 2.0**-14, (off, ref)
