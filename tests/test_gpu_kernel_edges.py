@@ -640,6 +640,59 @@ def test_gradient_stream_keeps_operands_until_their_stream_has_waited():
     group.close()
 
 
+@pytest.mark.parametrize("T,E,k", [(1, 1, 1), (511, 64, 8), (512, 64, 8), (513, 3, 2), (520, 33, 7), (4091, 16, 2), (8192, 9, 1)])
+def test_routing_in_one_block_and_in_a_cluster(T, E, k):
+    """Last size of one block, first of a cluster, shares that do not divide, a block without tokens, every number of experts."""
+    from oneccl_b200.parallel.ep import route_device
+
+    g = torch.Generator(device="cuda").manual_seed(T + E)
+    logits = torch.randn(T, E, generator=g, device="cuda")
+    idx, wts, counts, order, pos = route_device(logits, k)
+    ref = torch.topk(logits, k, dim=-1)
+    assert torch.equal(idx, ref.indices) and torch.equal(counts, torch.bincount(ref.indices.flatten(), minlength=E))
+    torch.testing.assert_close(wts, torch.softmax(ref.values, -1), rtol=1e-5, atol=1e-6)
+    assert torch.equal(order[pos], torch.arange(T * k, device="cuda")) and torch.equal(pos[order], torch.arange(T * k, device="cuda"))
+    assert bool((idx.flatten()[order].diff() >= 0).all())
+
+
+@pytest.mark.parametrize("W,T,H,k,skew", [(3, 77, 520, 1, 9.0), (3, 700, 264, 3, 2.0), (8, 600, 2056, 2, 5.0), (8, 5, 4096, 2, 0.0)])
+def test_moe_exchange_of_uneven_loads(W, T, H, k, skew):
+    """Experts with most, few and none of the rows, ranks that do not divide the parts of the lists: every row arrives once, in
+    the order of `order`, and nothing else is written."""
+    from oneccl_b200.ops.device_group import DeviceGroup
+    from oneccl_b200.parallel.ep import fused_combine, fused_dispatch, route_device
+
+    g = torch.Generator(device="cuda").manual_seed(T + H)
+    cap = T * k * W
+    group = DeviceGroup.emulated(W, heap_bytes=cap * H * 2 + (40 << 20), staging_bytes=1 << 20)
+    recv = group.symm_empty((cap, H), dtype=torch.bfloat16)
+    table = group.symm_empty((256 * W * W,), dtype=torch.int32)
+    meta = [torch.zeros(2 * W + 2, dtype=torch.int32, device="cuda") for _ in range(W)]
+    bias = torch.zeros(W, device="cuda")
+    bias[1], bias[W - 1] = skew, -skew * 4
+    x = [_bf16(g, T, H) for _ in range(W)]
+    idx, wts, counts, order, pos = zip(*(route_device(torch.randn(T, W, generator=g, device="cuda") + bias, k) for _ in range(W)))
+    out = [torch.empty_like(t) for t in x]
+    for t in recv:
+        t.fill_(7.0)
+    fused_dispatch(group, x, order, counts, meta, recv, table, k)
+    torch.cuda.synchronize()
+    for e in range(W):
+        sent = []
+        for r in range(W):
+            first = int(counts[r][:e].sum())
+            sent.append(x[r][order[r][first:first + int(counts[r][e])] // k])
+        sent = torch.cat(sent)
+        assert int(meta[e][2 * W]) == len(sent) and int(meta[e][2 * W + 1]) == 0
+        assert torch.equal(recv[e][: len(sent)], sent) and bool((recv[e][len(sent):] == 7.0).all())
+    fused_combine(group, [i.view(-1) for i in idx], pos, [w.view(-1) for w in wts], out, meta, recv, k)
+    torch.cuda.synchronize()
+    group.check()
+    for r in range(W):  # the weights of a token sum to 1 within their rounding, its copies are equal
+        torch.testing.assert_close(out[r].float(), x[r].float(), rtol=2.0**-7, atol=2.0**-9)
+    group.close()
+
+
 @pytest.mark.parametrize("T,E,k", [(3, 3, 1), (5000, 5, 2), (4097, 63, 3)])
 def test_routing_outputs_are_aligned_and_nothing_else_is_written(T, E, k):
     """One block and two kernels, odd numbers of items and experts.  The C entry with another value between counts and scratch."""
