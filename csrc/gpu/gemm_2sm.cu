@@ -47,7 +47,6 @@ struct gemm2_params {
     uint32_t* err;
     int M, N, K, epilogue;
     int group_n; // tile columns per raster group
-    int wide; // rows of C begin at 32-byte sectors
     unsigned long long timeout_ns;
     const int* rows; // optional device word: only the first min(M, *rows) rows of A are multiplied
 };
@@ -71,6 +70,47 @@ __device__ __forceinline__ void g2_tile(int t, int tiles_m, int tiles_n, int gro
     const int width = min(group, tiles_n - grp * group);
     mi = in / width;
     ni = grp * group + in % width;
+}
+
+__device__ __forceinline__ void st_8(__nv_bfloat16* p, const uint32_t* w) { // 8 columns
+    *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ void st_16(__nv_bfloat16* p, const uint32_t* w) { // 16 columns, a whole sector
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+                 "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+}
+
+// 2 W columns of a row of C from column `col` on, a multiple of 16, in whole 32-byte sectors.  Where N is an odd number of eights every
+// other row begins in the middle of one: then the first and the last half sector go alone.
+template <int W>
+__device__ __forceinline__ void g2_store(const gemm2_params& P, int M, int row, int col, const uint32_t (&w)[W]) {
+    if (row >= M)
+        return;
+    __nv_bfloat16* p = P.C + (size_t)row * P.N + col;
+    const int left = P.N - col; // columns, a multiple of 8
+    if (((uintptr_t)p & 31) == 0) {
+#pragma unroll
+        for (int i = 0; i < W; i += 8) {
+            if (2 * i + 16 <= left)
+                st_16(p + 2 * i, w + i);
+            else if (2 * i < left)
+                st_8(p + 2 * i, w + i);
+        }
+    }
+    else {
+        if (left > 0)
+            st_8(p, w);
+#pragma unroll
+        for (int i = 4; i + 8 < W; i += 8) {
+            if (2 * i + 16 <= left)
+                st_16(p + 2 * i, w + i);
+            else if (2 * i < left)
+                st_8(p + 2 * i, w + i);
+        }
+        if (2 * (W - 4) < left)
+            st_8(p + 2 * (W - 4), w + W - 4);
+    }
 }
 
 // PAIRS: CTA pairs per cluster.  With two, the tiles of a last, less than half full round are cut along K between the pairs of a
@@ -206,9 +246,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) gemm2sm_kernel(const __grid_con
     }
     const int q = warp & 3; // TMEM lane quarter this warp may read
     const int part = (warp - 2) >> 2; // this warp's share of the columns
-    // 16 columns of a lane's own row: activation, bf16, a whole 32-byte sector
-    auto emit = [&](const uint32_t (&r)[16], int row, int col) {
-        uint32_t w[8];
+    auto convert = [&](const uint32_t (&r)[16], uint32_t* w) { // activation and bf16
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             float a0 = __uint_as_float(r[2 * i]), a1 = __uint_as_float(r[2 * i + 1]);
@@ -219,21 +257,6 @@ __global__ void __launch_bounds__(G2_THREADS, 1) gemm2sm_kernel(const __grid_con
             const __nv_bfloat162 h = __floats2bfloat162_rn(a0, a1);
             w[i] = *reinterpret_cast<const uint32_t*>(&h);
         }
-        __nv_bfloat16* p = P.C + (size_t)row * P.N + col;
-        if (row < M) {
-            if (P.wide) {
-                if (col < P.N)
-                    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]),
-                                 "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
-                                 : "memory");
-            }
-            else
-#pragma unroll
-                for (int h = 0; h < 8; h += 4)
-                    if (col + 2 * h < P.N)
-                        *reinterpret_cast<uint4*>(p + 2 * h) = make_uint4(w[h], w[h + 1], w[h + 2], w[h + 3]);
-        }
-        __syncwarp(); // lanes part where rows or columns end
     };
     bool good = warp >= 2;
     if (warp >= 2) {
@@ -256,6 +279,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) gemm2sm_kernel(const __grid_con
             g2_tile(tile_of(n), tiles_m, tiles_n, P.group_n, mi, ni);
             const int row = mi * 256 + (int)cr * G2_HALF + q * 32 + lane, col0 = ni * G2_BN + part * G2_PART;
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * G2_BN + part * G2_PART;
+            uint32_t w[G2_PART / 2];
 #pragma unroll
             for (int c = 0; c < G2_PART; c += 16) {
                 uint32_t r[16];
@@ -268,8 +292,10 @@ __global__ void __launch_bounds__(G2_THREADS, 1) gemm2sm_kernel(const __grid_con
                     if (lane == 0)
                         mbar_arrive_cluster(tempty_leader + acc * 8);
                 }
-                emit(r, row, col0 + c);
+                convert(r, w + c / 2);
             }
+            g2_store(P, M, row, col0, w);
+            __syncwarp(); // lanes part where rows or columns end
         }
     }
     if constexpr (PAIRS > 1) {
@@ -297,6 +323,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) gemm2sm_kernel(const __grid_con
             if (warp >= 2 && good && !__any_sync(0xffffffffu, *abort_flag != 0)) {
                 int mi, ni;
                 g2_tile(whole + cluster, tiles_m, tiles_n, P.group_n, mi, ni);
+                uint32_t w[HALF_PART / 2];
 #pragma unroll
                 for (int c = 0; c < HALF_PART; c += 16) {
                     uint32_t r[16];
@@ -312,9 +339,9 @@ __global__ void __launch_bounds__(G2_THREADS, 1) gemm2sm_kernel(const __grid_con
                         for (int k = 0; k < 4; k++)
                             r[i + k] = __float_as_uint(__uint_as_float(r[i + k]) + v[k]);
                     }
-                    emit(r, mi * 256 + (int)cr * G2_HALF + q * 32 + lane,
-                         ni * G2_BN + (int)pair * (G2_BN / 2) + part * HALF_PART + c);
+                    convert(r, w + c / 2);
                 }
+                g2_store(P, M, mi * 256 + (int)cr * G2_HALF + q * 32 + lane, ni * G2_BN + (int)pair * (G2_BN / 2) + part * HALF_PART, w);
             }
         }
     }
@@ -356,12 +383,12 @@ int most_clusters() {
     return n;
 }
 
-// Expected time in us: 5.6 for launch, start and output, 0.335 per step of 64 and round of tiles, 15 % more where the rows of a
-// box begin between the 32-byte sectors; a cut tile takes half a round and 1.7 for the exchange.  4096 x 4096 with 512 rows, 32
-// tiles: 26.3 us uncut, 19.1 cut; with 1024 rows, 64 tiles for 74 pairs, nothing is cut.  Clusters of four leave some SMs out, so
-// products of many rounds keep the pairs.
+// Expected time in us: 5.6 for launch, start and output, 0.35 per step of 64 and round of tiles, a sixth more where the rows of a
+// box begin between the 32-byte sectors; clusters of two pairs start 1.2 later, a cut tile takes half a round and 1.0 for the
+// exchange (rms of 13 % over 150 products).  4096 x 4096 with 512 rows, 32 tiles: 26.3 us uncut, 19.1 cut; with 1024 rows, 64 tiles
+// for 74 pairs, nothing is cut.  Clusters of four leave some SMs out, so products of many rounds keep the pairs.
 double estimate(int M, int N, int K, int pairs) {
-    const double step = (K % 16 ? 1.15 : 1.0) * 0.335 * ((K + GEMM_BK - 1) / GEMM_BK);
+    const double step = (K % 16 ? 1.165 : 1.0) * 0.35 * ((K + GEMM_BK - 1) / GEMM_BK);
     const long long tiles = (long long)((M + 255) / 256) * ((N + G2_BN - 1) / G2_BN);
     if (pairs == 1) {
         const int most = device_sms() / 2;
@@ -369,7 +396,7 @@ double estimate(int M, int N, int K, int pairs) {
     }
     const long long clusters = std::min<long long>(most_clusters<2>(), tiles), left = tiles % (2 * clusters);
     const bool cut = left > 0 && left <= clusters;
-    return 5.8 + (tiles / (2 * clusters) + (cut ? 0.5 : left > 0 ? 1.0 : 0.0)) * step + (cut ? 1.7 : 0);
+    return 6.8 + (tiles / (2 * clusters) + (cut ? 0.5 : left > 0 ? 1.0 : 0.0)) * step + (cut ? 1.0 : 0);
 }
 
 template <int PAIRS>
@@ -410,7 +437,6 @@ void gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, i
     P.K = K;
     P.epilogue = epilogue;
     P.rows = rows_dev;
-    P.wide = N % 16 == 0 && ((uintptr_t)C & 31) == 0;
     P.timeout_ns = (unsigned long long)env_data::get().wait_timeout_ms * 1000000ull;
     const int tiles_n = (N + G2_BN - 1) / G2_BN;
     const int most = (int)std::min<size_t>(std::max<size_t>(G2_GROUP_BYTES / ((size_t)G2_BN * K * 2), 4), 32);

@@ -1,7 +1,7 @@
 // bf16 GEMM for products that leave the CTA-pair kernel's 256 x 256 tiles without enough of them: few rows of A
 // (decoding, a lightly loaded expert), or a small C.  C[M,N] = act(A[M,K] * B[N,K]^T), fp32 accumulation.
 //
-// The operands change places: 128 rows of B are the M side of tcgen05.mma and TN = 16 ... 256 rows of A its N side, so
+// The operands change places: 128 rows of B are the M side of tcgen05.mma and TN = 16 ... 128 rows of A its N side, so
 // two dozen tokens cost 32 columns, not 128 rows of which most are padding.  K is cut over the S CTAs of a cluster;
 // each reads its own part of B once and accumulates in its tensor memory, then every CTA of the cluster adds up
 // TN / S columns from the partial sums the others stored into its shared memory (fixed order, fp32), applies the
@@ -57,8 +57,12 @@ struct gs_layout {
     static constexpr int A_STAGE = TN * GEMM_BK * 2;
     static constexpr int STAGE = A_STAGE + B_STAGE;
     static constexpr int TMEM_COLS = TN < 32 ? 32 : TN;
-    static constexpr int BLOCKS = TN == 256 || STAGES > 4 ? 1 : 2; // per SM
+    static constexpr int BLOCKS = STAGES > 4 ? 1 : 2; // per SM
     static constexpr int UNITS = TN / 4; // of four columns: what the CTAs of a cluster share out
+    // of four epilogue warps, a share of the columns each: 200 x 1752 x 11840 took 22.8 us with one of them, 313 x 1720 x 864 7.3,
+    // now 20.8 and 6.8
+    static constexpr int GROUPS = TN >= 64 ? 2 : 1;
+    static constexpr int THREADS = 64 + 128 * GROUPS;
     static constexpr int TOTAL = 1024 + STAGES * STAGE + 128;
     // the ring also holds the partial sums afterwards: a source's units for one CTA, rounded up, times up to 8 sources
     static_assert((UNITS + 7) * GS_BN * 16 <= STAGES * STAGE, "the partial sums must fit the ring");
@@ -96,11 +100,14 @@ __device__ __forceinline__ void gs_store(const gemm_small_params& P, int M, int 
         *reinterpret_cast<__nv_bfloat162*>(dst + P.N) = odd ? __floats2bfloat162_rn(g1, k1) : __floats2bfloat162_rn(k1, g1);
 }
 
-// adds the S partial sums of this CTA's units of four columns in order and stores the result; one thread per row of B
-__device__ __forceinline__ void gs_reduce(const gemm_small_params& P, int S, int M, uint32_t part, int pitch, int units, int tok,
-                                          int n0, int row) {
+// adds the S partial sums of every GROUPS-th of this CTA's units of four columns, from `first` on, in order and stores the result;
+// one thread of a group per row of B
+template <int GROUPS>
+__device__ __forceinline__ void gs_reduce(const gemm_small_params& P, int S, int M, uint32_t part, int pitch, int first, int units,
+                                          int tok, int n0, int row) {
     const uint32_t step = (uint32_t)pitch * GS_BN * 16;
-    for (int u = 0; u < units && tok + 4 * u < M; u++, part += GS_BN * 16) {
+    part += first * GS_BN * 16;
+    for (int u = first; u < units && tok + 4 * u < M; u += GROUPS, part += GROUPS * GS_BN * 16) {
         float v[8][4];
 #pragma unroll
         for (int s = 0; s < 8; s++)
@@ -119,7 +126,7 @@ __device__ __forceinline__ void gs_reduce(const gemm_small_params& P, int S, int
 }
 
 template <int TN, int STAGES>
-__global__ void __launch_bounds__(GEMM_THREADS, gs_layout<TN, STAGES>::BLOCKS)
+__global__ void __launch_bounds__(gs_layout<TN, STAGES>::THREADS, gs_layout<TN, STAGES>::BLOCKS)
     gemm_small_kernel(const __grid_constant__ gemm_small_params P) {
     using namespace sm100;
     typedef gs_layout<TN, STAGES> L;
@@ -235,15 +242,17 @@ __global__ void __launch_bounds__(GEMM_THREADS, gs_layout<TN, STAGES>::BLOCKS)
     auto first_unit = [&](uint32_t s) { return (uint32_t)L::UNITS * s * P.inv_splits >> 16; };
     const int pitch = P.pitch;
     const int q = warp & 3; // quarter of the tensor memory's lanes this warp may read
-    const int row = q * 32 + lane;
+    const int grp = (warp - 2) >> 2, row = q * 32 + lane;
+    constexpr int COLS = TN / L::GROUPS; // of this warp
     if (warp >= 2 && good) {
         // Partial sums travel as [source][unit][row] packs of four floats: a warp stores 512 contiguous bytes,
         // and the reader's lanes take consecutive rows.  An undivided K needs no exchange.
         const uint32_t base = smem_u32(smem) + (uint32_t)(split * pitch * GS_BN + row) * 16;
-        uint32_t owner = 0, end = first_unit(1), dst = S > 1 ? map_to_cta(base, 0) : 0; // of the next unit
-        constexpr int CH = TN < 32 ? 16 : 32;
+        uint32_t unit = grp * COLS / 4, owner = ((unit + 1) * S - 1) / L::UNITS, end = first_unit(owner + 1);
+        uint32_t dst = S > 1 ? map_to_cta(base + (unit - first_unit(owner)) * GS_BN * 16, owner) : 0;
+        constexpr int CH = COLS < 32 ? 16 : 32;
 #pragma unroll 1
-        for (int c0 = 0; c0 < TN; c0 += CH) {
+        for (int c0 = grp * COLS; c0 < (grp + 1) * COLS; c0 += CH) {
             uint32_t r[CH];
             if constexpr (CH == 16)
                 tmem_ld_32x16(tmem + ((uint32_t)(q * 32) << 16) + c0, r);
@@ -258,13 +267,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, gs_layout<TN, STAGES>::BLOCKS)
                     gs_store(P, M, tok0 + c0 + i, n0, row, v);
                 }
                 else {
-                    if ((uint32_t)(c0 + i) / 4 == end) {
+                    if (unit == end) {
                         owner++;
                         end = first_unit(owner + 1);
                         dst = map_to_cta(base, owner);
                     }
                     st_cluster_v4(dst, r[i], r[i + 1], r[i + 2], r[i + 3]);
                     dst += GS_BN * 16;
+                    unit++;
                 }
             }
         }
@@ -277,7 +287,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, gs_layout<TN, STAGES>::BLOCKS)
     if (S > 1 && warp >= 2 && !*abort_flag) {
         const uint32_t part = smem_u32(smem) + row * 16;
         const int u0 = first_unit(split), units = first_unit(split + 1) - u0, tok = tok0 + 4 * u0;
-        gs_reduce(P, S, M, part, pitch, units, tok, n0, row);
+        gs_reduce<L::GROUPS>(P, S, M, part, pitch, grp, units, tok, n0, row);
     }
     if (warp == 2) { // all reads of the accumulator lie in front of the last barrier
         tc_fence_after_sync();
@@ -299,7 +309,7 @@ int resident_clusters(int splits) {
         allow_smem<gemm_small_kernel<128, GS_STAGES_ALONE>>(L::TOTAL);
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(splits);
-        cfg.blockDim = dim3(GEMM_THREADS);
+        cfg.blockDim = dim3(L::THREADS);
         cfg.dynamicSmemBytes = L::TOTAL;
         cudaLaunchAttribute attr{};
         attr.id = cudaLaunchAttributeClusterDimension;
@@ -321,7 +331,7 @@ void launch_small(const gemm_small_params& P, int tiles_n, int tiles_m, cudaStre
     allow_smem<gemm_small_kernel<TN, STAGES>>(L::TOTAL);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(tiles_n * P.splits, tiles_m);
-    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.blockDim = dim3(L::THREADS);
     cfg.dynamicSmemBytes = L::TOTAL;
     cfg.stream = st;
     cudaLaunchAttribute attr[2]{};
@@ -337,18 +347,19 @@ void launch_small(const gemm_small_params& P, int tiles_n, int tiles_m, cudaStre
 
 // What a product costs with tiles of TN rows of A, in us: `fixed` from launch to output, `exchange` if K is cut, a step of 64
 // of K with one CTA on an SM or with two, another round of resident CTAs, the factor on the steps where K is no multiple
-// of 16, so that the rows of a box begin between the 32-byte sectors, and a round of CTAs that find no rows.  Fitted to 8200 times
-// of 420 products of 1 to 700 rows, 520 to 14000 columns and K of 520 to 14300, then moved a little to where they choose best: the
-// chosen plan takes 2 to 3 % longer than the best one, 3 to 5 % where the device alone knows the rows; the rule this replaces
-// (1, 2, 4 or 8 parts, estimated cycles) 9 %.
+// of 16, so that the rows of a box begin between the 32-byte sectors, and a round of CTAs that find no rows.  Fitted to the times
+// of 300 products of 1 to 3000 rows, 520 to 14000 columns and K of 520 to 14300, then moved a little to where they choose best: the
+// chosen plan takes 2.3 % longer than the best one, 7 % where the device alone knows the rows; the rule this replaces (1, 2, 4 or 8
+// parts, estimated cycles) 9 %.
 struct small_cost {
     int tn;
     double fixed, exchange, alone, two, round, ragged, idle;
 };
 constexpr small_cost SMALL_COSTS[] = {
-    { 16, 3.23, 0.80, 0.274, 0.396, 2.0, 1.06, 0.6 },  { 32, 3.75, 0.72, 0.286, 0.430, 3.3, 1.12, 0.7 },
-    { 64, 4.68, 0.71, 0.275, 0.432, 4.1, 1.18, 0.6 },  { 128, 6.75, 0.72, 0.303, 0.609, 7.0, 1.14, 0.6 },
-    { 256, 10.56, 0.3, 0.385, 0.385, 10.5, 1.40, 0.8 },
+    { 16, 2.76, 0.87, 0.275, 0.396, 1.1, 1.04, 0.6 },
+    { 32, 3.64, 0.59, 0.274, 0.408, 2.8, 1.15, 0.8 },
+    { 64, 4.00, 0.82, 0.233, 0.417, 3.3, 1.22, 0.9 },
+    { 128, 4.98, 1.31, 0.279, 0.583, 5.7, 1.30, 0.8 },
 };
 constexpr double SMALL_BYTES_PER_US = 6.3e6; // of B, from memory
 constexpr double SMALL_L2_BYTES = 64e6; // of B that a second row of tiles still finds in the L2
@@ -369,7 +380,7 @@ void plan_small(int M, int rows, int N, int K, gemm_choice& best) {
         const double stream = (bytes > SMALL_L2_BYTES ? bytes * down : bytes) / SMALL_BYTES_PER_US;
         for (int s = 1; s <= std::min(8, c.tn / 4) && (s == 1 || kb / s >= 2); s++) {
             // clusters that run at the same time, with one CTA per SM and with the most
-            const long long one = resident[s], most = c.tn == 256 ? one : 2 * one;
+            const long long one = resident[s], most = 2 * one;
             if (s > 2 && launched > most) // a second round of wide clusters waits for whole groups of SMs
                 break;
             const long long rounds = (tiles + most - 1) / most, idle = (launched + most - 1) / most - rounds;
@@ -438,13 +449,12 @@ void gemm_bf16_small(const void* A, const void* B, void* C, int M, int N, int K,
         case 16: launch_small<16, 4>(P, tiles_n, tiles_m, st); break;
         case 32: launch_small<32, 4>(P, tiles_n, tiles_m, st); break;
         case 64: launch_small<64, 4>(P, tiles_n, tiles_m, st); break;
-        case 128:
+        default:
             if ((long long)tiles_n * tiles_m <= resident_clusters(plan.splits))
                 launch_small<128, GS_STAGES_ALONE>(P, tiles_n, tiles_m, st);
             else
                 launch_small<128, 3>(P, tiles_n, tiles_m, st);
             break;
-        default: launch_small<256, 4>(P, tiles_n, tiles_m, st); break;
     }
 }
 
