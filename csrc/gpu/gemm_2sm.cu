@@ -24,6 +24,7 @@
 #include "gpu/fused_gemm.cuh"
 #include "gpu/fused_gemm.hpp"
 #include "gpu/launch_util.cuh"
+#include "gpu/row_store.cuh"
 
 namespace cclx {
 namespace gpu {
@@ -47,6 +48,7 @@ struct gemm2_params {
     uint32_t* err;
     int M, N, K, epilogue;
     int group_n; // tile columns per raster group
+    int trade; // lanes trade sectors before they store
     unsigned long long timeout_ns;
     const int* rows; // optional device word: only the first min(M, *rows) rows of A are multiplied
 };
@@ -72,19 +74,15 @@ __device__ __forceinline__ void g2_tile(int t, int tiles_m, int tiles_n, int gro
     ni = grp * group + in % width;
 }
 
-__device__ __forceinline__ void st_8(__nv_bfloat16* p, const uint32_t* w) { // 8 columns
-    *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
-}
-__device__ __forceinline__ void st_16(__nv_bfloat16* p, const uint32_t* w) { // 16 columns, a whole sector
-    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
-                 "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
-                 : "memory");
-}
-
-// 2 W columns of a row of C from column `col` on, a multiple of 16, in whole 32-byte sectors.  Where N is an odd number of eights every
-// other row begins in the middle of one: then the first and the last half sector go alone.
+// 2 W columns of rows row0 + lane of C from column `col` on, a multiple of 16, in whole 32-byte sectors.  Where N is an odd number of
+// eights every other row begins in the middle of one: then each lane writes its own row, the first and the last half sector alone.
 template <int W>
-__device__ __forceinline__ void g2_store(const gemm2_params& P, int M, int row, int col, const uint32_t (&w)[W]) {
+__device__ __forceinline__ void g2_store(const gemm2_params& P, int M, int row0, int col, int lane, uint32_t (&w)[W]) {
+    if (P.trade) {
+        store_rows(P.C, M, P.N, row0, col, lane, w);
+        return;
+    }
+    const int row = row0 + lane;
     if (row >= M)
         return;
     __nv_bfloat16* p = P.C + (size_t)row * P.N + col;
@@ -277,7 +275,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) gemm2sm_kernel(const __grid_con
                 break;
             int mi, ni;
             g2_tile(tile_of(n), tiles_m, tiles_n, P.group_n, mi, ni);
-            const int row = mi * 256 + (int)cr * G2_HALF + q * 32 + lane, col0 = ni * G2_BN + part * G2_PART;
+            const int row0 = mi * 256 + (int)cr * G2_HALF + q * 32, col0 = ni * G2_BN + part * G2_PART;
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * G2_BN + part * G2_PART;
             uint32_t w[G2_PART / 2];
 #pragma unroll
@@ -294,7 +292,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) gemm2sm_kernel(const __grid_con
                 }
                 convert(r, w + c / 2);
             }
-            g2_store(P, M, row, col0, w);
+            g2_store(P, M, row0, col0, lane, w);
             __syncwarp(); // lanes part where rows or columns end
         }
     }
@@ -341,7 +339,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) gemm2sm_kernel(const __grid_con
                     }
                     convert(r, w + c / 2);
                 }
-                g2_store(P, M, mi * 256 + (int)cr * G2_HALF + q * 32 + lane, ni * G2_BN + (int)pair * (G2_BN / 2) + part * HALF_PART, w);
+                g2_store(P, M, mi * 256 + (int)cr * G2_HALF + q * 32, ni * G2_BN + (int)pair * (G2_BN / 2) + part * HALF_PART, lane, w);
             }
         }
     }
@@ -437,6 +435,10 @@ void gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, i
     P.K = K;
     P.epilogue = epilogue;
     P.rows = rows_dev;
+    // Rows that begin at a sector, but not at a 128-byte line: a lane's 64 columns lie in two lines then.  5728 x 5616 x 6024 387 us,
+    // 379 with the trade, 2966 x 12240 x 904 77.8 and 76.1.  Rows of whole lines are better off without: 8192 x 4096 x 4096 201 and
+    // 204 with it, under the power cap.
+    P.trade = N % 16 == 0 && N % 64 != 0 && ((uintptr_t)C & 31) == 0;
     P.timeout_ns = (unsigned long long)env_data::get().wait_timeout_ms * 1000000ull;
     const int tiles_n = (N + G2_BN - 1) / G2_BN;
     const int most = (int)std::min<size_t>(std::max<size_t>(G2_GROUP_BYTES / ((size_t)G2_BN * K * 2), 4), 32);
