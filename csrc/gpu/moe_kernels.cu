@@ -434,6 +434,22 @@ struct piece_walk {
 };
 
 constexpr int MOE_THREADS = 512;
+
+// A rank's tables in shared memory, read at once by all threads: followed pointer by pointer, their lines come one after the other through
+// the caches in front of every barrier and address. Dispatch and combine of 8 emulated ranks together, K = 2: 62 tokens x 1112
+// 83.8 -> 82.4 us, 1024 x 4096 127.3 -> 125.8; 2 ranks, 2048 x 4096 69.3 -> 68.4.
+__device__ __forceinline__ void fetch_tables(const comm_dev* tab, const moe_args& a, comm_dev& c, moe_rank_args& ra) {
+    const int er = a.emu ? (int)blockIdx.y : 0;
+    static_assert(sizeof(comm_dev) % 8 == 0 && sizeof(moe_rank_args) % 8 == 0 && sizeof(comm_dev) / 8 <= MOE_THREADS / 2, "copied by words");
+    const int i = threadIdx.x, j = threadIdx.x - MOE_THREADS / 2;
+    if (i < (int)(sizeof(comm_dev) / 8))
+        reinterpret_cast<unsigned long long*>(&c)[i] = reinterpret_cast<const unsigned long long*>(tab + er)[i];
+    if (a.emu && j >= 0 && j < (int)(sizeof(moe_rank_args) / 8))
+        reinterpret_cast<unsigned long long*>(&ra)[j] = reinterpret_cast<const unsigned long long*>(a.emu_tab + er)[j];
+    if (!a.emu && j == 0)
+        ra = a.r0;
+    __syncthreads();
+}
 constexpr int MOE_SEGMENTS = 256;
 
 // Bound by memory (every row read once, written topk times).  The rows stand grouped by expert, but are not sent in that order:
@@ -442,9 +458,9 @@ constexpr int MOE_SEGMENTS = 256;
 // Eight ranks with 1024 tokens of 4096 each, top-2, on one GPU: 48.2 us in order of experts with one piece per warp in flight,
 // 39.6 now; 16 tokens of 512, the barriers alone, 15.5 and 10.0.
 __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(const comm_dev* tab, moe_args a) {
-    const int er = a.emu ? (int)blockIdx.y : 0;
-    const comm_dev& c = tab[er];
-    const moe_rank_args& ra = a.emu ? a.emu_tab[er] : a.r0;
+    __shared__ comm_dev c;
+    __shared__ moe_rank_args ra;
+    fetch_tables(tab, a, c, ra);
     block_sync s;
     sync_begin(c, s);
     const int W = c.world;
@@ -583,9 +599,9 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(const comm_de
 // for all slots, now 43.4); 0, any number of slots, two packs of two slots.
 template <int TOPK>
 __global__ void __launch_bounds__(MOE_THREADS) moe_combine_kernel(const comm_dev* tab, moe_args a) {
-    const int er = a.emu ? (int)blockIdx.y : 0;
-    const comm_dev& c = tab[er];
-    const moe_rank_args& ra = a.emu ? a.emu_tab[er] : a.r0;
+    __shared__ comm_dev c;
+    __shared__ moe_rank_args ra;
+    fetch_tables(tab, a, c, ra);
     block_sync s;
     sync_begin(c, s);
     const int W = c.world;
