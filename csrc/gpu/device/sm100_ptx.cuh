@@ -222,9 +222,15 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, uint32_t a,
                  : "memory");
 }
 // all threads of all CTAs of the cluster; not time-bounded, so every code path must reach it
-__device__ __forceinline__ void cluster_sync_all() {
+__device__ __forceinline__ void cluster_arrive() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    cluster_arrive();
+    cluster_wait();
 }
 // one arrival on a barrier given by its shared::cluster address (may be the peer's)
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {

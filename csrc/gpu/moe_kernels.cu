@@ -218,6 +218,8 @@ __global__ void __launch_bounds__(1024)
     for (int e = threadIdx.x; e < n_experts; e += blockDim.x)
         count[e] = 0;
     __syncthreads();
+    if constexpr (C > 1)
+        sm100::cluster_arrive(); // this block runs: the others may write its shared memory
     gpu::pdl_wait(); // launched while the kernel in front still runs
     for (int t = threadIdx.x; t < n; t += blockDim.x)
         route_token<E>(logits + (size_t)(t0 + t) * n_experts, n_experts, topk, idx + (size_t)(t0 + t) * topk,
@@ -227,6 +229,7 @@ __global__ void __launch_bounds__(1024)
                        });
     __syncthreads();
     if constexpr (C > 1) {
+        sm100::cluster_wait();
         for (int i = threadIdx.x; i < C * n_experts; i += blockDim.x) {
             const int to = i / n_experts, e = i - to * n_experts;
             sm100::st_cluster_u32(sm100::map_to_cta(sm100::smem_u32(&all[me][e]), to), count[e]);
