@@ -324,7 +324,7 @@ CCLX_API int cclx_gemm_bf16_2sm(const void* A, const void* B, void* C, int M, in
                                 void* err_words, void* stream) {
     return capi::guard(
         [&] {
-            const int pairs = clusters == 0 && M > 0 && N > 0 && K > 0 ? choose_gemm(M, N, K, false).pairs : 1;
+            const int pairs = clusters == 0 ? choose_gemm(M, N, K, false).pairs : 1;
             gemm_bf16_2sm(A, B, C, M, N, K, epilogue, clusters, (uint32_t*)err_words, (cudaStream_t)stream, nullptr, pairs);
         });
 }

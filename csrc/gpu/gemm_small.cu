@@ -405,6 +405,7 @@ void plan_small(int M, int rows, int N, int K, gemm_choice& best) {
 // that only the device knows lies somewhere below M: half of it is taken.  The answer depends on the sizes and the kind of device
 // alone and takes 2 us to work out, half a small product: each thread keeps its latest ones.
 gemm_choice choose_gemm(int M, int N, int K, bool rows_on_device) {
+    CCL_THROW_IF_NOT(M > 0 && N > 0 && K > 0 && N % 8 == 0 && K % 8 == 0, "unsupported GEMM shape ", M, "x", N, "x", K);
     struct entry {
         int dev = -1, M, N, K;
         bool rows;

@@ -1,0 +1,20 @@
+"""Sizes that the product's C entries refuse, found before anything is asked of a GPU."""
+import ctypes as C
+
+import pytest
+
+from oneccl_b200 import _lib
+
+_ENTRIES = {  # arguments behind the sizes and the epilogue
+    "cclx_gemm_bf16": (C.c_int(0), None, None),
+    "cclx_gemm_bf16_2sm": (C.c_int(0), None, None),
+    "cclx_gemm_bf16_rows": (None, None, None),
+}
+
+
+@pytest.mark.parametrize("M,N,K", [(0, 64, 64), (64, 0, 64), (64, 64, 0), (0, 0, 0), (-1, 64, 64), (3, 12, 64), (3, 64, 12)])
+@pytest.mark.parametrize("entry", sorted(_ENTRIES))
+def test_empty_and_odd_products_are_refused(entry, M, N, K):
+    lib = _lib.load()
+    assert getattr(lib, entry)(None, None, None, M, N, K, 0, *_ENTRIES[entry]) != 0
+    assert b"unsupported GEMM shape" in lib.cclx_last_error()
