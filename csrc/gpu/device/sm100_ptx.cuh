@@ -69,6 +69,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
 }
 
+// The same for whole warps that go on with warp-wide instructions: a lane that gives up takes the others with it, so that all
+// succeed or none.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort, unsigned long long limit_ns) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort, limit_ns));
+}
+// whether any lane of a whole warp sees the flag that another role sets when it fails
+__device__ __forceinline__ bool warp_sees(volatile int* flag) {
+    return __any_sync(0xffffffffu, *flag != 0);
+}
+
 // ---- proxies / fences ------------------------------------------------------------
 __device__ __forceinline__ void fence_proxy_async() {
     asm volatile("fence.proxy.async;" ::: "memory");

@@ -343,11 +343,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             uint8_t* stage = sEpi + (warp - 2) * 32 * GEMM_EPI_ROW_BYTES;
             uint32_t tc = 0;
             const int M_per = P.M / W;
-            for (int t = g; t < total_tiles && !*abort_flag; t += G, tc++) {
+            for (int t = g; t < total_tiles && !warp_sees(abort_flag); t += G, tc++) {
                 const int mi = (t / tiles_n + m_rot) % tiles_m;
                 const int ni = t % tiles_n;
                 const uint32_t acc = tc & 1, aph = (tc >> 1) & 1;
-                if (!mbar_wait(&tfull[acc], aph, abort_flag, limit)) {
+                if (!mbar_wait_warp(&tfull[acc], aph, abort_flag, limit)) {
                     if (lane == 0)
                         gemm_fail(fr, abort_flag, GE_MBAR_TIMEOUT, 5);
                     break;

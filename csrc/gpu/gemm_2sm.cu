@@ -259,17 +259,14 @@ __global__ void __launch_bounds__(G2_THREADS, 1) gemm2sm_kernel(const __grid_con
     bool good = warp >= 2;
     if (warp >= 2) {
         const uint32_t tempty_leader = smem_u32(&tempty[0]) & PEER_BIT_MASK;
-        for (int n = 0; n < items && !*abort_flag; n++) {
+        for (int n = 0; n < items && !warp_sees(abort_flag); n++) {
             const uint32_t acc = n & 1, aph = (n >> 1) & 1;
-            if (!mbar_wait(&tfull[acc], aph, abort_flag, limit)) {
+            good = mbar_wait_warp(&tfull[acc], aph, abort_flag, limit);
+            if (!good) {
                 if (lane == 0)
                     g2_fail(P, abort_flag, GE_MBAR_TIMEOUT, 5);
-                good = false;
-            }
-            // a lane may see the flag of another role's failure and leave alone: the warp goes on together or not at all
-            good = __all_sync(0xffffffffu, good);
-            if (!good)
                 break;
+            }
             tc_fence_after_sync();
             if (n == mine) // the cut tile
                 break;
@@ -295,6 +292,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) gemm2sm_kernel(const __grid_con
             g2_store(P, M, row0, col0, lane, w);
             __syncwarp(); // lanes part where rows or columns end
         }
+        __syncwarp();
     }
     if constexpr (PAIRS > 1) {
         if (cut) {
@@ -318,7 +316,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) gemm2sm_kernel(const __grid_con
                 }
             }
             cluster_sync_all();
-            if (warp >= 2 && good && !__any_sync(0xffffffffu, *abort_flag != 0)) {
+            if (warp >= 2 && good && !warp_sees(abort_flag)) {
                 int mi, ni;
                 g2_tile(whole + cluster, tiles_m, tiles_n, P.group_n, mi, ni);
                 uint32_t w[HALF_PART / 2];

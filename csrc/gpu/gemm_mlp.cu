@@ -281,7 +281,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GM_THREADS, 1) mlp_k
                         in[c / 2 + i + 3] = b.w;
                     }
             }
-            if (!mbar_wait(&tfull[acc], aph, abort_flag, limit)) {
+            if (!mbar_wait_warp(&tfull[acc], aph, abort_flag, limit)) {
                 *abort_flag = 1;
                 ok = false;
             }
@@ -312,7 +312,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GM_THREADS, 1) mlp_k
                     store(P.out, row, col0 + c, o);
                     const float total = warp_totals(v, lane);
                     if ((lane & 1) == 0)
-                        sums[((tc & 1) * 4 + q) * GM_BN + c0 * 64 + c + lane / 2] = total;
+                        sums[((tc & 1) * 4 + q) * GM_BN + c0 * 64 + c + lane / 2] = ok ? total : __uint_as_float(0x7fc00000u);
                 }
                 else {
 #pragma unroll

@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(gs_layout<TN, STAGES>::THREADS, gs_layout<TN, 
     }
     bool good = true;
     if (warp >= 2) {
-        good = mbar_wait(tfull, 0, abort_flag, limit);
+        good = mbar_wait_warp(tfull, 0, abort_flag, limit);
         if (!good && lane == 0)
             gs_fail(P, abort_flag, 5);
         tc_fence_after_sync();
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(gs_layout<TN, STAGES>::THREADS, gs_layout<TN, 
         cluster_sync_all();
     else
         __syncthreads();
-    if (S > 1 && warp >= 2 && !*abort_flag) {
+    if (S > 1 && warp >= 2 && !warp_sees(abort_flag)) {
         const uint32_t part = smem_u32(smem) + row * 16;
         const int u0 = first_unit(split), units = first_unit(split + 1) - u0, tok = tok0 + 4 * u0;
         gs_reduce<L::GROUPS>(P, S, M, part, pitch, grp, units, tok, n0, row);

@@ -32,3 +32,11 @@ def test_other_blocks_shared_memory_is_written_between_cluster_barriers(kernel):
 def test_the_kernels_with_remote_stores_are_found():
     names = {k[1] for k in _kernels() if "st_cluster_" in k[2]}
     assert {"route_one_block_kernel", "gemm_small_kernel", "gemm2sm_kernel"} <= names
+
+
+@pytest.mark.parametrize("kernel", [k for k in _kernels() if "tmem_ld_32x" in k[2]], ids=lambda k: f"{k[0]}:{k[1]}")
+def test_warps_that_read_accumulators_give_up_together(kernel):
+    """Another role's failure is seen lane by lane: a warp that goes on with instructions of whole warps asks for all of its lanes."""
+    epilogue = kernel[2][kernel[2].index("const int q = warp & 3"):]
+    assert "!*abort_flag" not in epilogue and not re.search(r"\bmbar_wait\(", epilogue)
+    assert "mbar_wait(&tfull" not in kernel[2] and "mbar_wait(tfull" not in kernel[2]
