@@ -324,7 +324,7 @@ CCLX_API int cclx_gemm_bf16_2sm(const void* A, const void* B, void* C, int M, in
                                 void* err_words, void* stream) {
     return capi::guard(
         [&] {
-            const int pairs = clusters == 0 ? choose_gemm(M, N, K, false).pairs : 1;
+            const int pairs = clusters == 0 ? choose_gemm(C, M, N, K, false).pairs : 1;
             gemm_bf16_2sm(A, B, C, M, N, K, epilogue, clusters, (uint32_t*)err_words, (cudaStream_t)stream, nullptr, pairs);
         });
 }
@@ -334,7 +334,7 @@ CCLX_API int cclx_gemm_bf16_2sm(const void* A, const void* B, void* C, int M, in
 CCLX_API int cclx_gemm_bf16_rows(const void* A, const void* B, void* C, int M, int N, int K, int epilogue,
                                  const void* rows_dev, void* err_words, void* stream) {
     return capi::guard([&] {
-        const gemm_choice choice = choose_gemm(M, N, K, true);
+        const gemm_choice choice = choose_gemm(C, M, N, K, true);
         if (choice.small)
             gemm_bf16_small(A, B, C, M, N, K, epilogue, (uint32_t*)err_words, (cudaStream_t)stream, (const int*)rows_dev, choice);
         else

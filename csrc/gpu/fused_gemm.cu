@@ -95,7 +95,7 @@ void gemm_bf16_plain(const void* A, const void* B, void* C, int M, int N, int K,
     CCL_THROW_IF_NOT(M > 0 && N > 0 && K > 0 && N % 8 == 0 && K % 8 == 0, "unsupported GEMM shape ", M, "x", N, "x", K);
     // Without a grid asked for: the K-splitting kernel where it is expected to be faster (few rows, small C), else CTA
     // pairs (two-SM MMA).  A negative `ctas` forces the single-CTA kernel, CCL_CUDA_GEMM_2SM=0 turns the pairs off.
-    const gemm_choice choice = ctas == 0 ? choose_gemm(M, N, K, false) : gemm_choice{};
+    const gemm_choice choice = ctas == 0 ? choose_gemm(C, M, N, K, false) : gemm_choice{};
     if (choice.small) {
         gemm_bf16_small(A, B, C, M, N, K, epilogue, err, st, nullptr, choice);
         return;
@@ -104,6 +104,7 @@ void gemm_bf16_plain(const void* A, const void* B, void* C, int M, int N, int K,
         gemm_bf16_2sm(A, B, C, M, N, K, epilogue, ctas / 2, err, st, nullptr, choice.pairs);
         return;
     }
+    CCL_THROW_IF_NOT(((uintptr_t)C & 15) == 0, "GEMM output must be 16-byte aligned");
     if (ctas < 0)
         ctas = -ctas - 1; // -(n + 1) asks for the single-CTA kernel on n CTAs (0 = all SMs)
     const int bn = pick_bn(N);

@@ -22,7 +22,7 @@ struct gemm_choice {
     int pairs; // of the first: per cluster
     double us; // estimate of the second
 };
-gemm_choice choose_gemm(int M, int N, int K, bool rows_on_device);
+gemm_choice choose_gemm(const void* C, int M, int N, int K, bool rows_on_device);
 
 // the same product on CTA pairs (tcgen05.mma.cta_group::2, 256 x 256 tiles); `clusters` 0: as many clusters as the device takes, of
 // `pairs` pairs each

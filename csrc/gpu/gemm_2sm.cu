@@ -420,6 +420,7 @@ CUtensorMap make_bf16_kmajor_map(const void* base, uint64_t rows, uint64_t cols,
 void gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int clusters,
                    uint32_t* err, cudaStream_t st, const int* rows_dev, int pairs) {
     CCL_THROW_IF_NOT(M > 0 && N > 0 && K > 0 && N % 8 == 0 && K % 8 == 0, "unsupported GEMM shape ", M, "x", N, "x", K);
+    CCL_THROW_IF_NOT(((uintptr_t)C & 15) == 0, "GEMM output must be 16-byte aligned");
     allow_smem<gemm2sm_kernel<1>>(G2_SMEM);
     allow_smem<gemm2sm_kernel<2>>(G2_SMEM);
     gemm2_params P;

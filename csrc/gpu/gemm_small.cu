@@ -404,7 +404,7 @@ void plan_small(int M, int rows, int N, int K, gemm_choice& best) {
 // 18.5 with pairs) and 512 (22.6 and 19.1), at 1024 x 4096 between 1024 rows (16.2 and 17.8) and 2048 (21.9 and 18.8).  A row count
 // that only the device knows lies somewhere below M: half of it is taken.  The answer depends on the sizes and the kind of device
 // alone and takes 2 us to work out, half a small product: each thread keeps its latest ones.
-gemm_choice choose_gemm(int M, int N, int K, bool rows_on_device) {
+static gemm_choice choose_by_sizes(int M, int N, int K, bool rows_on_device) {
     CCL_THROW_IF_NOT(M > 0 && N > 0 && K > 0 && N % 8 == 0 && K % 8 == 0, "unsupported GEMM shape ", M, "x", N, "x", K);
     struct entry {
         int dev = -1, M, N, K;
@@ -424,6 +424,14 @@ gemm_choice choose_gemm(int M, int N, int K, bool rows_on_device) {
     c.pairs = two < one ? 2 : 1;
     c.small = rows <= 128 || c.us < std::min(one, two);
     e = { dev, M, N, K, rows_on_device, c };
+    return c;
+}
+
+// This kernel stores pairs of columns, the others packs of eight: an output between 16-byte boundaries is its own.
+gemm_choice choose_gemm(const void* C, int M, int N, int K, bool rows_on_device) {
+    gemm_choice c = choose_by_sizes(M, N, K, rows_on_device);
+    CCL_THROW_IF_NOT(((uintptr_t)C & 3) == 0, "GEMM output must be 4-byte aligned");
+    c.small |= ((uintptr_t)C & 15) != 0;
     return c;
 }
 

@@ -61,6 +61,35 @@ def test_gemm_plans(shape, rows):
             assert ((out[:n].double() - ref[:n]).abs() <= bound[:n]).all(), (n, kernel)
             assert (out[n:] == 7.0).all(), (n, kernel)
 
+
+@pytest.mark.parametrize("shape", [(40, 520, 264), (300, 1040, 520), (512, 4096, 1032), (700, 104, 72), (1024, 8192, 256)])
+def test_gemm_output_between_pack_boundaries(shape):
+    """An output that starts at a pair of columns only: right with the library's choice, refused where packs are stored."""
+    from oneccl_b200._lib import CclError
+    from oneccl_b200.ops.gemm import gemm_bf16
+
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(4)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    ref, sums = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+    for offset in (2, 6):
+        room = torch.full((M * N + 16,), 7.0, dtype=torch.bfloat16, device="cuda")
+        out = room[offset:offset + M * N].view(M, N)
+        for rows in (None, torch.tensor([M - 1], dtype=torch.int32, device="cuda")):
+            room.fill_(7.0)
+            n = M if rows is None else M - 1
+            gemm_bf16(a, w, out=out, check=True, rows=rows)
+            # one rounding of the result to bf16, K roundings of the fp32 sum
+            assert ((out[:n].double() - ref[:n]).abs() <= ref[:n].abs() * 2.0**-8 + K * 2.0**-23 * sums[:n]).all()
+            assert (out[n:] == 7.0).all() and (room[:offset] == 7.0).all() and (room[offset + M * N:] == 7.0).all()
+        for kernel in ("1sm", "2sm"):
+            with pytest.raises(CclError, match="16-byte aligned"):
+                gemm_bf16(a, w, out=out, kernel=kernel)
+    with pytest.raises(CclError, match="4-byte aligned"):
+        gemm_bf16(a, w, out=room[1:1 + M * N].view(M, N))
+
+
 @pytest.mark.parametrize("kernel", ["1sm", "2sm"])
 def test_gemm_silu_and_persistence(kernel):
     """More tiles than CTAs (each CTA loops, both TMEM accumulators are reused) + SiLU epilogue."""
