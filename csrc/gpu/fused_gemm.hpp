@@ -20,7 +20,6 @@ struct gemm_choice {
     bool small; // the second
     int tn, splits; // of the second: rows of A per tile, parts of K
     int pairs; // of the first: per cluster
-    double us; // estimate of the second
 };
 gemm_choice choose_gemm(const void* C, int M, int N, int K, bool rows_on_device);
 

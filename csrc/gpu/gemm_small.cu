@@ -16,6 +16,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <iterator>
 
 #include "core/env.hpp"
 #include "core/log.hpp"
@@ -364,46 +365,34 @@ constexpr small_cost SMALL_COSTS[] = {
 constexpr double SMALL_BYTES_PER_US = 6.3e6; // of B, from memory
 constexpr double SMALL_L2_BYTES = 64e6; // of B that a second row of tiles still finds in the L2
 
-// The cheapest tiles and split of K for `rows` expected rows of the M that the grid covers.
-void plan_small(int M, int rows, int N, int K, gemm_choice& best) {
-    const int kb = (K + GEMM_BK - 1) / GEMM_BK, across = (N + GS_BN - 1) / GS_BN;
-    int resident[9];
-    for (int s = 1; s <= 8; s++)
-        resident[s] = resident_clusters(s);
-    best.us = 1e30;
-    for (const small_cost& c : SMALL_COSTS) {
-        if (c.tn >= 4 * std::max(rows, 16)) // mostly padding
-            break;
-        const int down = (rows + c.tn - 1) / c.tn;
-        const long long tiles = (long long)across * down, launched = (long long)across * ((M + c.tn - 1) / c.tn);
-        const double bytes = (double)N * K * 2;
-        const double stream = (bytes > SMALL_L2_BYTES ? bytes * down : bytes) / SMALL_BYTES_PER_US;
-        for (int s = 1; s <= std::min(8, c.tn / 4) && (s == 1 || kb / s >= 2); s++) {
-            // clusters that run at the same time, with one CTA per SM and with the most
-            const long long one = resident[s], most = 2 * one;
-            if (s > 2 && launched > most) // a second round of wide clusters waits for whole groups of SMs
-                break;
-            const long long rounds = (tiles + most - 1) / most, idle = (launched + most - 1) / most - rounds;
-            const double steps = (double)rounds * ((kb + s - 1) / s) * (tiles <= one ? c.alone : c.two) * (K % 16 ? c.ragged : 1.0);
-            // both limits are felt where they are close: the fourth root of the sum of the fourth powers
-            const double s2 = steps * steps, m2 = stream * stream;
-            const double us = c.fixed + (s > 1 ? c.exchange : 0) + std::sqrt(std::sqrt(s2 * s2 + m2 * m2)) + c.round * (rounds - 1) +
-                              c.idle * idle;
-            if (us < best.us) {
-                best.tn = c.tn;
-                best.splits = s;
-                best.us = us;
-            }
-        }
-    }
+// Expected time in us of `rows` of the M rows that the grid covers.
+double small_us(const small_cost& c, int s, int M, int rows, int N, int K, const int* resident) {
+    const int kb = (K + GEMM_BK - 1) / GEMM_BK, across = (N + GS_BN - 1) / GS_BN, down = (rows + c.tn - 1) / c.tn;
+    const long long tiles = (long long)across * down, launched = (long long)across * ((M + c.tn - 1) / c.tn);
+    const double bytes = (double)N * K * 2;
+    const double stream = (bytes > SMALL_L2_BYTES ? bytes * down : bytes) / SMALL_BYTES_PER_US;
+    // clusters that run at the same time, with one CTA per SM and with the most
+    const long long one = resident[s], most = 2 * one;
+    const long long rounds = (tiles + most - 1) / most, idle = (launched + most - 1) / most - rounds;
+    const double steps = (double)rounds * ((kb + s - 1) / s) * (tiles <= one ? c.alone : c.two) * (K % 16 ? c.ragged : 1.0);
+    // both limits are felt where they are close: the fourth root of the sum of the fourth powers
+    const double s2 = steps * steps, m2 = stream * stream;
+    return c.fixed + (s > 1 ? c.exchange : 0) + std::sqrt(std::sqrt(s2 * s2 + m2 * m2)) + c.round * (rounds - 1) + c.idle * idle;
 }
 
 } // namespace
 
 // Up to 128 rows this kernel, beyond that by the estimates.  The line this draws at 4096 x 4096 lies between 256 rows (17.2 us here,
-// 18.5 with pairs) and 512 (22.6 and 19.1), at 1024 x 4096 between 1024 rows (16.2 and 17.8) and 2048 (21.9 and 18.8).  A row count
-// that only the device knows lies somewhere below M: half of it is taken.  The answer depends on the sizes and the kind of device
-// alone and takes 2 us to work out, half a small product: each thread keeps its latest ones.
+// 18.5 with pairs) and 512 (22.6 and 19.1), at 1024 x 4096 between 1024 rows (16.2 and 17.8) and 2048 (21.9 and 18.8).
+//
+// A row count that only the device knows is M at most, and what it is depends on the caller (a layer that gathers from W ranks: M / W).
+// The plan is the one that loses least in the worst of M / 8, M / 4, M / 2 and M rows, measured by the best plan of each.  Over 79
+// products of five counts each its times are 5.1 % above the best plans'; with the best plan of M / 2 7.5 %, and then up to 1.7 times
+// where B is read again for a second row of tiles (92 x 12680 x 11464, all rows: 109 us, now 76; 99 x 10664 x 6136: 62 and 38);
+// with the best plan of M 8.5 %.
+//
+// The answer depends on the sizes and the kind of device alone and takes some us to work out, as long as a small product: each
+// thread keeps its latest ones.
 static gemm_choice choose_by_sizes(int M, int N, int K, bool rows_on_device) {
     CCL_THROW_IF_NOT(M > 0 && N > 0 && K > 0 && N % 8 == 0 && K % 8 == 0, "unsupported GEMM shape ", M, "x", N, "x", K);
     struct entry {
@@ -417,12 +406,56 @@ static gemm_choice choose_by_sizes(int M, int N, int K, bool rows_on_device) {
     entry& e = known[((unsigned)M * 31 + (unsigned)N * 17 + (unsigned)K * 5 + rows_on_device) / 8 % 64];
     if (e.dev == dev && e.M == M && e.N == N && e.K == K && e.rows == rows_on_device)
         return e.c;
-    const int rows = rows_on_device ? (M + 1) / 2 : M;
-    gemm_choice c;
-    plan_small(M, rows, N, K, c);
-    const double one = gemm_2sm_estimate(rows, N, K, 1), two = gemm_2sm_estimate(rows, N, K, 2);
-    c.pairs = two < one ? 2 : 1;
-    c.small = rows <= 128 || c.us < std::min(one, two);
+
+    struct plan {
+        int tn, splits, pairs; // pairs > 0: that kernel
+        double us[4];
+    } plans[8 * std::size(SMALL_COSTS) + 2];
+    int n = 0;
+    const int counts = rows_on_device ? 4 : 1;
+    double best[4] = { 1e30, 1e30, 1e30, 1e30 };
+    auto consider = [&](int tn, int splits, int pairs, auto&& us) {
+        plan& p = plans[n++] = { tn, splits, pairs, {} };
+        for (int i = 0; i < counts; i++) {
+            p.us[i] = us((int)(((long long)M + (1 << i) - 1) >> i)); // M, M / 2, M / 4, M / 8
+            best[i] = std::min(best[i], p.us[i]);
+        }
+    };
+    const int kb = (K + GEMM_BK - 1) / GEMM_BK, across = (N + GS_BN - 1) / GS_BN;
+    int resident[9];
+    for (int s = 1; s <= 8; s++)
+        resident[s] = resident_clusters(s);
+    for (const small_cost& c : SMALL_COSTS) {
+        if (c.tn >= 4 * std::max(M, 16)) // mostly padding
+            break;
+        for (int s = 1; s <= std::min(8, c.tn / 4) && (s == 1 || kb / s >= 2); s++) {
+            if (s > 2 && (long long)across * ((M + c.tn - 1) / c.tn) > 2 * resident[s]) // a second round of wide clusters waits for
+                break; // whole groups of SMs
+            consider(c.tn, s, 0, [&](int rows) { return small_us(c, s, M, rows, N, K, resident); });
+        }
+    }
+    if (M > 128)
+        for (int pairs = 1; pairs <= 2; pairs++)
+            consider(0, 0, pairs, [&](int rows) { return gemm_2sm_estimate(rows, N, K, pairs); });
+
+    gemm_choice c{ true, 0, 0, gemm_2sm_estimate(M, N, K, 2) < gemm_2sm_estimate(M, N, K, 1) ? 2 : 1 };
+    double small = 1e30, pairs = 1e30;
+    for (int i = 0; i < n; i++) {
+        double worst = 0;
+        for (int k = 0; k < counts; k++)
+            worst = std::max(worst, plans[i].us[k] / best[k]);
+        double& least = plans[i].pairs ? pairs : small;
+        if (worst >= least)
+            continue;
+        least = worst;
+        if (plans[i].pairs)
+            c.pairs = plans[i].pairs;
+        else {
+            c.tn = plans[i].tn;
+            c.splits = plans[i].splits;
+        }
+    }
+    c.small = small < pairs;
     e = { dev, M, N, K, rows_on_device, c };
     return c;
 }
