@@ -347,37 +347,54 @@ void launch_small(const gemm_small_params& P, int tiles_n, int tiles_m, cudaStre
 }
 
 // What a product costs with tiles of TN rows of A, in us: `fixed` from launch to output, `exchange` if K is cut, a step of 64
-// of K with one CTA on an SM or with two, another round of resident CTAs, the factor on the steps where K is no multiple
-// of 16, so that the rows of a box begin between the 32-byte sectors, and a round of CTAs that find no rows.  Fitted to the times
-// of 300 products of 1 to 3000 rows, 520 to 14000 columns and K of 520 to 14300, then moved a little to where they choose best: the
-// chosen plan takes 2.3 % longer than the best one, 7 % where the device alone knows the rows; the rule this replaces (1, 2, 4 or 8
-// parts, estimated cycles) 9 %.
+// of K with one CTA on an SM or with two, `crowd` once where some SM holds two, another round of resident CTAs, the factors on the
+// steps where K is no multiple of 16, so that the rows of a box begin between the 32-byte sectors, and a round of CTAs that find no
+// rows.  `drawn`: what a CTA that is alone on its SM draws from memory, in bytes per us; the ring limits that (64 x 14336 x
+// 4096 on 112 CTAs of four stages 28.2 us, with K in two parts on 224 24.1).
+//
+// Fitted to 7800 times: 255 products of sizes that models have (1 to 2048 rows, N and K of 768 to 14336) and 380 drawn ones of 1 to
+// 8000 rows, 500 to 14300 columns and K.  The chosen plan takes 0.7 % longer than the best one for the first, 1.3 % for the others,
+// at most 1.2 times.  The fit before it, to drawn ones alone, took rows of tiles that run beside one another to read B once each
+// and knew neither `crowd` nor `drawn`: 3.6 % and 1.5 %, at most 1.4 times (64 x 14336 x
+// 4096 28.2 us, now 24.1; 128 x 2304 x 768 7.4 and 5.4; 192 x 4096 x 14336 45 and 39).
 struct small_cost {
     int tn;
-    double fixed, exchange, alone, two, round, ragged, idle;
+    double fixed, exchange, alone, two, crowd, round, ragged, ragged_two, idle, drawn;
 };
 constexpr small_cost SMALL_COSTS[] = {
-    { 16, 2.76, 0.87, 0.275, 0.396, 1.1, 1.04, 0.6 },
-    { 32, 3.64, 0.59, 0.274, 0.408, 2.8, 1.15, 0.8 },
-    { 64, 4.00, 0.82, 0.233, 0.417, 3.3, 1.22, 0.9 },
-    { 128, 4.98, 1.31, 0.279, 0.583, 5.7, 1.30, 0.8 },
+    { 16, 2.64, 0.91, 0.245, 0.287, 0.63, 0.48, 1.21, 1.43, 0.31, 52e3 },
+    { 32, 3.00, 0.83, 0.245, 0.308, 0.87, 2.45, 1.22, 1.43, 0.64, 52e3 },
+    { 64, 3.20, 1.12, 0.244, 0.329, 1.40, 3.33, 1.31, 1.68, 0.69, 49e3 },
+    { 128, 3.95, 1.71, 0.323, 0.455, 1.90, 5.35, 1.50, 1.65, 0.55, 39e3 },
 };
-constexpr double SMALL_BYTES_PER_US = 6.3e6; // of B, from memory
-constexpr double SMALL_L2_BYTES = 64e6; // of B that a second row of tiles still finds in the L2
+constexpr small_cost SMALL_COST_ALONE = { 128, 3.95, 1.71, 0.251, 0, 0, 0, 1.50, 0, 0, 82e3 }; // GS_STAGES_ALONE
+constexpr double SMALL_BYTES_PER_US = 6.5e6; // of B, from memory
+constexpr double SMALL_L2_BYTES = 64e6; // of B that a later round of tiles still finds in the L2
 
 // Expected time in us of `rows` of the M rows that the grid covers.
-double small_us(const small_cost& c, int s, int M, int rows, int N, int K, const int* resident) {
-    const int kb = (K + GEMM_BK - 1) / GEMM_BK, across = (N + GS_BN - 1) / GS_BN, down = (rows + c.tn - 1) / c.tn;
-    const long long tiles = (long long)across * down, launched = (long long)across * ((M + c.tn - 1) / c.tn);
-    const double bytes = (double)N * K * 2;
-    const double stream = (bytes > SMALL_L2_BYTES ? bytes * down : bytes) / SMALL_BYTES_PER_US;
+double small_us(const small_cost& cost, int s, int M, int rows, int N, int K, const int* resident) {
+    const int kb = (K + GEMM_BK - 1) / GEMM_BK, across = (N + GS_BN - 1) / GS_BN, down = (rows + cost.tn - 1) / cost.tn;
+    const long long tiles = (long long)across * down, launched = (long long)across * ((M + cost.tn - 1) / cost.tn);
     // clusters that run at the same time, with one CTA per SM and with the most
     const long long one = resident[s], most = 2 * one;
+    const small_cost& c = cost.tn == SMALL_COST_ALONE.tn && launched <= one ? SMALL_COST_ALONE : cost;
     const long long rounds = (tiles + most - 1) / most, idle = (launched + most - 1) / most - rounds;
-    const double steps = (double)rounds * ((kb + s - 1) / s) * (tiles <= one ? c.alone : c.two) * (K % 16 ? c.ragged : 1.0);
+    const bool alone = tiles <= one;
+    double steps = (double)rounds * ((kb + s - 1) / s) * (alone ? c.alone : c.two);
+    if (K % 16)
+        steps *= alone ? c.ragged : c.ragged_two;
+    double bytes = (double)N * K * 2, rate = SMALL_BYTES_PER_US;
+    if (bytes > SMALL_L2_BYTES) {
+        // rows of tiles that run beside one another read B from memory once, but do not keep step to the end
+        const double reads = (double)std::min<long long>(down, rounds);
+        bytes *= reads + 0.1 * (down - reads);
+        if (alone)
+            rate = std::min(rate, c.drawn * (double)(tiles * s));
+    }
     // both limits are felt where they are close: the fourth root of the sum of the fourth powers
-    const double s2 = steps * steps, m2 = stream * stream;
-    return c.fixed + (s > 1 ? c.exchange : 0) + std::sqrt(std::sqrt(s2 * s2 + m2 * m2)) + c.round * (rounds - 1) + c.idle * idle;
+    const double stream = bytes / rate, s2 = steps * steps, m2 = stream * stream;
+    return c.fixed + (s > 1 ? c.exchange : 0) + std::sqrt(std::sqrt(s2 * s2 + m2 * m2)) + (alone ? 0 : c.crowd) +
+           c.round * (rounds - 1) + c.idle * idle;
 }
 
 } // namespace

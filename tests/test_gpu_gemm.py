@@ -86,6 +86,31 @@ def test_gemm_row_count_on_the_device_costs_little_when_all_rows_are_there():
     assert best(count) < 1.25 * best(None)  # 1.04; with the plan for half of the rows 1.5
 
 
+def test_gemm_of_a_few_more_rows_still_streams_the_weights():
+    """Weights of 117 MB bound 24 rows and 64 alike: the tiles for 64 must keep as much of them in flight."""
+    from oneccl_b200.ops.gemm import gemm_bf16
+
+    N, K = 14336, 4096
+    g = torch.Generator(device="cuda").manual_seed(7)
+    ws = [torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2)]
+
+    def best(M):
+        a, out = torch.ones(M, K, dtype=torch.bfloat16, device="cuda"), torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+        times = []
+        for _ in range(10):
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            start.record()
+            for i in range(20):
+                gemm_bf16(a, ws[i & 1], out=out)
+            end.record()
+            end.synchronize()
+            times.append(start.elapsed_time(end))
+        return min(times)
+
+    best(24)
+    assert best(64) < 1.12 * best(24)  # 1.04; with one part of K on 112 CTAs 1.21
+
+
 @pytest.mark.parametrize("shape", [(40, 520, 264), (300, 1040, 520), (512, 4096, 1032), (700, 104, 72), (1024, 8192, 256)])
 def test_gemm_output_between_pack_boundaries(shape):
     """An output that starts at a pair of columns only: right with the library's choice, refused where packs are stored."""
