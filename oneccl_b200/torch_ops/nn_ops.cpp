@@ -462,9 +462,10 @@ struct Mlp : torch::autograd::Function<Mlp> {
                 check(cclx_partial_sums(ws.data_ptr<float>(), n, (int)N, 1, db.ptr(), nullptr, nullptr, db.add, st));
         });
         d2.product(dy, g, ctx->needs_input_grad(3));
-        db.done();
+        // in the order of the operators of their own: ranks with batches of different sizes reduce their buckets in the same order
         if (sinks[2])
             sinks[2]->report();
+        db.done();
         WeightGrad d1(sinks[0], du);
         Tensor dx;
         if (ctx->needs_input_grad(0))

@@ -147,6 +147,33 @@ def test_data_parallel_gradient_sinks_match_autograd():
     group.close()
 
 
+def test_mlp_reports_its_gradients_in_the_order_of_the_operators_of_their_own():
+    """Whether a rank's batch is large enough for the products with the GELU inside must not show in the order of its buckets."""
+    from oneccl_b200.ops import nn as K
+    from oneccl_b200.torch_ops import native
+
+    g = torch.Generator(device="cuda").manual_seed(8)
+    rows, D, N = 4608, 64, 1024
+    x, dy = (torch.randn(rows, D, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    params = {"w1": (N, D), "b1": (N,), "w2": (D, N), "b2": (D,)}
+    params = {k: torch.nn.Parameter((torch.randn(*s, generator=g, device="cuda") * 0.1).to(torch.bfloat16)) for k, s in params.items()}
+    seen = []
+    for name, p in params.items():
+        p._grad_sink = native().GradSink(torch.zeros_like(p), lambda name=name: seen.append(name))
+    w1, b1, w2, b2 = params.values()
+    orders, grads = [], []
+    for y in (native().mlp(x, w1, b1, w2, b2), K.linear(K.gelu(K.linear(x, w1, b1, defer_bias=True), b1), w2, b2, defer_bias=True)):
+        seen.clear()
+        for p in params.values():
+            p._grad_sink.fresh = True
+        y.backward(dy)
+        orders.append(list(seen))
+        grads.append([p._grad_sink.grad.clone() for p in (w1, b1, w2)])
+    assert orders[0] == orders[1] and sorted(orders[0]) == ["b1", "w1", "w2"]
+    for a, b in zip(*grads):  # each side rounds the sums, the activations and their gradient to bf16 once
+        assert float((a.double() - b.double()).norm() / b.double().norm()) <= 2.0**-7
+
+
 @pytest.mark.parametrize("shape", [(4608, 64, 1024, 136), (1999, 1032, 2056, 8), (2305, 768, 3072, 768), (3, 600, 264, 2200, 64)])
 def test_mlp(shape):
     """Two linear layers with the GELU inside the products against the same chain of operators of their own, and both against
