@@ -6,6 +6,7 @@
 // does not need and returns its gradient; `linear` is then called with defer_bias.
 #include "torch_ops.hpp"
 
+#include <ATen/autocast_mode.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
 
@@ -485,6 +486,9 @@ pybind11::object mlp(const Tensor& x, const pybind11::object& w1_, const pybind1
         w1.device() != x.device() || w2.device() != x.device() || w1.size(1) != x.size(-1) || w2.size(1) != w1.size(0) ||
         w1.size(0) % 8 != 0 || w1.size(1) % 8 != 0 || w2.size(0) % 8 != 0 || x.numel() == 0 || w1.numel() == 0 || w2.numel() == 0 ||
         !bias_ok(b1, x, w1.size(0)) || !bias_ok(b2, x, w2.size(0)))
+        return pybind11::none();
+    // autocast to another type gives the second product, and so its gradient, that type
+    if (at::autocast::is_autocast_enabled(at::kCUDA) && at::autocast::get_autocast_dtype(at::kCUDA) != at::kBFloat16)
         return pybind11::none();
     const int64_t rows = x.numel() / x.size(-1);
     if (rows * std::max(w1.size(0), w2.size(0)) >= (int64_t)1 << 31 ||

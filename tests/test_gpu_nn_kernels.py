@@ -174,6 +174,22 @@ def test_mlp_reports_its_gradients_in_the_order_of_the_operators_of_their_own():
         assert float((a.double() - b.double()).norm() / b.double().norm()) <= 2.0**-7
 
 
+def test_mlp_under_autocast_to_another_type():
+    """The products with the GELU inside know bf16 alone: under fp16 autocast the operators of their own run, under bf16 both agree."""
+    from oneccl_b200.ops import nn as K
+    from oneccl_b200.torch_ops import native
+
+    g = torch.Generator(device="cuda").manual_seed(9)
+    x, w1, b1, w2, b2 = ((torch.randn(*s, generator=g, device="cuda") * 0.1).to(torch.bfloat16)
+                         for s in ((4608, 64), (1024, 64), (1024,), (64, 1024), (64,)))
+    with torch.autocast("cuda", torch.float16):
+        assert native().mlp(x, w1, b1, w2, b2) is None
+        assert K.mlp(x, w1, b1, w2, b2).dtype == torch.float16
+    with torch.autocast("cuda", torch.bfloat16):
+        inside = native().mlp(x, w1, b1, w2, b2)
+    assert torch.equal(inside, native().mlp(x, w1, b1, w2, b2))
+
+
 @pytest.mark.parametrize("shape", [(4608, 64, 1024, 136), (1999, 1032, 2056, 8), (2305, 768, 3072, 768), (3, 600, 264, 2200, 64)])
 def test_mlp(shape):
     """Two linear layers with the GELU inside the products against the same chain of operators of their own, and both against
