@@ -389,9 +389,12 @@ using namespace cclx;
 // tiles fill at least three quarters of their rounds.  Forward and backward of 3072 x 768 (0.97 of two rounds) 85.6 against
 // 92.3 us, 2560 x 1024 (0.72 of three) 123.4 against 130.4, 3200 x 768 (0.70 of three) 101.7 against 100.0, 1280 x 1024 (0.54 of
 // two) 84.2 against 80.7.
-CCLX_API int cclx_mlp_preferred(int M, int N) {
-    const long long tiles = (M + 255ll) / 256 * ((N + 255) / 256), pairs = gpu::device_sms() / 2;
-    return tiles * 4 >= (tiles + pairs - 1) / pairs * pairs * 3;
+// `preferred` is left alone where the device cannot be asked.
+CCLX_API int cclx_mlp_preferred(int M, int N, int* preferred) {
+    return capi::guard([&] {
+        const long long tiles = (M + 255ll) / 256 * ((N + 255) / 256), pairs = std::max(1, gpu::device_sms() / 2);
+        *preferred = tiles * 4 >= (tiles + pairs - 1) / pairs * pairs * 3;
+    });
 }
 
 // u = x W1^T + bias and g = gelu(u): x [M,K], W1 [N,K], bias [N], u and g [M,N]; bf16, 16-byte aligned

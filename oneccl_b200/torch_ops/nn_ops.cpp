@@ -491,8 +491,12 @@ pybind11::object mlp(const Tensor& x, const pybind11::object& w1_, const pybind1
     if (at::autocast::is_autocast_enabled(at::kCUDA) && at::autocast::get_autocast_dtype(at::kCUDA) != at::kBFloat16)
         return pybind11::none();
     const int64_t rows = x.numel() / x.size(-1);
-    if (rows * std::max(w1.size(0), w2.size(0)) >= (int64_t)1 << 31 ||
-        !cclx_mlp_preferred((int)rows, (int)w1.size(0)))
+    if (rows * std::max(w1.size(0), w2.size(0)) >= (int64_t)1 << 31)
+        return pybind11::none();
+    set_device(x.get_device()); // whose SMs are counted
+    int preferred = 0;
+    check(cclx_mlp_preferred((int)rows, (int)w1.size(0), &preferred));
+    if (!preferred)
         return pybind11::none();
     std::vector<SinkRef> sinks{ sink_of(w1_), sink_of(b1_), sink_of(w2_) };
     pybind11::gil_scoped_release nogil;

@@ -2,6 +2,7 @@
 import ctypes as C
 
 import pytest
+import torch
 
 from oneccl_b200 import _lib
 
@@ -10,6 +11,14 @@ _ENTRIES = {  # arguments behind the sizes and the epilogue
     "cclx_gemm_bf16_2sm": (C.c_int(0), None, None),
     "cclx_gemm_bf16_rows": (None, None, None),
 }
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="what happens without a device")
+def test_without_a_device_the_question_for_the_faster_mlp_is_an_error():
+    """An exception that left the C entry would end the process."""
+    lib, answer = _lib.load(), C.c_int(-7)
+    assert lib.cclx_mlp_preferred(8192, 4096, C.byref(answer)) != 0 and answer.value == -7
+    assert b"CUDA" in lib.cclx_last_error()
 
 
 @pytest.mark.parametrize("M,N,K", [(0, 64, 64), (64, 0, 64), (64, 64, 0), (0, 0, 0), (-1, 64, 64), (3, 12, 64), (3, 64, 12)])
