@@ -392,6 +392,10 @@ using namespace cclx;
 // `preferred` is left alone where the device cannot be asked.
 CCLX_API int cclx_mlp_preferred(int M, int N, int* preferred) {
     return capi::guard([&] {
+        if (!env_data::get().gemm_2sm) { // no CTA pairs
+            *preferred = 0;
+            return;
+        }
         const long long tiles = (M + 255ll) / 256 * ((N + 255) / 256), pairs = std::max(1, gpu::device_sms() / 2);
         *preferred = tiles * 4 >= (tiles + pairs - 1) / pairs * pairs * 3;
     });
