@@ -62,6 +62,30 @@ def test_gemm_plans(shape, rows):
             assert (out[n:] == 7.0).all(), (n, kernel)
 
 
+@pytest.mark.parametrize("rows", [False, True], ids=["all-rows", "rows-on-device"])
+@pytest.mark.parametrize("shape", [(300, 4112, 1096), (513, 2096, 1032), (1900, 5008, 136), (1000, 1056, 264), (2300, 3104, 72)])
+def test_gemm_rows_of_c_that_begin_between_lines(shape, rows):
+    """N a multiple of 16 but not of 64: lanes of the CTA pairs trade sectors before they store, 64 columns at a time or 32 of a tile cut
+    between pairs (the first two).  Eight elements further on nothing begins at a sector and every lane stores its own row."""
+    from oneccl_b200.ops.gemm import gemm_bf16
+
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(5)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    ref = a.double() @ w.double().t()
+    # one rounding of the result to bf16, K roundings of the fp32 sum
+    bound = ref.abs() * 2.0**-8 + K * 2.0**-23 * (a.double().abs() @ w.double().abs().t()) + 1e-30
+    for offset in (0, 8):
+        for n in (M - 130, M - 1, M) if rows else (M,):
+            room = torch.full((M * N + 16,), 7.0, dtype=torch.bfloat16, device="cuda")
+            out = room[offset:offset + M * N].view(M, N)
+            count = torch.tensor([n], dtype=torch.int32, device="cuda") if rows else None
+            gemm_bf16(a, w, out=out, check=True, kernel="auto" if rows else "2sm", rows=count)
+            assert ((out[:n].double() - ref[:n]).abs() <= bound[:n]).all(), (n, offset)
+            assert (out[n:] == 7.0).all() and (room[:offset] == 7.0).all() and (room[offset + M * N:] == 7.0).all()
+
+
 def test_gemm_row_count_on_the_device_costs_little_when_all_rows_are_there():
     """B larger than the L2 and more than half of the rows: tiles that were planned for half of them would read B twice."""
     from oneccl_b200.ops.gemm import gemm_bf16

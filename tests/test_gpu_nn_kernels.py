@@ -147,6 +147,53 @@ def test_data_parallel_gradient_sinks_match_autograd():
     group.close()
 
 
+def test_data_parallel_with_the_gelu_inside_the_products():
+    """Batches large enough for the MLP's own kernels: weight gradients beside backward, deferred bias sums, accumulation over two
+    passes, a graphed step; against the plain module's autograd."""
+    from oneccl_b200.models.gpt2 import GPT2, GPT2Config
+    from oneccl_b200.ops.device_group import DeviceGroup
+    from oneccl_b200.parallel.ddp import DataParallel, GraphedTrainStep
+    from oneccl_b200.torch_ops import native
+
+    cfg = GPT2Config(2, 4, 256, 512, 1000)
+    models = []
+    for _ in range(2):
+        torch.manual_seed(0)
+        models.append(GPT2(cfg, fused_ops=True).cuda().to(torch.bfloat16))
+    plain, wrapped = models
+    block, x = plain.blocks[0], torch.zeros(4096, 256, dtype=torch.bfloat16, device="cuda")
+    assert native().mlp(x, block.fc.weight, block.fc.bias, block.fc2.weight, block.fc2.bias) is not None
+    idx, tgt = (torch.randint(0, cfg.vocab, (8, 512), device="cuda") for _ in range(2))
+    group = DeviceGroup.emulated(1, heap_bytes=64 << 20, staging_bytes=1 << 20)
+    ddp = DataParallel(wrapped, group, bucket_mb=0.25)
+
+    def compare(passes):
+        plain.zero_grad(set_to_none=True)
+        for _ in range(passes):
+            plain(idx, tgt).backward()
+        torch.cuda.synchronize()
+        assert all(b.pending == 0 for b in ddp.buckets)
+        for (n, a), (_, b) in zip(plain.named_parameters(), wrapped.named_parameters()):
+            # the same kernels: they differ where autograd rounds a second contribution before it adds it
+            off = float((b.grad.double() - a.grad.double()).norm() / a.grad.double().norm())
+            assert off <= 2.0**-7, (n, off)
+
+    for _ in range(2):
+        ddp.begin_step()
+        ddp(idx, tgt).backward()
+        ddp.finish()
+        compare(1)
+    ddp.zero_grad()
+    for _ in range(2):
+        ddp(idx, tgt).backward()
+    ddp.finish()
+    compare(2)
+    step = GraphedTrainStep(ddp, ddp.make_optimizer(device_step=True, lr=0.0, weight_decay=0.0), idx, tgt)
+    step(idx, tgt)
+    compare(1)
+    group.close()
+
+
 def test_mlp_reports_its_gradients_in_the_order_of_the_operators_of_their_own():
     """Whether a rank's batch is large enough for the products with the GELU inside must not show in the order of its buckets."""
     from oneccl_b200.ops import nn as K
