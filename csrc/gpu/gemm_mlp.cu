@@ -385,19 +385,21 @@ void launch_mlp(const void* a, const void* b, const void* bias, void* u, void* o
 
 using namespace cclx;
 
-// Whether the products with the activation inside are expected to be faster than library products and passes of their own: if the
-// tiles fill at least three quarters of their rounds.  Forward and backward of 3072 x 768 (0.97 of two rounds) 85.6 against
-// 92.3 us, 2560 x 1024 (0.72 of three) 123.4 against 130.4, 3200 x 768 (0.70 of three) 101.7 against 100.0, 1280 x 1024 (0.54 of
-// two) 84.2 against 80.7.
-// `preferred` is left alone where the device cannot be asked.
-CCLX_API int cclx_mlp_preferred(int M, int N, int* preferred) {
+// *answer: 0 if the products with the activation inside may not run (no CTA pairs), 1 if they may, 2 if they are expected to be faster
+// than library products and passes of their own: if the result fills at least three quarters of the rounds of tiles and its rows begin
+// at 32-byte sectors.  Forward and backward of 8192 x 1024 x 4096 (rows, width, hidden width; 0.99 of seven rounds) 322 against
+// 370 us, 2048 x 512 x 2048 (0.86 of one) 49.7 against 50.9, 666 x 1280 x 5120 (0.70 of one, though its tiles fill 0.81) 75.6 against
+// 73.7, 300 x 4096 x 16384 (0.51 of two) 291 against 262; between sectors, 8192 x 768 x 3064 270 against 238, 2048 x 1024 x 4104 113
+// against 108.  Of 119 sizes of 300 to 16384 rows and widths of 64 to 4096 the line gives up two that gained more than 2 % (4096 and
+// 8192 x 1600 x 1600, 0.68, 5 and 7 %); of the 102 on this side three lose more than 1.5 % (666 x 3072 x 12288 2.5 %).
+CCLX_API int cclx_mlp_preferred(int M, int N, int* answer) {
     return capi::guard([&] {
-        if (!env_data::get().gemm_2sm) { // no CTA pairs
-            *preferred = 0;
+        *answer = 0;
+        if (!env_data::get().gemm_2sm)
             return;
-        }
         const long long tiles = (M + 255ll) / 256 * ((N + 255) / 256), pairs = std::max(1, gpu::device_sms() / 2);
-        *preferred = tiles * 4 >= (tiles + pairs - 1) / pairs * pairs * 3;
+        const double room = 65536.0 * pairs * ((tiles + pairs - 1) / pairs);
+        *answer = N % 16 == 0 && (double)M * N >= 0.75 * room ? 2 : 1;
     });
 }
 

@@ -76,9 +76,9 @@ def gelu(u, bias):
 
 
 def mlp(x, w1, b1, w2, b2):
-    """``gelu(x @ w1.T + b1) @ w2.T + b2`` with the tanh-form GELU and its gradient inside the products where the batch is large
-    enough, else as ``linear``, ``gelu``, ``linear``.  ``b2``'s gradient is left to the operator that consumes the output."""
-    y = native().mlp(x, w1, b1, w2, b2)
+    """``gelu(x @ w1.T + b1) @ w2.T + b2`` with the tanh-form GELU and its gradient inside the products where that is expected to
+    be faster, else as ``linear``, ``gelu``, ``linear``.  ``b2``'s gradient is left to the operator that consumes the output."""
+    y = native().mlp(x, w1, b1, w2, b2, True)
     if y is None:
         return linear(gelu(linear(x, w1, b1, defer_bias=True), b1), w2, b2, defer_bias=True)
     return y

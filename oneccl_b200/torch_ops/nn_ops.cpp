@@ -478,9 +478,9 @@ struct Mlp : torch::autograd::Function<Mlp> {
     }
 };
 
-// None where the operator does not take the call, or products of their own are expected to be faster
+// None where the operator does not take the call, and with `if_faster` where products of their own are expected to be faster
 pybind11::object mlp(const Tensor& x, const pybind11::object& w1_, const pybind11::object& b1_, const pybind11::object& w2_,
-                     const pybind11::object& b2_) {
+                     const pybind11::object& b2_, bool if_faster) {
     const Tensor w1 = tensor_of(w1_), b1 = tensor_of(b1_), w2 = tensor_of(w2_), b2 = tensor_of(b2_);
     if (!bf16_cuda(x) || x.dim() < 1 || !bf16_cuda(w1) || !bf16_cuda(w2) || w1.dim() != 2 || w2.dim() != 2 ||
         w1.device() != x.device() || w2.device() != x.device() || w1.size(1) != x.size(-1) || w2.size(1) != w1.size(0) ||
@@ -494,9 +494,9 @@ pybind11::object mlp(const Tensor& x, const pybind11::object& w1_, const pybind1
     if (rows * std::max(w1.size(0), w2.size(0)) >= (int64_t)1 << 31)
         return pybind11::none();
     set_device(x.get_device()); // whose SMs are counted
-    int preferred = 0;
-    check(cclx_mlp_preferred((int)rows, (int)w1.size(0), &preferred));
-    if (!preferred)
+    int answer = 0;
+    check(cclx_mlp_preferred((int)rows, (int)w1.size(0), &answer));
+    if (answer < (if_faster ? 2 : 1))
         return pybind11::none();
     std::vector<SinkRef> sinks{ sink_of(w1_), sink_of(b1_), sink_of(w2_) };
     pybind11::gil_scoped_release nogil;
@@ -635,7 +635,8 @@ void bind_nn(pybind11::module_& m) {
           pybind11::arg("bias"), pybind11::arg("eps"), pybind11::arg("res_bias") = pybind11::none());
     m.def("linear", &linear);
     m.def("bias_gelu", &bias_gelu);
-    m.def("mlp", &mlp);
+    m.def("mlp", &mlp, pybind11::arg("x"), pybind11::arg("w1"), pybind11::arg("b1"), pybind11::arg("w2"), pybind11::arg("b2"),
+          pybind11::arg("if_faster") = false);
     m.def("split_qkv", &split_qkv);
     m.def("embed", &embed);
     m.def("embed_check", &embed_check);

@@ -60,7 +60,7 @@ int cclx_gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int 
                        void* err_words, void* stream);
 int cclx_gemm_bf16_rows(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, const void* rows_dev,
                         void* err_words, void* stream);
-int cclx_mlp_preferred(int M, int N, int* preferred);
+int cclx_mlp_preferred(int M, int N, int* answer);
 int cclx_linear_gelu(const void* x, const void* w1, const void* bias, void* u, void* g, int M, int N, int K, void* stream);
 int cclx_linear_gelu_bwd_rows(int M);
 int cclx_linear_gelu_bwd(const void* dy, const void* w2, const void* u, void* du, float* partial, int M, int N, int K, void* stream);

@@ -221,6 +221,17 @@ def test_mlp_reports_its_gradients_in_the_order_of_the_operators_of_their_own():
         assert float((a.double() - b.double()).norm() / b.double().norm()) <= 2.0**-7
 
 
+@pytest.mark.parametrize("rows,D,N,inside", [(4096, 256, 1024, True), (2048, 512, 2048, True), (300, 64, 16384, False),
+                                             (666, 64, 5120, False), (8192, 64, 3064, False), (2048, 64, 4104, False)])
+def test_mlp_keeps_to_the_operators_of_their_own_where_they_are_faster(rows, D, N, inside):
+    """Rows of tiles that are mostly padding, and rows of the result that begin between sectors."""
+    from oneccl_b200.torch_ops import native
+
+    x, w1, b1, w2, b2 = (torch.zeros(*s, dtype=torch.bfloat16, device="cuda") for s in ((rows, D), (N, D), (N,), (D, N), (D,)))
+    assert native().mlp(x, w1, b1, w2, b2) is not None
+    assert (native().mlp(x, w1, b1, w2, b2, True) is not None) == inside
+
+
 def test_mlp_under_autocast_to_another_type():
     """The products with the GELU inside know bf16 alone: under fp16 autocast the operators of their own run, under bf16 both agree."""
     from oneccl_b200.ops import nn as K
