@@ -241,6 +241,22 @@ __device__ __forceinline__ bool peer_barrier(const comm_dev& c, block_sync& s, u
     return s.ok;
 }
 
+// The barrier in two halves, without signatures: between them a block does what needs nothing from its peers, while the flags travel.
+__device__ __forceinline__ void peer_arrive(const comm_dev& c, block_sync& s) {
+    __syncthreads();
+    s.used++;
+    if (s.ok && threadIdx.x < (unsigned)c.world)
+        st_release_sys(c.flags[threadIdx.x] + blockIdx.x * MAX_RANKS + c.rank, s.epoch + s.used);
+}
+__device__ __forceinline__ bool peer_wait(const comm_dev& c, block_sync& s) {
+    const int p = threadIdx.x;
+    const int fail = s.ok && p < c.world &&
+                     !wait_flag_sys(c, c.flags[c.rank] + blockIdx.x * MAX_RANKS + p, s.epoch + s.used, p, ST_BARRIER_TIMEOUT);
+    if (__syncthreads_or(fail))
+        s.ok = false;
+    return s.ok;
+}
+
 // Hash of the arguments of a zero-copy collective that every rank must pass alike (never zero).
 __device__ __forceinline__ uint32_t arg_signature(uint32_t kind, size_t in_off, size_t out_off, size_t count,
                                                   uint32_t flags) {

@@ -458,8 +458,10 @@ constexpr int MOE_SEGMENTS = 256;
 // Bound by memory (every row read once, written topk times).  The rows stand grouped by expert, but are not sent in that order:
 // each expert's rows are cut into the same number of parts and the parts are taken in turn, so that all peers receive all the time,
 // and the topk copies of a token, which is found at about the same depth of every list, are read while it is still in the L2.
-// Eight ranks with 1024 tokens of 4096 each, top-2, on one GPU: 48.2 us in order of experts with one piece per warp in flight,
-// 39.6 now; 16 tokens of 512, the barriers alone, 15.5 and 10.0.
+// The table of parts is made while the barrier's flags travel: in front of it, it cost an exchange of few rows what the order gains.
+// Eight ranks on one GPU, top-2, each launch by itself: 1024 tokens of 4096 47.7 us in order of experts with one piece per warp in
+// flight, 42.8 with the table in front of the barrier, 41.0 now; 256 of 4096 21.8, 22.9 and 21.7; 62 of 1112 16.2, 16.5 and 15.3; one of
+// 512 15.5, 15.4 and 14.5, the barriers alone.
 __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(const comm_dev* tab, moe_args a) {
     __shared__ comm_dev c;
     __shared__ moe_rank_args ra;
@@ -479,7 +481,7 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(const comm_de
         if (p == 0)
             s_own[e] = v;
     }
-    __syncthreads();
+    peer_arrive(c, s);
     const int shift = 31 - __clz(MOE_SEGMENTS / W), n_seg = W << shift; // 2^shift parts
     auto upto = [&](int e, int part) { return (unsigned)(((unsigned long long)(unsigned)s_own[e] * (unsigned)part) >> shift); };
     for (int i = threadIdx.x; i < MOE_SEGMENTS; i += blockDim.x) {
@@ -555,7 +557,7 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_dispatch_kernel(const comm_de
     look();
     fetch(p0, v0);
 
-    bool ok = peer_barrier(c, s);
+    const bool ok = peer_wait(c, s);
     // The table is read by all threads at once and worked on in shared memory: one thread that walked it in global memory
     // waited W * W times for the L2, some 40 us for eight ranks, in every block.
     for (int i = threadIdx.x; i < W * W; i += blockDim.x)
