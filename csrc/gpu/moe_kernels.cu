@@ -213,13 +213,13 @@ __global__ void __launch_bounds__(1024)
     __shared__ unsigned short ticket[ITEMS];
     __shared__ unsigned char expert[ITEMS];
     gpu::pdl_trigger();
+    if constexpr (C > 1)
+        sm100::cluster_arrive_relaxed(); // this block runs: the others may write its shared memory
     const int lane = threadIdx.x & 31, me = C > 1 ? (int)blockIdx.x : 0;
     const int per = (n_tokens + C - 1) / C, t0 = me * per, n = max(0, min(per, n_tokens - t0)); // tokens of this block
     for (int e = threadIdx.x; e < n_experts; e += blockDim.x)
         count[e] = 0;
     __syncthreads();
-    if constexpr (C > 1)
-        sm100::cluster_arrive(); // this block runs: the others may write its shared memory
     gpu::pdl_wait(); // launched while the kernel in front still runs
     for (int t = threadIdx.x; t < n; t += blockDim.x)
         route_token<E>(logits + (size_t)(t0 + t) * n_experts, n_experts, topk, idx + (size_t)(t0 + t) * topk,
