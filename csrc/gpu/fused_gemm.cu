@@ -15,10 +15,7 @@
 namespace cclx {
 namespace gpu {
 
-namespace {
-
-// [rows, cols] row-major bf16 matrix, box = 64 columns x box_rows rows, 128-byte swizzle
-CUtensorMap make_map(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+CUtensorMap make_bf16_map(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
     const driver_api& d = driver();
     CCL_THROW_IF_NOT(d.loaded && d.TensorMapEncodeTiled, "CUDA driver not available: ", d.error);
     CCL_THROW_IF_NOT(((uintptr_t)base & 15) == 0, "GEMM operand must be 16-byte aligned");
@@ -32,15 +29,6 @@ CUtensorMap make_map(const void* base, uint64_t rows, uint64_t cols, uint32_t bo
                                     box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
     return m;
-}
-
-} // namespace
-
-CUtensorMap make_bf16_map(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
-    return make_map(base, rows, cols, box_rows);
-}
-CUtensorMap make_bf16_kmajor_map(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
-    return make_map(base, rows, cols, box_rows);
 }
 
 namespace {
@@ -110,8 +98,8 @@ void gemm_bf16_plain(const void* A, const void* B, void* C, int M, int N, int K,
     const int bn = pick_bn(N);
     fused_params P;
     std::memset(&P, 0, sizeof(P));
-    P.r[0].tmA = make_map(A, M, K, GEMM_BM);
-    P.r[0].tmB = make_map(B, N, K, bn);
+    P.r[0].tmA = make_bf16_map(A, M, K, GEMM_BM);
+    P.r[0].tmB = make_bf16_map(B, N, K, bn);
     P.r[0].C = (__nv_bfloat16*)C;
     P.r[0].err = err;
     P.r[0].plan_state = nullptr;
@@ -292,11 +280,11 @@ void fused_plan_run(fused_plan* p, const void* const* A, const void* const* B, v
     for (int e = 0; e < p->entries; e++) {
         const void* a = p->mode == GM_AG ? fused_plan_x_full(p, e) : A[e];
         if (a != p->lastA[e]) {
-            p->P.r[e].tmA = make_map(a, p->M, p->K, GEMM_BM);
+            p->P.r[e].tmA = make_bf16_map(a, p->M, p->K, GEMM_BM);
             p->lastA[e] = a;
         }
         if (B[e] != p->lastB[e]) {
-            p->P.r[e].tmB = make_map(B[e], p->N, p->K, p->two_sm ? 128 : p->bn); // a pair's CTA stages half of the B tile
+            p->P.r[e].tmB = make_bf16_map(B[e], p->N, p->K, p->two_sm ? 128 : p->bn); // a pair's CTA stages half of the B tile
             p->lastB[e] = B[e];
         }
         p->P.r[e].C = (__nv_bfloat16*)C[e];

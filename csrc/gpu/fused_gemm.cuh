@@ -38,6 +38,9 @@
 namespace cclx {
 namespace gpu {
 
+// [rows, cols] row-major bf16 matrix, box = 64 columns x box_rows rows, 128-byte swizzle
+CUtensorMap make_bf16_map(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
+
 constexpr int GEMM_BM = 128;
 constexpr int GEMM_BK = 64;
 constexpr int GEMM_UMMA_K = 16;

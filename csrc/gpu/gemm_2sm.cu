@@ -299,6 +299,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1) gemm2sm_kernel(const __grid_con
             // Pair p finishes columns [128 p, 128 p + 128) of the tile: the other pair's half sums of them arrive in the ring, which
             // nobody uses any more, as packs of four columns per row.  The sum of two halves does not depend on their order.
             constexpr int HALF_PART = G2_PART / 2;
+            static_assert(G2_BN / 2 / 4 * G2_HALF * 16 <= G2_RING, "the half sums must fit the ring");
             const uint32_t acc = mine & 1;
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * G2_BN + part * HALF_PART;
             const uint32_t here = smem_u32(smem) + (uint32_t)(q * 32 + lane + part * (HALF_PART / 4) * G2_HALF) * 16;
@@ -415,8 +416,6 @@ void launch_2sm(const gemm2_params& P, int clusters, cudaStream_t st) {
 
 } // namespace
 
-CUtensorMap make_bf16_kmajor_map(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
-
 void gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, int epilogue, int clusters,
                    uint32_t* err, cudaStream_t st, const int* rows_dev, int pairs) {
     CCL_THROW_IF_NOT(M > 0 && N > 0 && K > 0 && N % 8 == 0 && K % 8 == 0, "unsupported GEMM shape ", M, "x", N, "x", K);
@@ -425,8 +424,8 @@ void gemm_bf16_2sm(const void* A, const void* B, void* C, int M, int N, int K, i
     allow_smem<gemm2sm_kernel<2>>(G2_SMEM);
     gemm2_params P;
     std::memset(&P, 0, sizeof(P));
-    P.tmA = make_bf16_kmajor_map(A, M, K, G2_HALF);
-    P.tmB = make_bf16_kmajor_map(B, N, K, G2_HALF);
+    P.tmA = make_bf16_map(A, M, K, G2_HALF);
+    P.tmB = make_bf16_map(B, N, K, G2_HALF);
     P.C = (__nv_bfloat16*)C;
     P.err = err;
     P.M = M;

@@ -28,8 +28,6 @@
 namespace cclx {
 namespace gpu {
 
-CUtensorMap make_bf16_map(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
-
 namespace {
 
 constexpr int GM_STAGES = 6;

@@ -28,8 +28,6 @@
 namespace cclx {
 namespace gpu {
 
-CUtensorMap make_bf16_kmajor_map(const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
-
 namespace {
 
 constexpr int GS_BN = 128; // rows of B per tile
@@ -490,8 +488,8 @@ void gemm_bf16_small(const void* A, const void* B, void* C, int M, int N, int K,
     CCL_THROW_IF_NOT(M > 0 && N > 0 && K > 0 && N % 8 == 0 && K % 8 == 0, "unsupported GEMM shape ", M, "x", N, "x", K);
     gemm_small_params P;
     std::memset(&P, 0, sizeof(P));
-    P.tmA = make_bf16_kmajor_map(A, M, K, plan.tn);
-    P.tmB = make_bf16_kmajor_map(B, N, K, GS_BN);
+    P.tmA = make_bf16_map(A, M, K, plan.tn);
+    P.tmB = make_bf16_map(B, N, K, GS_BN);
     P.C = (__nv_bfloat16*)C;
     P.err = err;
     P.M = M;

@@ -194,21 +194,21 @@ __global__ void __launch_bounds__(256)
             atomicAdd(&counts[e], (unsigned long long)hist[e]);
 }
 
-// The whole routing of a batch of up to ROUTE_ONE_BLOCK items in one launch: selection, counts, offsets and placement with the
+// The whole routing of a batch of up to ROUTE_ONE_LAUNCH items in one launch: selection, counts, offsets and placement with the
 // counters in shared memory, in one block or in a cluster of C that exchange their counts.  Latency is what it costs; the selection
 // takes some 300 instructions per token, 2.5 us for 1024 tokens on one SM.  From 512 tokens on a cluster is
-// faster: 1024 tokens among 8 experts, top-2, 2.6 us instead of 4.1 in a chain of such calls, 4096 tokens 3.4 instead of 12.1; 256
+// faster: 1024 tokens among 8 experts, top-2, 2.5 us instead of 4.0 in a chain of such calls, 4096 tokens 3.4 instead of 12.0; 256
 // tokens take 2.2 in one block.
-constexpr int ROUTE_ONE_BLOCK = 8192;
+constexpr int ROUTE_ONE_LAUNCH = 8192;
 constexpr int ROUTE_CLUSTER = 8;
 constexpr int ROUTE_CLUSTER_TOKENS = 512; // from so many tokens on
 
 template <int E, int C>
 __global__ void __launch_bounds__(1024)
-    route_one_block_kernel(const float* logits, int n_tokens, int n_experts, int topk, long long* __restrict__ idx,
+    route_one_launch_kernel(const float* logits, int n_tokens, int n_experts, int topk, long long* __restrict__ idx,
                            float* __restrict__ wts, unsigned long long* __restrict__ counts, long long* __restrict__ order,
                            long long* __restrict__ pos) {
-    constexpr int ITEMS = C > 1 ? ROUTE_ONE_BLOCK / C + ROUTE_MAX_TOPK : ROUTE_CLUSTER_TOKENS * ROUTE_MAX_TOPK;
+    constexpr int ITEMS = C > 1 ? ROUTE_ONE_LAUNCH / C + ROUTE_MAX_TOPK : ROUTE_CLUSTER_TOKENS * ROUTE_MAX_TOPK;
     __shared__ unsigned int count[ROUTE_MAX_EXPERTS], offs[ROUTE_MAX_EXPERTS], all[C][ROUTE_MAX_EXPERTS];
     __shared__ unsigned short ticket[ITEMS];
     __shared__ unsigned char expert[ITEMS];
@@ -289,7 +289,7 @@ void launch_route(const float* logits, int n_tokens, int n_experts, int topk, lo
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = wide ? 2 : 1;
-    CUDA_CHECK(cudaLaunchKernelEx(&cfg, wide ? route_one_block_kernel<E, ROUTE_CLUSTER> : route_one_block_kernel<E, 1>, logits, n_tokens,
+    CUDA_CHECK(cudaLaunchKernelEx(&cfg, wide ? route_one_launch_kernel<E, ROUTE_CLUSTER> : route_one_launch_kernel<E, 1>, logits, n_tokens,
                                   n_experts, topk, idx, wts, counts, order, pos));
 }
 
@@ -331,9 +331,9 @@ __global__ void __launch_bounds__(256)
 }
 } // namespace
 
-// items (token, slot) up to which one block does the whole routing
+// items (token, slot) up to which one launch does the whole routing: a block, or a cluster of eight
 CCLX_API int cclx_moe_route_one_block() {
-    return ROUTE_ONE_BLOCK;
+    return ROUTE_ONE_LAUNCH;
 }
 
 // logits [n_tokens, n_experts] fp32 -> idx [n_tokens, topk] (int64), wts [n_tokens, topk] (fp32),
@@ -347,7 +347,7 @@ CCLX_API int cclx_moe_route(const float* logits, int n_tokens, int n_experts, in
         CCL_THROW_IF_NOT(topk >= 1 && topk <= ROUTE_MAX_TOPK && topk <= n_experts, "top-k must be between 1 and min(",
                          ROUTE_MAX_TOPK, ", experts)");
         cudaStream_t st = (cudaStream_t)stream;
-        if (n_tokens > 0 && (size_t)n_tokens * topk <= ROUTE_ONE_BLOCK) {
+        if (n_tokens > 0 && (size_t)n_tokens * topk <= ROUTE_ONE_LAUNCH) {
             auto launch = n_experts <= 8 ? launch_route<8> : n_experts <= 16 ? launch_route<16> : launch_route<0>;
             launch(logits, n_tokens, n_experts, topk, idx, wts, (unsigned long long*)counts, order, pos, st);
             return;

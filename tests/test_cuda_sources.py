@@ -31,7 +31,7 @@ def test_other_blocks_shared_memory_is_written_between_cluster_barriers(kernel):
 
 def test_the_kernels_with_remote_stores_are_found():
     names = {k[1] for k in _kernels() if "st_cluster_" in k[2]}
-    assert {"route_one_block_kernel", "gemm_small_kernel", "gemm2sm_kernel"} <= names
+    assert {"route_one_launch_kernel", "gemm_small_kernel", "gemm2sm_kernel"} <= names
 
 
 @pytest.mark.parametrize("kernel", [k for k in _kernels() if "tmem_ld_32x" in k[2]], ids=lambda k: f"{k[0]}:{k[1]}")
