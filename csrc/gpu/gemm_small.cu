@@ -294,18 +294,25 @@ __global__ void __launch_bounds__(gs_layout<TN, STAGES>::THREADS, gs_layout<TN, 
     }
 }
 
-// clusters of `splits` CTAs that run at the same time with one CTA per SM: fewer than SMs / splits, since a cluster
-// stays within a group of SMs
+// Stands for the kernels above when the runtime is asked how many clusters fit: for kernels with tensor memory it answers for one CTA
+// per SM whatever shared memory allows, but two run (24 rows, K = 14336 in eight parts: 22.7 us for 4096 columns, 32 clusters, and
+// 32.9 for 4352, 34 clusters where 33 fit in twos and 15 alone).
+template <int TN, int STAGES>
+__global__ void __launch_bounds__(gs_layout<TN, STAGES>::THREADS, gs_layout<TN, STAGES>::BLOCKS) gs_shape_kernel() {}
+
+// Clusters of `splits` CTAs that run at the same time.  A cluster stays within a group of SMs, so there are fewer than SMs / splits with
+// one CTA per SM, but more than twice as many with two: 15 and 33 clusters of eight, 33 and 71 of four.
+template <int TN, int STAGES>
 int resident_clusters(int splits) {
+    typedef gs_layout<TN, STAGES> L;
     static std::atomic<int> known[64][9];
     if (splits == 1)
-        return device_sms();
+        return L::BLOCKS * device_sms();
     int dev = 0;
     CUDA_CHECK(cudaGetDevice(&dev));
     int n = dev < 64 ? known[dev][splits].load(std::memory_order_relaxed) : 0;
     if (n == 0) {
-        typedef gs_layout<128, GS_STAGES_ALONE> L;
-        allow_smem<gemm_small_kernel<128, GS_STAGES_ALONE>>(L::TOTAL);
+        allow_smem<gs_shape_kernel<TN, STAGES>>(L::TOTAL);
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(splits);
         cfg.blockDim = dim3(L::THREADS);
@@ -316,12 +323,18 @@ int resident_clusters(int splits) {
         attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
-        CUDA_CHECK(cudaOccupancyMaxActiveClusters(&n, gemm_small_kernel<128, GS_STAGES_ALONE>, &cfg));
+        CUDA_CHECK(cudaOccupancyMaxActiveClusters(&n, gs_shape_kernel<TN, STAGES>, &cfg));
         n = std::max(n, 1);
         if (dev < 64)
             known[dev][splits].store(n, std::memory_order_relaxed);
     }
     return n;
+}
+int clusters_alone(int splits) {
+    return resident_clusters<128, GS_STAGES_ALONE>(splits);
+}
+int clusters_in_twos(int splits) {
+    return resident_clusters<64, 4>(splits);
 }
 
 template <int TN, int STAGES>
@@ -351,7 +364,7 @@ void launch_small(const gemm_small_params& P, int tiles_n, int tiles_m, cudaStre
 // 4096 on 112 CTAs of four stages 28.2 us, with K in two parts on 224 24.1).
 //
 // Fitted to 7800 times: 255 products of sizes that models have (1 to 2048 rows, N and K of 768 to 14336) and 380 drawn ones of 1 to
-// 8000 rows, 500 to 14300 columns and K.  The chosen plan takes 0.7 % longer than the best one for the first, 1.3 % for the others,
+// 8000 rows, 500 to 14300 columns and K.  The chosen plan takes 0.7 % longer than the best one for the first, 1.0 % for the others,
 // at most 1.2 times.  The fit before it, to drawn ones alone, took rows of tiles that run beside one another to read B once each
 // and knew neither `crowd` nor `drawn`: 3.6 % and 1.5 %, at most 1.4 times (64 x 14336 x
 // 4096 28.2 us, now 24.1; 128 x 2304 x 768 7.4 and 5.4; 192 x 4096 x 14336 45 and 39).
@@ -370,11 +383,10 @@ constexpr double SMALL_BYTES_PER_US = 6.5e6; // of B, from memory
 constexpr double SMALL_L2_BYTES = 64e6; // of B that a later round of tiles still finds in the L2
 
 // Expected time in us of `rows` of the M rows that the grid covers.
-double small_us(const small_cost& cost, int s, int M, int rows, int N, int K, const int* resident) {
+double small_us(const small_cost& cost, int s, int M, int rows, int N, int K) {
     const int kb = (K + GEMM_BK - 1) / GEMM_BK, across = (N + GS_BN - 1) / GS_BN, down = (rows + cost.tn - 1) / cost.tn;
     const long long tiles = (long long)across * down, launched = (long long)across * ((M + cost.tn - 1) / cost.tn);
-    // clusters that run at the same time, with one CTA per SM and with the most
-    const long long one = resident[s], most = 2 * one;
+    const long long one = clusters_alone(s), most = clusters_in_twos(s);
     const small_cost& c = cost.tn == SMALL_COST_ALONE.tn && launched <= one ? SMALL_COST_ALONE : cost;
     const long long rounds = (tiles + most - 1) / most, idle = (launched + most - 1) / most - rounds;
     const bool alone = tiles <= one;
@@ -402,7 +414,7 @@ double small_us(const small_cost& cost, int s, int M, int rows, int N, int K, co
 //
 // A row count that only the device knows is M at most, and what it is depends on the caller (a layer that gathers from W ranks: M / W).
 // The plan is the one that loses least in the worst of M / 8, M / 4, M / 2 and M rows, measured by the best plan of each.  Over 79
-// products of five counts each its times are 5.1 % above the best plans'; with the best plan of M / 2 7.5 %, and then up to 1.7 times
+// products of five counts each its times are 5.0 % above the best plans'; with the best plan of M / 2 7.5 %, and then up to 1.7 times
 // where B is read again for a second row of tiles (92 x 12680 x 11464, all rows: 109 us, now 76; 99 x 10664 x 6136: 62 and 38);
 // with the best plan of M 8.5 %.
 //
@@ -437,16 +449,14 @@ static gemm_choice choose_by_sizes(int M, int N, int K, bool rows_on_device) {
         }
     };
     const int kb = (K + GEMM_BK - 1) / GEMM_BK, across = (N + GS_BN - 1) / GS_BN;
-    int resident[9];
-    for (int s = 1; s <= 8; s++)
-        resident[s] = resident_clusters(s);
     for (const small_cost& c : SMALL_COSTS) {
         if (c.tn >= 4 * std::max(M, 16)) // mostly padding
             break;
         for (int s = 1; s <= std::min(8, c.tn / 4) && (s == 1 || kb / s >= 2); s++) {
-            if (s > 2 && (long long)across * ((M + c.tn - 1) / c.tn) > 2 * resident[s]) // a second round of wide clusters waits for
-                break; // whole groups of SMs
-            consider(c.tn, s, 0, [&](int rows) { return small_us(c, s, M, rows, N, K, resident); });
+            // a second round of wide clusters waits for whole groups of SMs
+            if (s > 2 && (long long)across * ((M + c.tn - 1) / c.tn) > clusters_in_twos(s))
+                break;
+            consider(c.tn, s, 0, [&](int rows) { return small_us(c, s, M, rows, N, K); });
         }
     }
     if (M > 128)
@@ -507,7 +517,7 @@ void gemm_bf16_small(const void* A, const void* B, void* C, int M, int N, int K,
         case 32: launch_small<32, 4>(P, tiles_n, tiles_m, st); break;
         case 64: launch_small<64, 4>(P, tiles_n, tiles_m, st); break;
         default:
-            if ((long long)tiles_n * tiles_m <= resident_clusters(plan.splits))
+            if ((long long)tiles_n * tiles_m <= clusters_alone(plan.splits))
                 launch_small<128, GS_STAGES_ALONE>(P, tiles_n, tiles_m, st);
             else
                 launch_small<128, 3>(P, tiles_n, tiles_m, st);
