@@ -24,6 +24,7 @@
 #include "gpu/fused_gemm.cuh"
 #include "gpu/gelu.cuh"
 #include "gpu/launch_util.cuh"
+#include "gpu/row_store.cuh"
 
 namespace cclx {
 namespace gpu {
@@ -246,15 +247,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GM_THREADS, 1) mlp_k
             const bool on = row < P.M && col < P.N;
             if (P.wide) {
                 if (on)
-                    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]),
-                                 "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
-                                 : "memory");
+                    st_16(p, w);
             }
             else
 #pragma unroll
                 for (int h = 0; h < 8; h += 4)
                     if (on && col + h * 2 < P.N)
-                        *reinterpret_cast<uint4*>(p + h * 2) = make_uint4(w[h], w[h + 1], w[h + 2], w[h + 3]);
+                        st_8(p + h * 2, w + h);
         };
         uint32_t tc = 0;
         // all of these warps see every tile, whatever happens to the other roles: they meet at a barrier

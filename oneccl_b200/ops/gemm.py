@@ -37,7 +37,8 @@ def gemm_bf16(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None,
     """``kernel``: "auto" (the library decides), "1sm" (one CTA per 128 x 256 tile) or "2sm" (CTA pairs,
     tcgen05 cta_group::2, 256 x 256 tiles; ``ctas`` then counts CTAs, two per pair).  ``rows``: an int32
     device tensor whose first element says how many of ``a``'s rows to multiply (read by the kernel, so the
-    host never learns it; the other rows of ``out`` stay as they are)."""
+    host never learns it; the other rows of ``out`` stay as they are).  ``out`` starts at a multiple of 4 bytes, of 16
+    where ``kernel`` or ``ctas`` asks for the kernels of whole tiles."""
     assert a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and a.is_cuda and w.is_cuda
     assert a.dim() == 2 and w.dim() == 2 and a.shape[1] == w.shape[1]
     assert rows is None or (rows.dtype == torch.int32 and rows.is_cuda)
