@@ -303,13 +303,11 @@ __global__ void __launch_bounds__(gs_layout<TN, STAGES>::THREADS, gs_layout<TN, 
 // Clusters of `splits` CTAs that run at the same time.  A cluster stays within a group of SMs, so there are fewer than SMs / splits with
 // one CTA per SM, but more than twice as many with two: 15 and 33 clusters of eight, 33 and 71 of four.
 template <int TN, int STAGES>
-int resident_clusters(int splits) {
+int resident_clusters(int dev, int splits) {
     typedef gs_layout<TN, STAGES> L;
     static std::atomic<int> known[64][9];
     if (splits == 1)
         return L::BLOCKS * device_sms();
-    int dev = 0;
-    CUDA_CHECK(cudaGetDevice(&dev));
     int n = dev < 64 ? known[dev][splits].load(std::memory_order_relaxed) : 0;
     if (n == 0) {
         allow_smem<gs_shape_kernel<TN, STAGES>>(L::TOTAL);
@@ -330,11 +328,11 @@ int resident_clusters(int splits) {
     }
     return n;
 }
-int clusters_alone(int splits) {
-    return resident_clusters<128, GS_STAGES_ALONE>(splits);
-}
-int clusters_in_twos(int splits) {
-    return resident_clusters<64, 4>(splits);
+struct fits {
+    int alone, in_twos;
+};
+fits clusters_that_fit(int dev, int splits) { // on the current device
+    return { resident_clusters<128, GS_STAGES_ALONE>(dev, splits), resident_clusters<64, 4>(dev, splits) };
 }
 
 template <int TN, int STAGES>
@@ -383,10 +381,10 @@ constexpr double SMALL_BYTES_PER_US = 6.5e6; // of B, from memory
 constexpr double SMALL_L2_BYTES = 64e6; // of B that a later round of tiles still finds in the L2
 
 // Expected time in us of `rows` of the M rows that the grid covers.
-double small_us(const small_cost& cost, int s, int M, int rows, int N, int K) {
+double small_us(const small_cost& cost, int s, const fits& clusters, int M, int rows, int N, int K) {
     const int kb = (K + GEMM_BK - 1) / GEMM_BK, across = (N + GS_BN - 1) / GS_BN, down = (rows + cost.tn - 1) / cost.tn;
     const long long tiles = (long long)across * down, launched = (long long)across * ((M + cost.tn - 1) / cost.tn);
-    const long long one = clusters_alone(s), most = clusters_in_twos(s);
+    const long long one = clusters.alone, most = clusters.in_twos; // at the same time
     const small_cost& c = cost.tn == SMALL_COST_ALONE.tn && launched <= one ? SMALL_COST_ALONE : cost;
     const long long rounds = (tiles + most - 1) / most, idle = (launched + most - 1) / most - rounds;
     const bool alone = tiles <= one;
@@ -418,8 +416,8 @@ double small_us(const small_cost& cost, int s, int M, int rows, int N, int K) {
 // where B is read again for a second row of tiles (92 x 12680 x 11464, all rows: 109 us, now 76; 99 x 10664 x 6136: 62 and 38);
 // with the best plan of M 8.5 %.
 //
-// The answer depends on the sizes and the kind of device alone and takes some us to work out, as long as a small product: each
-// thread keeps its latest ones.
+// The answer depends on the sizes and the kind of device alone and takes 0.5 us to work out, 2 us where the count is on the device, of
+// the 4.2 us of a call: each thread keeps its latest ones.
 static gemm_choice choose_by_sizes(int M, int N, int K, bool rows_on_device) {
     CCL_THROW_IF_NOT(M > 0 && N > 0 && K > 0 && N % 8 == 0 && K % 8 == 0, "unsupported GEMM shape ", M, "x", N, "x", K);
     struct entry {
@@ -449,14 +447,17 @@ static gemm_choice choose_by_sizes(int M, int N, int K, bool rows_on_device) {
         }
     };
     const int kb = (K + GEMM_BK - 1) / GEMM_BK, across = (N + GS_BN - 1) / GS_BN;
+    fits clusters[9];
+    for (int s = 1; s <= 8; s++)
+        clusters[s] = clusters_that_fit(dev, s);
     for (const small_cost& c : SMALL_COSTS) {
         if (c.tn >= 4 * std::max(M, 16)) // mostly padding
             break;
         for (int s = 1; s <= std::min(8, c.tn / 4) && (s == 1 || kb / s >= 2); s++) {
             // a second round of wide clusters waits for whole groups of SMs
-            if (s > 2 && (long long)across * ((M + c.tn - 1) / c.tn) > clusters_in_twos(s))
+            if (s > 2 && (long long)across * ((M + c.tn - 1) / c.tn) > clusters[s].in_twos)
                 break;
-            consider(c.tn, s, 0, [&](int rows) { return small_us(c, s, M, rows, N, K); });
+            consider(c.tn, s, 0, [&](int rows) { return small_us(c, s, clusters[s], M, rows, N, K); });
         }
     }
     if (M > 128)
@@ -516,12 +517,14 @@ void gemm_bf16_small(const void* A, const void* B, void* C, int M, int N, int K,
         case 16: launch_small<16, 4>(P, tiles_n, tiles_m, st); break;
         case 32: launch_small<32, 4>(P, tiles_n, tiles_m, st); break;
         case 64: launch_small<64, 4>(P, tiles_n, tiles_m, st); break;
-        default:
-            if ((long long)tiles_n * tiles_m <= clusters_alone(plan.splits))
+        default: {
+            int dev = 0;
+            CUDA_CHECK(cudaGetDevice(&dev));
+            if ((long long)tiles_n * tiles_m <= clusters_that_fit(dev, plan.splits).alone)
                 launch_small<128, GS_STAGES_ALONE>(P, tiles_n, tiles_m, st);
             else
                 launch_small<128, 3>(P, tiles_n, tiles_m, st);
-            break;
+        }
     }
 }
 
